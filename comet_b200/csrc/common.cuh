@@ -76,6 +76,7 @@ int widen_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t st);
 int narrow_f64_to_f32(const double *src, float *dst, int64_t n, cudaStream_t st);
 // out[0..n] = exclusive prefix sum of in[0..n-1], out[n] = total
 int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st);
+int exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st);
 // sorted COO row coordinates -> row pointer; *sorted_flag_dev set to 0 if rows are not ascending
 int coo_rows_to_pos(const int64_t *rows, int64_t nnz, int64_t nrows, int64_t *pos, int *flag_dev,
                     cudaStream_t st);

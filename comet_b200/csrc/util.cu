@@ -141,7 +141,8 @@ __device__ __forceinline__ int64_t block_exclusive_scan(int64_t v, int64_t *tota
     return r;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) scan_tile_sums(const int64_t *__restrict__ in,
+template <typename InT>
+__global__ void __launch_bounds__(SCAN_THREADS) scan_tile_sums(const InT *__restrict__ in,
                                                                int64_t *__restrict__ sums, int64_t n)
 {
     int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
@@ -169,7 +170,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_sums_inplace(int64_t *sums,
     if (threadIdx.x == 0) *grand_total = carry;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) scan_apply(const int64_t *__restrict__ in,
+template <typename InT>
+__global__ void __launch_bounds__(SCAN_THREADS) scan_apply(const InT *__restrict__ in,
                                                            const int64_t *__restrict__ sums,
                                                            int64_t *__restrict__ out, int64_t n)
 {
@@ -190,7 +192,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply(const int64_t *__rest
     }
 }
 
-int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st)
+template <typename InT>
+static int exclusive_scan(const InT *in, int64_t *out, int64_t n, cudaStream_t st)
 {
     if (n <= 0) {
         CB_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), st));
@@ -208,6 +211,9 @@ int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t 
     CB_LAUNCH_CHECK();
     return 0;
 }
+
+int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st) { return exclusive_scan(in, out, n, st); }
+int exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st) { return exclusive_scan(in, out, n, st); }
 
 // ---------------------------------------------------------------------------
 // COO adapter: row coordinates sorted ascending (the reference reader sorts by
