@@ -110,6 +110,7 @@ for _op in ("spmv", "spmm", "sddmm", "spgemm_symbolic", "spgemm_numeric"):
         SIGNATURES["comet_b200_%s_f32_%s" % (_op, _w)] = SIGNATURES["comet_b200_%s_f64_i64" % _op]
 
 _lib = None
+_address = {}
 
 
 class CometB200Error(RuntimeError):
@@ -125,6 +126,10 @@ def load():
                 "libcomet_b200.so is missing (%s). Build it with `python -m comet_b200.build`; "
                 "there is no CPU fallback." % LIB_PATH)
         lib = ctypes.CDLL(LIB_PATH)
+        try:
+            from . import _pycall  # noqa: F401
+        except ImportError as e:
+            raise CometB200Error("_pycall.so is missing or does not load (%s). Build it with `python -m comet_b200.build`." % e)
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(lib, name)
             fn.restype = res
@@ -133,6 +138,14 @@ def load():
         lib.comet_b200_set_error_mode(1)
         _lib = lib
     return _lib
+
+
+def address(name):
+    """Address of an entry point, for ``_pycall.call`` / ``call_i32``."""
+    a = _address.get(name)
+    if a is None:
+        a = _address[name] = ctypes.cast(getattr(load(), name), c_void_p).value
+    return a
 
 
 def check(status=0):

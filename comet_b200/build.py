@@ -1,4 +1,4 @@
-"""Builds ``libcomet_b200.so`` in-tree with nvcc for sm_100a (no GPU needed to compile).
+"""Builds ``libcomet_b200.so`` (nvcc, sm_100a) and the Python call module ``_pycall.so`` in-tree (no GPU needed to compile).
 
     python -m comet_b200.build [--force] [--verbose]
 """
@@ -7,11 +7,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libcomet_b200.so")
+PYCALL = os.path.join(HERE, "_pycall.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -68,7 +70,21 @@ def build_library(force=False, verbose=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout)
             raise RuntimeError("link of libcomet_b200.so failed")
+    build_pycall(force)
     return LIB
+
+
+def build_pycall(force=False):
+    src = os.path.join(CSRC, "pycall.cpp")
+    if not force and not _stale(PYCALL, [src]):
+        return PYCALL
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           "-I" + sysconfig.get_paths()["include"], src, "-o", PYCALL]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout)
+        raise RuntimeError("build of _pycall.so failed")
+    return PYCALL
 
 
 if __name__ == "__main__":

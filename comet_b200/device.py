@@ -45,27 +45,43 @@ def to_device(A, device="cuda", pin=False):
 
 
 def _p(t):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # torch.cuda.current_stream() builds a Stream object (2 us); the handle is all that is needed
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _check_cuda(*ts):
     for t in ts:
-        if t is not None and (not t.is_cuda or not t.is_contiguous()):
+        if t is not None and not (t.is_cuda and t.is_contiguous()):
             raise ValueError("device entry points need contiguous CUDA tensors")
+
+
+_ready = None
+
+
+def _call(name, *args):
+    """Calls a device entry point (integers and addresses only); raises on a non-zero status."""
+    global _ready
+    if _ready is None:
+        _lib.load()
+        from . import _pycall
+        _ready = _pycall.call_i32
+    st = _ready(_lib.address(name), *args)
+    if st:
+        _lib.check(st)
 
 
 def spmv(A, x, y=None, semiring=PLUS_TIMES, accumulate=False):
     _check_cuda(A.pos, A.crd, A.val, x, y)
     if y is None:
-        y = torch.zeros(A.nrows, dtype=torch.float64, device=x.device)
-    lib = _lib.load()
-    st = lib.comet_b200_dev_spmv_f64_i64(A.nstored, A.nnz, _p(A.row_ids), _p(A.pos), _p(A.crd),
-                                         _p(A.val), _p(x), _p(y), semiring, int(accumulate), _stream())
-    _lib.check(st)
+        # rows a DCSR matrix does not store, and the values that are added to, start at zero; any other row is written
+        new = torch.zeros if A.row_ids is not None or accumulate else torch.empty
+        y = new(A.nrows, dtype=torch.float64, device=x.device)
+    _call("comet_b200_dev_spmv_f64_i64", A.nstored, A.nnz, _p(A.row_ids), A.pos.data_ptr(), A.crd.data_ptr(),
+          A.val.data_ptr(), x.data_ptr(), y.data_ptr(), semiring, int(accumulate), _stream())
     return y
 
 
@@ -79,11 +95,9 @@ def spmm(A, B, C=None, semiring=PLUS_TIMES, accumulate=False, variant=0):
         C = torch.empty((A.nrows, k), dtype=torch.float64, device=B.device)
         if A.row_ids is not None:
             C.zero_()
-    lib = _lib.load()
-    st = lib.comet_b200_dev_spmm_f64_i64(A.nstored, A.ncols, A.nnz, k, _p(A.row_ids), _p(A.pos),
-                                         _p(A.crd), _p(A.val), _p(B), B.stride(0), _p(C), C.stride(0),
-                                         semiring, int(accumulate), int(variant), _stream())
-    _lib.check(st)
+    _call("comet_b200_dev_spmm_f64_i64", A.nstored, A.ncols, A.nnz, k, _p(A.row_ids), A.pos.data_ptr(),
+          A.crd.data_ptr(), A.val.data_ptr(), B.data_ptr(), B.stride(0), C.data_ptr(), C.stride(0),
+          semiring, int(accumulate), int(variant), _stream())
     return C
 
 
@@ -92,10 +106,8 @@ def sddmm(S, X, Y, out=None):
     _check_cuda(S.pos, S.crd, S.val, X, Y, out)
     if out is None:
         out = torch.empty(S.nnz, dtype=torch.float64, device=X.device)
-    lib = _lib.load()
-    st = lib.comet_b200_dev_sddmm_f64_i64(S.nrows, S.nnz, X.shape[1], _p(S.pos), _p(S.crd), _p(S.val),
-                                          _p(X), X.stride(0), _p(Y), Y.stride(0), _p(out), _stream())
-    _lib.check(st)
+    _call("comet_b200_dev_sddmm_f64_i64", S.nrows, S.nnz, X.shape[1], S.pos.data_ptr(), S.crd.data_ptr(),
+          S.val.data_ptr(), X.data_ptr(), X.stride(0), Y.data_ptr(), Y.stride(0), out.data_ptr(), _stream())
     return out
 
 
@@ -108,25 +120,21 @@ class SpgemmResult:
 def spgemm_symbolic(A, B, M=None, semiring=PLUS_TIMES):
     """Returns (handle, cpos tensor, nnz)."""
     _check_cuda(A.pos, A.crd, A.val, B.pos, B.crd, B.val)
-    lib = _lib.load()
     cpos = torch.empty(A.nrows + 1, dtype=torch.int64, device=A.pos.device)
-    nnz = ctypes.c_int64(0)
-    handle = ctypes.c_int64(0)
-    st = lib.comet_b200_dev_spgemm_symbolic_f64_i64(
-        A.nrows, B.ncols, B.nnz, _p(A.pos), _p(A.crd), _p(A.val), _p(B.pos), _p(B.crd), _p(B.val),
-        _p(M.pos if M is not None else None), _p(M.crd if M is not None else None), semiring, _p(cpos),
-        ctypes.byref(nnz), ctypes.byref(handle), _stream())
-    _lib.check(st)
-    return handle.value, cpos, nnz.value
+    out = (ctypes.c_int64 * 2)()
+    at = ctypes.addressof(out)
+    _call("comet_b200_dev_spgemm_symbolic_f64_i64",
+          A.nrows, B.ncols, B.nnz, A.pos.data_ptr(), A.crd.data_ptr(), A.val.data_ptr(), B.pos.data_ptr(),
+          B.crd.data_ptr(), B.val.data_ptr(), M.pos.data_ptr() if M is not None else 0,
+          M.crd.data_ptr() if M is not None else 0, semiring, cpos.data_ptr(), at, at + 8, _stream())
+    return out[1], cpos, out[0]
 
 
 def spgemm_numeric(handle, nnz, device, keep=False, crd=None, val=None):
-    lib = _lib.load()
     if crd is None:
         crd = torch.empty(max(nnz, 1), dtype=torch.int64, device=device)[:nnz]
         val = torch.empty(max(nnz, 1), dtype=torch.float64, device=device)[:nnz]
-    st = lib.comet_b200_dev_spgemm_numeric_f64_i64(handle, _p(crd), _p(val), int(keep), _stream())
-    _lib.check(st)
+    _call("comet_b200_dev_spgemm_numeric_f64_i64", handle, crd.data_ptr(), val.data_ptr(), int(keep), _stream())
     return crd, val
 
 
@@ -141,10 +149,8 @@ def masked_pair_count(A, B, M, row_lo=0, row_hi=None, out=None):
     _check_cuda(A.pos, A.crd, B.pos, B.crd, M.pos, M.crd)
     row_hi = A.nrows if row_hi is None else row_hi
     if out is None:
-        out = torch.zeros(1, dtype=torch.int64, device=A.pos.device)
-    lib = _lib.load()
-    st = lib.comet_b200_dev_masked_spgemm_count_f64_i64(
-        row_lo, row_hi, B.ncols, A.nnz, B.nnz, M.nnz, _p(A.pos), _p(A.crd), _p(B.pos), _p(B.crd),
-        _p(M.pos), _p(M.crd), _p(out), _stream())
-    _lib.check(st)
+        out = torch.empty(1, dtype=torch.int64, device=A.pos.device)       # cleared by the call
+    _call("comet_b200_dev_masked_spgemm_count_f64_i64", row_lo, row_hi, B.ncols, A.nnz, B.nnz, M.nnz,
+          A.pos.data_ptr(), A.crd.data_ptr(), B.pos.data_ptr(), B.crd.data_ptr(), M.pos.data_ptr(), M.crd.data_ptr(),
+          out.data_ptr(), _stream())
     return out
