@@ -22,7 +22,6 @@ import ctypes
 import numpy as np
 
 from . import _lib
-from ._lib import MemRef1D, MemRef2D
 
 PLUS_TIMES, PLUS_PAIR, PLUS_FIRST, PLUS_SECOND, MIN_PLUS, MIN_FIRST, MIN_SECOND, ANY_PAIR = range(8)
 MASK_NONE = 0
@@ -121,43 +120,76 @@ def as_sparse(m):
 
 
 class _Packer:
-    """Builds the (rank, descriptor*) argument pairs and keeps the arrays alive."""
+    """Builds the (rank, descriptor address) argument pairs.  The descriptors of a call are the rows of one int64 array
+    ({allocated, aligned, offset, sizes..., strides...}); the arrays they point to are kept alive with it."""
+
+    _ROOM = 64                 # descriptors; a masked sparse product has 32
+    _WORDS = 7                 # 64-bit words of the largest one
 
     def __init__(self):
-        self.keep = []
+        self.words = (ctypes.c_int64 * (self._ROOM * self._WORDS))()
+        self.at = ctypes.addressof(self.words)
+        self.n = 0
+        self.keep = [self.words]
+
+    def _put(self, arr, *shape):
+        i = self.n * self._WORDS
+        self.n += 1
+        p = arr.__array_interface__["data"][0]
+        self.words[i:i + 3 + len(shape)] = (p, p, 0) + shape
+        self.keep.append(arr)
+        return self.at + 8 * i
 
     def m1(self, arr):
-        arr = np.ascontiguousarray(arr)
-        d = MemRef1D()
-        d.allocated = d.aligned = arr.ctypes.data
-        d.offset = 0
-        d.sizes[0] = arr.shape[0]
-        d.strides[0] = 1
-        self.keep += [arr, d]
-        return [1, ctypes.addressof(d)]
+        if not (arr.__class__ is np.ndarray and arr.ndim == 1 and arr.flags.c_contiguous):
+            arr = np.ascontiguousarray(arr)
+        return [1, self._put(arr, arr.shape[0], 1)]
 
     def m2(self, arr, transposed_view=False):
-        d = MemRef2D()
-        d.allocated = d.aligned = arr.ctypes.data
-        d.offset = 0
+        s0, s1 = arr.strides[0] // arr.itemsize, arr.strides[1] // arr.itemsize
         if transposed_view:       # present row-major [n, k] as a {k, n} memref with strides {1, ld}
-            d.sizes[0], d.sizes[1] = arr.shape[1], arr.shape[0]
-            d.strides[0], d.strides[1] = 1, arr.strides[0] // arr.itemsize
-        else:
-            d.sizes[0], d.sizes[1] = arr.shape
-            d.strides[0], d.strides[1] = arr.strides[0] // arr.itemsize, arr.strides[1] // arr.itemsize
-        self.keep += [arr, d]
-        return [2, ctypes.addressof(d)]
+            return [2, self._put(arr, arr.shape[1], arr.shape[0], 1, s0)]
+        return [2, self._put(arr, arr.shape[0], arr.shape[1], s0, s1)]
 
     def sparse(self, t):
         f1, f2 = _FMT[t.format]
-        empty = np.zeros(0, dtype=t.index_dtype)
+        none = self.m1(_EMPTY)    # the tile arrays: no elements
         dims = np.array([t.nrows, t.ncols], dtype=np.int64)
-        args = [f1, -1, f2, -1]
-        args += self.m1(t.a1pos) + self.m1(t.a1crd) + self.m1(empty) + self.m1(empty)
-        args += self.m1(t.a2pos) + self.m1(t.a2crd) + self.m1(empty) + self.m1(empty)
-        args += self.m1(t.val) + self.m1(dims)
-        return args
+        return [f1, -1, f2, -1, *self.m1(t.a1pos), *self.m1(t.a1crd), *none, *none, *self.m1(t.a2pos),
+                *self.m1(t.a2crd), *none, *none, *self.m1(t.val), *self.m1(dims)]
+
+
+_EMPTY = np.zeros(0, dtype=np.int64)
+
+
+class _ResultBlock:
+    """Page-locked memory of the library's pool; goes back when the array made from it is gone."""
+    __slots__ = ("address", "free", "__array_interface__")
+
+    def __init__(self, address, nbytes):
+        self.address = address
+        self.free = _lib.load().comet_b200_result_free      # arrays may outlive this module's globals
+        self.__array_interface__ = {"data": (address, False), "shape": (nbytes,), "typestr": "|u1", "version": 3}
+
+    def __del__(self):
+        self.free(self.address)
+
+
+_RESULT_MIN = 1 << 18          # smaller results are not worth a block
+
+
+def _result(shape, dtype):
+    """A new array for a result that the call writes completely: in page-locked memory when the library has a block,
+    which the device then fills by DMA (an ordinary new array is first faulted in page by page)."""
+    dtype = np.dtype(dtype)
+    n = dtype.itemsize
+    for d in (shape if isinstance(shape, tuple) else (shape,)):
+        n *= d
+    if n >= _RESULT_MIN:
+        p = _lib.load().comet_b200_result_alloc(n)
+        if p:
+            return np.asarray(_ResultBlock(p, n)).view(dtype).reshape(shape)
+    return np.empty(shape, dtype=dtype)
 
 
 _F32_OPS = ("spmv", "spmm", "sddmm", "spgemm_symbolic", "spgemm_numeric")
@@ -206,7 +238,10 @@ def spmv(A, x, y0=None, semiring=PLUS_TIMES):
     fn, _, (A,) = _entry(lib, "spmv", A, dense=(x,) if y0 is None else (x, y0))
     vt = fn.value_dtype
     x = np.ascontiguousarray(x, dtype=vt)
-    y = np.zeros(A.nrows, dtype=vt) if y0 is None else np.array(y0, dtype=vt)
+    if y0 is not None:
+        y = np.array(y0, dtype=vt)
+    else:
+        y = np.zeros(A.nrows, dtype=vt) if A.format == "DCSR" else _result(A.nrows, vt)     # DCSR leaves rows out
     fn(*pk.sparse(A), *pk.m1(x), *pk.m1(y), _dense_semiring(semiring), 0 if y0 is None else 1)
     _lib.check()
     return y
@@ -227,7 +262,10 @@ def spmm(A, B, C0=None, semiring=PLUS_TIMES, sharded=False):
     fn, _, (A,) = _entry(lib, _name("spmm", sharded), A, dense=(B,) if C0 is None else (B, C0))
     vt = fn.value_dtype
     B = np.ascontiguousarray(B, dtype=vt)
-    C = np.zeros((A.nrows, B.shape[1]), dtype=vt) if C0 is None else np.array(C0, dtype=vt, order="C")
+    if C0 is not None:
+        C = np.array(C0, dtype=vt, order="C")
+    else:
+        C = (np.zeros if A.format == "DCSR" else _result)((A.nrows, B.shape[1]), dtype=vt)   # DCSR leaves rows out
     fn(*pk.sparse(A), *pk.m2(B), *pk.m2(C), _dense_semiring(semiring), 0 if C0 is None else 1)
     _lib.check()
     return C
@@ -299,8 +337,7 @@ def _finish_sparse_out(lib, handle, nrows, ncols, cpos, sizes, vt=np.float64):
     _lib.check()
     nnz = int(sizes[8])
     dt = cpos.dtype
-    ccrd = np.zeros(nnz, dtype=dt)
-    cval = np.zeros(nnz, dtype=vt)
+    ccrd, cval = _result(nnz, dt), _result(nnz, vt)
     pk = _Packer()
     fn = getattr(lib, "comet_b200_spgemm_numeric_%s_%s" % ("f32" if vt == np.float32 else "f64",
                                                            "i32" if dt == np.int32 else "i64"))
@@ -418,23 +455,17 @@ def from_coordinates(rows, cols, vals, shape):
     """CSR from coordinate entries in any order, sorted on the device the way the reference reader sorts
     them on the host (by row, then column; entries with equal coordinates stay in input order and are
     kept, lib/ExecutionEngine/SparseUtils.cpp:360-533)."""
-    import torch
-    lib = _lib.load()
     nrows, ncols = int(shape[0]), int(shape[1])
-    r = torch.from_numpy(_i64(rows)).cuda()
-    c = torch.from_numpy(_i64(cols)).cuda()
-    v = torch.from_numpy(_f64(vals)).cuda()
-    nnz = int(r.shape[0])
-    pos = torch.empty(nrows + 1, dtype=torch.int64, device="cuda")
-    crd = torch.empty(nnz, dtype=torch.int64, device="cuda")
-    val = torch.empty(nnz, dtype=torch.float64, device="cuda")
-    st = lib.comet_b200_dev_coo_to_csr_f64_i64(nrows, ncols, nnz, r.data_ptr(), c.data_ptr(), v.data_ptr(),
-                                               pos.data_ptr(), crd.data_ptr(), val.data_ptr(),
-                                               torch.cuda.current_stream().cuda_stream)
-    _lib.check(st)
-    torch.cuda.synchronize()
-    return SparseTensor("CSR", nrows, ncols, np.array([nrows], dtype=np.int64), np.array([-1], dtype=np.int64),
-                        pos.cpu().numpy(), crd.cpu().numpy(), val.cpu().numpy())
+    rows, cols, vals = _i64(rows), _i64(cols), _f64(vals)
+    nnz = rows.shape[0]
+    if cols.shape[0] != nnz or vals.shape[0] != nnz:
+        raise ValueError("from_coordinates: rows, cols and vals have different lengths")
+    pos, crd, val = _result(nrows + 1, np.int64), _result(nnz, np.int64), _result(nnz, np.float64)
+    at = lambda a: a.__array_interface__["data"][0]
+    _lib.check(_lib.load().comet_b200_host_coo_to_csr(nrows, ncols, nnz, at(rows), at(cols), at(vals), at(pos), at(crd),
+                                                      at(val)))
+    return SparseTensor("CSR", nrows, ncols, np.array([nrows], dtype=np.int64), np.array([-1], dtype=np.int64), pos, crd,
+                        val)
 
 
 def reduce_sum(vals):

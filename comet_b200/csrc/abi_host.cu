@@ -156,7 +156,41 @@ struct DevBag {
     cudaStream_t st;
     std::vector<void *> ptrs;
     explicit DevBag(cudaStream_t s) : st(s) {}
-    ~DevBag() { for (void *p : ptrs) cudaFreeAsync(p, st); }
+    ~DevBag()
+    {
+        if (open) uploads_join();          // an early return: the copies still read the caller's arrays
+        for (void *p : ptrs) cudaFreeAsync(p, st);
+    }
+    // Between begin() and commit() the uploads below run side by side; what is made from them on the device (widened
+    // indices and values) is launched by commit(), and so must be everything else that reads them.
+    struct Widen {
+        bool index;
+        const void *src;
+        void *dst;
+        int64_t n;
+    };
+    bool open = false;
+    std::vector<Widen> later;
+    void begin() { open = uploads_begin(); }
+    int commit()
+    {
+        if (open) {
+            open = false;
+            CB_TRY(uploads_join());
+        }
+        for (const Widen &w : later) CB_TRY(widen(w));
+        later.clear();
+        return 0;
+    }
+    int widen(const Widen &w)
+    {
+        if (open) {
+            later.push_back(w);
+            return 0;
+        }
+        return w.index ? widen_i32_to_i64((const int32_t *)w.src, (int64_t *)w.dst, w.n, st)
+                       : widen_f32_to_f64((const float *)w.src, (double *)w.dst, w.n, st);
+    }
     int alloc(void **p, size_t bytes)
     {
         if (bytes == 0) bytes = 8;
@@ -188,6 +222,10 @@ struct DevBag {
             const size_t n = bytes - lo < s ? bytes - lo : s;
             CB_TRY(h2d((char *)*p + lo, (const char *)host + lo, n, st));
         }
+        if (open) {                        // the exchange reads this rank's slice
+            CB_TRY(uploads_join());
+            open = uploads_begin();
+        }
         return comm_allgather_inplace(cm, *p, s, st);
     }
     // n VALUES of the entry point's width -> double on the device
@@ -197,7 +235,7 @@ struct DevBag {
         void *narrow = nullptr;
         CB_TRY(upload_rep(&narrow, host, n * 4, cm));
         CB_TRY(alloc((void **)p, n * 8));
-        return widen_f32_to_f64((const float *)narrow, *p, (int64_t)n, st);
+        return widen({false, narrow, *p, (int64_t)n});
     }
     // n doubles on the device -> VALUES of the entry point's width in the host array
     int download_val(void *host, const double *dev, size_t n)
@@ -216,7 +254,7 @@ struct DevBag {
         void *narrow = nullptr;
         CB_TRY(upload_rep(&narrow, host, (size_t)n * 4, cm));
         CB_TRY(alloc((void **)p, (size_t)n * 8));
-        return widen_i32_to_i64((const int32_t *)narrow, *p, n, st);
+        return widen({true, narrow, *p, n});
     }
 };
 
@@ -242,37 +280,38 @@ static int pool_keep()
     return 0;
 }
 
-// Uploads a sparse operand; for COO it also derives the row pointer on the device.  The column
-// coordinates (and DCSR's row coordinates) are range-checked on the device and the stream is
-// synchronised, so a coordinate outside the matrix is reported here, before any kernel that gathers
-// through it has been launched.
-static int upload_sparse(const char *what, const HostSparse &h, DevBag &bag, DevSparse *d,
-                         bool need_val = true, Comm *rep = nullptr)
+// Uploads the arrays of a sparse operand (inside begin() / commit() with others, or on its own).
+static int stage_sparse(const HostSparse &h, DevBag &bag, DevSparse *d, bool need_val = true, Comm *rep = nullptr)
 {
     memset(d, 0, sizeof(*d));
-    cudaStream_t st = bag.st;
     CB_TRY(bag.upload_idx(&d->crd, h.a2crd, h.nnz, h.isz, rep));
     if (need_val) CB_TRY(bag.upload_val(&d->val, h.val, (size_t)h.nnz, rep));
+    d->nrows_k = h.fmt == F_DCSR ? h.nstored : h.nrows;
+    if (h.fmt != F_COO) CB_TRY(bag.upload_idx(&d->pos, h.a2pos, d->nrows_k + 1, h.isz, rep));
+    if (h.fmt == F_DCSR) CB_TRY(bag.upload_idx(&d->row_ids, h.a1crd, h.nstored, h.isz, rep));
+    if (h.fmt == F_COO) CB_TRY(bag.upload_idx(&d->rows, h.a1crd, h.nnz, h.isz, rep));
+    return 0;
+}
+
+// For COO derives the row pointer on the device.  The column coordinates (and DCSR's row coordinates) are
+// range-checked on the device and the stream is synchronised, so a coordinate outside the matrix is reported here,
+// before any kernel that gathers through it has been launched.
+static int check_sparse(const char *what, const HostSparse &h, DevBag &bag, DevSparse *d)
+{
+    cudaStream_t st = bag.st;
+    PinnedWords words;
+    if (!words.p) return fail("%s: no page-locked memory for the operand check", what);
     int *flags = nullptr;                     // [0] coordinates in range, [1] COO rows ascending and in range
     CB_TRY(bag.alloc((void **)&flags, 2 * sizeof(int)));
-    int got[2] = {1, 1};
-    CB_CUDA(cudaMemcpyAsync(flags, got, sizeof(got), cudaMemcpyHostToDevice, st));
+    CB_CUDA(cudaMemsetAsync(flags, 1, 2 * sizeof(int), st));          // any value but 0
     CB_TRY(check_index_range(d->crd, h.nnz, h.ncols, flags, st));
-    if (h.fmt == F_CSR) {
-        d->nrows_k = h.nrows;
-        CB_TRY(bag.upload_idx(&d->pos, h.a2pos, h.nrows + 1, h.isz, rep));
-    } else if (h.fmt == F_DCSR) {
-        d->nrows_k = h.nstored;
-        CB_TRY(bag.upload_idx(&d->pos, h.a2pos, h.nstored + 1, h.isz, rep));
-        CB_TRY(bag.upload_idx(&d->row_ids, h.a1crd, h.nstored, h.isz, rep));
-        CB_TRY(check_index_range(d->row_ids, h.nstored, h.nrows, flags, st));
-    } else {
-        d->nrows_k = h.nrows;
-        CB_TRY(bag.upload_idx(&d->rows, h.a1crd, h.nnz, h.isz, rep));
+    if (h.fmt == F_DCSR) CB_TRY(check_index_range(d->row_ids, h.nstored, h.nrows, flags, st));
+    if (h.fmt == F_COO) {
         CB_TRY(bag.alloc((void **)&d->pos, (size_t)(h.nrows + 1) * 8));
         CB_TRY(coo_rows_to_pos(d->rows, h.nnz, h.nrows, d->pos, flags + 1, st));
     }
-    CB_CUDA(cudaMemcpyAsync(got, flags, sizeof(got), cudaMemcpyDeviceToHost, st));
+    int *got = (int *)words.p;
+    CB_CUDA(cudaMemcpyAsync(got, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CB_CUDA(cudaStreamSynchronize(st));
     if (!got[1])
         return fail("%s: COO row coordinates must be ascending and inside [0, rows) "
@@ -281,6 +320,15 @@ static int upload_sparse(const char *what, const HostSparse &h, DevBag &bag, Dev
         return fail("%s: a coordinate lies outside the matrix (crd must be in [0, %lld)%s)", what,
                     (long long)h.ncols, h.fmt == F_DCSR ? ", stored row coordinates in [0, rows)" : "");
     return 0;
+}
+
+static int upload_sparse(const char *what, const HostSparse &h, DevBag &bag, DevSparse *d,
+                         bool need_val = true, Comm *rep = nullptr)
+{
+    bag.begin();
+    CB_TRY(stage_sparse(h, bag, d, need_val, rep));
+    CB_TRY(bag.commit());
+    return check_sparse(what, h, bag, d);
 }
 
 // Range check (then a stream synchronisation) of coordinate arrays uploaded outside upload_sparse:
@@ -376,12 +424,15 @@ static int spmv_host(const HostSparse &A, Arr x, Arr y, int semiring, int accumu
     CB_TRY(need_stream(&st));
     DevBag bag(st);
     DevSparse dA;
-    CB_TRY(upload_sparse("spmv", A, bag, &dA));
     double *dx, *dy;
+    bag.begin();
+    CB_TRY(stage_sparse(A, bag, &dA));
     CB_TRY(bag.upload_val(&dx, x.data, (size_t)A.ncols));
     bool keep_old = accumulate || A.fmt == F_DCSR;   // rows DCSR does not store keep their value
     if (keep_old) CB_TRY(bag.upload_val(&dy, y.data, (size_t)A.nrows));
     else CB_TRY(bag.alloc((void **)&dy, (size_t)A.nrows * 8));
+    CB_TRY(bag.commit());
+    CB_TRY(check_sparse("spmv", A, bag, &dA));
     if (!accumulate && A.fmt == F_DCSR) CB_CUDA(cudaMemsetAsync(dy, 0, (size_t)A.nrows * 8, st));
     CB_TRY(comet_b200_dev_spmv_f64_i64(dA.nrows_k, A.nnz, dA.row_ids, dA.pos, dA.crd, dA.val, dx, dy,
                                        semiring, accumulate, st));
@@ -516,14 +567,11 @@ static int spmm_host(const HostSparse &A, const Mat &B, const Mat &C, int semiri
     trace("spmm: begin (%lld rows, %lld entries, rank %d of %d)", (long long)A.nrows, (long long)A.nnz,
           cm ? cm->rank : 0, cm ? cm->nranks : 1);
     int rc = spmm_check(A, B, C);
-    if (!rc) rc = upload_sparse("spmm", A, bag, &dA);
-    trace("spmm: A uploaded and checked");
-    CB_TRY(guard.agree(rc));
-    trace("spmm: ranks agreed");
     const int64_t k = B.cols;
+    bool panels = false;
+    int64_t panel = 32;
     {
         // panels of 32 columns (256-byte rows) once the dense operands are big enough to matter
-        int64_t panel = 32;
         const char *env = getenv("COMET_B200_SPMM_PANEL");
         if (env) panel = atoll(env);
         double min_bytes = 256e6;
@@ -539,16 +587,29 @@ static int spmm_host(const HostSparse &A, const Mat &B, const Mat &C, int semiri
         // and pageable operands must force one mode with COMET_B200_SPMM_PANEL, since the all-gather of the
         // two paths differs.)
         const bool pinned = env || (!host_is_pageable(B.data) && !host_is_pageable(C.data));
-        if (!accumulate && A.fmt != F_DCSR && panel >= 2 && panel % 2 == 0 && k >= 2 * panel && big &&
-            semiring == COMET_B200_PLUS_TIMES && g_vsz == 8 && pinned)
-            return spmm_host_panels(A, dA, bag, B, C, semiring, panel, st, cm);
+        panels = !accumulate && A.fmt != F_DCSR && panel >= 2 && panel % 2 == 0 && k >= 2 * panel && big &&
+                 semiring == COMET_B200_PLUS_TIMES && g_vsz == 8 && pinned;
     }
     double *dB, *dC;
-    CB_TRY(bag.upload_val(&dB, B.data, (size_t)((A.ncols - 1) * B.s0 + k) * (A.ncols > 0), cm));
     size_t cbytes = A.nrows > 0 ? (size_t)((A.nrows - 1) * C.s0 + k) * 8 : 0;
-    bool keep_old = accumulate || A.fmt == F_DCSR || C.s0 != k;
-    if (keep_old) CB_TRY(bag.upload_val(&dC, C.data, cbytes / 8));
-    else CB_TRY(bag.alloc((void **)&dC, cbytes));
+    const bool keep_old = accumulate || A.fmt == F_DCSR || C.s0 != k;
+    auto stage_dense = [&]() {
+        CB_TRY(bag.upload_val(&dB, B.data, (size_t)((A.ncols - 1) * B.s0 + k) * (A.ncols > 0), cm));
+        if (keep_old) CB_TRY(bag.upload_val(&dC, C.data, cbytes / 8));
+        else CB_TRY(bag.alloc((void **)&dC, cbytes));
+        return 0;
+    };
+    const bool together = !cm && !panels;         // ranks agree on A before they exchange B; panels upload B themselves
+    bag.begin();
+    if (!rc) rc = stage_sparse(A, bag, &dA);
+    if (!rc && together) rc = stage_dense();
+    if (!rc) rc = bag.commit();
+    if (!rc) rc = check_sparse("spmm", A, bag, &dA);
+    trace("spmm: A uploaded and checked");
+    CB_TRY(guard.agree(rc));
+    trace("spmm: ranks agreed");
+    if (panels) return spmm_host_panels(A, dA, bag, B, C, semiring, panel, st, cm);
+    if (!together) CB_TRY(stage_dense());
     if (!accumulate && A.fmt == F_DCSR) CB_CUDA(cudaMemsetAsync(dC, 0, cbytes, st));
     CB_TRY(comet_b200_dev_spmm_f64_i64(dA.nrows_k, A.ncols, A.nnz, k, dA.row_ids, dA.pos, dA.crd,
                                        dA.val, dB, B.s0, dC, C.s0, semiring, accumulate, 0, st));
@@ -665,17 +726,23 @@ static void sddmm_impl(int mode, COMET_B200_SPARSE2D(S), int64_t X_rank, void *X
     int rc = GET_SPARSE("sddmm: S", S, &S) || GET_SPARSE("sddmm: O", O, &O) ||
              get2d("sddmm: X", X_rank, X_ptr, &X) || get2d("sddmm: D", D_rank, D_ptr, &D);
     if (!rc) rc = sddmm_check(S, O, X, D);
-    if (!rc) rc = upload_sparse("sddmm", S, bag, &dS);
     const int64_t k = rc ? 0 : X.cols;
+    double *dD = nullptr;
+    auto stage_d = [&]() {
+        if (D.s0 == 1)                        // a row-major [cols, K] matrix viewed transposed
+            return bag.upload_val(&dY, D.data, S.ncols > 0 ? (size_t)((S.ncols - 1) * D.s1 + k) : 0, cm);
+        return bag.upload_val(&dD, D.data, k > 0 ? (size_t)((k - 1) * D.s0 + S.ncols) : 0, cm);
+    };
+    bag.begin();
+    if (!rc) rc = stage_sparse(S, bag, &dS);
     if (!rc) rc = bag.upload_val(&dX, X.data, S.nrows > 0 ? (size_t)((S.nrows - 1) * X.s0 + k) : 0);
+    if (!rc && !cm) rc = stage_d();           // ranks agree before they exchange D
+    if (!rc) rc = bag.commit();
+    if (!rc) rc = check_sparse("sddmm", S, bag, &dS);
     if (guard.agree(rc)) return;
-    int64_t ldy;
-    if (D.s0 == 1) {                          // a row-major [cols, K] matrix viewed transposed
-        ldy = D.s1;
-        if (bag.upload_val(&dY, D.data, S.ncols > 0 ? (size_t)((S.ncols - 1) * ldy + k) : 0, cm)) return;
-    } else {                                  // D[k, j]: transpose on the device
-        double *dD;
-        if (bag.upload_val(&dD, D.data, k > 0 ? (size_t)((k - 1) * D.s0 + S.ncols) : 0, cm)) return;
+    if (cm && stage_d()) return;
+    int64_t ldy = D.s1;
+    if (D.s0 != 1) {                          // D[k, j]: transpose on the device
         ldy = k + (k & 1);
         if (bag.alloc((void **)&dY, (size_t)S.ncols * ldy * 8)) return;
         if (comet_b200_dev_transpose_f64(k, S.ncols, dD, D.s0, dY, ldy, st)) return;
@@ -1261,3 +1328,29 @@ SHARDED_WIDTHS(void, masked_spgemm_count, masked_count_impl,
 
 extern "C" void comet_b200_transpose_2D_f64_i64(TRANSPOSE_ARGS) { TRANSPOSE_BODY(8); }
 extern "C" void comet_b200_transpose_2D_f64_i32(TRANSPOSE_ARGS) { TRANSPOSE_BODY(4); }
+
+extern "C" int32_t comet_b200_host_coo_to_csr(int64_t nrows, int64_t ncols, int64_t nnz, const int64_t *rows,
+                                              const int64_t *cols, const double *vals, int64_t *pos, int64_t *crd, double *val)
+{
+    clear_error();
+    if (nrows < 0 || ncols < 0 || nnz < 0) return fail("coo_to_csr: negative size");
+    cudaStream_t st;
+    CB_TRY(need_stream(&st));
+    DevBag bag(st);
+    const size_t bytes = (size_t)nnz * 8;
+    void *dr, *dc, *dv, *dpos, *dcrd, *dval;
+    bag.begin();
+    CB_TRY(bag.upload(&dr, rows, bytes));
+    CB_TRY(bag.upload(&dc, cols, bytes));
+    CB_TRY(bag.upload(&dv, vals, bytes));
+    CB_TRY(bag.commit());
+    CB_TRY(bag.alloc(&dpos, (size_t)(nrows + 1) * 8));
+    CB_TRY(bag.alloc(&dcrd, bytes));
+    CB_TRY(bag.alloc(&dval, bytes));
+    CB_TRY(comet_b200_dev_coo_to_csr_f64_i64(nrows, ncols, nnz, (const int64_t *)dr, (const int64_t *)dc, (const double *)dv,
+                                             (int64_t *)dpos, (int64_t *)dcrd, (double *)dval, st));
+    CB_TRY(d2h(crd, dcrd, bytes, st));
+    CB_TRY(d2h(val, dval, bytes, st));
+    CB_TRY(d2h(pos, dpos, (size_t)(nrows + 1) * 8, st));
+    return finish(st);
+}

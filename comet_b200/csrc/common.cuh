@@ -61,6 +61,7 @@ enum Slot {
 };
 int scratch(Slot slot, size_t bytes, void **ptr);   // status; *ptr valid until the slot grows
 void scratch_release_all();
+void result_release_kept();                          // page-locked result blocks that are not in use (hostmem.cu)
 
 int sm_count();
 cudaStream_t lib_stream();   // the library's own stream for the host-memref entry points

@@ -161,6 +161,10 @@ void comet_b200_set_error_mode(int32_t return_instead_of_exit)
 
 int32_t comet_b200_version(void) { return 100; }
 
-void comet_b200_release_scratch(void) { cb200::scratch_release_all(); }
+void comet_b200_release_scratch(void)
+{
+    cb200::scratch_release_all();
+    cb200::result_release_kept();
+}
 
 }

@@ -626,7 +626,19 @@ COMET_B200_EXPORT int32_t comet_b200_dev_gather_probe_f64_i64(int64_t nnz, const
 /* Measurement aid: launches an empty kernel on `stream` (the launch floor of back-to-back small calls). */
 COMET_B200_EXPORT int32_t comet_b200_dev_noop(void *stream);
 
-/* Frees the library's scratch memory on the current device. */
+/* Coordinate entries in host memory, in any order -> CSR arrays in host memory (pos[nrows+1], crd[nnz], val[nnz]):
+   upload, comet_b200_dev_coo_to_csr_f64_i64 on the library's stream, download.  Returns 0 on success. */
+COMET_B200_EXPORT int32_t comet_b200_host_coo_to_csr(int64_t nrows, int64_t ncols, int64_t nnz, const int64_t *rows,
+                                                     const int64_t *cols, const double *vals, int64_t *pos, int64_t *crd,
+                                                     double *val);
+
+/* Page-locked memory for a result of `bytes` bytes, from a pool of at most 1 GiB that is kept between calls; NULL when the
+   pool has no block of that size (it may have one the next time): use ordinary memory then.  Contents are undefined.
+   result_free gives a block back; both may be called from any thread. */
+COMET_B200_EXPORT void *comet_b200_result_alloc(int64_t bytes);
+COMET_B200_EXPORT void comet_b200_result_free(void *p);
+
+/* Frees the library's scratch memory on the current device, and the kept result blocks. */
 COMET_B200_EXPORT void comet_b200_release_scratch(void);
 
 #ifdef __cplusplus
