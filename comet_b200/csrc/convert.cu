@@ -4,174 +4,239 @@
 // COMET does these on the host with one thread: the reader sorts the parsed entries with
 // std::stable_sort by (row, col) and keeps duplicates (lib/ExecutionEngine/SparseUtils.cpp:360-367,
 // 404-533), and transpose_2D turns CSR into coordinates, sorts them by (col, row) and rebuilds the
-// row pointer (lib/ExecutionEngine/TransposeUtils.cpp:738-812).  Here both are one radix sort of
-// 64-bit keys major * extent + minor carrying the entry's position (least significant digit first,
-// stable, so equal coordinates keep their input order like stable_sort), a gather of the values, and
-// the row pointer from the sorted majors.
+// row pointer (lib/ExecutionEngine/TransposeUtils.cpp:738-812).  Here both are one radix sort (least significant
+// digit first, stable, so equal coordinates keep their input order like stable_sort) of keys major | minor in as
+// many bits as the two extents need, carrying the entry's position, then a gather of the values and
+// the row pointer by binary search in the sorted keys.  A CSR matrix is already in row order, so its
+// transpose sorts by the column alone.
 //
-// The sort is this file's own: per 8-bit digit, a counting kernel (digit histogram per tile), one
-// exclusive scan over the digit-major table of counts, and a scatter kernel that ranks every key
-// inside its tile.  Ranking is what makes it stable: a warp walks its part of the tile 32
-// consecutive keys at a time, `__match_any_sync` names the lanes that hold the same digit, a key's
-// rank is the number of such lanes below it plus the count its warp has already seen for the digit,
-// and warps are ordered by a prefix over their counts.
+// The sort is this file's own.  One kernel makes the keys and counts the digits of all passes; a pass is one kernel:
+// a CTA ranks a tile of keys by their digit, learns from the tiles before it where its runs of equal digits
+// start (each tile publishes its digit counts, then their sums over all tiles so far, and looks back until it meets
+// such a sum), orders the tile in shared memory and writes it out run by run.  Tiles are numbered in the order in
+// which CTAs start, so the tiles looked back at are running or done; the wait is bounded all the same.  Ranking
+// is what makes it stable: a warp walks its part of the tile 32 consecutive keys at a time, `__match_any_sync`
+// names the lanes that hold the same digit, a key's rank is the number of such lanes below it plus the
+// count its warp has already seen for the digit, and warps are ordered by a prefix over their counts.
 //
-// Bound: HBM (a pass reads 32 and writes 16 bytes per entry; passes = key bits / 8).
+// Bound: HBM or L2 (a pass reads and writes key and position once: 2 x 12 bytes per entry for keys above 32 bits and fewer
+// than 2^32 entries; passes = key bits / 8, rounded up).  Measured on B200: 4.2 M entries with 36-bit keys 28 us for the keys,
+// 67 us a pass, 47 us for gather and row pointer (a count, three scan and a scatter kernel per pass before); 1000 entries
+// from and to host arrays 735 -> 141 us.
 #include "common.cuh"
+#include "hostcopy.cuh"
 
 namespace cb200 {
 
 // ---------------------------------------------------------------------------
-// Stable LSD radix sort of (uint64 key, int64 payload) pairs.
+// Stable LSD radix sort of (key, position) pairs.
 // ---------------------------------------------------------------------------
 static const int RS_THREADS = 256;                    // 8 warps
+static const int RS_WARPS = RS_THREADS / 32;
 static const int RS_ROUNDS = 16;                      // rounds of 32 keys per warp
 static const int RS_TILE = RS_THREADS * RS_ROUNDS;    // keys per CTA
 static const int RS_DIGITS = 256;
+static const int RS_MAX_PASSES = 8;
+static const int RS_COPIES = 8;                       // histograms a CTA keeps while counting: equal digits meet 4 lanes at most
+static const uint64_t RS_COUNT = 1ull << 62;          // state word: the tile's own count
+static const uint64_t RS_SUM = 2ull << 62;            // state word: sum over all tiles up to this one
+static const int RS_SPIN_LIMIT = 1 << 24;
 
-// Walks this warp's part of the tile in order.  On return cnt[d] (this warp's row of shared counters) holds
-// the number of keys with digit d, and offs[r] the rank of the key of round r among the warp's keys with the
-// same digit.  SCATTER = false only counts.
-template <bool SCATTER>
-__device__ __forceinline__ void rs_rank_warp(const uint64_t *__restrict__ keys, int64_t base, int64_t n, int shift,
-                                             unsigned *cnt, uint64_t (&k)[RS_ROUNDS], unsigned (&offs)[RS_ROUNDS])
+struct SortPlan {
+    int passes, width;                                // digits of `width` bits
+    int64_t ntiles;
+    int *bad;                                         // [0] coordinate outside the matrix, [1] a look-back gave up
+    unsigned *ticket;                                 // one per pass
+    uint64_t *hist;                                   // [pass][digit] counts, then their exclusive sums
+    uint64_t *state;                                  // [pass][tile][digit]
+};
+
+// Counts the digits of every pass of one key into the CTA's histograms.
+template <typename KeyT>
+__device__ __forceinline__ void rs_count_key(unsigned *h, KeyT key, int passes, int width)
 {
-    const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
+    const int copy = threadIdx.x & (RS_COPIES - 1);
+    for (int p = 0; p < passes; p++)
+        atomicAdd(&h[((p * RS_DIGITS) + ((unsigned)(key >> (p * width)) & ((1u << width) - 1u))) * RS_COPIES + copy], 1u);
+}
+
+__device__ __forceinline__ void rs_count_flush(const unsigned *h, int passes, uint64_t *hist)
+{
+    for (int i = threadIdx.x; i < passes * RS_DIGITS; i += blockDim.x) {
+        unsigned t = 0;
+        for (int c = 0; c < RS_COPIES; c++) t += h[i * RS_COPIES + c];
+        if (t) atomicAdd((unsigned long long *)hist + i, (unsigned long long)t);
+    }
+}
+
+// keys of coordinate entries; `minor` null: the major coordinate alone
+template <typename KeyT>
+__global__ void __launch_bounds__(256)
+rs_make_keys_kernel(int64_t n, const int64_t *__restrict__ major, const int64_t *__restrict__ minor, int64_t nmajor,
+                    int64_t nminor, int minor_bits, KeyT *__restrict__ keys, SortPlan sp)
+{
+    extern __shared__ unsigned s_hist[];
+    for (int i = threadIdx.x; i < sp.passes * RS_DIGITS * RS_COPIES; i += blockDim.x) s_hist[i] = 0;
+    __syncthreads();
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t a = __ldcs((const long long *)major + i), b = minor ? __ldcs((const long long *)minor + i) : 0;
+        KeyT key = 0;                                 // reported by the host; the key stays in range
+        if (a < 0 || a >= nmajor || b < 0 || b >= nminor) *sp.bad = 1;
+        else key = (KeyT)(((uint64_t)a << minor_bits) | (uint64_t)b);
+        keys[i] = key;
+        rs_count_key(s_hist, key, sp.passes, sp.width);
+    }
+    __syncthreads();
+    rs_count_flush(s_hist, sp.passes, sp.hist);
+}
+
+// counts -> exclusive sums, a CTA per pass
+__global__ void __launch_bounds__(RS_DIGITS)
+rs_scan_kernel(uint64_t *hist)
+{
+    __shared__ uint64_t s[RS_DIGITS];
+    uint64_t *h = hist + blockIdx.x * RS_DIGITS;
+    const uint64_t own = h[threadIdx.x];
+    s[threadIdx.x] = own;
+    __syncthreads();
+    for (int o = 1; o < RS_DIGITS; o <<= 1) {
+        const uint64_t v = (int)threadIdx.x >= o ? s[threadIdx.x - o] : 0;
+        __syncthreads();
+        s[threadIdx.x] += v;
+        __syncthreads();
+    }
+    h[threadIdx.x] = s[threadIdx.x] - own;
+}
+
+// One pass.  FIRST: the position of key i is i.
+template <typename KeyT, typename IdxT, bool FIRST>
+__global__ void __launch_bounds__(RS_THREADS)
+rs_pass_kernel(int64_t n, const KeyT *__restrict__ keys, const IdxT *__restrict__ idx, KeyT *__restrict__ keys_out,
+               IdxT *__restrict__ idx_out, int pass, SortPlan sp)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    KeyT *s_keys = (KeyT *)s_raw;
+    IdxT *s_idx = (IdxT *)(s_keys + RS_TILE);
+    __shared__ unsigned cnt[RS_WARPS][RS_DIGITS];
+    __shared__ unsigned local[RS_DIGITS];             // first place of the digit's run in the ordered tile
+    __shared__ int64_t start[RS_DIGITS];              // first place of the tile's run of the digit in the output
+    __shared__ unsigned warp_sum[RS_WARPS];
+    __shared__ unsigned s_tile;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, d0 = threadIdx.x;
+    const int shift = pass * sp.width;
+    const unsigned mask = (1u << sp.width) - 1u, below = (1u << lane) - 1u;
+    if (threadIdx.x == 0) s_tile = atomicAdd(sp.ticket + pass, 1u);
+    for (int i = threadIdx.x; i < RS_WARPS * RS_DIGITS; i += RS_THREADS) (&cnt[0][0])[i] = 0;
+    __syncthreads();
+    const int64_t tile = s_tile;
+    const int64_t base = tile * RS_TILE + (int64_t)w * 32 * RS_ROUNDS + lane;
+    KeyT k[RS_ROUNDS];
+    IdxT v[RS_ROUNDS];
+    unsigned rank[RS_ROUNDS];
 #pragma unroll
     for (int r = 0; r < RS_ROUNDS; r++) {
-        const int64_t i = base + r * 32 + lane;
-        const bool live = i < n;
-        const uint64_t key = live ? keys[i] : 0;
-        const unsigned d = live ? (unsigned)((key >> shift) & (RS_DIGITS - 1)) : RS_DIGITS;   // dead lanes form their own group
+        const int64_t i = base + r * 32;
+        k[r] = i < n ? keys[i] : 0;
+        v[r] = FIRST ? (IdxT)i : (i < n ? idx[i] : 0);
+    }
+#pragma unroll
+    for (int r = 0; r < RS_ROUNDS; r++) {
+        const bool live = base + r * 32 < n;
+        const unsigned d = live ? (unsigned)(k[r] >> shift) & mask : RS_DIGITS;    // dead lanes form their own group
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         const int leader = __ffs(peers) - 1;
         unsigned old = 0;
         if (live && lane == leader) {
-            old = cnt[d];
-            cnt[d] = old + __popc(peers);
+            old = cnt[w][d];
+            cnt[w][d] = old + __popc(peers);
         }
         old = __shfl_sync(0xffffffffu, old, leader);
         __syncwarp();
-        if (SCATTER) {
-            k[r] = key;
-            offs[r] = old + __popc(peers & below);
-        }
+        rank[r] = old + __popc(peers & below);
     }
-}
-
-// hist[d * ntiles + tile] = number of keys of the tile with digit d
-__global__ void __launch_bounds__(RS_THREADS)
-rs_count_kernel(const uint64_t *__restrict__ keys, int64_t n, int shift, int64_t ntiles, int64_t *__restrict__ hist)
-{
-    __shared__ unsigned cnt[RS_THREADS / 32][RS_DIGITS];
-    const int w = threadIdx.x >> 5;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        for (int i = threadIdx.x; i < (RS_THREADS / 32) * RS_DIGITS; i += RS_THREADS) (&cnt[0][0])[i] = 0;
-        __syncthreads();
-        uint64_t k[RS_ROUNDS];
-        unsigned offs[RS_ROUNDS];
-        rs_rank_warp<false>(keys, tile * RS_TILE + (int64_t)w * 32 * RS_ROUNDS, n, shift, cnt[w], k, offs);
-        __syncthreads();
-        if (threadIdx.x < RS_DIGITS) {
-            unsigned t = 0;
-            for (int i = 0; i < RS_THREADS / 32; i++) t += cnt[i][threadIdx.x];
-            hist[(int64_t)threadIdx.x * ntiles + tile] = t;
-        }
-        __syncthreads();
+    __syncthreads();
+    unsigned total = 0;                               // this thread's digit: keys of it in the tile
+    for (int i = 0; i < RS_WARPS; i++) {
+        const unsigned c = cnt[i][d0];
+        cnt[i][d0] = total;
+        total += c;
     }
-}
-
-// base[d * ntiles + tile] = first output position of the tile's keys with digit d (exclusive scan of hist)
-__global__ void __launch_bounds__(RS_THREADS)
-rs_scatter_kernel(const uint64_t *__restrict__ keys, const int64_t *__restrict__ vals, int64_t n, int shift,
-                  int64_t ntiles, const int64_t *__restrict__ base, uint64_t *__restrict__ keys_out,
-                  int64_t *__restrict__ vals_out)
-{
-    __shared__ unsigned cnt[RS_THREADS / 32][RS_DIGITS];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        for (int i = threadIdx.x; i < (RS_THREADS / 32) * RS_DIGITS; i += RS_THREADS) (&cnt[0][0])[i] = 0;
-        __syncthreads();
-        uint64_t k[RS_ROUNDS];
-        unsigned offs[RS_ROUNDS];
-        const int64_t wbase = tile * RS_TILE + (int64_t)w * 32 * RS_ROUNDS;
-        rs_rank_warp<true>(keys, wbase, n, shift, cnt[w], k, offs);
-        __syncthreads();
-        if (threadIdx.x < RS_DIGITS) {        // counts per warp -> start of each warp's keys inside the tile's run of the digit
-            unsigned run = 0;
-            for (int i = 0; i < RS_THREADS / 32; i++) {
-                const unsigned c = cnt[i][threadIdx.x];
-                cnt[i][threadIdx.x] = run;
-                run += c;
-            }
-        }
-        __syncthreads();
+    volatile uint64_t *state = sp.state + ((int64_t)pass * sp.ntiles) * RS_DIGITS;
+    state[tile * RS_DIGITS + d0] = (tile == 0 ? RS_SUM : RS_COUNT) | total;
+    unsigned incl = total;
 #pragma unroll
-        for (int r = 0; r < RS_ROUNDS; r++) {
-            const int64_t i = wbase + r * 32 + lane;
-            if (i < n) {
-                const unsigned d = (unsigned)((k[r] >> shift) & (RS_DIGITS - 1));
-                const int64_t at = base[(int64_t)d * ntiles + tile] + cnt[w][d] + offs[r];
-                keys_out[at] = k[r];
-                vals_out[at] = vals[i];
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_sum[w] = incl;
+    __syncthreads();
+    unsigned off = incl - total;
+    for (int i = 0; i < w; i++) off += warp_sum[i];
+    local[d0] = off;
+    uint64_t before = 0;                              // keys of the digit in earlier tiles
+    for (int64_t t = tile - 1; t >= 0; t--) {
+        uint64_t s = 0;
+        for (int spin = 0; (s = state[t * RS_DIGITS + d0]) < RS_COUNT; spin++)
+            if (spin > RS_SPIN_LIMIT) {
+                sp.bad[1] = 1;
+                s = RS_SUM;
+                break;
             }
+        before += s & (RS_COUNT - 1);
+        if (s >= RS_SUM) break;
+    }
+    if (tile > 0) state[tile * RS_DIGITS + d0] = RS_SUM | (before + total);
+    start[d0] = (int64_t)(sp.hist[pass * RS_DIGITS + d0] + before) - off;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RS_ROUNDS; r++) {
+        if (base + r * 32 >= n) continue;
+        const unsigned d = (unsigned)(k[r] >> shift) & mask;
+        const unsigned at = local[d] + cnt[w][d] + rank[r];
+        s_keys[at] = k[r];
+        s_idx[at] = v[r];
+    }
+    __syncthreads();
+    const int64_t left = n - tile * RS_TILE;
+    const int live = left < RS_TILE ? (int)left : RS_TILE;
+    for (int i = threadIdx.x; i < live; i += RS_THREADS) {
+        const KeyT key = s_keys[i];
+        const int64_t at = start[(unsigned)(key >> shift) & mask] + i;
+        if (at >= 0 && at < n) {                      // always, unless a look-back gave up
+            keys_out[at] = key;
+            idx_out[at] = s_idx[i];
         }
-        __syncthreads();
     }
 }
 
-// Sorts n pairs by the low `bits` bits of the key.  The result is in (keys, vals) or (keys2, vals2): *in_second
-// tells which.  hist / base: scratch of 256 * ntiles + 1 int64 each.
-static int radix_sort_pairs(uint64_t *keys, uint64_t *keys2, int64_t *vals, int64_t *vals2, int64_t n, int bits,
-                            int64_t *hist, int64_t *base, bool *in_second, cudaStream_t st)
-{
-    const int64_t ntiles = ceil_div(n, RS_TILE);
-    int64_t grid = ntiles;
-    const int64_t cap = (int64_t)sm_count() * 8;
-    if (grid > cap) grid = cap;
-    bool second = false;
-    for (int shift = 0; shift < bits; shift += 8) {
-        uint64_t *kin = second ? keys2 : keys, *kout = second ? keys : keys2;
-        int64_t *vin = second ? vals2 : vals, *vout = second ? vals : vals2;
-        rs_count_kernel<<<(unsigned)grid, RS_THREADS, 0, st>>>(kin, n, shift, ntiles, hist);
-        CB_LAUNCH_CHECK();
-        CB_TRY(exclusive_scan_i64(hist, base, RS_DIGITS * ntiles, st));
-        rs_scatter_kernel<<<(unsigned)grid, RS_THREADS, 0, st>>>(kin, vin, n, shift, ntiles, base, kout, vout);
-        CB_LAUNCH_CHECK();
-        second = !second;
-    }
-    *in_second = second;
-    return 0;
-}
-
+template <typename KeyT, typename IdxT>
 __global__ void __launch_bounds__(256)
-make_keys_kernel(int64_t n, const int64_t *__restrict__ major, const int64_t *__restrict__ minor,
-                 int64_t nmajor, int64_t nminor, uint64_t *__restrict__ keys, int64_t *__restrict__ idx,
-                 int *__restrict__ bad)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = major[i], b = minor[i];
-        if (a < 0 || a >= nmajor || b < 0 || b >= nminor) {
-            *bad = 1;                                   // reported by the host; the key stays in range
-            keys[i] = 0;
-        } else {
-            keys[i] = (uint64_t)a * (uint64_t)nminor + (uint64_t)b;
-        }
-        idx[i] = i;
-    }
-}
-
-__global__ void __launch_bounds__(256)
-gather_sorted_kernel(int64_t n, const uint64_t *__restrict__ keys, const int64_t *__restrict__ idx,
-                     int64_t nminor, const double *__restrict__ vals, int64_t *__restrict__ major_out,
-                     int64_t *__restrict__ minor_out, double *__restrict__ vals_out)
+rs_gather_kernel(int64_t n, const KeyT *__restrict__ keys, const IdxT *__restrict__ idx, int minor_bits,
+                 const double *__restrict__ vals, const int64_t *__restrict__ payload, int64_t *__restrict__ major_out,
+                 int64_t *__restrict__ minor_out, double *__restrict__ vals_out)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t k = keys[i];
-        if (major_out) major_out[i] = (int64_t)(k / (uint64_t)nminor);
-        if (minor_out) minor_out[i] = (int64_t)(k % (uint64_t)nminor);
-        if (vals_out) vals_out[i] = vals[idx[i]];
+        const int64_t from = vals_out || payload ? (int64_t)idx[i] : 0;
+        if (major_out) major_out[i] = (int64_t)(k >> minor_bits);
+        if (minor_out) minor_out[i] = payload ? payload[from] : (int64_t)(k & ((1ull << minor_bits) - 1ull));
+        if (vals_out) vals_out[i] = vals[from];
+    }
+}
+
+// pos[r] = first sorted key whose major coordinate is r or more
+template <typename KeyT>
+__global__ void __launch_bounds__(256)
+rs_pos_kernel(int64_t n, const KeyT *__restrict__ keys, int minor_bits, int64_t nmajor, int64_t *__restrict__ pos)
+{
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= nmajor; r += (int64_t)gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = n;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if ((int64_t)((uint64_t)keys[mid] >> minor_bits) < r) lo = mid + 1; else hi = mid;
+        }
+        pos[r] = lo;
     }
 }
 
@@ -193,64 +258,99 @@ static unsigned grid_for(int64_t work)
     return (unsigned)(blocks > cap ? cap : blocks);
 }
 
-static int key_bits(int64_t nmajor, int64_t nminor, int *bits)
+static int extent_bits(int64_t n)
 {
-    if (nmajor <= 0 || nminor <= 0) return fail("sort: empty coordinate space");
-    const unsigned __int128 space = (unsigned __int128)nmajor * (unsigned __int128)nminor;
-    if (space >> 63) return fail("sort: rows x cols = %lld x %lld does not fit a 63-bit key", (long long)nmajor,
-                                 (long long)nminor);
-    int b = 1;
-    while (b < 63 && ((unsigned __int128)1 << b) < space) b++;
-    *bits = b;
-    return 0;
+    int b = 0;
+    while (b < 63 && ((int64_t)1 << b) < n) b++;
+    return b;
 }
 
-// Entries sorted by (major, minor), equal coordinates in input order.  Any of the outputs may be null.
+struct SortOut {
+    int64_t *major, *minor, *pos;                     // pos: row pointer over the major coordinate
+    double *vals;
+};
+
+template <typename KeyT, typename IdxT>
+static int sort_entries(int64_t n, int64_t nmajor, int64_t nminor, int bits, int minor_bits, const int64_t *major,
+                        const int64_t *minor, const double *vals, const int64_t *payload, const SortOut &out, cudaStream_t st)
+{
+    SortPlan sp;
+    sp.passes = bits > 0 ? (bits + 7) / 8 : 1;
+    sp.width = bits > 0 ? (bits + sp.passes - 1) / sp.passes : 1;
+    sp.ntiles = ceil_div(n, RS_TILE);
+    auto pad = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t head = 256, hist = sizeof(uint64_t) * RS_DIGITS * sp.passes,
+                 state = sizeof(uint64_t) * RS_DIGITS * sp.passes * (size_t)sp.ntiles, cleared = pad(head + hist + state);
+    char *mem = nullptr;
+    const size_t bytes = cleared + 2 * pad((size_t)n * sizeof(KeyT)) + 2 * pad((size_t)n * sizeof(IdxT));
+    if (cudaMallocAsync((void **)&mem, bytes, st) != cudaSuccess) return fail("sort: device allocation of %zu bytes failed", bytes);
+    sp.bad = (int *)mem;
+    sp.ticket = (unsigned *)(mem + 64);
+    sp.hist = (uint64_t *)(mem + head);
+    sp.state = sp.hist + RS_DIGITS * sp.passes;
+    KeyT *keys[2];
+    IdxT *idx[2];
+    keys[0] = (KeyT *)(mem + cleared);
+    keys[1] = (KeyT *)((char *)keys[0] + pad((size_t)n * sizeof(KeyT)));
+    idx[0] = (IdxT *)((char *)keys[1] + pad((size_t)n * sizeof(KeyT)));
+    idx[1] = (IdxT *)((char *)idx[0] + pad((size_t)n * sizeof(IdxT)));
+    cudaMemsetAsync(mem, 0, cleared, st);
+    int64_t grid = ceil_div(n, 2048);
+    if (grid > sm_count() * 4) grid = sm_count() * 4;
+    const size_t hist_smem = sizeof(unsigned) * sp.passes * RS_DIGITS * RS_COPIES;
+    const size_t tile_smem = (size_t)RS_TILE * (sizeof(KeyT) + sizeof(IdxT));
+    cudaFuncSetAttribute(rs_make_keys_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_smem);
+    cudaFuncSetAttribute(rs_pass_kernel<KeyT, IdxT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem);
+    cudaFuncSetAttribute(rs_pass_kernel<KeyT, IdxT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem);
+    rs_make_keys_kernel<KeyT><<<(unsigned)grid, 256, hist_smem, st>>>(n, major, minor, nmajor, nminor, minor_bits, keys[0], sp);
+    rs_scan_kernel<<<(unsigned)sp.passes, RS_DIGITS, 0, st>>>(sp.hist);
+    int from = 0;
+    for (int p = 0; p < sp.passes; p++, from ^= 1) {
+        if (p == 0)
+            rs_pass_kernel<KeyT, IdxT, true><<<(unsigned)sp.ntiles, RS_THREADS, tile_smem, st>>>(
+                n, keys[0], nullptr, keys[1], idx[1], p, sp);
+        else
+            rs_pass_kernel<KeyT, IdxT, false><<<(unsigned)sp.ntiles, RS_THREADS, tile_smem, st>>>(
+                n, keys[from], idx[from], keys[from ^ 1], idx[from ^ 1], p, sp);
+    }
+    rs_gather_kernel<KeyT, IdxT><<<grid_for(n), 256, 0, st>>>(n, keys[from], idx[from], minor_bits, vals, payload, out.major,
+                                                             out.minor, vals ? out.vals : nullptr);
+    if (out.pos) rs_pos_kernel<KeyT><<<grid_for(nmajor + 1), 256, 0, st>>>(n, keys[from], minor_bits, nmajor, out.pos);
+    int rc = 0;
+    PinnedWords words;
+    int *bad = (int *)words.p;
+    if (!bad || cudaMemcpyAsync(bad, sp.bad, 2 * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess)
+        rc = fail("sort: kernels failed");
+    else if (bad[1])
+        rc = fail("sort: a tile did not see its predecessors' counts");
+    else if (bad[0])
+        rc = fail("sort: a coordinate lies outside %lld x %lld", (long long)nmajor, (long long)nminor);
+    cudaFreeAsync(mem, st);
+    return rc;
+}
+
+// Entries sorted by (major, minor), equal coordinates in input order; `minor` null: by the major coordinate alone, and the
+// minor output is payload[] of the entry.  Any of the outputs may be null.
+static int sort_into(int64_t n, int64_t nmajor, int64_t nminor, const int64_t *major, const int64_t *minor, const double *vals,
+                     const int64_t *payload, const SortOut &out, cudaStream_t st)
+{
+    if (nmajor <= 0 || nminor <= 0) return fail("sort: empty coordinate space");
+    const int minor_bits = minor ? extent_bits(nminor) : 0, bits = minor_bits + extent_bits(nmajor);
+    if (bits > 64) return fail("sort: rows x cols = %lld x %lld does not fit a 64-bit key", (long long)nmajor, (long long)nminor);
+    const bool wide = n >= 0xffffffffLL;
+#define GO(K, I) return sort_entries<K, I>(n, nmajor, nminor, bits, minor_bits, major, minor, vals, payload, out, st)
+    if (bits <= 32) { if (wide) GO(uint32_t, uint64_t); GO(uint32_t, uint32_t); }
+    if (wide) GO(uint64_t, uint64_t);
+    GO(uint64_t, uint32_t);
+#undef GO
+}
+
 int sort_coo(int64_t n, int64_t nmajor, int64_t nminor, const int64_t *major, const int64_t *minor,
              const double *vals, int64_t *major_out, int64_t *minor_out, double *vals_out, cudaStream_t st)
 {
     if (n <= 0) return 0;
-    int bits = 0;
-    CB_TRY(key_bits(nmajor, nminor, &bits));
-    uint64_t *keys = nullptr, *keys2 = nullptr;
-    int64_t *idx = nullptr, *idx2 = nullptr, *hist = nullptr, *base = nullptr;
-    int *bad = nullptr;
-    const size_t table = (size_t)RS_DIGITS * (size_t)ceil_div(n, RS_TILE) + 1;
-    int rc = 0;
-    auto alloc = [&](void **p, size_t bytes) {
-        if (rc) return;
-        if (cudaMallocAsync(p, bytes ? bytes : 8, st) != cudaSuccess) {
-            *p = nullptr;
-            rc = fail("sort: device allocation of %zu bytes failed", bytes);
-        }
-    };
-    alloc((void **)&keys, (size_t)n * 8);
-    alloc((void **)&keys2, (size_t)n * 8);
-    alloc((void **)&idx, (size_t)n * 8);
-    alloc((void **)&idx2, (size_t)n * 8);
-    alloc((void **)&bad, sizeof(int));
-    alloc((void **)&hist, table * 8);
-    alloc((void **)&base, table * 8);
-    int bad_host = 0;
-    bool second = false;
-    if (!rc) {
-        cudaMemsetAsync(bad, 0, sizeof(int), st);
-        make_keys_kernel<<<grid_for(n), 256, 0, st>>>(n, major, minor, nmajor, nminor, keys, idx, bad);
-        rc = radix_sort_pairs(keys, keys2, idx, idx2, n, bits, hist, base, &second, st);
-    }
-    if (!rc) {
-        gather_sorted_kernel<<<grid_for(n), 256, 0, st>>>(n, second ? keys2 : keys, second ? idx2 : idx, nminor, vals,
-                                                          major_out, minor_out, vals ? vals_out : nullptr);
-        if (cudaMemcpyAsync(&bad_host, bad, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess)
-            rc = fail("sort: kernels failed");
-        else if (bad_host)
-            rc = fail("sort: a coordinate lies outside %lld x %lld", (long long)nmajor, (long long)nminor);
-    }
-    void *all[] = {keys, keys2, idx, idx2, bad, hist, base};
-    for (void *p : all)
-        if (p) cudaFreeAsync(p, st);
-    return rc;
+    return sort_into(n, nmajor, nminor, major, minor, vals, nullptr, {major_out, minor_out, nullptr, vals_out}, st);
 }
 
 }  // namespace cb200
@@ -276,19 +376,7 @@ extern "C" int32_t comet_b200_dev_coo_to_csr_f64_i64(int64_t nrows, int64_t ncol
         CB_CUDA(cudaMemsetAsync(pos, 0, (size_t)(nrows + 1) * 8, st));
         return 0;
     }
-    int64_t *srows = nullptr;
-    int *flag = nullptr;
-    CB_CUDA(cudaMallocAsync((void **)&srows, (size_t)nnz * 8, st));
-    int rc = sort_coo(nnz, nrows, ncols, rows, cols, vals, srows, crd, val, st);
-    if (!rc && cudaMallocAsync((void **)&flag, sizeof(int), st) != cudaSuccess) rc = fail("coo_to_csr: allocation failed");
-    if (!rc) {
-        int one = 1;
-        cudaMemcpyAsync(flag, &one, sizeof(int), cudaMemcpyHostToDevice, st);
-        rc = coo_rows_to_pos(srows, nnz, nrows, pos, flag, st);
-    }
-    cudaFreeAsync(srows, st);
-    if (flag) cudaFreeAsync(flag, st);
-    return rc;
+    return sort_into(nnz, nrows, ncols, rows, cols, vals, nullptr, {nullptr, crd, pos, val}, st);
 }
 
 extern "C" int32_t comet_b200_dev_csr_transpose_f64_i64(int64_t nrows, int64_t ncols, int64_t nnz, const int64_t *pos,
@@ -302,24 +390,11 @@ extern "C" int32_t comet_b200_dev_csr_transpose_f64_i64(int64_t nrows, int64_t n
         CB_CUDA(cudaMemsetAsync(tpos, 0, (size_t)(ncols + 1) * 8, st));
         return 0;
     }
-    int64_t *rows = nullptr, *scols = nullptr;
-    int *flag = nullptr;
+    int64_t *rows = nullptr;
     CB_CUDA(cudaMallocAsync((void **)&rows, (size_t)nnz * 8, st));
-    if (cudaMallocAsync((void **)&scols, (size_t)nnz * 8, st) != cudaSuccess) {
-        cudaFreeAsync(rows, st);
-        return fail("transpose: allocation failed");
-    }
     expand_rows_kernel<<<grid_for(nrows * 8), 256, 0, st>>>(nrows, pos, rows);
-    // major = column of the input, minor = its row: the transposed matrix in row-major order
-    int rc = sort_coo(nnz, ncols, nrows, crd, rows, val, scols, tcrd, tval, st);
-    if (!rc && cudaMallocAsync((void **)&flag, sizeof(int), st) != cudaSuccess) rc = fail("transpose: allocation failed");
-    if (!rc) {
-        int one = 1;
-        cudaMemcpyAsync(flag, &one, sizeof(int), cudaMemcpyHostToDevice, st);
-        rc = coo_rows_to_pos(scols, nnz, ncols, tpos, flag, st);
-    }
+    // the entries are in row order already: a stable sort by column leaves every column's rows ascending
+    const int rc = sort_into(nnz, ncols, nrows, crd, nullptr, val, rows, {nullptr, tcrd, tpos, tval}, st);
     cudaFreeAsync(rows, st);
-    cudaFreeAsync(scols, st);
-    if (flag) cudaFreeAsync(flag, st);
     return rc;
 }

@@ -42,3 +42,17 @@ def test_results_that_are_kept_do_not_share_memory():
     _lib.load().comet_b200_release_scratch()
     assert np.array_equal(view, np.full(100, 3.0))
     assert np.array_equal(api.spmv(A, np.full(40000, 2.0)), np.full(40000, 2.0))
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (1, 70000), (70000, 1), (3, 1 << 40), (1 << 20, 1 << 12)])
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 40000])
+def test_sort_keys_of_every_width(shape, n):
+    """One digit, keys of up to 32 bits, wider ones; tiles of 4096 keys."""
+    rng = np.random.default_rng(n)
+    rows, cols = rng.integers(0, shape[0], n), rng.integers(0, shape[1], n)
+    cols[::3] = cols[0]
+    vals = rng.uniform(-1, 1, n)
+    C = api.from_coordinates(rows, cols, vals, shape)
+    order = np.lexsort((np.arange(n), cols, rows))
+    assert np.array_equal(C.a2pos, np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=shape[0]))]))
+    assert np.array_equal(C.a2crd, cols[order]) and np.array_equal(C.val, vals[order])
