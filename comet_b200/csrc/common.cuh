@@ -77,10 +77,17 @@ int widen_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t st);
 int narrow_f64_to_f32(const double *src, float *dst, int64_t n, cudaStream_t st);
 // out[0..n] = exclusive prefix sum of in[0..n-1], out[n] = total
 int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st);
+int exclusive_scan_nonzero(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st);   // counts entries that are not 0
 int exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st);
 // sorted COO row coordinates -> row pointer; *sorted_flag_dev set to 0 if rows are not ascending
 int coo_rows_to_pos(const int64_t *rows, int64_t nnz, int64_t nrows, int64_t *pos, int *flag_dev,
                     cudaStream_t st);
+
+// Entry indices of a CSR matrix in column order (rows ascending inside a column), without a synchronisation: tpos[ncols+1],
+// trow = row_of[] of the entry, tidx = its place.  Entries from *limit on (device memory; null: none) are left out of
+// tpos.  *err (device memory) becomes 1 if it failed.  n < 2^31, ncols < 2^31.
+int transpose_index(int64_t n, const int64_t *limit, int64_t ncols, const int64_t *crd, const int32_t *row_of, int64_t *tpos,
+                    int32_t *trow, int32_t *tidx, int *err, cudaStream_t st);
 
 // *flag_dev (preset to 1 by the caller) becomes 0 if some idx[i] is outside [0, limit)
 int check_index_range(const int64_t *idx, int64_t n, int64_t limit, int *flag_dev, cudaStream_t st);

@@ -69,11 +69,12 @@ __device__ __forceinline__ void rs_count_flush(const unsigned *h, int passes, ui
     }
 }
 
-// keys of coordinate entries; `minor` null: the major coordinate alone
+// keys of coordinate entries; `minor` null: the major coordinate alone; entries from *limit on (limit not null) get the last
+// major coordinate
 template <typename KeyT>
 __global__ void __launch_bounds__(256)
 rs_make_keys_kernel(int64_t n, const int64_t *__restrict__ major, const int64_t *__restrict__ minor, int64_t nmajor,
-                    int64_t nminor, int minor_bits, KeyT *__restrict__ keys, SortPlan sp)
+                    int64_t nminor, int minor_bits, const int64_t *limit, KeyT *__restrict__ keys, SortPlan sp)
 {
     extern __shared__ unsigned s_hist[];
     for (int i = threadIdx.x; i < sp.passes * RS_DIGITS * RS_COPIES; i += blockDim.x) s_hist[i] = 0;
@@ -81,7 +82,8 @@ rs_make_keys_kernel(int64_t n, const int64_t *__restrict__ major, const int64_t 
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a = __ldcs((const long long *)major + i), b = minor ? __ldcs((const long long *)minor + i) : 0;
         KeyT key = 0;                                 // reported by the host; the key stays in range
-        if (a < 0 || a >= nmajor || b < 0 || b >= nminor) *sp.bad = 1;
+        if (limit && i >= *limit) key = (KeyT)(nmajor - 1);
+        else if (a < 0 || a >= nmajor || b < 0 || b >= nminor) *sp.bad = 1;
         else key = (KeyT)(((uint64_t)a << minor_bits) | (uint64_t)b);
         keys[i] = key;
         rs_count_key(s_hist, key, sp.passes, sp.width);
@@ -270,9 +272,18 @@ struct SortOut {
     double *vals;
 };
 
+// Sorted keys and positions of n entries in memory that the caller frees (sp.bad is its first byte).
 template <typename KeyT, typename IdxT>
-static int sort_entries(int64_t n, int64_t nmajor, int64_t nminor, int bits, int minor_bits, const int64_t *major,
-                        const int64_t *minor, const double *vals, const int64_t *payload, const SortOut &out, cudaStream_t st)
+struct Sorted {
+    char *mem = nullptr;
+    SortPlan sp;
+    KeyT *keys;
+    IdxT *idx;
+};
+
+template <typename KeyT, typename IdxT>
+static int sort_keys(int64_t n, int64_t nmajor, int64_t nminor, int bits, int minor_bits, const int64_t *major,
+                     const int64_t *minor, const int64_t *limit, Sorted<KeyT, IdxT> *out, cudaStream_t st)
 {
     SortPlan sp;
     sp.passes = bits > 0 ? (bits + 7) / 8 : 1;
@@ -302,7 +313,7 @@ static int sort_entries(int64_t n, int64_t nmajor, int64_t nminor, int bits, int
     cudaFuncSetAttribute(rs_make_keys_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_smem);
     cudaFuncSetAttribute(rs_pass_kernel<KeyT, IdxT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem);
     cudaFuncSetAttribute(rs_pass_kernel<KeyT, IdxT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem);
-    rs_make_keys_kernel<KeyT><<<(unsigned)grid, 256, hist_smem, st>>>(n, major, minor, nmajor, nminor, minor_bits, keys[0], sp);
+    rs_make_keys_kernel<KeyT><<<(unsigned)grid, 256, hist_smem, st>>>(n, major, minor, nmajor, nminor, minor_bits, limit, keys[0], sp);
     rs_scan_kernel<<<(unsigned)sp.passes, RS_DIGITS, 0, st>>>(sp.hist);
     int from = 0;
     for (int p = 0; p < sp.passes; p++, from ^= 1) {
@@ -313,9 +324,24 @@ static int sort_entries(int64_t n, int64_t nmajor, int64_t nminor, int bits, int
             rs_pass_kernel<KeyT, IdxT, false><<<(unsigned)sp.ntiles, RS_THREADS, tile_smem, st>>>(
                 n, keys[from], idx[from], keys[from ^ 1], idx[from ^ 1], p, sp);
     }
-    rs_gather_kernel<KeyT, IdxT><<<grid_for(n), 256, 0, st>>>(n, keys[from], idx[from], minor_bits, vals, payload, out.major,
+    out->mem = mem;
+    out->sp = sp;
+    out->keys = keys[from];
+    out->idx = idx[from];
+    return 0;
+}
+
+template <typename KeyT, typename IdxT>
+static int sort_entries(int64_t n, int64_t nmajor, int64_t nminor, int bits, int minor_bits, const int64_t *major,
+                        const int64_t *minor, const double *vals, const int64_t *payload, const SortOut &out, cudaStream_t st)
+{
+    Sorted<KeyT, IdxT> s;
+    CB_TRY((sort_keys<KeyT, IdxT>(n, nmajor, nminor, bits, minor_bits, major, minor, nullptr, &s, st)));
+    char *mem = s.mem;
+    const SortPlan sp = s.sp;
+    rs_gather_kernel<KeyT, IdxT><<<grid_for(n), 256, 0, st>>>(n, s.keys, s.idx, minor_bits, vals, payload, out.major,
                                                              out.minor, vals ? out.vals : nullptr);
-    if (out.pos) rs_pos_kernel<KeyT><<<grid_for(nmajor + 1), 256, 0, st>>>(n, keys[from], minor_bits, nmajor, out.pos);
+    if (out.pos) rs_pos_kernel<KeyT><<<grid_for(nmajor + 1), 256, 0, st>>>(n, s.keys, minor_bits, nmajor, out.pos);
     int rc = 0;
     PinnedWords words;
     int *bad = (int *)words.p;
@@ -351,6 +377,31 @@ int sort_coo(int64_t n, int64_t nmajor, int64_t nminor, const int64_t *major, co
 {
     if (n <= 0) return 0;
     return sort_into(n, nmajor, nminor, major, minor, vals, nullptr, {major_out, minor_out, nullptr, vals_out}, st);
+}
+
+// trow[q], tidx[q]: row and place of the q-th entry in column order; *err = 1 if the sort failed
+__global__ void __launch_bounds__(256)
+rs_index_kernel(int64_t n, const uint32_t *__restrict__ idx, const int32_t *__restrict__ row_of, int32_t *__restrict__ trow,
+                int32_t *__restrict__ tidx, const int *bad, int *err)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (bad[0] || bad[1])) *err = 1;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t from = idx[i];
+        trow[i] = row_of[from];
+        tidx[i] = (int32_t)from;
+    }
+}
+
+int transpose_index(int64_t n, const int64_t *limit, int64_t ncols, const int64_t *crd, const int32_t *row_of, int64_t *tpos,
+                    int32_t *trow, int32_t *tidx, int *err, cudaStream_t st)
+{
+    Sorted<uint32_t, uint32_t> s;
+    CB_TRY((sort_keys<uint32_t, uint32_t>(n, ncols + 1, 1, extent_bits(ncols + 1), 0, crd, nullptr, limit, &s, st)));
+    rs_index_kernel<<<grid_for(n), 256, 0, st>>>(n, s.idx, row_of, trow, tidx, s.sp.bad, err);
+    rs_pos_kernel<uint32_t><<<grid_for(ncols + 1), 256, 0, st>>>(n, s.keys, 0, ncols, tpos);
+    cudaFreeAsync(s.mem, st);
+    CB_LAUNCH_CHECK();
+    return 0;
 }
 
 }  // namespace cb200

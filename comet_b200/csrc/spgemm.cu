@@ -27,6 +27,9 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "hostcopy.cuh"
+#include "masked.cuh"
+#include "semiring.cuh"
 
 namespace cb200 {
 
@@ -53,6 +56,7 @@ struct Plan {
     unsigned n1, n2;
     uint32_t *bm_store;      // n2 * words, or null
     int words;
+    MaskedPlan *masked;      // not null: the product is formed by dot products over the mask
     cudaStream_t last;       // stream of the latest call on this plan: its arrays are released in that stream's order
 };
 
@@ -69,6 +73,7 @@ static void plan_free(Plan *p, cudaStream_t st)
     if (p->list2) cudaFreeAsync(p->list2, st);
     if (p->bin_counts) cudaFreeAsync(p->bin_counts, st);
     if (p->bm_store) cudaFreeAsync(p->bm_store, st);
+    masked_free(p->masked, st);
     delete p;
 }
 
@@ -112,45 +117,6 @@ __device__ __forceinline__ bool in_mask(const int64_t *__restrict__ mcrd, int64_
         if (v < j) ms = mid + 1; else me = mid;
     }
     return false;
-}
-
-// --------------------------------------------------------------------------
-// Semiring arithmetic (codes of include/comet_b200.h).  The second operator
-// combines A[i,k] and B[k,j]; the first one folds the products of one output.
-// "any" is only offered with "pair", where every product is 1, so it can share
-// the min fold.
-// --------------------------------------------------------------------------
-__device__ __forceinline__ double sr_combine(int semi, double a, double b)
-{
-    switch (semi) {
-    case COMET_B200_PLUS_PAIR: case COMET_B200_ANY_PAIR: return 1.0;
-    case COMET_B200_PLUS_FIRST: case COMET_B200_MIN_FIRST: return a;
-    case COMET_B200_PLUS_SECOND: case COMET_B200_MIN_SECOND: return b;
-    case COMET_B200_MIN_PLUS: return a + b;
-    default: return a * b;
-    }
-}
-
-__host__ __device__ __forceinline__ bool sr_is_min(int semi) { return semi >= COMET_B200_MIN_PLUS; }
-
-__device__ __forceinline__ double sr_identity(int semi) { return sr_is_min(semi) ? __longlong_as_double(0x7ff0000000000000LL) : 0.0; }
-
-// min fold on an f64 in shared or global memory (there is no native one)
-__device__ __forceinline__ void atomic_min_f64(double *addr, double v)
-{
-    unsigned long long *a = (unsigned long long *)addr;
-    unsigned long long old = *a;
-    while (v < __longlong_as_double((long long)old)) {
-        const unsigned long long assumed = old;
-        old = atomicCAS(a, assumed, (unsigned long long)__double_as_longlong(v));
-        if (old == assumed) break;
-    }
-}
-
-__device__ __forceinline__ void sr_fold(int semi, double *addr, double v)
-{
-    if (sr_is_min(semi)) atomic_min_f64(addr, v);
-    else atomicAdd(addr, v);
 }
 
 // --------------------------------------------------------------------------
@@ -798,8 +764,28 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     int rc = 0;
 #define STEP(expr) do { if (!rc) rc = (expr); } while (0)
 #define STEP_CUDA(expr) do { if (!rc) { cudaError_t e_ = (expr); if (e_ != cudaSuccess) rc = fail("%s failed: %s", #expr, cudaGetErrorString(e_)); } } while (0)
-    STEP(dev_alloc(&p->bcrd32, (size_t)nnz_b, st));
+    if (mpos) {
+        STEP(masked_symbolic(nrows, ncols_b, nnz_b, apos, acrd, bpos, bcrd, mpos, mcrd, cpos, &p->masked, st));
+        if (!rc && p->masked) {
+            PinnedWords words;
+            if (!rc && !words.p) rc = fail("spgemm: no page-locked memory");
+            STEP_CUDA(cudaMemcpyAsync(words.p, cpos + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+            STEP_CUDA(cudaMemcpyAsync((int64_t *)words.p + 1, masked_checks(p->masked), 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+            STEP_CUDA(cudaStreamSynchronize(st));
+            if (rc) { plan_free(p, st); return rc; }
+            const int *ok = (const int *)((int64_t *)words.p + 1);
+            if (ok[0] == 0 && ok[1] == ok[2]) {
+                p->nnz_c = *(int64_t *)words.p;
+                *nnz_host = p->nnz_c;
+                *handle_out = register_plan(p);
+                return 0;
+            }
+            masked_free(p->masked, st);    // rows of B that do not ascend strictly: push
+            p->masked = nullptr;
+        }
+    }
     STEP(dev_alloc(&p->cnt, (size_t)nrows + 1, st));
+    STEP(dev_alloc(&p->bcrd32, (size_t)nnz_b, st));
     STEP(dev_alloc(&p->list1, (size_t)nrows, st));
     STEP(dev_alloc(&p->list2, (size_t)nrows, st));
     STEP(dev_alloc(&p->bin_counts, 2, st));
@@ -897,7 +883,9 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
     if (!p) return fail("numeric phase: unknown handle %lld", (long long)handle);
     p->last = st;
     int rc = 0;
-    if (p->kind == 1) {
+    if (p->masked) {
+        rc = masked_numeric(p->masked, p->aval, p->bval, p->mcrd, p->semi, ccrd, cval, st);
+    } else if (p->kind == 1) {
         if (p->nrows > 0) {
             elews_ss_kernel<true><<<(unsigned)ceil_div(p->nrows, 256), 256, 0, st>>>(
                 p->nrows, p->apos, p->acrd, p->aval, p->bpos, p->bcrd, p->bval, nullptr, p->cpos, ccrd,

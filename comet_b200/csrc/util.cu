@@ -213,6 +213,16 @@ static int exclusive_scan(const InT *in, int64_t *out, int64_t n, cudaStream_t s
 }
 
 int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st) { return exclusive_scan(in, out, n, st); }
+
+// positions of the non-zero entries
+struct NonZero {
+    int32_t v;
+    __device__ operator int64_t() const { return v != 0; }
+};
+int exclusive_scan_nonzero(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st)
+{
+    return exclusive_scan((const NonZero *)in, out, n, st);
+}
 int exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st) { return exclusive_scan(in, out, n, st); }
 
 // ---------------------------------------------------------------------------
