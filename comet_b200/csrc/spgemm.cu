@@ -24,6 +24,7 @@
 // Accumulation order inside a row is not fixed (atomics); structure (pos, crd)
 // is exact and values agree with a sequential sum to rounding.
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "common.cuh"
@@ -34,11 +35,12 @@
 namespace cb200 {
 
 static const int HASH_ROW_MAX = 256;        // bound for bin 1
-static const int HASH_SLOTS = 512;          // table size per warp (load factor <= 0.5)
+static const int HASH_SLOTS = 512;          // table size per warp with sums (load factor <= 0.5); twice that without
 static const int HASH_WARPS = 4;            // warps per CTA in the hash kernels
 static const int BM_THREADS = 512;          // CTA size of the bitmap kernels
 static const size_t BM_SMEM_LIMIT = 200 * 1024;
 static const size_t BM_STORE_BUDGET = (size_t)12 << 30;
+static const size_t BM_STORE_SMALL = (size_t)64 << 20;
 
 struct Plan {
     int kind;                // 0 = spgemm, 1 = elementwise CSR .* CSR
@@ -48,11 +50,11 @@ struct Plan {
     int semi;                // semiring code
     int64_t *cpos;           // caller's array
     int64_t nnz_c;
-    // owned device memory
-    int32_t *bcrd32;
+    void *mem;               // owned device memory: the next five arrays
+    unsigned *bin_counts;    // [2]
     int64_t *cnt;            // per-row distinct count
+    int32_t *bcrd32;
     int32_t *list1, *list2;  // rows of bin 1 / bin 2
-    unsigned *bin_counts;    // [2] on device
     unsigned n1, n2;
     uint32_t *bm_store;      // n2 * words, or null
     int words;
@@ -67,11 +69,7 @@ static int64_t g_next_handle = 1;
 static void plan_free(Plan *p, cudaStream_t st)
 {
     if (!p) return;
-    if (p->bcrd32) cudaFreeAsync(p->bcrd32, st);
-    if (p->cnt) cudaFreeAsync(p->cnt, st);
-    if (p->list1) cudaFreeAsync(p->list1, st);
-    if (p->list2) cudaFreeAsync(p->list2, st);
-    if (p->bin_counts) cudaFreeAsync(p->bin_counts, st);
+    if (p->mem) cudaFreeAsync(p->mem, st);
     if (p->bm_store) cudaFreeAsync(p->bm_store, st);
     masked_free(p->masked, st);
     delete p;
@@ -209,29 +207,105 @@ bin_rows_kernel(int64_t nrows, const int64_t *__restrict__ apos, const int64_t *
 
 // --------------------------------------------------------------------------
 // Bin 1: warp per row, hash table in shared memory.
+//
+// The products of 32 entries of the A row at a time are laid end to end and dealt to the lanes, 32 per step (short rows
+// of B would otherwise leave most lanes idle, and every one of them cost its own chain of dependent loads), the next
+// step's loads ahead of the current step's insertions.  The keys that an insertion created are numbered and listed, so a
+// row ends by clearing its own slots and not the table, and the sums are kept by number.  The numeric call sorts key |
+// number in registers (a bitonic network of 32 x E words; 64-bit ones from 2^24 columns on); ranking each key against
+// all others was two thirds of the kernel before (16384 rows of 256 products: 207 us).
 // --------------------------------------------------------------------------
-__device__ __forceinline__ int hash_slot(int32_t j)
-{
-    return (int)(((uint32_t)j * 0x9E3779B1u) >> 23);   // top 9 bits: 0..511
-}
 
 // Inserts j; returns the slot, sets *fresh when this call created the entry.
+template <int SLOTS>
 __device__ __forceinline__ int hash_insert(int32_t *keys, int32_t j, bool *fresh)
 {
-    int h = hash_slot(j);
+    int h = (int)(((uint64_t)((uint32_t)j * 0x9E3779B1u) * SLOTS) >> 32);
     *fresh = false;
-    for (int probe = 0; probe < HASH_SLOTS; probe++) {
+    for (int probe = 0; probe < SLOTS; probe++) {
         int32_t old = atomicCAS(&keys[h], -1, j);
         if (old == -1) { *fresh = true; return h; }
         if (old == j) return h;
-        h = (h + 1) & (HASH_SLOTS - 1);
+        h = (h + 1) & (SLOTS - 1);
     }
-    return -1;   // cannot happen: at most HASH_ROW_MAX distinct keys in HASH_SLOTS slots
+    return -1;   // cannot happen: at most HASH_ROW_MAX distinct keys in two or four times as many slots
 }
 
-template <bool NUMERIC>
-__global__ void __launch_bounds__(HASH_WARPS * 32)
-hash_rows_kernel(unsigned nlist, const int32_t *__restrict__ list, const int64_t *__restrict__ apos,
+// Sorts the 32 * E words v[r] of lane l (place l * E + r) ascending: a bitonic network.  The blocks that a level sorts
+// downwards are complemented for its duration, so that every exchange puts the smaller word first.
+template <int E, typename T>
+__device__ __forceinline__ void warp_sort(T (&v)[E], int lane)
+{
+#pragma unroll
+    for (int k = 2; k <= 32 * E; k <<= 1) {
+        // complemented at the level before: place & (k / 2); at this one: place & k
+#pragma unroll
+        for (int r = 0; r < E; r++) {
+            const int place = lane * E + r;
+            v[r] ^= (T)0 - (T)(((place & k) != 0) != (k > 2 && (place & (k >> 1)) != 0));
+        }
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= E) {
+                const bool low = (lane & (j / E)) == 0;
+#pragma unroll
+                for (int r = 0; r < E; r++) {
+                    const T o = __shfl_xor_sync(0xffffffffu, v[r], j / E);
+                    v[r] = low ? min(v[r], o) : max(v[r], o);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < E; r++) {
+                    if (r & j) continue;
+                    const T a = min(v[r], v[r | j]), b = max(v[r], v[r | j]);
+                    v[r] = a;
+                    v[r | j] = b;
+                }
+            }
+        }
+    }
+    // the last level complemented nothing (place < 32 E), the one before it the upper half, taken back above
+}
+
+// Writes a row's n listed keys in ascending order, and the value of each, to C.  The sorted words go through `list` so
+// that the stores are coalesced.
+template <int E, typename T>
+__device__ __forceinline__ void write_sorted(T *list, const int32_t *row_keys, const double *vals, int n, int lane,
+                                             int64_t *__restrict__ ccrd, double *__restrict__ cval)
+{
+    T v[E];
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const int at = lane + 32 * r;                  // any order goes in
+        v[r] = at < n ? (T)row_keys[at] << 8 | (T)at : ~(T)0;
+    }
+    __syncwarp();
+    warp_sort<E>(v, lane);
+#pragma unroll
+    for (int r = 0; r < E; r++)
+        if (lane * E + r < n) list[lane * E + r] = v[r];
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+        const T x = list[i];
+        ccrd[i] = (int64_t)(x >> 8);
+        cval[i] = vals[(int)(x & 255)];
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ void write_row(T *list, const int32_t *row_keys, const double *vals, int n, int lane,
+                                          int64_t *__restrict__ ccrd, double *__restrict__ cval)
+{
+    if (n <= 32) write_sorted<1>(list, row_keys, vals, n, lane, ccrd, cval);
+    else if (n <= 64) write_sorted<2>(list, row_keys, vals, n, lane, ccrd, cval);
+    else if (n <= 128) write_sorted<4>(list, row_keys, vals, n, lane, ccrd, cval);
+    else write_sorted<8>(list, row_keys, vals, n, lane, ccrd, cval);
+}
+
+// WIDE: columns from 2^24 on, sorted as 64-bit words.
+template <bool NUMERIC, bool WIDE>
+__global__ void __launch_bounds__(HASH_WARPS * 32, NUMERIC && !WIDE ? 7 : 1)
+hash_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restrict__ list, const int64_t *__restrict__ apos,
                  const int64_t *__restrict__ acrd, const double *__restrict__ aval,
                  const int64_t *__restrict__ bpos, const int32_t *__restrict__ bcrd,
                  const double *__restrict__ bval, const int64_t *__restrict__ mpos,
@@ -239,62 +313,204 @@ hash_rows_kernel(unsigned nlist, const int32_t *__restrict__ list, const int64_t
                  const int64_t *__restrict__ cpos, int64_t *__restrict__ ccrd,
                  double *__restrict__ cval)
 {
-    __shared__ int32_t s_keys[HASH_WARPS][HASH_SLOTS];
-    __shared__ double s_vals[NUMERIC ? HASH_WARPS : 1][NUMERIC ? HASH_SLOTS : 1];
-    __shared__ int32_t s_ckeys[NUMERIC ? HASH_WARPS : 1][NUMERIC ? HASH_ROW_MAX : 1];
-    __shared__ unsigned short s_cslot[NUMERIC ? HASH_WARPS : 1][NUMERIC ? HASH_ROW_MAX : 1];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    using Word = typename std::conditional<WIDE, unsigned long long, unsigned>::type;
+    constexpr int SLOTS = NUMERIC ? HASH_SLOTS : 2 * HASH_SLOTS;
+    __shared__ int32_t s_keys[HASH_WARPS][SLOTS];
+    __shared__ unsigned short s_slot[HASH_WARPS][HASH_ROW_MAX];      // slots of the row's keys, by number
+    __shared__ unsigned short s_number[NUMERIC ? HASH_WARPS : 1][NUMERIC ? SLOTS : 1];
+    __shared__ double s_vals[NUMERIC ? HASH_WARPS : 1][NUMERIC ? HASH_ROW_MAX : 1];
+    __shared__ int32_t s_list[NUMERIC ? HASH_WARPS : 1][NUMERIC ? HASH_ROW_MAX : 1];
+    __shared__ Word s_sorted[NUMERIC ? HASH_WARPS : 1][NUMERIC ? HASH_ROW_MAX : 1];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, wn = NUMERIC ? w : 0;
+    const unsigned below = (1u << lane) - 1u;
     int32_t *keys = s_keys[w];
-    const unsigned nwarps = gridDim.x * HASH_WARPS;
+    double *vals = s_vals[wn];
+    int32_t *row_keys = s_list[wn];
+    const double ident = sr_identity(semi);
+    for (int s = lane; s < SLOTS; s += 32) keys[s] = -1;
+    if (NUMERIC)
+        for (int s = lane; s < HASH_ROW_MAX; s += 32) vals[s] = ident;
+    __syncwarp();
+    const unsigned nwarps = gridDim.x * HASH_WARPS, nlist = *nlist_dev;
     for (unsigned it = blockIdx.x * HASH_WARPS + w; it < nlist; it += nwarps) {
         const int64_t r = list[it];
-        for (int s = lane; s < HASH_SLOTS; s += 32) {
-            keys[s] = -1;
-            if (NUMERIC) s_vals[w][s] = sr_identity(semi);
-        }
-        __syncwarp();
         int64_t ms = 0, me = 0;
         if (mpos) { ms = mpos[r]; me = mpos[r + 1]; }
-        int fresh_count = 0;
-        for (int64_t p = apos[r]; p < apos[r + 1]; p++) {
-            const int64_t k = acrd[p];
-            const double av = NUMERIC ? aval[p] : 0.0;
-            for (int64_t q = bpos[k] + lane; q < bpos[k + 1]; q += 32) {
-                int32_t j = bcrd[q];
-                if (mpos && !in_mask(mcrd, ms, me, j)) continue;
-                bool fresh;
-                int h = hash_insert(keys, j, &fresh);
-                fresh_count += fresh ? 1 : 0;
-                if (NUMERIC && h >= 0) sr_fold(semi, &s_vals[w][h], sr_combine(semi, av, bval[q]));
+        int n = 0;                                     // distinct columns so far
+        const int64_t ae = apos[r + 1];
+        for (int64_t p0 = apos[r]; p0 < ae; p0 += 32) {
+            int64_t s = 0;
+            int len = 0;
+            double av = 0.0;
+            if (p0 + lane < ae) {
+                const int64_t k = acrd[p0 + lane];
+                if (NUMERIC) av = aval[p0 + lane];
+                s = bpos[k];
+                len = (int)(bpos[k + 1] - s);
+            }
+            int upto = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const int total = __shfl_sync(0xffffffffu, upto, 31);
+            const int64_t rel = s - (upto - len);      // product x of the batch is entry rel + x of B, for its own A entry
+            auto fetch = [&](int x, int32_t &j, double &bv, double &a) {
+                int t = 0;                             // first A entry whose prefix sum exceeds x
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, upto, t + step - 1) <= x) t += step;
+                const int64_t q = __shfl_sync(0xffffffffu, (long long)rel, t) + x;
+                if (NUMERIC) a = shfl_f64(av, t, 32);
+                j = -1;
+                if (x < total) {
+                    j = bcrd[q];
+                    if (NUMERIC) bv = bval[q];
+                }
+            };
+            int32_t j1;
+            double bv1 = 0.0, a1 = 0.0;
+            fetch(lane, j1, bv1, a1);
+            for (int x0 = 0; x0 < total; x0 += 32) {
+                const int32_t j = j1;
+                const double bv = bv1, a = a1;
+                if (x0 + 32 < total) fetch(x0 + 32 + lane, j1, bv1, a1);
+                bool fresh = false;
+                int h = -1;
+                if (j >= 0 && (!mpos || in_mask(mcrd, ms, me, j))) {
+                    h = hash_insert<SLOTS>(keys, j, &fresh);
+                }
+                const unsigned made = __ballot_sync(0xffffffffu, fresh);
+                if (fresh) {
+                    const int at = n + __popc(made & below);
+                    s_slot[w][at] = (unsigned short)h;
+                    if (NUMERIC) {
+                        row_keys[at] = j;
+                        s_number[wn][h] = (unsigned short)at;
+                    }
+                }
+                n += __popc(made);
+                if (NUMERIC) {
+                    __syncwarp();                      // the new keys' numbers
+                    if (h >= 0) sr_fold(semi, &vals[s_number[wn][h]], sr_combine(semi, a, bv));
+                }
             }
         }
         __syncwarp();
         if (!NUMERIC) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) fresh_count += __shfl_xor_sync(0xffffffffu, fresh_count, o);
-            if (lane == 0) cnt[r] = fresh_count;
+            if (lane == 0) cnt[r] = n;
         } else {
-            // compact the occupied slots, then place each key at its rank among them
-            int n = 0;
-            for (int s0 = 0; s0 < HASH_SLOTS; s0 += 32) {
-                int32_t key = keys[s0 + lane];
-                unsigned occ = __ballot_sync(0xffffffffu, key != -1);
-                if (key != -1) {
-                    int at = n + __popc(occ & ((1u << lane) - 1u));
-                    s_ckeys[w][at] = key;
-                    s_cslot[w][at] = (unsigned short)(s0 + lane);
-                }
-                n += __popc(occ);
-            }
-            __syncwarp();
             const int64_t base = cpos[r];
-            for (int i = lane; i < n; i += 32) {
-                int32_t key = s_ckeys[w][i];
-                int rank = 0;
-                for (int t = 0; t < n; t++) rank += s_ckeys[w][t] < key ? 1 : 0;
-                ccrd[base + rank] = key;
-                cval[base + rank] = s_vals[w][s_cslot[w][i]];
+            write_row(s_sorted[wn], row_keys, vals, n, lane, ccrd + base, cval + base);
+            __syncwarp();
+        }
+        for (int i = lane; i < n; i += 32) {
+            keys[s_slot[w][i]] = -1;
+            if (NUMERIC) vals[i] = ident;
+        }
+        __syncwarp();
+    }
+}
+
+// --------------------------------------------------------------------------
+// Bin 1 without a mask, numeric call: the row has at most HASH_ROW_MAX products, so they are sorted by column in registers, and equal
+// neighbours are added up.  A word is column | place of the product in the row (8 bits), so equal columns keep the order
+// of the products and the sums are those of the sequential loop.  Products are dealt to the lanes as in the hash
+// kernel.  Against hashing and sorting the distinct keys: no insertion loops, no atomics (16384 rows of 256
+// products: 66 -> 47 us; counting alone, the table is the faster one: 26 against 34 us).
+// --------------------------------------------------------------------------
+template <int E, typename T>
+__device__ __forceinline__ void sort_words(T *list, int n, int lane)
+{
+    T v[E];
+#pragma unroll
+    for (int r = 0; r < E; r++) v[r] = lane + 32 * r < n ? list[lane + 32 * r] : ~(T)0;      // any order goes in
+    __syncwarp();
+    warp_sort<E>(v, lane);
+#pragma unroll
+    for (int r = 0; r < E; r++) list[lane * E + r] = v[r];
+    __syncwarp();
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(HASH_WARPS * 32)
+short_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restrict__ rows, const int64_t *__restrict__ apos,
+                  const int64_t *__restrict__ acrd, const double *__restrict__ aval, const int64_t *__restrict__ bpos,
+                  const int32_t *__restrict__ bcrd, const double *__restrict__ bval, int semi,
+                  const int64_t *__restrict__ cpos, int64_t *__restrict__ ccrd, double *__restrict__ cval)
+{
+    using Word = typename std::conditional<WIDE, unsigned long long, unsigned>::type;
+    __shared__ Word s_list[HASH_WARPS][HASH_ROW_MAX];
+    __shared__ double s_vals[HASH_WARPS][HASH_ROW_MAX];
+    __shared__ unsigned short s_head[HASH_WARPS][HASH_ROW_MAX + 1];     // first word of every column
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    Word *list = s_list[w];
+    double *vals = s_vals[w];
+    unsigned short *head = s_head[w];
+    const unsigned nwarps = gridDim.x * HASH_WARPS, nlist = *nlist_dev;
+    for (unsigned it = blockIdx.x * HASH_WARPS + w; it < nlist; it += nwarps) {
+        const int64_t r = rows[it];
+        const int64_t ae = apos[r + 1];
+        int n = 0;                                     // products so far
+        for (int64_t p0 = apos[r]; p0 < ae; p0 += 32) {
+            int64_t s = 0;
+            int len = 0;
+            double av = 0.0;
+            if (p0 + lane < ae) {
+                const int64_t k = acrd[p0 + lane];
+                av = aval[p0 + lane];
+                s = bpos[k];
+                len = (int)(bpos[k + 1] - s);
             }
+            int upto = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const int total = __shfl_sync(0xffffffffu, upto, 31);
+            const int64_t rel = s - (upto - len);      // product x of the batch is entry rel + x of B, for its own A entry
+#pragma unroll 2
+            for (int x0 = 0; x0 < total; x0 += 32) {
+                const int x = x0 + lane;
+                int t = 0;                             // first A entry whose prefix sum exceeds x
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, upto, t + step - 1) <= x) t += step;
+                const int64_t q = __shfl_sync(0xffffffffu, (long long)rel, t) + x;
+                const double a = shfl_f64(av, t, 32);
+                if (x < total) {
+                    list[n + x] = (Word)bcrd[q] << 8 | (Word)(n + x);
+                    vals[n + x] = sr_combine(semi, a, bval[q]);
+                }
+            }
+            n += total;
+        }
+        __syncwarp();
+        if (n <= 32) sort_words<1>(list, n, lane);
+        else if (n <= 64) sort_words<2>(list, n, lane);
+        else if (n <= 128) sort_words<4>(list, n, lane);
+        else sort_words<8>(list, n, lane);
+        int distinct = 0;
+        for (int x0 = 0; x0 < n; x0 += 32) {
+            const int x = x0 + lane;
+            const bool first = x < n && (x == 0 || (list[x] >> 8) != (list[x - 1] >> 8));
+            const unsigned firsts = __ballot_sync(0xffffffffu, first);
+            if (first) head[distinct + __popc(firsts & below)] = (unsigned short)x;
+            distinct += __popc(firsts);
+        }
+        if (lane == 0) head[distinct] = (unsigned short)n;
+        __syncwarp();
+        const int64_t base = cpos[r];
+        for (int i = lane; i < distinct; i += 32) {
+            const int b = head[i], e = head[i + 1];
+            const Word x = list[b];
+            double sum = vals[(int)(x & 255)];
+            for (int y = b + 1; y < e; y++) sum = sr_fold_value(semi, sum, vals[(int)(list[y] & 255)]);
+            ccrd[base + i] = (int64_t)(x >> 8);
+            cval[base + i] = sum;
         }
         __syncwarp();
     }
@@ -454,7 +670,7 @@ __device__ __forceinline__ void mark_products(uint32_t *bm, int64_t r, const int
 
 template <bool SMEM>
 __global__ void __launch_bounds__(BM_THREADS)
-bitmap_symbolic_kernel(unsigned nlist, const int32_t *__restrict__ list, int words,
+bitmap_symbolic_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restrict__ list, int words,
                        uint32_t *__restrict__ gbm, const int64_t *__restrict__ apos,
                        const int64_t *__restrict__ acrd, const int64_t *__restrict__ bpos,
                        const int32_t *__restrict__ bcrd, const int64_t *__restrict__ mpos,
@@ -466,6 +682,7 @@ bitmap_symbolic_kernel(unsigned nlist, const int32_t *__restrict__ list, int wor
     __shared__ int s_long[LONG_LIST];
     __shared__ unsigned s_ctl[2];
     uint32_t *bm = SMEM ? s_dyn : gbm + (size_t)blockIdx.x * words;
+    const unsigned nlist = *nlist_dev;
     for (unsigned it = blockIdx.x; it < nlist; it += gridDim.x) {
         const int64_t r = list[it];
         for (int w = threadIdx.x; w < words; w += BM_THREADS) bm[w] = 0;
@@ -784,11 +1001,16 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
             p->masked = nullptr;
         }
     }
-    STEP(dev_alloc(&p->cnt, (size_t)nrows + 1, st));
-    STEP(dev_alloc(&p->bcrd32, (size_t)nnz_b, st));
-    STEP(dev_alloc(&p->list1, (size_t)nrows, st));
-    STEP(dev_alloc(&p->list2, (size_t)nrows, st));
-    STEP(dev_alloc(&p->bin_counts, 2, st));
+    auto pad = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+    const size_t b_cnt = pad(((size_t)nrows + 1) * 8), b_crd = pad((size_t)nnz_b * 4 + 8), b_list = pad((size_t)nrows * 4);
+    char *mem = nullptr;
+    STEP(dev_alloc(&mem, 256 + b_cnt + b_crd + 2 * b_list, st));
+    p->mem = mem;
+    p->bin_counts = (unsigned *)mem;
+    p->cnt = (int64_t *)(mem + 256);
+    p->bcrd32 = (int32_t *)(mem + 256 + b_cnt);
+    p->list1 = (int32_t *)(mem + 256 + b_cnt + b_crd);
+    p->list2 = (int32_t *)((char *)p->list1 + b_list);
     STEP_CUDA(cudaMemsetAsync(p->bin_counts, 0, 2 * sizeof(unsigned), st));
     STEP(narrow_i64_to_i32(bcrd, p->bcrd32, nnz_b, st));
     if (!rc && nrows > 0) {
@@ -796,16 +1018,23 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
             nrows, apos, acrd, bpos, mpos, p->cnt, p->list1, p->list2, p->bin_counts);
         STEP_CUDA(cudaGetLastError());
     }
-    unsigned counts[2] = {0, 0};
-    STEP_CUDA(cudaMemcpyAsync(counts, p->bin_counts, sizeof(counts), cudaMemcpyDeviceToHost, st));
-    STEP_CUDA(cudaStreamSynchronize(st));
-    p->n1 = counts[0]; p->n2 = counts[1];
+    PinnedWords words;
+    if (!rc && !words.p) rc = fail("spgemm: no page-locked memory");
+    unsigned *counts = (unsigned *)words.p;
+    // The bitmaps of the bin-2 rows are kept for the numeric call, so their number is needed to allocate them: after a
+    // synchronisation, unless bitmaps for every row are small change (then the kernels read the bin sizes themselves).
+    p->n1 = p->n2 = (unsigned)nrows;
+    if ((size_t)nrows * p->words * 4 > BM_STORE_SMALL) {
+        STEP_CUDA(cudaMemcpyAsync(counts, p->bin_counts, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        STEP_CUDA(cudaStreamSynchronize(st));
+        if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; }
+    }
     if (!rc && p->n1) {
         unsigned grid = (unsigned)ceil_div(p->n1, HASH_WARPS);
         unsigned cap = (unsigned)sm_count() * 16;
         if (grid > cap) grid = cap;
-        hash_rows_kernel<false><<<grid, HASH_WARPS * 32, 0, st>>>(
-            p->n1, p->list1, apos, acrd, aval, bpos, p->bcrd32, bval, mpos, p->mcrd, p->semi, p->cnt,
+        hash_rows_kernel<false, false><<<grid, HASH_WARPS * 32, 0, st>>>(
+            p->bin_counts, p->list1, apos, acrd, aval, bpos, p->bcrd32, bval, mpos, p->mcrd, p->semi, p->cnt,
             nullptr, nullptr, nullptr);
         STEP_CUDA(cudaGetLastError());
     }
@@ -826,7 +1055,7 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             if (!rc)
                 bitmap_symbolic_kernel<true><<<grid, BM_THREADS, smem, st>>>(
-                    p->n2, p->list2, p->words, nullptr, apos, acrd, bpos, p->bcrd32, mpos, p->mcrd,
+                    p->bin_counts + 1, p->list2, p->words, nullptr, apos, acrd, bpos, p->bcrd32, mpos, p->mcrd,
                     p->cnt, p->bm_store);
         } else {
             int grid = bitmap_grid(p->n2, 0);
@@ -834,14 +1063,19 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
             STEP(scratch(SLOT_BITMAP, (size_t)grid * 2 * smem, &gbm));
             if (!rc)
                 bitmap_symbolic_kernel<false><<<grid, BM_THREADS, 0, st>>>(
-                    p->n2, p->list2, p->words, (uint32_t *)gbm, apos, acrd, bpos, p->bcrd32, mpos,
+                    p->bin_counts + 1, p->list2, p->words, (uint32_t *)gbm, apos, acrd, bpos, p->bcrd32, mpos,
                     p->mcrd, p->cnt, p->bm_store);
         }
         STEP_CUDA(cudaGetLastError());
     }
     STEP(exclusive_scan_i64(p->cnt, cpos, nrows, st));
-    STEP_CUDA(cudaMemcpyAsync(&p->nnz_c, cpos + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    STEP_CUDA(cudaMemcpyAsync(counts, p->bin_counts, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    STEP_CUDA(cudaMemcpyAsync(counts + 2, cpos + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     STEP_CUDA(cudaStreamSynchronize(st));
+    if (!rc) {
+        p->n1 = counts[0]; p->n2 = counts[1];
+        p->nnz_c = *(int64_t *)(counts + 2);
+    }
 #undef STEP
 #undef STEP_CUDA
     if (rc) { plan_free(p, st); return rc; }
@@ -862,6 +1096,7 @@ int elews_ss_symbolic(int64_t nrows, const int64_t *apos, const int64_t *acrd, c
     p->apos = apos; p->acrd = acrd; p->aval = aval; p->bpos = bpos; p->bcrd = bcrd; p->bval = bval;
     p->cpos = cpos;
     int rc = dev_alloc(&p->cnt, (size_t)nrows + 1, st);
+    p->mem = p->cnt;
     if (!rc && nrows > 0) {
         elews_ss_kernel<false><<<(unsigned)ceil_div(nrows, 256), 256, 0, st>>>(
             nrows, apos, acrd, aval, bpos, bcrd, bval, p->cnt, nullptr, nullptr, nullptr);
@@ -897,9 +1132,15 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
             unsigned grid = (unsigned)ceil_div(p->n1, HASH_WARPS);
             unsigned cap = (unsigned)sm_count() * 16;
             if (grid > cap) grid = cap;
-            hash_rows_kernel<true><<<grid, HASH_WARPS * 32, 0, st>>>(
-                p->n1, p->list1, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32, p->bval, p->mpos,
-                p->mcrd, p->semi, nullptr, p->cpos, ccrd, cval);
+            if (!p->mpos) {
+                auto k = p->ncols <= (1 << 24) ? short_rows_kernel<false> : short_rows_kernel<true>;
+                k<<<grid, HASH_WARPS * 32, 0, st>>>(p->bin_counts, p->list1, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32,
+                                                    p->bval, p->semi, p->cpos, ccrd, cval);
+            } else {
+                auto k = p->ncols <= (1 << 24) ? hash_rows_kernel<true, false> : hash_rows_kernel<true, true>;
+                k<<<grid, HASH_WARPS * 32, 0, st>>>(p->bin_counts, p->list1, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32,
+                                                    p->bval, p->mpos, p->mcrd, p->semi, nullptr, p->cpos, ccrd, cval);
+            }
             if (cudaGetLastError() != cudaSuccess) rc = fail("spgemm numeric (hash) launch failed");
         }
         if (!rc && p->n2) {
