@@ -1,5 +1,9 @@
 // SpMM  C[a,:] = C[a,:] (+) sum_b A[a,b] (x) B[b,:]   (CSR / DCSR rows, dense row-major B and C).
 //
+// spmm_rows picks the kernels: spmm_short.cu for matrices without long rows, spmm_pieces.cu and spmm_stream.cu for the
+// others.  This file holds the row panels, which a caller can ask for by the variant and which the allocation-free entry
+// point runs, as their long-row list has a bounded size.
+//
 // Row-panel design.  A group of T lanes owns one row of A and a panel of W
 // columns of B/C (2*NI doubles per lane, 128-bit loads); it loads T (crd, val)
 // pairs at a time with one coalesced streaming load and broadcasts them with
@@ -15,6 +19,7 @@
 //
 // Bound: HBM.  Algorithmic bytes = 8(n+1) + 16 nnz + 8 ncols K + 8 nrows K.
 #include "common.cuh"
+#include "spmm.cuh"
 
 namespace cb200 {
 
@@ -189,8 +194,8 @@ spmm_chunks_kernel(const int64_t *__restrict__ row_ids, const int64_t *__restric
     }
 }
 
-// Any K, any alignment: one thread per output element.  Correctness path for
-// shapes the panel kernels do not take (odd K, unaligned or odd leading dimensions).
+// Any size: one thread per output element.  For operands beyond 32-bit column numbers or row offsets, which no other kernel
+// here takes.
 __global__ void __launch_bounds__(256)
 spmm_scalar_kernel(int64_t nrows, const int64_t *__restrict__ row_ids,
                    const int64_t *__restrict__ pos, const int64_t *__restrict__ crd,
@@ -209,21 +214,32 @@ spmm_scalar_kernel(int64_t nrows, const int64_t *__restrict__ row_ids,
     }
 }
 
-int spmm_stream(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const int64_t *row_ids, const int64_t *pos,
-                const int64_t *crd, const double *val, const double *b, int64_t ldb, double *c, int64_t ldc,
-                int accumulate, bool forced, cudaStream_t st);
 int spmm_stream_tma(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const int64_t *row_ids, const int64_t *pos,
                     const int64_t *crd, const double *val, const double *b, int64_t ldb, double *c, int64_t ldc,
                     int accumulate, bool gather4, cudaStream_t st);
 
-// Shapes the entry-stream path takes without being asked.
-// From 64 columns on a row of B fills the lanes of a warp and the stream wins on uniform and
-// skewed matrices alike (R-MAT scale 20, K = 128: 1.19 ms against 1.83 ms); below that the
-// lane groups of the panel kernels waste less.
-static bool spmm_stream_preferred(int64_t nrows, int64_t nnz, int64_t k)
+// The call without a variant.  Matrices without long rows go to spmm_short_rows; which ones those are only the device knows,
+// so the kernels for the others are launched too and return at once.  Of these the entry stream takes over from the pieces
+// where a row of B fills a warp, from 64 columns (R-MAT scale 20: K = 48 894 us against 880, K = 64 833 against 900, K = 65
+// 1421 against 1685).  From 96 columns on it is as fast as spmm_short_rows where that takes a call (400,000 rows of 8, K = 128:
+// 477 us against 502; 50,021 rows of up to 24: 55 against 54) and is launched alone.
+static int spmm_auto(const SpmmCall &a)
 {
-    (void)nrows; (void)nnz;
-    return k >= 64;
+    const bool stream = !a.pair && a.k >= 64 && a.nnz > 0;
+    LongRows lr = {nullptr, 0};
+    if (!stream || !a.vec || a.k < 96) CB_TRY(spmm_short_rows(a, &lr));
+    if (!stream) return spmm_pieces(a, lr);
+    const int64_t slices = ceil_div(a.k, 256), width = ceil_div(ceil_div(a.k, slices), 2) * 2;
+    for (int64_t col0 = 0; col0 < a.k; col0 += width) {
+        SpmmCall part = a;
+        part.k = a.k - col0 < width ? a.k - col0 : width;
+        part.b += col0;
+        part.c += col0;
+        const int took = spmm_stream(part, lr);
+        if (took < 0) return -1;
+        if (took == 0) CB_TRY(spmm_pieces(part, lr));
+    }
+    return 0;
 }
 
 struct SpmmArgs {
@@ -294,6 +310,14 @@ int spmm_rows(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const int64_
     int pair = semiring == COMET_B200_PLUS_PAIR;
     bool vec_ok = (k % 2 == 0) && (ldb % 2 == 0) && (ldc % 2 == 0) &&
                   ((((uintptr_t)b | (uintptr_t)c) & 15) == 0) && k <= (1 << 24);
+    const SpmmCall call = {nrows, ncols, nnz, k, row_ids, pos, crd, val, b, ldb, c, ldc, pair != 0, vec_ok, accumulate, st};
+    // bits 24-25 of the variant pick the path: 0 = by shape, 1 = entry stream (rows of B staged in shared memory by
+    // cp.async), 2 = row panels, 3 = entry stream with the rows staged by TMA bulk copies (bit 26 in addition: one
+    // tile::gather4 tensor copy per stage instead of one bulk copy per row); its low bits ask for panels of a given shape
+    const int path = (variant >> 24) & 3;
+    // row offsets and column numbers are 32-bit in the kernels below
+    const bool narrow_ids = ncols <= 0xffffffffLL && ldb < (1LL << 29) && k <= (1 << 24);
+    if (narrow_ids && (!vec_ok || (path == 0 && ((variant & 0xffffff) == 0 || (!pair && k >= 64))))) return spmm_auto(call);
     if (!vec_ok) {
         int64_t blocks = ceil_div(nrows * k, 256);
         int64_t cap = (int64_t)sm_count() * 32;
@@ -303,18 +327,14 @@ int spmm_rows(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const int64_
         CB_LAUNCH_CHECK();
         return 0;
     }
-    // bits 24-25 of the variant pick the path: 0 = by shape, 1 = entry stream (rows of B staged in shared memory by
-    // cp.async), 2 = row panels, 3 = entry stream with the rows staged by TMA bulk copies (bit 26 in addition: one
-    // tile::gather4 tensor copy per stage instead of one bulk copy per row)
-    const int path = (variant >> 24) & 3;
     if (!pair && path == 3) {
         const int took = spmm_stream_tma(nrows, ncols, nnz, k, row_ids, pos, crd, val, b, ldb, c, ldc, accumulate,
                                          ((variant >> 26) & 1) != 0, st);
         if (took < 0) return -1;
         if (took > 0) return 0;
     }
-    if (!pair && path != 2 && (path == 1 || spmm_stream_preferred(nrows, nnz, k))) {
-        const int took = spmm_stream(nrows, ncols, nnz, k, row_ids, pos, crd, val, b, ldb, c, ldc, accumulate, path == 1, st);
+    if (!pair && path == 1) {
+        const int took = spmm_stream(call, LongRows{nullptr, 0});
         if (took < 0) return -1;
         if (took > 0) return 0;
     }

@@ -1,0 +1,29 @@
+// The automatic SpMM: a call's operands, and the kernels that take it.
+#pragma once
+#include "common.cuh"
+#include "stream.cuh"
+
+namespace cb200 {
+
+struct SpmmCall {
+    int64_t nrows, ncols, nnz, k;
+    const int64_t *row_ids, *pos, *crd;
+    const double *val, *b;
+    int64_t ldb;
+    double *c;
+    int64_t ldc;
+    bool pair;
+    bool vec;                 // K, both leading dimensions and both addresses allow 16-byte accesses
+    int accumulate;
+    cudaStream_t st;
+};
+
+// Takes the call if no row is long, which only the device knows; `lr` is for the kernels that take it otherwise (spmm_short.cu).
+int spmm_short_rows(const SpmmCall &a, LongRows *lr);
+// Equal pieces of A's path, a group of lanes each; any K and alignment (spmm_pieces.cu).
+int spmm_pieces(const SpmmCall &a, LongRows lr);
+// Rows of B staged in shared memory (spmm_stream.cu).  Returns 1 when it took the call, 0 when the shape is not one that
+// it handles, -1 on error.
+int spmm_stream(const SpmmCall &a, LongRows lr);
+
+}  // namespace cb200

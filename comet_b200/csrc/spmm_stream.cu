@@ -1,13 +1,11 @@
 // SpMM over the entry stream, rows of B staged in shared memory by asynchronous copies.
 //
-// The row-panel kernels of spmm.cu keep the gathered rows of B in flight in
-// registers and hand out whole rows of A, so a power-law matrix needs a second
-// pass for its hub rows and the bytes in flight follow occupancy.  Here every
-// warp owns a ring of shared-memory stages (SB_G rows of B each) and a piece of
+// Every warp owns a ring of shared-memory stages (G rows of B each) and a piece of
 // the ENTRY stream of A: per stored entry its lanes issue 16-byte cp.async
 // copies of B[crd, :] into the ring, several stages ahead of the stage being
 // multiplied, so the gather runs ahead of the arithmetic without holding
-// registers.  (One bulk copy per row -- cp.async.bulk completing on an
+// registers (the row panels of spmm.cu keep them in flight in registers, so
+// that the bytes in flight follow occupancy).  (One bulk copy per row -- cp.async.bulk completing on an
 // mbarrier -- was measured first and was slower: 1 KB per copy is too little
 // work per copy instruction, 6.1 ms against 1.2 ms on R-MAT scale 20, K = 128.)
 //
@@ -20,94 +18,72 @@
 // accumulate), so its summation order is not fixed and differences stay at
 // rounding level.
 //
-// Bound: HBM.  Algorithmic bytes = 8(n+1) + 16 nnz + 8 ncols K + 8 nrows K.
+// Bound: the L2 -> SM rate (17 TB/s) for the gathered rows of B; the arrays alone would take 370 us of HBM time at R-MAT
+// scale 20, K = 128, the gather 960 us.  Constant offsets in the ring, short pieces for small matrices (stream_plan) and a plan
+// kernel with a thread per row instead of a search per piece: 1240 -> 1140 us there, 111 -> 28 us at scale 14.
 #include "common.cuh"
-#include "stream.cuh"
+#include "spmm.cuh"
 
 namespace cb200 {
 
 static const int SB_WARPS = 16;                // warps per CTA, one CTA per SM
-static const int SB_G = 4;                     // rows of B per stage (one copy group)
-static const int SB_MAX_STAGES = 8;
 static const int SB_RING_BYTES = 12 * 1024;    // per warp
 static const int SB_SIDE_BYTES = 512;           // per warp: 32 column indices, 32 values of A, 32 row ends
 
-// Blocks are equal pieces of the path that walks A row by row: one step per stored entry and one
-// step per row end (a row costs about as much as an entry: its result is written, or zeros for an
-// empty row).  One warp per block boundary b finds where the path stands after b*q steps: inside
-// row block_row[b], at entry block_ent[b].  When the call does not accumulate, a row that a
-// boundary cuts gets zeros here: its parts are added with atomics.
-__global__ void __launch_bounds__(256)
-spmm_stream_plan_kernel(int64_t nrows, int64_t nnz, int64_t q, int64_t nblocks, const int64_t *__restrict__ row_ids,
-                        const int64_t *__restrict__ pos, double *__restrict__ c, int64_t ldc, int k, int accumulate,
-                        int64_t *__restrict__ block_row, int64_t *__restrict__ block_ent)
+// One copy of sizeof(V) bytes global -> shared.  16-byte ones bypass L1; operands with odd widths or addresses take 8.
+template <typename V>
+__device__ __forceinline__ void sb_copy(uint32_t dst, const void *src);
+template <>
+__device__ __forceinline__ void sb_copy<double2>(uint32_t dst, const void *src) { sb_copy16(dst, src); }
+template <>
+__device__ __forceinline__ void sb_copy<double>(uint32_t dst, const void *src)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t b = warp; b <= nblocks; b += nwarps) {
-        int64_t d = b * q;
-        if (d > nnz + nrows) d = nnz + nrows;
-        // largest r in [0, nrows] with pos[r] + r <= d: the 32 lanes probe 32 points of the range per step
-        int64_t lo = 0, hi = nrows;
-        while (lo < hi) {
-            const int64_t step = (hi - lo + 31) / 32;
-            int64_t probe = lo + (lane + 1) * step;
-            if (probe > hi) probe = hi;
-            const int k = __popc(__ballot_sync(0xffffffffu, pos[probe] + probe <= d));   // the first k probes hold
-            const int64_t fail_at = lo + (int64_t)(k + 1) * step;                             // probe k does not (if k < 32)
-            if (k > 0) { lo += (int64_t)k * step; if (lo > hi) lo = hi; }
-            if (k < 32) hi = (fail_at < hi ? fail_at : hi) - 1;                               // the answer lies before probe k
-        }
-        int64_t r = lo, e = d - lo;
-        if (b > 0 && r < nrows && e >= pos[r + 1]) {   // the boundary is the end of row r: start at the next row
-            e = pos[r + 1];
-            r += 1;
-        }
-        if (lane == 0) {
-            block_row[b] = r;
-            block_ent[b] = e;
-        }
-        if (!accumulate && b > 0 && b < nblocks && r < nrows && e > pos[r]) {
-            const int64_t out = row_ids ? row_ids[r] : r;
-            double2 *crow = (double2 *)(c + out * ldc);
-            for (int j = lane; j < k / 2; j += 32) crow[j] = make_double2(0.0, 0.0);
-        }
-    }
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 
-template <int NI, bool FULLK>
+// NI vectors V per lane cover the columns; FULLK: exactly.  A row takes 32 NI vectors in the ring whether it fills them or
+// not, so that every offset is a constant; a stage is four rows, two when rows are longer than 1 KB.
+template <typename V, int NI>
+struct StreamShape {
+    static const int ROW = 32 * NI * (int)sizeof(V);
+    static const int G = ROW <= 1024 ? 4 : 2;
+    static const int STAGE = ROW * G;
+    static const int STAGES = SB_RING_BYTES / STAGE;
+    static const int RING = STAGE * STAGES;
+    static const int WARP = RING + SB_SIDE_BYTES;
+};
+
+template <typename V, int NI, bool FULLK>
 __global__ void __launch_bounds__(SB_WARPS * 32, 1)
-spmm_stream_kernel(int64_t nrows, int64_t nnz, int64_t q, unsigned nblocks, const int64_t *__restrict__ row_ids,
+spmm_stream_kernel(int64_t nrows, unsigned nblocks, const int64_t *__restrict__ row_ids,
                    const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, const double *__restrict__ val,
-                   const double *__restrict__ b, int64_t ldb, double *__restrict__ c, int64_t ldc, int k, int stages_arg,
+                   const double *__restrict__ b, int64_t ldb, double *__restrict__ c, int64_t ldc, int k,
                    int accumulate, WorkHeader *hdr, const int64_t *__restrict__ block_row,
-                   const int64_t *__restrict__ block_ent)
+                   const int64_t *__restrict__ block_ent, LongRows lr)
 {
+    wait_for_previous();
+    if (not_this(lr)) return;
+    using S = StreamShape<V, NI>;
+    constexpr int SB_G = S::G, stages = S::STAGES;
+    constexpr uint32_t rowbytes = S::ROW, stagebytes = S::STAGE, ringbytes = S::RING;
     // per warp: a ring of `stages` stages of SB_G rows of B, then 32 column indices and 32 values of A
     extern __shared__ __align__(128) unsigned char sb_smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    // K = 64 NI is the common case: every size below is then a compile-time constant
-    const int stages = FULLK ? SB_RING_BYTES / (SB_G * NI * 512) : stages_arg;
-    const int k2 = FULLK ? NI * 32 : (k >> 1);          // double2 vectors per row
-    const uint32_t rowbytes = FULLK ? (uint32_t)NI * 512u : (uint32_t)k * 8u;
-    const uint32_t stagebytes = rowbytes * SB_G;
-    const uint32_t warpbytes = (uint32_t)stages * stagebytes + SB_SIDE_BYTES;
-    unsigned char *ring = sb_smem_raw + (size_t)warp * warpbytes;
-    int32_t *cs = (int32_t *)(ring + (size_t)stages * stagebytes);
+    const int kv = FULLK ? NI * 32 : k / Vec<V>::N;     // vectors per row
+    unsigned char *ring = sb_smem_raw + (size_t)warp * S::WARP;
+    int32_t *cs = (int32_t *)(ring + S::RING);
     double *vs = (double *)(cs + 32);
     int *ps = (int *)(vs + 32);                         // block-local end positions of 32 consecutive rows
-    const uint32_t ring_s = sb_smem(ring) + (uint32_t)lane * 16u;
-    const char *bl = (const char *)b + lane * 16;
+    const uint32_t ring_s = sb_smem(ring) + (uint32_t)lane * (uint32_t)sizeof(V);
+    const char *bl = (const char *)b + lane * sizeof(V);
     const int64_t ldb8 = ldb * 8;
     bool on[NI];
 #pragma unroll
-    for (int i = 0; i < NI; i++) on[i] = FULLK || (lane + i * 32 < k2);
+    for (int i = 0; i < NI; i++) on[i] = FULLK || (lane + i * 32 < kv);
 
     uint32_t pofs = 0;               // byte offset of the stage the next issue fills
     uint32_t cofs = 0;               // byte offset of the stage the next wait reads
-    const uint32_t ringbytes = (uint32_t)stages * stagebytes;
 
     while (true) {
         unsigned blk = 0;
@@ -143,42 +119,27 @@ spmm_stream_kernel(int64_t nrows, int64_t nnz, int64_t q, unsigned nblocks, cons
         int32_t cnext = (lane < cnt) ? (int32_t)ld_stream(crd0 + lane) : 0;
         double vnext = (lane < cnt) ? ld_stream(val0 + lane) : 0.0;
 
-        double2 acc[NI];
+        V acc[NI];
 #pragma unroll
-        for (int i = 0; i < NI; i++) acc[i] = make_double2(0.0, 0.0);
+        for (int i = 0; i < NI; i++) acc[i] = Vec<V>::zero();
 
         // write out the finished row r and clear the accumulators
         auto flush = [&](bool whole) {
             const int64_t out = row_ids ? row_ids[r] : r;
             double *crow = c + out * ldc;
-            if (whole) {
-                if (!accumulate || rs < re) {
+            if (whole && accumulate && rs == re) return;       // an empty row adds nothing
 #pragma unroll
-                    for (int i = 0; i < NI; i++) {
-                        const int j = lane + i * 32;
-                        if (on[i]) {
-                            double2 o = acc[i];
-                            if (accumulate) {
-                                const double2 old = __ldcs((const double2 *)crow + j);
-                                o.x += old.x;
-                                o.y += old.y;
-                            }
-                            __stcs((double2 *)crow + j, o);
-                        }
+            for (int i = 0; i < NI; i++) {
+                V *at = (V *)crow + lane + i * 32;
+                if (on[i]) {
+                    if (!whole) Vec<V>::atomic_to(at, acc[i]);
+                    else {
+                        if (accumulate) Vec<V>::add_to(acc[i], __ldcs(at));
+                        __stcs(at, acc[i]);
                     }
                 }
-            } else {
-#pragma unroll
-                for (int i = 0; i < NI; i++) {
-                    const int j = lane + i * 32;
-                    if (on[i]) {
-                        atomicAdd(crow + 2 * j, acc[i].x);
-                        atomicAdd(crow + 2 * j + 1, acc[i].y);
-                    }
-                }
+                acc[i] = Vec<V>::zero();
             }
-#pragma unroll
-            for (int i = 0; i < NI; i++) acc[i] = make_double2(0.0, 0.0);
         };
         auto next_row = [&]() {
             flush(rs >= 0);
@@ -202,8 +163,14 @@ spmm_stream_kernel(int64_t nrows, int64_t nnz, int64_t q, unsigned nblocks, cons
                     cnext = (nb < cnt) ? (int32_t)ld_stream(crd0 + nb) : 0;
                     __syncwarp();
                 }
-                const int4 c4 = *(const int4 *)(cs + off);          // broadcast read of four column indices
-                const int cc[4] = {c4.x, c4.y, c4.z, c4.w};
+                int cc[SB_G];                                       // broadcast read of the column indices
+                if (SB_G == 4) {
+                    const int4 c4 = *(const int4 *)(cs + off);
+                    cc[0] = c4.x; cc[1] = c4.y; cc[SB_G - 2] = c4.z; cc[SB_G - 1] = c4.w;
+                } else {
+                    const int2 c2 = *(const int2 *)(cs + off);
+                    cc[0] = c2.x; cc[1] = c2.y;
+                }
                 const uint32_t dst = ring_s + pofs;
                 const int m = cnt - g * SB_G;
                 if (m >= SB_G) {
@@ -212,7 +179,7 @@ spmm_stream_kernel(int64_t nrows, int64_t nnz, int64_t q, unsigned nblocks, cons
                         const char *src = bl + (int64_t)cc[t] * ldb8;
 #pragma unroll
                         for (int i = 0; i < NI; i++)
-                            if (on[i]) sb_copy16(dst + (uint32_t)t * rowbytes + (uint32_t)i * 512u, src + i * 512);
+                            if (on[i]) sb_copy<V>(dst + (uint32_t)t * rowbytes + (uint32_t)(i * 32 * (int)sizeof(V)), src + i * 32 * (int)sizeof(V));
                     }
                 } else {
 #pragma unroll
@@ -221,7 +188,7 @@ spmm_stream_kernel(int64_t nrows, int64_t nnz, int64_t q, unsigned nblocks, cons
                             const char *src = bl + (int64_t)cc[t] * ldb8;
 #pragma unroll
                             for (int i = 0; i < NI; i++)
-                                if (on[i]) sb_copy16(dst + (uint32_t)t * rowbytes + (uint32_t)i * 512u, src + i * 512);
+                                if (on[i]) sb_copy<V>(dst + (uint32_t)t * rowbytes + (uint32_t)(i * 32 * (int)sizeof(V)), src + i * 32 * (int)sizeof(V));
                         }
                     }
                 }
@@ -241,37 +208,33 @@ spmm_stream_kernel(int64_t nrows, int64_t nnz, int64_t q, unsigned nblocks, cons
                 vnext = (nb < cnt) ? ld_stream(val0 + nb) : 0.0;
             }
             issue(g + stages - 1);
-            if (FULLK && NI == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");        // stages - 1
-            else if (FULLK && NI == 1) asm volatile("cp.async.wait_group 5;" ::: "memory");
-            else sb_wait_pending(stages - 1);
+            sb_wait<stages - 1>();
             __syncwarp();                               // the other lanes' copies of this stage have landed too
-            const double2 *src = (const double2 *)(ring + cofs) + lane;
-            double2 bv[SB_G][NI];
+            const V *src = (const V *)(ring + cofs) + lane;
+            V bv[SB_G][NI];
 #pragma unroll
             for (int t = 0; t < SB_G; t++)
 #pragma unroll
-                for (int i = 0; i < NI; i++) bv[t][i] = on[i] ? src[t * k2 + i * 32] : make_double2(0.0, 0.0);
-            const double2 v01 = *(const double2 *)(vs + off), v23 = *(const double2 *)(vs + off + 2);
-            const double vv[4] = {v01.x, v01.y, v23.x, v23.y};
+                for (int i = 0; i < NI; i++) bv[t][i] = on[i] ? src[(t * NI + i) * 32] : Vec<V>::zero();
+            double vv[SB_G];
+#pragma unroll
+            for (int t = 0; t < SB_G; t += 2) {
+                const double2 v2 = *(const double2 *)(vs + off + t);
+                vv[t] = v2.x; vv[t + 1] = v2.y;
+            }
             const int j0 = g * SB_G;
             if (j0 + SB_G <= re && j0 + SB_G <= cnt) {  // the four entries belong to the row in progress
 #pragma unroll
                 for (int t = 0; t < SB_G; t++)
 #pragma unroll
-                    for (int i = 0; i < NI; i++) {
-                        acc[i].x = fma(vv[t], bv[t][i].x, acc[i].x);
-                        acc[i].y = fma(vv[t], bv[t][i].y, acc[i].y);
-                    }
+                    for (int i = 0; i < NI; i++) Vec<V>::fma_to(acc[i], vv[t], bv[t][i]);
             } else {
 #pragma unroll
                 for (int t = 0; t < SB_G; t++) {
                     if (j0 + t < cnt) {
                         while (j0 + t >= re) next_row();
 #pragma unroll
-                        for (int i = 0; i < NI; i++) {
-                            acc[i].x = fma(vv[t], bv[t][i].x, acc[i].x);
-                            acc[i].y = fma(vv[t], bv[t][i].y, acc[i].y);
-                        }
+                        for (int i = 0; i < NI; i++) Vec<V>::fma_to(acc[i], vv[t], bv[t][i]);
                     }
                 }
             }
@@ -287,89 +250,49 @@ spmm_stream_kernel(int64_t nrows, int64_t nnz, int64_t q, unsigned nblocks, cons
     }
 }
 
-// Cuts the (entries + rows) path of a CSR matrix into pieces for `warps` persistent warps and runs the plan
-// kernel.  c != null and accumulate == 0: rows cut by a boundary get zeros (k columns).  Returns 1, 0 when the
-// piece count does not fit 32 bits, -1 on error.  The plan lives in the work-list scratch slot of the device.
-int stream_plan(int64_t nrows, int64_t nnz, int64_t warps, const int64_t *row_ids, const int64_t *pos, double *c,
-                int64_t ldc, int k, int accumulate, cudaStream_t st, StreamPlan *out)
+template <typename V, int NI, bool FULLK>
+static int launch_stream(const SpmmCall &a, LongRows lr)
 {
-    const int64_t steps = nnz + nrows;                 // path length: one step per entry, one per row end
-    int64_t q = ceil_div(steps, warps * 8);
-    if (q < 512) q = 512;
-    const int64_t nblocks = ceil_div(steps, q);
-    if (nblocks > 0x7ffffff0LL) return 0;
-    void *wl = nullptr;
-    if (scratch(SLOT_WORKLIST, sizeof(WorkHeader) + (size_t)(nblocks + 1) * 2 * sizeof(int64_t), &wl)) return -1;
-    out->hdr = (WorkHeader *)wl;
-    out->block_row = (int64_t *)((char *)wl + sizeof(WorkHeader));
-    out->block_ent = out->block_row + (nblocks + 1);
-    out->q = q;
-    out->nblocks = nblocks;
-    if (cudaMemsetAsync(out->hdr, 0, sizeof(WorkHeader), st) != cudaSuccess) {
-        fail("clearing the block counter failed");
+    StreamPlan plan;
+    const int planned = stream_plan(a.nrows, a.nnz, (int64_t)sm_count() * SB_WARPS, a.row_ids, a.pos, a.c, a.ldc, a.k,
+                                    a.accumulate, lr, a.st, &plan);
+    if (planned <= 0) return planned;
+    auto kernel = spmm_stream_kernel<V, NI, FULLK>;
+    const size_t smem = (size_t)SB_WARPS * StreamShape<V, NI>::WARP;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        fail("spmm: shared memory size refused");
         return -1;
     }
-    const int64_t pgrid = ceil_div((nblocks + 1) * 32, 256);
-    spmm_stream_plan_kernel<<<(unsigned)pgrid, 256, 0, st>>>(nrows, nnz, q, nblocks, row_ids, pos, c, ldc, k,
-                                                            c ? accumulate : 1, out->block_row, out->block_ent);
-    return 1;
-}
-
-// Returns 1 when this path took the call, 0 when the shape is not one it handles, -1 on error.
-int spmm_stream(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const int64_t *row_ids, const int64_t *pos,
-                const int64_t *crd, const double *val, const double *b, int64_t ldb, double *c, int64_t ldc,
-                int accumulate, bool forced, cudaStream_t st)
-{
-    // 16-byte copies need aligned rows; the lane layout covers up to 256 columns
-    if (k < 2 || k > 256 || (k & 1) || (ldb & 1) || (ldc & 1) || ((((uintptr_t)b | (uintptr_t)c) & 15) != 0)) return 0;
-    if (nnz < (forced ? 1 : (1 << 16)) || nrows <= 0 || ncols > 0x7fffffffLL) return 0;   // column indices travel as int32
-    const int rowbytes = (int)k * 8;
-    int stages = SB_RING_BYTES / (SB_G * rowbytes);
-    if (stages > SB_MAX_STAGES) stages = SB_MAX_STAGES;
-    if (stages < 2) return 0;
-    const size_t smem = (size_t)SB_WARPS * ((size_t)stages * SB_G * rowbytes + SB_SIDE_BYTES);
-
-    StreamPlan plan;
-    const int planned = stream_plan(nrows, nnz, (int64_t)sm_count() * SB_WARPS, row_ids, pos, c, ldc, (int)k, accumulate,
-                                    st, &plan);
-    if (planned <= 0) return planned;
-    WorkHeader *hdr = plan.hdr;
-    const int64_t *block_row = plan.block_row, *block_ent = plan.block_ent;
-    const int64_t q = plan.q, nblocks = plan.nblocks;
-    int64_t grid = ceil_div(nblocks, SB_WARPS);
+    int64_t grid = ceil_div(plan.nblocks, SB_WARPS);
     if (grid > sm_count()) grid = sm_count();
-    const int ni = k <= 64 ? 1 : (k <= 128 ? 2 : 4);
-#define SB_LAUNCH(NN, FK)                                                                                              \
-    do {                                                                                                           \
-        static bool attr_set[64] = {false};                                                                        \
-        int d = 0;                                                                                                 \
-        cudaGetDevice(&d);                                                                                         \
-        if (d >= 0 && d < 64 && !attr_set[d]) {                                                                    \
-            if (cudaFuncSetAttribute(spmm_stream_kernel<NN, FK>, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
-                                     SB_WARPS * (SB_RING_BYTES + SB_SIDE_BYTES)) != cudaSuccess) {                    \
-                fail("spmm: shared memory size refused");                                                          \
-                return -1;                                                                                         \
-            }                                                                                                      \
-            attr_set[d] = true;                                                                                    \
-        }                                                                                                          \
-        spmm_stream_kernel<NN, FK><<<(unsigned)grid, SB_WARPS * 32, smem, st>>>(                                       \
-            nrows, nnz, q, (unsigned)nblocks, row_ids, pos, crd, val, b, ldb, c, ldc, (int)k, stages, accumulate,  \
-            hdr, block_row, block_ent);                                                                                       \
-    } while (0)
-    const bool fullk = (k == 64 * ni);
-    if (ni == 1 && fullk) SB_LAUNCH(1, true);
-    else if (ni == 1) SB_LAUNCH(1, false);
-    else if (ni == 2 && fullk) SB_LAUNCH(2, true);
-    else if (ni == 2) SB_LAUNCH(2, false);
-    else if (fullk) SB_LAUNCH(4, true);
-    else SB_LAUNCH(4, false);
-#undef SB_LAUNCH
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_behind(kernel, dim3((unsigned)grid), SB_WARPS * 32, smem, a.st, a.nrows, (unsigned)plan.nblocks,
+                                        a.row_ids, a.pos, a.crd, a.val, a.b, a.ldb, a.c, a.ldc, (int)a.k, a.accumulate,
+                                        plan.hdr, plan.block_row, plan.block_ent, lr);
     if (e != cudaSuccess) {
         fail("spmm: launch failed: %s", cudaGetErrorString(e));
         return -1;
     }
     return 1;
+}
+
+int spmm_stream(const SpmmCall &a, LongRows lr)
+{
+    if (a.k < 1 || a.k > 256 || a.nnz < 1 || a.nrows <= 0 || a.ncols > 0x7fffffffLL) return 0;    // columns travel as int32
+    if (a.vec) {
+        if (a.k == 64) return launch_stream<double2, 1, true>(a, lr);
+        if (a.k < 64) return launch_stream<double2, 1, false>(a, lr);
+        if (a.k == 128) return launch_stream<double2, 2, true>(a, lr);
+        if (a.k < 128) return launch_stream<double2, 2, false>(a, lr);
+        if (a.k <= 192) return launch_stream<double2, 3, false>(a, lr);
+        if (a.k == 256) return launch_stream<double2, 4, true>(a, lr);
+        return launch_stream<double2, 4, false>(a, lr);
+    }
+    if (a.k <= 32) return launch_stream<double, 1, false>(a, lr);
+    if (a.k <= 64) return launch_stream<double, 2, false>(a, lr);
+    if (a.k <= 96) return launch_stream<double, 3, false>(a, lr);
+    if (a.k <= 128) return launch_stream<double, 4, false>(a, lr);
+    if (a.k <= 192) return launch_stream<double, 6, false>(a, lr);
+    return launch_stream<double, 8, false>(a, lr);
 }
 
 }  // namespace cb200

@@ -488,8 +488,8 @@ COMET_B200_EXPORT int32_t comet_b200_dev_spmv_f64_i64(int64_t nrows, int64_t nnz
                                                       int32_t semiring, int32_t accumulate,
                                                       void *stream);
 
-/* variant: 0 = automatic.  Bits 24-25 pick the kernel family: 0 = by shape (the entry-stream kernel
-   from 64 columns and 65536 stored entries on, for plus-times; the row-panel kernels otherwise),
+/* variant: 0 = automatic.  Bits 24-25 pick the kernel family: 0 = by shape and row lengths (row
+   panels if the low bits ask for them and K < 64),
    1 = entry stream whenever the shape allows it (K even, at most 256; worth asking for with
    narrow B and a power-law A, where it is several times faster than the panels),
    2 = row panels, 3 = the entry stream with the rows of B staged by TMA bulk copies
