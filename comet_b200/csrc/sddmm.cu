@@ -1,225 +1,229 @@
 // SDDMM  out[p] = S.val[p] * sum_k X[i,k] * Y[j,k]   for every stored (i,j) of S (CSR).
 //
-// Two launches share the work by row length.
-//   rows of at most LONG_ROW entries: warps draw blocks of BLOCK_ROWS consecutive rows from a
-//     counter and walk the block's entries as ONE stream, 32 entries per batch; the row of every
-//     entry is found once per batch by a shuffle binary search over the block's row pointers, the
-//     next batch's coordinates are fetched before the current one is worked on, and groups of G
-//     lanes gather X[i,:] and Y[j,:] with 128-bit loads and finish each dot product with
-//     xor-shuffles.  The 32 results of a batch are scaled by S.val and leave in one coalesced store.
-//   longer rows: cut into CHUNK-entry pieces on a work list in scratch memory by the first launch;
-//     the second launch gives every piece to a warp that keeps X[i,:] in registers.  On power-law
-//     matrices this balanced path carries most of the entries.
+// Every entry is a dot product of its own, so the entries are cut into equal pieces whatever rows they belong to, one warp
+// per piece.  A warp takes 32 entries at a time: a lane each loads their columns and values, one batch ahead, and finds
+// their rows among 32 row ends that the lanes hold (six shuffles; the ends are replaced when a batch runs past them).
+// Groups of G lanes then take G consecutive entries each: NI vectors per lane cover the columns, X[i,:] stays in registers
+// while the row does not change, and the products of U entries are in flight.  An entry's sum is finished with
+// xor-shuffles and lands in the lane that holds its place, so results leave in one coalesced store.
 //
-// Bound: HBM.  Algorithmic bytes = 8(n+1) + 24 nnz + 8 K (nrows + ncols).
+// A batch of one row (long rows: most of a power-law matrix) takes a path with X[i,:] loaded once and nothing but Y in flight.
+//
+// V = double2 where K, both leading dimensions and both addresses allow 16-byte accesses, otherwise double: an odd number of
+// columns costs twice the load instructions and no more.  K beyond one pass of a warp is walked in slices (LOOP).
+//
+// Bound: HBM for the arrays, 8(n+1) + 24 nnz + 8 K (nrows + ncols) bytes; with wide rows the L2 -> SM rate (17 TB/s) for the
+// gathered rows of Y.
 #include "common.cuh"
+#include "stream.cuh"
 
 namespace cb200 {
 
-static const int SDDMM_THREADS = 256;
-static const int64_t SDDMM_LONG_ROW = 32;
-static const int64_t SDDMM_CHUNK = 64;
-static const int SDDMM_BLOCK_ROWS = 8;     // consecutive rows a warp draws at a time (power of two <= 32)
+static const int SD_THREADS = 256;
 
-// Entries [s, e) of row `row`; xr holds this lane's part of X[row,:].
-template <int G, int NI>
-__device__ __forceinline__ void sample_range(const double2 (&xr)[NI], const int64_t *__restrict__ crd,
-                                             const double *__restrict__ sval,
-                                             const double *__restrict__ y, int64_t ldy,
-                                             double *__restrict__ out, int64_t s, int64_t e, int lane,
-                                             int k2)
+// piece_row[b]: the row of entry b * 2^s.  A thread per row, a warp together for a row with many pieces.
+__global__ void __launch_bounds__(256)
+sddmm_plan_kernel(int64_t nrows, int s, int64_t npieces, const int64_t *__restrict__ pos, int32_t *__restrict__ piece_row)
 {
-    constexpr int P = 32 / G;                 // entries in flight per step
-    const int g = lane / G, l = lane % G;
-    for (int64_t base = s; base < e; base += 32) {
-        const int64_t p = base + lane;
-        int64_t c = 0;
-        if (p < e) c = ld_stream(crd + p);
-        const int n = (e - base) < 32 ? (int)(e - base) : 32;
-        double mine = 0.0;
-        const int steps = (n + P - 1) / P;
-#pragma unroll 2
-        for (int t = 0; t < steps; t++) {
-            const int idx = t * P + g;        // entry of this batch handled by my group
-            const int64_t cc = __shfl_sync(0xffffffffu, (long long)c, idx & 31);
-            double d0 = 0.0, d1 = 0.0;
-            if (idx < n) {
-                const double2 *yr = (const double2 *)(y + cc * ldy);
-#pragma unroll
-                for (int i = 0; i < NI; i++) {
-                    if (l + i * G < k2) {
-                        double2 yy = __ldg(yr + l + i * G);
-                        d0 = fma(xr[i].x, yy.x, d0);
-                        d1 = fma(xr[i].y, yy.y, d1);
-                    }
-                }
-            }
-            double d = d0 + d1;
-#pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            // a batch has at most 32 / P = G steps, so lane l == t of each group can keep step t's result
-            if (l == t) mine = d;
+    let_next_start();
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, mask = ((int64_t)1 << s) - 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) piece_row[npieces] = (int32_t)(nrows - 1);
+    for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; r0 < nrows; r0 += stride) {
+        int64_t b0 = 0, b1 = 0;
+        if (r0 + lane < nrows) {
+            b0 = (pos[r0 + lane] + mask) >> s;
+            b1 = (pos[r0 + lane + 1] + mask) >> s;
+            if (b1 > npieces) b1 = npieces;
         }
-        // lane (g, l) now holds the result of batch entry l*P + g: a permutation of the batch,
-        // so the store below is one coalesced 256-byte write per warp
-        const int idx = l * P + g;
-        if (idx < n) out[base + idx] = ld_stream(sval + base + idx) * mine;
+        if (b1 - b0 <= 4)
+            for (int64_t b = b0; b < b1; b++) piece_row[b] = (int32_t)(r0 + lane);
+        unsigned many = __ballot_sync(0xffffffffu, b1 - b0 > 4);
+        while (many) {
+            const int t = __ffs(many) - 1;
+            many &= many - 1;
+            const int64_t tb = __shfl_sync(0xffffffffu, (long long)b0, t), te = __shfl_sync(0xffffffffu, (long long)b1, t);
+            for (int64_t b = tb + lane; b < te; b += 32) piece_row[b] = (int32_t)(r0 + t);
+        }
     }
 }
 
-template <int G, int NI>
-__device__ __forceinline__ void load_x(double2 (&xr)[NI], const double *__restrict__ x, int64_t ldx,
-                                       int64_t row, int l, int k2)
-{
-    const double2 *xp = (const double2 *)(x + row * ldx);
-#pragma unroll
-    for (int i = 0; i < NI; i++)
-        xr[i] = (l + i * G < k2) ? __ldg(xp + l + i * G) : make_double2(0.0, 0.0);
-}
+__device__ __forceinline__ void dot_to(double (&d)[2], double2 a, double2 b) { d[0] = fma(a.x, b.x, d[0]); d[1] = fma(a.y, b.y, d[1]); }
+__device__ __forceinline__ void dot_to(double (&d)[2], double a, double b) { d[0] = fma(a, b, d[0]); }
 
-// Entries [a, b) of a run of consecutive rows, as one stream: a batch of 32
-// consecutive entries may span several rows, so each entry carries its row
-// (found once per batch by a shuffle binary search over the 32 row pointers the
-// lanes hold) and X[row,:] is read through L1 next to Y[col,:].  The next
-// batch's coordinates and rows are fetched before the current batch is worked
-// on, so no load depends on another one inside the loop.
-template <int G, int NI>
-__device__ __forceinline__ void sample_stream(int64_t row0, int64_t rp, const int64_t *__restrict__ crd,
-                                              const double *__restrict__ sval,
-                                              const double *__restrict__ x, int64_t ldx,
-                                              const double *__restrict__ y, int64_t ldy,
-                                              double *__restrict__ out, int64_t a, int64_t b, int lane,
-                                              int k2)
+// A column number.  Y has more than 2^32 rows only if they are short.
+template <bool SHORT>
+struct Columns { using type = uint32_t; };
+template <>
+struct Columns<true> { using type = unsigned long long; };
+
+template <typename V, int G, int NI, int U, int UF, int MINB, bool LOOP>
+__global__ void __launch_bounds__(SD_THREADS, MINB)
+sddmm_kernel(int64_t nrows, int64_t nnz, int s, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd,
+             const double *__restrict__ sval, const double *__restrict__ x0, uint32_t ldx8, const double *__restrict__ y0,
+             uint32_t ldy8, double *__restrict__ out, int kv, const int32_t *__restrict__ piece_row, int64_t npieces)
 {
-    constexpr int P = 32 / G;
-    const int g = lane / G, l = lane % G;
-    auto fetch = [&](int64_t base, int64_t &c, int &row) {
-        const int64_t p = base + lane;
-        c = 0;
-        if (p < b) c = ld_stream(crd + p);
-        // last t in [0, BLOCK_ROWS) with pos[row0 + t] <= p  (rp = this lane's row pointer)
-        int lo = 0;
+    using Col = typename Columns<(G * NI <= 8)>::type;
+    const int lane = threadIdx.x & 31, g = lane / G, l = lane % G;
+    const int64_t piece = ((int64_t)blockIdx.x * SD_THREADS + threadIdx.x) >> 5;
+    const char *x = (const char *)((const V *)x0 + l), *y = (const char *)((const V *)y0 + l);
+    bool on[NI];
 #pragma unroll
-        for (int step = SDDMM_BLOCK_ROWS / 2; step > 0; step >>= 1) {
-            const int64_t v = __shfl_sync(0xffffffffu, (long long)rp, lo + step);
-            if (v <= p) lo += step;
-        }
-        row = lo;
+    for (int i = 0; i < NI; i++) on[i] = LOOP || l + i * G < kv;
+    wait_for_previous();
+    if (piece >= npieces) return;
+
+    const int64_t p0 = piece << s;
+    const int n = nnz - p0 < ((int64_t)1 << s) ? (int)(nnz - p0) : 1 << s;
+    const int rlast = piece_row[piece + 1];            // no entry of the piece lies in a later row
+    int w0 = piece_row[piece];                         // lane i holds the end of row w0 + i, counted from the piece's start
+    int end;
+    auto load_ends = [&]() {
+        const int64_t e = w0 + lane < nrows ? pos[w0 + lane + 1] - p0 : n;
+        end = e < n ? (int)e : n;
     };
-    int64_t c_next;
-    int row_next;
-    fetch(a, c_next, row_next);
-    for (int64_t base = a; base < b; base += 32) {
-        const int64_t c = c_next;
-        const int row = row_next;
-        if (base + 32 < b) fetch(base + 32, c_next, row_next);
-        const int n = (b - base) < 32 ? (int)(b - base) : 32;
-        const int steps = (n + P - 1) / P;
+    load_ends();
+    crd += p0;
+    sval += p0;
+    out += p0;
+
+    // columns, values and rows of the batch at e
+    auto fetch = [&](int e, Col &c, double &v, int &row) {
+        const int p = e + lane < n ? e + lane : n - 1;
+        c = (Col)ld_stream(crd + p);
+        v = ld_stream(sval + p);
+        bool open = true;
+        while (true) {
+            int lo = 0;                                // ends at or before p
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, end, lo + step - 1) <= p) lo += step;
+            if (__shfl_sync(0xffffffffu, end, lo) <= p) lo++;
+            if (open && lo < 32) {
+                row = w0 + lo;
+                open = false;
+            }
+            const unsigned left = __ballot_sync(0xffffffffu, open);
+            if (!left) break;
+            // the first row whose end lies behind the first entry without a row: 32 probes at a time where empty rows lie between
+            const int64_t want = p0 + __shfl_sync(0xffffffffu, p, __ffs(left) - 1);
+            int64_t a = (int64_t)w0 + 32, b = (int64_t)rlast + 1;
+            while (b - a > 32) {
+                const int64_t step = (b - a + 31) / 32, at = a + lane * step;
+                const int k = __popc(__ballot_sync(0xffffffffu, at < b && pos[at < b ? at + 1 : a] <= want));
+                if (k == 0) break;                     // row a itself
+                b = a + k * step + 1 < b ? a + k * step + 1 : b;
+                a += (k - 1) * step + 1;
+            }
+            w0 = (int)a;
+            load_ends();
+        }
+    };
+
+    Col cn;
+    double vn;
+    int rn, cur = -1;
+    V xr[NI];
+#pragma unroll
+    for (int i = 0; i < NI; i++) xr[i] = Vec<V>::zero();
+    fetch(0, cn, vn, rn);
+    for (int e = 0; e < n; e += 32) {
+        const Col c = cn;
+        const double v = vn;
+        const int row = rn;
+        if (e + 32 < n) fetch(e + 32, cn, vn, rn);
+        const int m = n - e;
         double mine = 0.0;
-#pragma unroll 2
-        for (int t = 0; t < steps; t++) {
-            const int idx = t * P + g;
-            const int64_t cc = __shfl_sync(0xffffffffu, (long long)c, idx & 31);
-            const int rr = __shfl_sync(0xffffffffu, row, idx & 31);
-            double d0 = 0.0, d1 = 0.0;
-            if (idx < n) {
-                const double2 *yr = (const double2 *)(y + cc * ldy);
-                const double2 *xp = (const double2 *)(x + (row0 + rr) * ldx);
+        if (LOOP) {
+            for (int t = 0; t < G; t++) {
+                const int idx = g * G + t;
+                const Col cc = __shfl_sync(0xffffffffu, c, idx);
+                const int rr = __shfl_sync(0xffffffffu, row, idx);
+                double d[2] = {0.0, 0.0};
+                for (int k = 0; k < kv && idx < m; k += G * NI) {
+                    V a[NI], b[NI];
 #pragma unroll
-                for (int i = 0; i < NI; i++) {
-                    if (l + i * G < k2) {
-                        const double2 yy = __ldg(yr + l + i * G);
-                        const double2 xx = __ldg(xp + l + i * G);
-                        d0 = fma(xx.x, yy.x, d0);
-                        d1 = fma(xx.y, yy.y, d1);
+                    for (int i = 0; i < NI; i++) {
+                        const bool in = l + i * G + k < kv;
+                        a[i] = in ? __ldg((const V *)(x + (uint64_t)(uint32_t)rr * ldx8) + i * G + k) : Vec<V>::zero();
+                        b[i] = in ? __ldg((const V *)(y + (uint64_t)cc * ldy8) + i * G + k) : Vec<V>::zero();
                     }
-                }
-            }
-            double d = d0 + d1;
 #pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (l == t) mine = d;
-        }
-        const int idx = l * P + g;
-        if (idx < n) out[base + idx] = ld_stream(sval + base + idx) * mine;
-    }
-}
-
-// Warps draw blocks of SDDMM_BLOCK_ROWS consecutive rows from a counter and walk each block's
-// entries as a stream; rows longer than LONG_ROW are cut out of the stream and
-// go to the chunk list.
-template <int G, int NI>
-__global__ void __launch_bounds__(SDDMM_THREADS)
-sddmm_rows_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd,
-                  const double *__restrict__ sval, const double *__restrict__ x, int64_t ldx,
-                  const double *__restrict__ y, int64_t ldy, double *__restrict__ out, int k,
-                  WorkHeader *hdr, Chunk *chunks, unsigned chunk_cap)
-{
-    const int lane = threadIdx.x & 31;
-    const int k2 = k / 2;
-    const int64_t nblocks = (nrows + SDDMM_BLOCK_ROWS - 1) / SDDMM_BLOCK_ROWS;
-    while (true) {
-        unsigned blk = 0;
-        if (lane == 0) blk = atomicAdd(&hdr->pad[0], 1u);
-        blk = __shfl_sync(0xffffffffu, blk, 0);
-        if ((int64_t)blk >= nblocks) break;
-        const int64_t row0 = (int64_t)blk * SDDMM_BLOCK_ROWS;
-        const int nr = (nrows - row0) < SDDMM_BLOCK_ROWS ? (int)(nrows - row0) : SDDMM_BLOCK_ROWS;
-        const int64_t rp = pos[row0 + (lane < nr ? lane : nr)];      // lanes past the block hold its end
-        const int64_t rnext = pos[row0 + (lane < nr ? lane + 1 : nr)];
-        const bool is_long = lane < nr && (rnext - rp) > SDDMM_LONG_ROW;
-        if (is_long) {
-            unsigned n = (unsigned)((rnext - rp + SDDMM_CHUNK - 1) / SDDMM_CHUNK);
-            unsigned at = atomicAdd(&hdr->count, n);
-            if (at + n <= chunk_cap) {
-                for (unsigned i = 0; i < n; i++) {
-                    chunks[at + i].row = row0 + lane;
-                    chunks[at + i].begin = rp + (int64_t)i * SDDMM_CHUNK;
+                    for (int i = 0; i < NI; i++) dot_to(d, a[i], b[i]);
                 }
-            } else {
-                hdr->overflow = 1;
+                double sum = d[0] + d[1];
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (l == t) mine = sum;
+            }
+        } else if (UF > 0 && __all_sync(0xffffffffu, row == __shfl_sync(0xffffffffu, row, 0))) {
+            if (row != cur)
+#pragma unroll
+                for (int i = 0; i < NI; i++)
+                    xr[i] = on[i] ? __ldg((const V *)(x + (uint64_t)(uint32_t)row * ldx8) + i * G) : Vec<V>::zero();
+            cur = row;
+            constexpr int UU = UF > 0 ? UF : 1;
+#pragma unroll 1
+            for (int t0 = 0; t0 < G; t0 += UU) {
+                V yv[UU][NI];
+#pragma unroll
+                for (int u = 0; u < UU; u++) {
+                    const int idx = g * G + t0 + u;
+                    const Col cc = __shfl_sync(0xffffffffu, c, idx);
+#pragma unroll
+                    for (int i = 0; i < NI; i++)
+                        yv[u][i] = on[i] && idx < m ? __ldg((const V *)(y + (uint64_t)cc * ldy8) + i * G) : Vec<V>::zero();
+                }
+#pragma unroll
+                for (int u = 0; u < UU; u++) {
+                    double d[2] = {0.0, 0.0};
+#pragma unroll
+                    for (int i = 0; i < NI; i++) dot_to(d, xr[i], yv[u][i]);
+                    double sum = d[0] + d[1];
+#pragma unroll
+                    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                    if (l == t0 + u) mine = sum;
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int t0 = 0; t0 < G; t0 += U) {
+                V yv[U][NI], xv[U][NI];
+                int rr[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int idx = g * G + t0 + u;
+                    const Col cc = __shfl_sync(0xffffffffu, c, idx);
+                    rr[u] = __shfl_sync(0xffffffffu, row, idx);
+#pragma unroll
+                    for (int i = 0; i < NI; i++)
+                        yv[u][i] = on[i] && idx < m ? __ldg((const V *)(y + (uint64_t)cc * ldy8) + i * G) : Vec<V>::zero();
+                    if (rr[u] != (u ? rr[u - 1] : cur))
+#pragma unroll
+                        for (int i = 0; i < NI; i++)
+                            xv[u][i] = on[i] ? __ldg((const V *)(x + (uint64_t)(uint32_t)rr[u] * ldx8) + i * G) : Vec<V>::zero();
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (rr[u] != (u ? rr[u - 1] : cur))
+#pragma unroll
+                        for (int i = 0; i < NI; i++) xr[i] = xv[u][i];
+                    double d[2] = {0.0, 0.0};
+#pragma unroll
+                    for (int i = 0; i < NI; i++) dot_to(d, xr[i], yv[u][i]);
+                    double sum = d[0] + d[1];
+#pragma unroll
+                    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                    if (l == t0 + u) mine = sum;
+                }
+                cur = rr[U - 1];
             }
         }
-        const unsigned longmask = __ballot_sync(0xffffffffu, is_long);
-        int t0 = 0;
-        while (t0 < nr) {
-            const unsigned m = longmask >> t0;
-            const int run = m ? (__ffs(m) - 1) : (nr - t0);      // rows [t0, t0 + run) hold no long row
-            if (run > 0) {
-                const int64_t a = __shfl_sync(0xffffffffu, (long long)rp, t0);
-                const int last = t0 + run - 1;
-                const int64_t b = __shfl_sync(0xffffffffu, (long long)rnext, last);
-                if (b > a) sample_stream<G, NI>(row0, rp, crd, sval, x, ldx, y, ldy, out, a, b, lane, k2);
-            }
-            t0 += run + 1;
-        }
+        if (lane < m) out[e + lane] = v * mine;
     }
 }
 
-template <int G, int NI>
-__global__ void __launch_bounds__(SDDMM_THREADS)
-sddmm_chunks_kernel(const int64_t *__restrict__ pos, const int64_t *__restrict__ crd,
-                    const double *__restrict__ sval, const double *__restrict__ x, int64_t ldx,
-                    const double *__restrict__ y, int64_t ldy, double *__restrict__ out, int k,
-                    const WorkHeader *hdr, const Chunk *chunks, unsigned chunk_cap)
-{
-    const int lane = threadIdx.x & 31;
-    const int k2 = k / 2;
-    const unsigned warp = (blockIdx.x * SDDMM_THREADS + threadIdx.x) >> 5;
-    const unsigned nwarps = (gridDim.x * SDDMM_THREADS) >> 5;
-    unsigned count = hdr->count;
-    if (count > chunk_cap) count = 0;
-    for (unsigned w = warp; w < count; w += nwarps) {
-        const Chunk ch = chunks[w];
-        int64_t cend = pos[ch.row + 1];
-        if (cend > ch.begin + SDDMM_CHUNK) cend = ch.begin + SDDMM_CHUNK;
-        double2 xr[NI];
-        load_x<G, NI>(xr, x, ldx, ch.row, lane % G, k2);
-        sample_range<G, NI>(xr, crd, sval, y, ldy, out, ch.begin, cend, lane, k2);
-    }
-}
-
-// Any K and alignment: one thread per row (correctness path).
+// Any size: one thread per row.  For operands beyond 32-bit row and column numbers or row offsets.
 __global__ void __launch_bounds__(256)
 sddmm_scalar_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd,
                     const double *__restrict__ sval, const double *__restrict__ x, int64_t ldx,
@@ -236,24 +240,63 @@ sddmm_scalar_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_
     }
 }
 
-template <int G, int NI>
-static int launch_sddmm(int64_t nrows, int64_t nnz, const int64_t *pos, const int64_t *crd,
-                        const double *sval, const double *x, int64_t ldx, const double *y,
-                        int64_t ldy, double *out, int k, WorkHeader *hdr, Chunk *chunks,
-                        unsigned cap, cudaStream_t st)
+struct SddmmCall {
+    int64_t nrows, nnz, k;
+    const int64_t *pos, *crd;
+    const double *sval, *x;
+    int64_t ldx;
+    const double *y;
+    int64_t ldy;
+    double *out;
+    cudaStream_t st;
+};
+
+template <typename V, int G, int NI, int U, int UF, int MINB, bool LOOP>
+static int launch_sddmm(const SddmmCall &a)
 {
-    int64_t grid = ceil_div(nrows, SDDMM_THREADS / 32);
-    const int64_t full = (int64_t)sm_count() * 16;
-    if (grid > full) grid = full;
-    sddmm_rows_kernel<G, NI><<<(unsigned)grid, SDDMM_THREADS, 0, st>>>(nrows, pos, crd, sval, x, ldx, y, ldy,
-                                                                     out, k, hdr, chunks, cap);
+    const int64_t warps = (int64_t)sm_count() * 32;    // about what the registers let run at a time
+    int s = 5;                                         // 2^5 to 2^8 entries a piece, the most that still give four rounds
+    while (s < 8 && a.nnz >> (s + 1) >= warps * 4) s++;
+    const int64_t npieces = ceil_div(a.nnz, (int64_t)1 << s), blocks = ceil_div(npieces, SD_THREADS / 32);
+    if (blocks > 0x7fffffffLL) return fail("sddmm: too many entries");
+    void *rows = nullptr;
+    CB_TRY(scratch(SLOT_WORKLIST, (size_t)(npieces + 1) * sizeof(int32_t), &rows));
+    int64_t grid = ceil_div(a.nrows, 256);
+    if (grid > sm_count() * 8) grid = sm_count() * 8;
+    sddmm_plan_kernel<<<(unsigned)grid, 256, 0, a.st>>>(a.nrows, s, npieces, a.pos, (int32_t *)rows);
     CB_LAUNCH_CHECK();
-    if (nnz > SDDMM_LONG_ROW) {
-        sddmm_chunks_kernel<G, NI><<<(unsigned)sm_count() * 8, SDDMM_THREADS, 0, st>>>(
-            pos, crd, sval, x, ldx, y, ldy, out, k, hdr, chunks, cap);
-        CB_LAUNCH_CHECK();
-    }
+    CB_CUDA(launch_behind(sddmm_kernel<V, G, NI, U, UF, MINB, LOOP>, dim3((unsigned)blocks), SD_THREADS, 0, a.st, a.nrows, a.nnz, s, a.pos,
+                          a.crd, a.sval, a.x, (uint32_t)(a.ldx * 8), a.y, (uint32_t)(a.ldy * 8), a.out,
+                          (int)(a.k / Vec<V>::N), (const int32_t *)rows, npieces));
     return 0;
+}
+
+// G lanes x NI vectors just cover the columns; many vectors per lane and few lanes mean fewer shuffles per entry, as long as
+// a group's loads still fill whole 128-byte lines.  U and UF (0: no path of its own for batches of one row) are entries in
+// flight, MINB the CTAs per SM that the registers are limited for; taken from sweeps over R-MAT graphs of scale 14, 17 and
+// 20, 400,000 rows of 8 and ragged rectangles.  Microseconds, R-MAT scale 20 / scale 14 / 400,000 rows of 8, with the lane
+// group per 32 entries of short rows and chunk list for the others (even K) or the thread per row (odd K) before:
+//   K = 4   331 28 66 -> 199 14 34    K = 16  ...  29 95 -> 334 15 82      K = 13  53290 1549 ... -> 372 15 80
+//   K = 64  852 .. 320 -> 808 19 259  K = 128 1551 .. 589 -> 1406 25 535   K = 127 430553 11377 2469 -> 1846 27 625
+template <typename V>
+static int dispatch_sddmm(const SddmmCall &a)
+{
+    const int64_t kv = a.k / Vec<V>::N;
+    constexpr bool pairs = Vec<V>::N == 2;
+    if (kv <= 1) return launch_sddmm<V, 1, 2, 1, 0, 1, false>(a);
+    if (kv <= 2) return launch_sddmm<V, 2, 1, 2, 2, 1, false>(a);
+    if (kv <= 4) return launch_sddmm<V, 2, 2, 2, 0, 1, false>(a);
+    if (kv <= 8) return pairs ? launch_sddmm<V, 4, 2, 1, 2, 4, false>(a) : launch_sddmm<V, 4, 2, 2, 2, 1, false>(a);
+    if (kv <= (pairs ? 12 : 16)) return launch_sddmm<V, 4, 4, 1, 1, 1, false>(a);
+    if (kv <= 16) return launch_sddmm<V, 8, 2, 1, 2, 4, false>(a);
+    if (kv <= 32) return pairs ? launch_sddmm<V, 8, 4, 1, 1, 1, false>(a) : launch_sddmm<V, 8, 4, 2, 2, 4, false>(a);
+    if (kv <= 48) return pairs ? launch_sddmm<V, 16, 3, 1, 1, 1, false>(a) : launch_sddmm<V, 16, 3, 2, 2, 4, false>(a);
+    if (kv <= 64) return launch_sddmm<V, 16, 4, 1, 2, 3, false>(a);
+    if (!pairs && kv <= 96) return launch_sddmm<V, 32, 3, 2, 2, 4, false>(a);
+    if (kv <= 128) return pairs ? launch_sddmm<V, 32, 4, 2, 2, 1, false>(a) : launch_sddmm<V, 32, 4, 1, 2, 3, false>(a);
+    if (kv <= 192) return launch_sddmm<V, 32, 6, 1, 1, 1, false>(a);
+    if (kv <= 256) return launch_sddmm<V, 32, 8, 1, 1, 1, false>(a);
+    return launch_sddmm<V, 32, 4, 1, 0, 1, true>(a);
 }
 
 int sddmm_csr(int64_t nrows, int64_t nnz, int64_t k, const int64_t *pos, const int64_t *crd,
@@ -261,28 +304,16 @@ int sddmm_csr(int64_t nrows, int64_t nnz, int64_t k, const int64_t *pos, const i
               double *out, cudaStream_t st)
 {
     if (nrows <= 0 || nnz <= 0) return 0;
-    bool vec_ok = k > 0 && k % 2 == 0 && k <= 256 && ldx % 2 == 0 && ldy % 2 == 0 &&
-                  ((((uintptr_t)x | (uintptr_t)y) & 15) == 0);
-    if (!vec_ok) {
+    if (k <= 0 || k > (1 << 24) || nrows >= 0x7fffffe0LL || ldx >= (1LL << 29) || ldy >= (1LL << 29)) {
         int64_t blocks = ceil_div(nrows, 256);
+        if (blocks > 0x7fffffffLL) blocks = 0x7fffffffLL;
         sddmm_scalar_kernel<<<(unsigned)blocks, 256, 0, st>>>(nrows, pos, crd, sval, x, ldx, y, ldy, out, k);
         CB_LAUNCH_CHECK();
         return 0;
     }
-    size_t cap = (size_t)(nnz / SDDMM_CHUNK + nnz / SDDMM_LONG_ROW + 16);
-    void *wl = nullptr;
-    CB_TRY(scratch(SLOT_WORKLIST, sizeof(WorkHeader) + cap * sizeof(Chunk), &wl));
-    WorkHeader *hdr = (WorkHeader *)wl;
-    Chunk *chunks = (Chunk *)((char *)wl + sizeof(WorkHeader));
-    CB_CUDA(cudaMemsetAsync(hdr, 0, sizeof(WorkHeader), st));
-#define GO(GG, NN) return launch_sddmm<GG, NN>(nrows, nnz, pos, crd, sval, x, ldx, y, ldy, out, (int)k, hdr, chunks, (unsigned)cap, st)
-    if (k <= 8) GO(1, 4);
-    if (k <= 16) GO(2, 4);
-    if (k <= 32) GO(4, 4);
-    if (k <= 64) GO(8, 4);
-    if (k <= 128) GO(16, 4);
-    GO(32, 4);
-#undef GO
+    const SddmmCall a = {nrows, nnz, k, pos, crd, sval, x, ldx, y, ldy, out, st};
+    const bool vec = k % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+    return vec ? dispatch_sddmm<double2>(a) : dispatch_sddmm<double>(a);
 }
 
 }  // namespace cb200
