@@ -1,18 +1,26 @@
 // SpMV  y[a] = y[a] (+) sum_b A[a,b] (x) x[b]   (CSR / DCSR rows, f64 values, i64 indices).
 //
 // A group of T lanes (T chosen from the mean row length) walks one row with
-// 128-bit loads of crd and val (two entries per load).
-// Small matrices (< 2^20 stored entries): one launch, no scratch memory; rows
-// longer than LONG_ROW entries are left to the end of the CTA, where all 256
-// threads walk each of them together; the summation order per row is fixed.
-// Larger matrices: rows longer than DEFER_ROW entries are cut into chunks that
+// 128-bit loads of crd and val (two entries per load), the next row's pointers on their way.
+//
+// Up to 2^18 stored entries: one launch, no scratch memory; rows of more than 16 T entries are left to the end of the CTA,
+// where a warp, or for very long ones all 256 threads, walk them; the summation order per row is fixed.
+// From 2^20 on: rows longer than DEFER_ROW entries are cut into chunks that
 // go to a work list in scratch memory, and a second launch gives each chunk to
 // a warp that adds its partial sum to y with one f64 atomic -- on a power-law
 // matrix the long rows sit next to each other and would otherwise all land in
 // the first few CTAs.
+// Between: equal tiles of A's path.  A power-law matrix of this size has its hub rows in a CTA or two, which one launch
+// waits for, and too few others to hide a list and its launches.  Microseconds, one launch / list / tiles:
+//   even rows: 262,144 entries 5.5 / 9 / 9    600,000 8.2 / 12 / 10.5    3.2 M 26 / 25 / 29    36 M 201 / 182 / 232
+//   R-MAT:     120,000 entries 18 / -  / 7.6  728,000 84 / 25 / 12       3 M 500 / 43 / 28     16 M 1150 / 133 / 107
+// The tiles would take large power-law matrices too, but nothing known at the launch tells those from large even ones.
 //
-// Bound: HBM.  Algorithmic bytes per call = 8(n+1) + 16 nnz + 8 ncols + 8 nrows.
+// Bound: HBM, 8(n+1) + 16 nnz + 8 ncols + 8 nrows bytes per call, and the L1's rate for the gathered x, one line per entry
+// (57 us at one line a clock for 16 M entries of a power-law matrix).  Row pointers fetched a row ahead: R-MAT scale 20
+// 146 -> 133 us, 36 M entries in even rows 202 -> 182.
 #include "common.cuh"
+#include "stream.cuh"
 
 namespace cb200 {
 
@@ -22,6 +30,8 @@ static const int64_t LONG_ROW = 2048;
 static const int64_t DEFER_ROW = 64;       // with a work list: rows above this go to it
 static const int64_t SPMV_CHUNK = 256;     // entries per work-list chunk
 static const int64_t DEFER_MIN_NNZ = 1 << 20;
+static const int64_t TILES_MIN_NNZ = (1 << 18) + 1;
+static const int TILE_ITEMS = 8;           // steps per thread of a tile's CTA: 2^11 per tile
 
 template <bool PAIR>
 __device__ __forceinline__ double combine(double a, double b)
@@ -68,44 +78,30 @@ spmv_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *_
     constexpr int ROWS = GROUPS * SPMV_PASSES;
     __shared__ int64_t long_rows[ROWS];
     __shared__ int n_long;
+    __shared__ unsigned n_chunks, first[ROWS];
     __shared__ double warp_part[SPMV_THREADS / 32];
 
     const int g = threadIdx.x / T, l = threadIdx.x % T;
     const int lane = threadIdx.x & 31;
     const unsigned gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << (lane & ~(T - 1)));
-    if (threadIdx.x == 0) n_long = 0;
+    if (threadIdx.x == 0) n_long = n_chunks = 0;
     // Programmatic dependent launch: when the launch carries that attribute this grid may be set up while the
     // kernel before it in the stream is still running; nothing that kernel may have written (x, y, even A) is
     // touched before the wait, and the next kernel in the stream is allowed to set up from here on.  Without
     // the attribute both instructions do nothing.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_for_previous();
+    let_next_start();
     __syncthreads();
 
     const int64_t row0 = (int64_t)blockIdx.x * (GROUPS * passes);
+    int64_t s1 = 0, e1 = 0;
+    if (row0 + g < nrows) { s1 = pos[row0 + g]; e1 = pos[row0 + g + 1]; }
     for (int pass = 0; pass < passes; pass++) {
         int64_t r = row0 + pass * GROUPS + g;
         if (r >= nrows) break;
-        int64_t s = pos[r], e = pos[r + 1];
-        if (hdr && e - s > DEFER_ROW) {
-            if (l == 0) {
-                const unsigned n = (unsigned)((e - s + SPMV_CHUNK - 1) / SPMV_CHUNK);
-                const unsigned at = atomicAdd(&hdr->count, n);
-                if (at + n <= chunk_cap) {
-                    for (unsigned i = 0; i < n; i++) {
-                        chunks[at + i].row = r;
-                        chunks[at + i].begin = s + (int64_t)i * SPMV_CHUNK;
-                    }
-                    if (!accumulate) y[row_ids ? row_ids[r] : r] = 0.0;     // the chunks add into it
-                    continue;
-                }
-                hdr->overflow = 1;
-            }
-            // all lanes of the group must agree: the list cannot overflow (its capacity is a bound),
-            // so a deferred row is always skipped here
-            continue;
-        }
-        if (e - s > LONG_ROW) {
+        const int64_t s = s1, e = e1;
+        if (pass + 1 < passes && r + GROUPS < nrows) { s1 = pos[r + GROUPS]; e1 = pos[r + GROUPS + 1]; }   // on their way meanwhile
+        if (e - s > (hdr ? DEFER_ROW : T * 16)) {      // left to the end of the CTA, or to the chunks' kernel
             if (l == 0) long_rows[atomicAdd(&n_long, 1)] = r;
             continue;
         }
@@ -119,8 +115,42 @@ spmv_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *_
     }
     __syncthreads();
     const int nl = n_long;
+    if (hdr) {
+        // chunks of the CTA's long rows: room for all of them is taken at once (a counter that 50,000 rows went to one by
+        // one took 60 us), a warp writes a row's
+        for (int i = threadIdx.x; i < nl; i += SPMV_THREADS) {
+            const int64_t r = long_rows[i];
+            first[i] = atomicAdd(&n_chunks, (unsigned)((pos[r + 1] - pos[r] + SPMV_CHUNK - 1) / SPMV_CHUNK));
+            if (!accumulate) y[row_ids ? row_ids[r] : r] = 0.0;         // the chunks add into it
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && nl) n_chunks = atomicAdd(&hdr->count, n_chunks);
+        __syncthreads();
+        for (int i = threadIdx.x >> 5; i < nl; i += SPMV_THREADS / 32) {
+            const int64_t r = long_rows[i], s = pos[r], n = (pos[r + 1] - s + SPMV_CHUNK - 1) / SPMV_CHUNK;
+            const unsigned at = n_chunks + first[i];
+            if (at + n > chunk_cap) continue;          // cannot be: its capacity is a bound
+            for (int64_t k = lane; k < n; k += 32) {
+                chunks[at + k].row = r;
+                chunks[at + k].begin = s + k * SPMV_CHUNK;
+            }
+        }
+        return;
+    }
+    for (int i = threadIdx.x >> 5; i < nl; i += SPMV_THREADS / 32) {
+        const int64_t r = long_rows[i], s = pos[r], e = pos[r + 1];
+        if (e - s > LONG_ROW) continue;
+        double sum = row_partial<PAIR, VEC>(crd, val, x, s, e, lane, 32);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) {
+            const int64_t out = row_ids ? row_ids[r] : r;
+            y[out] = accumulate ? y[out] + sum : sum;
+        }
+    }
     for (int i = 0; i < nl; i++) {
         int64_t r = long_rows[i];
+        if (pos[r + 1] - pos[r] <= LONG_ROW) continue;
         double sum = row_partial<PAIR, VEC>(crd, val, x, pos[r], pos[r + 1], threadIdx.x, SPMV_THREADS);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -136,6 +166,111 @@ spmv_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *_
     }
 }
 
+// Equal tiles of A's path (one step per stored entry and one per row end), a CTA each.  The products of a tile's entries are
+// made with all loads in flight and put into shared memory; every thread then walks eight steps of the merged list of
+// entries and row ends, and sums of rows that reach over threads travel by a segmented scan.  A row cut by a tile boundary
+// is added with atomics onto a zero written by the plan.
+//
+// Bound: at the sizes it is used for, the latency of plan, entries and gathers (6 us) and then the L1's rate of line
+// accesses.  R-MAT scale 16, 728,000 entries: 86 -> 12 us.
+template <bool PAIR>
+__global__ void __launch_bounds__(SPMV_THREADS, 4)
+spmv_tiles_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
+                  const int64_t *__restrict__ crd, const double *__restrict__ val, const double *__restrict__ x,
+                  double *__restrict__ y, int accumulate, const int64_t *__restrict__ tile_row,
+                  const int64_t *__restrict__ tile_ent)
+{
+    constexpr int ITEMS = TILE_ITEMS, STEPS = SPMV_THREADS * ITEMS;
+    __shared__ double prod[STEPS + STEPS / ITEMS];     // entry i at i + i / ITEMS: a thread's run of ITEMS hits every bank once
+    __shared__ int ends[STEPS + 2];                    // ends of the rows that end in the tile, counted from its first entry
+    __shared__ double warp_sum[SPMV_THREADS / 32];
+    __shared__ int warp_end[SPMV_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    wait_for_previous();
+    const int64_t r0 = tile_row[blockIdx.x], e0 = tile_ent[blockIdx.x];
+    const int m = (int)(tile_row[blockIdx.x + 1] - r0), n = (int)(tile_ent[blockIdx.x + 1] - e0);
+
+    int64_t c[ITEMS];
+    double v[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        const int p = tid + i * SPMV_THREADS;
+        c[i] = 0;
+        v[i] = 0.0;
+        if (p < n) {
+            if (!PAIR) c[i] = ld_stream(crd + e0 + p);
+            v[i] = PAIR ? 1.0 : ld_stream(val + e0 + p);
+        }
+    }
+    for (int a = tid; a < m; a += SPMV_THREADS) ends[a] = (int)(pos[r0 + a + 1] - e0);
+    const bool cut = r0 < nrows && pos[r0] < e0;       // the first row starts in an earlier tile
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        const int p = tid + i * SPMV_THREADS;
+        if (p < n) prod[p + p / ITEMS] = PAIR ? 1.0 : v[i] * __ldg(x + c[i]);
+    }
+    __syncthreads();
+
+    // where this thread's steps start: after `a` row ends and `e` entries
+    const int d = tid * ITEMS < n + m ? tid * ITEMS : n + m;
+    const int last = tid == SPMV_THREADS - 1 || d + ITEMS > n + m ? n + m : d + ITEMS;
+    int lo = d > n ? d - n : 0, hi = d < m ? d : m;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ends[mid] <= d - 1 - mid) lo = mid + 1;
+        else hi = mid;
+    }
+    int a = lo, e = d - lo;
+    const int a0 = a;
+    double acc = 0.0, head = 0.0;                      // head: what this thread adds to the first row that ends here
+    auto store = [&](int64_t r, double sum, bool add) {
+        double *at = y + (row_ids ? row_ids[r] : r);
+        if (add) atomicAdd(at, sum);
+        else *at = accumulate ? *at + sum : sum;
+    };
+    int next = a < m ? ends[a] : n + 1;
+    for (int t = d; t < last; t++) {
+        if (e < next) {
+            acc += prod[e + e / ITEMS];
+            e++;
+        } else {
+            if (a == a0) head = acc;
+            else store(r0 + a, acc, false);
+            acc = 0.0;
+            a++;
+            next = a < m ? ends[a] : n + 1;
+        }
+    }
+    // sums of unfinished rows travel to the thread in which the row ends
+    const bool has = a > a0;
+    double sum = acc;
+    bool stop = has;                                   // the sum starts in this thread
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double up = __shfl_up_sync(0xffffffffu, sum, o);
+        const bool ups = __shfl_up_sync(0xffffffffu, (int)stop, o);
+        if (lane >= o && !stop) {
+            sum += up;
+            stop = ups;
+        }
+    }
+    if (lane == 31) {
+        warp_sum[warp] = sum;
+        warp_end[warp] = stop;
+    }
+    double in = __shfl_up_sync(0xffffffffu, sum, 1);
+    bool in_stop = __shfl_up_sync(0xffffffffu, (int)stop, 1);
+    if (lane == 0) { in = 0.0; in_stop = false; }
+    __syncthreads();
+    if (!in_stop)
+        for (int w = warp - 1; w >= 0; w--) {
+            in += warp_sum[w];
+            if (warp_end[w]) break;
+        }
+    if (has) store(r0 + a0, in + head, a0 == 0 && cut);
+    if (tid == SPMV_THREADS - 1 && r0 + m < nrows && e0 + n > pos[r0 + m]) store(r0 + m, has ? acc : in + acc, true);
+}
+
 template <bool PAIR, bool VEC>
 __global__ void __launch_bounds__(SPMV_THREADS)
 spmv_chunks_kernel(const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
@@ -146,6 +281,7 @@ spmv_chunks_kernel(const int64_t *__restrict__ row_ids, const int64_t *__restric
     const int lane = threadIdx.x & 31;
     const unsigned warp = (blockIdx.x * SPMV_THREADS + threadIdx.x) >> 5;
     const unsigned nwarps = (gridDim.x * SPMV_THREADS) >> 5;
+    wait_for_previous();
     unsigned count = hdr->count;
     if (count > chunk_cap) count = 0;
     for (unsigned w = warp; w < count; w += nwarps) {
@@ -204,7 +340,7 @@ static int launch_spmv(int64_t nrows, const int64_t *row_ids, const int64_t *pos
     CB_LAUNCH_CHECK();
     if (hdr) {
         const unsigned g2 = (unsigned)sm_count() * 8;
-#define GO2(P, V) spmv_chunks_kernel<P, V><<<g2, SPMV_THREADS, 0, st>>>(row_ids, pos, crd, val, x, y, hdr, chunks, (unsigned)cap)
+#define GO2(P, V) CB_CUDA(launch_behind(spmv_chunks_kernel<P, V>, dim3(g2), SPMV_THREADS, 0, st, row_ids, pos, crd, val, x, y, hdr, chunks, (unsigned)cap))
         if (pair) { if (vec) GO2(true, true); else GO2(true, false); }
         else      { if (vec) GO2(false, true); else GO2(false, false); }
 #undef GO2
@@ -221,15 +357,27 @@ int spmv_rows(int64_t nrows, int64_t nnz, const int64_t *row_ids, const int64_t 
     bool vec = (((uintptr_t)crd | (uintptr_t)val) & 15) == 0;
     bool pair = semiring == COMET_B200_PLUS_PAIR;
     double mean = (double)nnz / (double)nrows;
-    if (const char *env = getenv("COMET_B200_SPMV_LANES")) {        // tuning knob: lanes per row
-        const int t = atoi(env);
-        if (t == 2) mean = 4.0; else if (t == 4) mean = 8.0; else if (t == 8) mean = 24.0;
-        else if (t == 16) mean = 48.0; else if (t == 32) mean = 1e9;
+    int t = mean <= 4.0 ? 2 : mean <= 8.0 ? 4 : mean <= 24.0 ? 8 : mean <= 48.0 ? 16 : 32;
+    if (nnz < TILES_MIN_NNZ) {
+        // lanes that would idle otherwise shorten the longest rows (R-MAT scale 14: 28 -> 18 us)
+        while (t < 32 && nrows * t * 2 <= (int64_t)sm_count() * 2048) t *= 2;
     }
-    if (mean <= 4.0) return launch_spmv<2>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
-    if (mean <= 8.0) return launch_spmv<4>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
-    if (mean <= 24.0) return launch_spmv<8>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
-    if (mean <= 48.0) return launch_spmv<16>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
+    if (const char *env = getenv("COMET_B200_SPMV_LANES")) {        // tuning knob: lanes per row
+        const int want = atoi(env);
+        if (want == 2 || want == 4 || want == 8 || want == 16 || want == 32) t = want;
+    } else if (nnz >= TILES_MIN_NNZ && nnz < DEFER_MIN_NNZ) {
+        StreamPlan plan;
+        static_assert(SPMV_THREADS * TILE_ITEMS == 1 << 11, "steps per tile");
+        CB_TRY(piece_plan(nrows, nnz, 11, row_ids, pos, y, 1, 1, accumulate, LongRows{nullptr, 0}, st, &plan));
+        if (plan.nblocks > 0x7fffffffLL) return fail("spmv: too many rows");
+        CB_CUDA(launch_behind(pair ? spmv_tiles_kernel<true> : spmv_tiles_kernel<false>, dim3((unsigned)plan.nblocks),
+                              SPMV_THREADS, 0, st, nrows, row_ids, pos, crd, val, x, y, accumulate, plan.block_row, plan.block_ent));
+        return 0;
+    }
+    if (t == 2) return launch_spmv<2>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
+    if (t == 4) return launch_spmv<4>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
+    if (t == 8) return launch_spmv<8>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
+    if (t == 16) return launch_spmv<16>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
     return launch_spmv<32>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
 }
 
