@@ -28,6 +28,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "stream.cuh"
 #include "hostcopy.cuh"
 #include "masked.cuh"
 #include "semiring.cuh"
@@ -118,30 +119,45 @@ __device__ __forceinline__ bool in_mask(const int64_t *__restrict__ mcrd, int64_
 }
 
 // --------------------------------------------------------------------------
-// Binning: 8 lanes per row sum the lengths of the B rows it touches.
+// Binning: 8 lanes per row sum the lengths of the B rows it touches, 32 of them at a time, and stop when the sum has left
+// bin 1: a row's bin does not depend on more, and the hub rows of a power-law matrix leave it at once (R-MAT scale 13, 59,000
+// entries: 82 -> 6 us; scale 16 125 -> 9).  The CTAs behind those of the rows copy B's columns as 32-bit numbers.
 // --------------------------------------------------------------------------
 static const int BIN_THREADS = 256;
-static const int BIN_ROWS = (BIN_THREADS / 8) * 4;
+static const int BIN_PASS = BIN_THREADS / 8;            // rows at a time
+static const int BIN_ROWS = BIN_PASS * 4;
 static const int64_t BIN_LONG_ROW = 1024;
+static const int64_t NARROW_PART = 4096;                // entries per CTA
 
 __global__ void __launch_bounds__(BIN_THREADS)
-bin_rows_kernel(int64_t nrows, const int64_t *__restrict__ apos, const int64_t *__restrict__ acrd,
+bin_rows_kernel(int64_t nrows, int passes, unsigned row_ctas, const int64_t *__restrict__ apos, const int64_t *__restrict__ acrd,
                 const int64_t *__restrict__ bpos, const int64_t *__restrict__ mpos,
                 int64_t *__restrict__ cnt, int32_t *__restrict__ list1, int32_t *__restrict__ list2,
-                unsigned *__restrict__ bin_counts)
+                unsigned *__restrict__ bin_counts, const int64_t *__restrict__ bcrd, int32_t *__restrict__ bcrd32, int64_t nnz_b)
 {
+    if (blockIdx.x >= row_ctas) {
+        const int64_t first = (int64_t)(blockIdx.x - row_ctas) * NARROW_PART;
+        for (int64_t q = first + 2 * threadIdx.x; q < first + NARROW_PART && q < nnz_b; q += 2 * BIN_THREADS) {
+            if (q + 1 < nnz_b) {
+                const longlong2 c = __ldcs((const longlong2 *)(bcrd + q));
+                *(int2 *)(bcrd32 + q) = make_int2((int)c.x, (int)c.y);
+            } else {
+                bcrd32[q] = (int32_t)bcrd[q];
+            }
+        }
+        return;
+    }
     __shared__ unsigned char bin_of[BIN_ROWS];
     __shared__ unsigned short local_at[BIN_ROWS];
     __shared__ unsigned local_cnt[2], base[2], n_long;
     __shared__ unsigned short long_slot[BIN_ROWS];
-    __shared__ int64_t warp_sum[BIN_THREADS / 32];
     const int g = threadIdx.x / 8, l = threadIdx.x % 8;
     const unsigned gmask = 0xffu << ((threadIdx.x & 31) & ~7);
     if (threadIdx.x < 2) local_cnt[threadIdx.x] = 0;
     if (threadIdx.x == 2) n_long = 0;
     __syncthreads();
-    const int64_t row0 = (int64_t)blockIdx.x * BIN_ROWS;
-    // the bin of a row from the upper bound ub of its distinct columns
+    const int64_t row0 = (int64_t)blockIdx.x * (BIN_PASS * passes);
+    // the bin of a row from ub: its products, or more than HASH_ROW_MAX if it has more
     auto place = [&](int slot, int64_t r, int64_t ub) {
         if (mpos) {
             int64_t ml = mpos[r + 1] - mpos[r];
@@ -152,57 +168,82 @@ bin_rows_kernel(int64_t nrows, const int64_t *__restrict__ apos, const int64_t *
         if (b == 0) cnt[r] = 0;
         else local_at[slot] = (unsigned short)atomicAdd(&local_cnt[b - 1], 1u);
     };
-    for (int pass = 0; pass < 4; pass++) {
-        int slot = pass * (BIN_THREADS / 8) + g;
-        int64_t r = row0 + slot;
+    // lengths of the rows of B of entries p, p + lanes, ... (four of them) before `end`
+    auto four = [&](int64_t p, int64_t end, int lanes) {
+        int64_t k[4], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) k[i] = p + i * lanes < end ? acrd[p + i * lanes] : -1;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (k[i] >= 0) sum += bpos[k[i] + 1] - bpos[k[i]];
+        return sum;
+    };
+    for (int pass = 0; pass < passes; pass++) {
+        const int slot = pass * BIN_PASS + g;
+        const int64_t r = row0 + slot;
         if (r >= nrows) break;
         const int64_t as = apos[r], ae = apos[r + 1];
-        if (ae - as > BIN_LONG_ROW) {                    // a hub row: left to the whole CTA below
-            if (l == 0) long_slot[atomicAdd(&n_long, 1u)] = (unsigned short)slot;
-            continue;
-        }
         int64_t ub = 0;
-        for (int64_t p = as + l; p < ae; p += 8) {
-            int64_t k = acrd[p];
-            ub += bpos[k + 1] - bpos[k];
-        }
+        bool later = false;
+        for (int64_t p = as; p < ae; p += 32) {
+            if (p - as >= 64 && ae - p > BIN_LONG_ROW) {       // many entries and hardly a product: left to the whole CTA below
+                later = true;
+                break;
+            }
+            int64_t part = four(p + l, ae, 8);
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) ub += __shfl_xor_sync(gmask, (long long)ub, o, 8);
-        if (l == 0) place(slot, r, ub);
+            for (int o = 4; o > 0; o >>= 1) part += __shfl_xor_sync(gmask, (long long)part, o, 8);
+            ub += part;
+            if (ub > HASH_ROW_MAX) break;
+        }
+        if (l == 0) {
+            if (later) long_slot[atomicAdd(&n_long, 1u)] = (unsigned short)slot;
+            else place(slot, r, ub);
+        }
     }
     __syncthreads();
-    // rows of A with thousands of entries: eight lanes would walk them for a millisecond while the rest of
-    // the grid has finished
     const unsigned nl = n_long;
     for (unsigned i = 0; i < nl; i++) {
         const int slot = long_slot[i];
-        const int64_t r = row0 + slot;
+        const int64_t r = row0 + slot, ae = apos[r + 1];
         int64_t ub = 0;
-        for (int64_t p = apos[r] + threadIdx.x; p < apos[r + 1]; p += BIN_THREADS) {
-            int64_t k = acrd[p];
-            ub += bpos[k + 1] - bpos[k];
+        bool over = false;
+        for (int64_t p = apos[r]; p < ae && !over; p += 4 * BIN_THREADS) {
+            ub += four(p + threadIdx.x, ae, BIN_THREADS);
+            over = __syncthreads_or(ub > HASH_ROW_MAX);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ub += __shfl_xor_sync(0xffffffffu, (long long)ub, o);
-        if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = ub;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int64_t t = 0;
-            for (int w = 0; w < BIN_THREADS / 32; w++) t += warp_sum[w];
-            place(slot, r, t);
+        // without a thread over the limit, the sum of all: no more than 256 * HASH_ROW_MAX
+        int64_t total = over ? HASH_ROW_MAX + 1 : 0;
+        if (!over) {
+            __shared__ unsigned sum;
+            if (threadIdx.x == 0) sum = 0;
+            __syncthreads();
+            if (ub) atomicAdd(&sum, (unsigned)ub);
+            __syncthreads();
+            total = sum;
         }
+        if (threadIdx.x == 0) place(slot, r, total);
         __syncthreads();
     }
     __syncthreads();
-    if (threadIdx.x < 2) base[threadIdx.x] = atomicAdd(&bin_counts[threadIdx.x], local_cnt[threadIdx.x]);
+    if (threadIdx.x < 2 && local_cnt[threadIdx.x]) base[threadIdx.x] = atomicAdd(&bin_counts[threadIdx.x], local_cnt[threadIdx.x]);
     __syncthreads();
-    for (int slot = threadIdx.x; slot < BIN_ROWS; slot += BIN_THREADS) {
+    for (int slot = threadIdx.x; slot < BIN_PASS * passes; slot += BIN_THREADS) {
         int64_t r = row0 + slot;
         if (r >= nrows) break;
         int b = bin_of[slot];
         if (b == 1) list1[base[0] + local_at[slot]] = (int32_t)r;
         else if (b == 2) list2[base[1] + local_at[slot]] = (int32_t)r;
     }
+}
+
+// What the host waits for, written straight to its page-locked words (three copies cost 5 us more).
+__global__ void publish_kernel(const unsigned *__restrict__ bin_counts, const int64_t *__restrict__ nnz, unsigned *host)
+{
+    wait_for_previous();
+    host[0] = bin_counts[0];
+    host[1] = bin_counts[1];
+    if (nnz) *(int64_t *)(host + 2) = *nnz;
 }
 
 // --------------------------------------------------------------------------
@@ -331,6 +372,7 @@ hash_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restri
     if (NUMERIC)
         for (int s = lane; s < HASH_ROW_MAX; s += 32) vals[s] = ident;
     __syncwarp();
+    wait_for_previous();
     const unsigned nwarps = gridDim.x * HASH_WARPS, nlist = *nlist_dev;
     for (unsigned it = blockIdx.x * HASH_WARPS + w; it < nlist; it += nwarps) {
         const int64_t r = list[it];
@@ -449,6 +491,7 @@ short_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restr
     Word *list = s_list[w];
     double *vals = s_vals[w];
     unsigned short *head = s_head[w];
+    wait_for_previous();
     const unsigned nwarps = gridDim.x * HASH_WARPS, nlist = *nlist_dev;
     for (unsigned it = blockIdx.x * HASH_WARPS + w; it < nlist; it += nwarps) {
         const int64_t r = rows[it];
@@ -682,6 +725,7 @@ bitmap_symbolic_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__
     __shared__ int s_long[LONG_LIST];
     __shared__ unsigned s_ctl[2];
     uint32_t *bm = SMEM ? s_dyn : gbm + (size_t)blockIdx.x * words;
+    wait_for_previous();
     const unsigned nlist = *nlist_dev;
     for (unsigned it = blockIdx.x; it < nlist; it += gridDim.x) {
         const int64_t r = list[it];
@@ -762,6 +806,7 @@ team_clear_kernel(const TeamHeader *th, const uint64_t *__restrict__ items, unsi
                   const int32_t *__restrict__ list, const int64_t *__restrict__ cpos, int semi,
                   double *__restrict__ cval)
 {
+    wait_for_previous();
     unsigned n = th->nitems;
     if (n > cap) n = 0;
     const double ident = sr_identity(semi);
@@ -800,6 +845,7 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
     uint32_t *pre = bm + words;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NW = BM_THREADS / 32;
+    wait_for_previous();
     for (unsigned iter = blockIdx.x;; iter += gridDim.x) {
         // one row per CTA, or (with an item list) the next member of a team
         unsigned it = iter, part = 0, team = 1;
@@ -1012,10 +1058,13 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     p->list1 = (int32_t *)(mem + 256 + b_cnt + b_crd);
     p->list2 = (int32_t *)((char *)p->list1 + b_list);
     STEP_CUDA(cudaMemsetAsync(p->bin_counts, 0, 2 * sizeof(unsigned), st));
-    STEP(narrow_i64_to_i32(bcrd, p->bcrd32, nnz_b, st));
-    if (!rc && nrows > 0) {
-        bin_rows_kernel<<<(unsigned)ceil_div(nrows, BIN_ROWS), BIN_THREADS, 0, st>>>(
-            nrows, apos, acrd, bpos, mpos, p->cnt, p->list1, p->list2, p->bin_counts);
+    if (!rc && nrows + nnz_b > 0) {
+        const int passes = nrows >= (int64_t)sm_count() * 8 * BIN_ROWS ? 4 : 1;
+        const int64_t row_ctas = ceil_div(nrows, (int64_t)BIN_PASS * passes), ctas = row_ctas + ceil_div(nnz_b, NARROW_PART);
+        if (ctas > 0x7fffffffLL) rc = fail("spgemm: too many entries");
+        if (!rc)
+            bin_rows_kernel<<<(unsigned)ctas, BIN_THREADS, 0, st>>>(nrows, passes, (unsigned)row_ctas, apos, acrd, bpos, mpos, p->cnt,
+                                                                   p->list1, p->list2, p->bin_counts, bcrd, p->bcrd32, nnz_b);
         STEP_CUDA(cudaGetLastError());
     }
     PinnedWords words;
@@ -1025,7 +1074,7 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     // synchronisation, unless bitmaps for every row are small change (then the kernels read the bin sizes themselves).
     p->n1 = p->n2 = (unsigned)nrows;
     if ((size_t)nrows * p->words * 4 > BM_STORE_SMALL) {
-        STEP_CUDA(cudaMemcpyAsync(counts, p->bin_counts, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        STEP_CUDA(launch_behind(publish_kernel, dim3(1), 1, 0, st, p->bin_counts, nullptr, counts));
         STEP_CUDA(cudaStreamSynchronize(st));
         if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; }
     }
@@ -1033,10 +1082,8 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
         unsigned grid = (unsigned)ceil_div(p->n1, HASH_WARPS);
         unsigned cap = (unsigned)sm_count() * 16;
         if (grid > cap) grid = cap;
-        hash_rows_kernel<false, false><<<grid, HASH_WARPS * 32, 0, st>>>(
-            p->bin_counts, p->list1, apos, acrd, aval, bpos, p->bcrd32, bval, mpos, p->mcrd, p->semi, p->cnt,
-            nullptr, nullptr, nullptr);
-        STEP_CUDA(cudaGetLastError());
+        STEP_CUDA(launch_behind(hash_rows_kernel<false, false>, dim3(grid), HASH_WARPS * 32, 0, st, p->bin_counts, p->list1, apos, acrd,
+                                aval, bpos, p->bcrd32, bval, mpos, p->mcrd, p->semi, p->cnt, nullptr, nullptr, nullptr));
     }
     if (!rc && p->n2) {
         size_t store = (size_t)p->n2 * p->words * sizeof(uint32_t);
@@ -1053,10 +1100,8 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
             int grid = bitmap_grid(p->n2, smem);
             STEP_CUDA(cudaFuncSetAttribute(bitmap_symbolic_kernel<true>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            if (!rc)
-                bitmap_symbolic_kernel<true><<<grid, BM_THREADS, smem, st>>>(
-                    p->bin_counts + 1, p->list2, p->words, nullptr, apos, acrd, bpos, p->bcrd32, mpos, p->mcrd,
-                    p->cnt, p->bm_store);
+            STEP_CUDA(launch_behind(bitmap_symbolic_kernel<true>, dim3(grid), BM_THREADS, smem, st, p->bin_counts + 1, p->list2,
+                                    p->words, nullptr, apos, acrd, bpos, p->bcrd32, mpos, p->mcrd, p->cnt, p->bm_store));
         } else {
             int grid = bitmap_grid(p->n2, 0);
             void *gbm = nullptr;
@@ -1069,8 +1114,7 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
         STEP_CUDA(cudaGetLastError());
     }
     STEP(exclusive_scan_i64(p->cnt, cpos, nrows, st));
-    STEP_CUDA(cudaMemcpyAsync(counts, p->bin_counts, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    STEP_CUDA(cudaMemcpyAsync(counts + 2, cpos + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    STEP_CUDA(launch_behind(publish_kernel, dim3(1), 1, 0, st, p->bin_counts, cpos + nrows, counts));
     STEP_CUDA(cudaStreamSynchronize(st));
     if (!rc) {
         p->n1 = counts[0]; p->n2 = counts[1];
@@ -1164,20 +1208,20 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
                 if (!rc) {
                     team_items_kernel<<<(unsigned)ceil_div(p->n2, 256), 256, 0, st>>>(
                         p->n2, p->list2, p->cpos, per_entry, th, items, (unsigned)cap);
-                    team_clear_kernel<<<(unsigned)sm_count() * 8, 256, 0, st>>>(th, items, (unsigned)cap, p->list2,
-                                                                                p->cpos, p->semi, cval);
+                    launch_behind(team_clear_kernel, dim3((unsigned)sm_count() * 8), 256, 0, st, th, items, (unsigned)cap, p->list2,
+                                  p->cpos, p->semi, cval);
                     if (p->semi == COMET_B200_PLUS_TIMES) {
                         cudaFuncSetAttribute(bitmap_numeric_kernel<true, true>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                        bitmap_numeric_kernel<true, true><<<grid, BM_THREADS, smem, st>>>(
-                            p->n2, p->list2, p->words, nullptr, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32,
-                            p->bval, p->mpos, p->mcrd, p->semi, p->bm_store, p->cpos, ccrd, cval, th, items);
+                        launch_behind(bitmap_numeric_kernel<true, true>, dim3(grid), BM_THREADS, smem, st, p->n2, p->list2, p->words,
+                                      nullptr, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32, p->bval, p->mpos, p->mcrd,
+                                      p->semi, p->bm_store, p->cpos, ccrd, cval, th, items);
                     } else {
                         cudaFuncSetAttribute(bitmap_numeric_kernel<true, false>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                        bitmap_numeric_kernel<true, false><<<grid, BM_THREADS, smem, st>>>(
-                            p->n2, p->list2, p->words, nullptr, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32,
-                            p->bval, p->mpos, p->mcrd, p->semi, p->bm_store, p->cpos, ccrd, cval, th, items);
+                        launch_behind(bitmap_numeric_kernel<true, false>, dim3(grid), BM_THREADS, smem, st, p->n2, p->list2, p->words,
+                                      nullptr, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32, p->bval, p->mpos, p->mcrd,
+                                      p->semi, p->bm_store, p->cpos, ccrd, cval, th, items);
                     }
                 }
             } else {
