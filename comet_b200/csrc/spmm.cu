@@ -225,7 +225,7 @@ int spmm_stream_tma(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const 
 // 477 us against 502; 50,021 rows of up to 24: 55 against 54) and is launched alone.
 static int spmm_auto(const SpmmCall &a)
 {
-    const bool stream = !a.pair && a.k >= 64 && a.nnz > 0;
+    const bool stream = !a.pair && a.k >= 64 && a.nnz >= SPMM_FIXED_NNZ;
     LongRows lr = {nullptr, 0};
     if (!stream || !a.vec || a.k < 96) CB_TRY(spmm_short_rows(a, &lr));
     if (!stream) return spmm_pieces(a, lr);

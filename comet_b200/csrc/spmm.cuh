@@ -5,6 +5,9 @@
 
 namespace cb200 {
 
+// Calls with fewer entries (plus-times) give the same sums to the bit every time: no atomics.
+static const int64_t SPMM_FIXED_NNZ = 65536;
+
 struct SpmmCall {
     int64_t nrows, ncols, nnz, k;
     const int64_t *row_ids, *pos, *crd;

@@ -7,6 +7,10 @@
 // boundary cuts are added with f64 atomics onto zeros that the plan kernel has written, so hub rows are shared by as many
 // groups as they have pieces and no row waits for another.
 //
+// FIXED, for small matrices: a piece leaves its part of a cut row in scratch memory instead (the part of a row that started
+// before it in one slot, of a row that goes on after it in another), and a last kernel adds the parts up in the order of
+// the pieces, so the sums of every call are the same to the bit.  It costs 2 us.
+//
 // V = double2 where K, both leading dimensions and both addresses allow 16-byte accesses, otherwise double: an odd
 // number of columns costs twice the load instructions and no more.  K beyond one pass is walked in slices.
 //
@@ -119,12 +123,12 @@ int stream_plan(int64_t nrows, int64_t nnz, int64_t warps, const int64_t *row_id
     return piece_plan(nrows, nnz, s, row_ids, pos, c, ldc, k, accumulate, lr, st, out) ? -1 : 1;
 }
 
-template <typename V, int T, int NI, bool PAIR>
+template <typename V, int T, int NI, bool PAIR, bool FIXED>
 __global__ void __launch_bounds__(SP_THREADS, pieces_ctas<V>(NI))
 spmm_pieces_kernel(int64_t nrows, int64_t npieces, const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
                    const int64_t *__restrict__ crd, const double *__restrict__ val, const double *__restrict__ b0, uint32_t ldb8,
                    double *__restrict__ c0, int64_t ldc, int k, int accumulate, const int64_t *__restrict__ piece_row,
-                   const int64_t *__restrict__ piece_ent, LongRows lr)
+                   const int64_t *__restrict__ piece_ent, LongRows lr, double *__restrict__ parts, int64_t all_k)
 {
     wait_for_previous();
     if (not_this(lr)) return;
@@ -163,12 +167,14 @@ spmm_pieces_kernel(int64_t nrows, int64_t npieces, const int64_t *__restrict__ r
     for (int i = 0; i < NI; i++) acc[i] = Vec<V>::zero();
 
     auto flush = [&](bool store) {
-        V *crow = (V *)(c + (row_ids ? row_ids[r] : r) * ldc);
+        V *crow = FIXED && !store ? (V *)(parts + (2 * piece + (whole ? 1 : 0)) * all_k + col0)
+                                  : (V *)(c + (row_ids ? row_ids[r] : r) * ldc);
 #pragma unroll
         for (int i = 0; i < NI; i++) {
             if (on[i]) {
                 V *at = crow + l + i * T;
-                if (!store) Vec<V>::atomic_to(at, acc[i]);
+                if (!store && FIXED) *at = acc[i];
+                else if (!store) Vec<V>::atomic_to(at, acc[i]);
                 else {
                     if (accumulate) Vec<V>::add_to(acc[i], *at);
                     __stcs(at, acc[i]);                // written once, not read again here
@@ -243,24 +249,64 @@ spmm_pieces_kernel(int64_t nrows, int64_t npieces, const int64_t *__restrict__ r
     if (rend < nrows && e0 + n_ent > pos[rend]) flush(false);
 }
 
+// FIXED: the row that piece b starts and does not end, its parts in order.  A warp per piece.
+__global__ void __launch_bounds__(256)
+spmm_parts_kernel(int64_t nrows, int64_t npieces, const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
+                  double *__restrict__ c, int64_t ldc, int64_t k, int accumulate, const int64_t *__restrict__ piece_row,
+                  const int64_t *__restrict__ piece_ent, LongRows lr, const double *__restrict__ parts)
+{
+    wait_for_previous();
+    if (not_this(lr)) return;
+    const int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b >= npieces) return;
+    const int64_t r = piece_row[b + 1];
+    if (r >= nrows) return;
+    const int64_t start = pos[r];
+    if (start < piece_ent[b] || start >= piece_ent[b + 1]) return;      // starts in another piece, or none of it is in this one
+    int64_t last = b + 1;
+    while (last + 1 < npieces && piece_row[last + 1] <= r) last++;      // the piece in which the row ends
+    double *crow = c + (row_ids ? row_ids[r] : r) * ldc;
+    for (int64_t j = threadIdx.x & 31; j < k; j += 32) {
+        double sum = parts[(2 * b + 1) * k + j];
+#pragma unroll 4
+        for (int64_t q = b + 1; q <= last; q++) sum += parts[2 * q * k + j];
+        crow[j] = accumulate ? crow[j] + sum : sum;
+    }
+}
+
 template <typename V, int T, int NI>
 static int launch_pieces(const SpmmCall &a, LongRows lr)
 {
     const int64_t kv = a.k / Vec<V>::N;
     const int64_t groups = (int64_t)sm_count() * SP_THREADS * pieces_ctas<V>(NI) / T;      // on the chip at a time
     int s = 5;                                         // 2^5 to 2^8 steps, the longest that still give four rounds
-    while (s < 8 && (a.nnz + a.nrows) >> (s + 1) >= groups * 4) s++;
-    while ((a.nnz + a.nrows) >> s >= (1LL << 31)) s++;
+    // The same pieces at every K, so that a product taken in panels has the sums of the whole one
+    const bool fixed = a.nnz < SPMM_FIXED_NNZ && !a.pair;
+    double *parts = nullptr;
+    if (fixed) {
+        while ((a.nnz + a.nrows) >> s >= (1 << 13)) s++;               // parts of 64 MB at most
+        void *mem = nullptr;
+        CB_TRY(scratch(SLOT_MISC, (size_t)(ceil_div(a.nnz + a.nrows, (int64_t)1 << s) + 1) * 2 * (size_t)a.k * sizeof(double), &mem));
+        parts = (double *)mem;
+    } else {
+        while (s < 8 && (a.nnz + a.nrows) >> (s + 1) >= groups * 4) s++;
+        while ((a.nnz + a.nrows) >> s >= (1LL << 31)) s++;
+    }
     StreamPlan plan;
-    CB_TRY(piece_plan(a.nrows, a.nnz, s, a.row_ids, a.pos, a.c, a.ldc, a.k, a.accumulate, lr, a.st, &plan));
+    CB_TRY(piece_plan(a.nrows, a.nnz, s, a.row_ids, a.pos, fixed ? nullptr : a.c, a.ldc, a.k, a.accumulate, lr, a.st, &plan));
     const int64_t blocks = ceil_div(plan.nblocks * T, SP_THREADS), slices = ceil_div(kv, T * NI);
-    auto kernel = a.pair ? spmm_pieces_kernel<V, T, NI, true> : spmm_pieces_kernel<V, T, NI, false>;
+    auto kernel = a.pair  ? spmm_pieces_kernel<V, T, NI, true, false>
+                  : fixed ? spmm_pieces_kernel<V, T, NI, false, true>
+                          : spmm_pieces_kernel<V, T, NI, false, false>;
     for (int64_t first = 0; first < slices; first += 65535) {
         const int64_t n = slices - first < 65535 ? slices - first : 65535, col0 = first * T * NI * Vec<V>::N;
         CB_CUDA(launch_behind(kernel, dim3((unsigned)blocks, (unsigned)n), SP_THREADS, 0, a.st, a.nrows, plan.nblocks, a.row_ids,
                               a.pos, a.crd, a.val, a.b + col0, (uint32_t)(a.ldb * 8), a.c + col0, a.ldc, (int)(a.k - col0),
-                              a.accumulate, plan.block_row, plan.block_ent, lr));
+                              a.accumulate, plan.block_row, plan.block_ent, lr, parts ? parts + col0 : nullptr, a.k));
     }
+    if (fixed)
+        CB_CUDA(launch_behind(spmm_parts_kernel, dim3((unsigned)ceil_div(plan.nblocks * 32, 256)), 256, 0, a.st, a.nrows, plan.nblocks,
+                              a.row_ids, a.pos, a.c, a.ldc, a.k, a.accumulate, plan.block_row, plan.block_ent, lr, parts));
     return 0;
 }
 
@@ -285,6 +331,16 @@ static int dispatch_pieces(const SpmmCall &a, LongRows lr)
 
 int spmm_pieces(const SpmmCall &a, LongRows lr)
 {
+    if (a.k > 512 && a.nnz < SPMM_FIXED_NNZ) {         // the parts' memory grows with the columns
+        for (int64_t col0 = 0; col0 < a.k; col0 += 512) {
+            SpmmCall slab = a;
+            slab.k = a.k - col0 < 512 ? a.k - col0 : 512;
+            slab.b += col0;
+            slab.c += col0;
+            CB_TRY(spmm_pieces(slab, lr));
+        }
+        return 0;
+    }
     return a.vec ? dispatch_pieces<double2>(a, lr) : dispatch_pieces<double>(a, lr);
 }
 

@@ -65,3 +65,13 @@ def test_stored_rows_only(kind, k):
     C = dev.spmm(_device(m, ids, 3 * m.shape[0] + 1), torch.from_numpy(B).cuda())
     _same(C[1::3], m, m @ B, B)
     assert not C[0::3].any() and not C[2::3].any()
+
+
+@pytest.mark.parametrize("k", [1, 6, 33, 64, 200, 600])
+def test_small_products_are_the_same_to_the_bit(k):
+    m = _matrix("skewed")
+    A, B = _device(m), torch.rand((m.shape[1], k), device="cuda", dtype=torch.float64)
+    C = dev.spmm(A, B)
+    assert all(torch.equal(C, dev.spmm(A, B)) for _ in range(5))
+    if k > 6:                      # and a panel's sums are those of the whole product
+        assert torch.equal(C[:, :6], dev.spmm(A, B[:, :6]))
