@@ -312,14 +312,17 @@ static int launch_pieces(const SpmmCall &a, LongRows lr)
 
 // As few lanes as cover the columns with one vector each up to 16, then more vectors a lane: at 17 to 32 vectors 16 lanes x 2
 // beat 32 x 1 (R-MAT scale 20, K = 48: 890 against 1030 us), at 33 to 48 vectors 16 x 3 beat 32 x 2 (scale 17, K = 96: 128
-// against 227).  Beyond 128 vectors in slices as even as they go.
+// against 227).  On a small matrix narrow rows get lanes that would idle anyway: 16 of them load a piece's entries at once
+// (R-MAT scale 14, K = 4: 49 -> 27 us).  Beyond 128 vectors in slices as even as they go.
 template <typename V>
 static int dispatch_pieces(const SpmmCall &a, LongRows lr)
 {
     const int64_t kv = a.k / Vec<V>::N;
-    if (kv <= 2) return launch_pieces<V, 2, 1>(a, lr);
-    if (kv <= 4) return launch_pieces<V, 4, 1>(a, lr);
-    if (kv <= 8) return launch_pieces<V, 8, 1>(a, lr);
+    int64_t t = kv <= 2 ? 2 : kv <= 4 ? 4 : kv <= 8 ? 8 : 16;
+    while (t < 16 && ((a.nnz + a.nrows) >> 5) * t * 2 <= (int64_t)sm_count() * 1024) t *= 2;
+    if (t == 2) return launch_pieces<V, 2, 1>(a, lr);
+    if (t == 4) return launch_pieces<V, 4, 1>(a, lr);
+    if (t == 8) return launch_pieces<V, 8, 1>(a, lr);
     if (kv <= 16) return launch_pieces<V, 16, 1>(a, lr);
     if (kv <= 32) return launch_pieces<V, 16, 2>(a, lr);
     if (kv <= 48) return launch_pieces<V, 16, 3>(a, lr);
