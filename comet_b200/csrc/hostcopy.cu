@@ -35,11 +35,13 @@ namespace cb200 {
 namespace {
 
 // Measured on this host (16 virtual cores): one core copies 16 GB/s, eight 35 to 40, PCIe moves 53; the driver's own
-// staging 14.  Waking a worker takes 12 us, so a copy is cut into pieces of at least 512 KB (30 us of copying).
+// staging 14.  Waking a worker takes 12 us and the DMA engine reads the chunks while others are written, so few threads with
+// large pieces beat many with small ones (4.3 MB / 17 MB / 70 MB in and out: five threads and pieces of 1.5 MB 225 / 601 /
+// 3500 us, eight and 512 KB 272 / 639 / 3580).
 const size_t CHUNK = (size_t)2 << 20;     // bytes per page-locked chunk
 const int SLAB_CHUNKS = 8;                // chunks are allocated 16 MiB at a time (7 ms each),
 const int MAX_SLABS = 4;                  // at most 64 MiB per device
-const size_t PIECE_MIN = (size_t)512 << 10;
+const size_t PIECE_MIN = (size_t)1536 << 10;
 const size_t STAGE_MIN_DEFAULT = (size_t)96 << 10;  // smaller copies are left to the driver
 
 struct Slot {
@@ -56,12 +58,12 @@ class Pool {
   public:
     explicit Pool(int device) : device_(device)
     {
-        // half of the cores this process can count on: launchers that start one process per GPU export
+        // a third of the cores this process can count on: launchers that start one process per GPU export
         // LOCAL_WORLD_SIZE, and the processes of one node share its cores
         int share = 1;
         const char *lws = getenv("LOCAL_WORLD_SIZE");
         if (lws && atoi(lws) > 1) share = atoi(lws);
-        int n = (int)std::thread::hardware_concurrency() / (2 * share);
+        int n = (int)std::thread::hardware_concurrency() / (3 * share);
         const char *env = getenv("COMET_B200_COPY_THREADS");
         if (env) n = atoi(env);
         if (n < 2) n = 2;
