@@ -7,6 +7,8 @@
 //   bin 1  bound <= HASH_ROW_MAX           -> one warp per row, hash table in
 //          shared memory (int32 keys + f64 accumulators); output order by rank
 //          counting among the row's distinct keys
+//   bin 3  bound <= MID_ROW_MAX, no mask, not too many columns -> 128 threads per row, a bitmap over the columns of B and
+//          sums by rank in shared memory
 //   bin 2  everything else                 -> one CTA per row, a bitmap over the
 //          columns of B in shared memory (global memory when B has too many
 //          columns); popcounts give the row's count, prefix popcounts give each
@@ -52,11 +54,11 @@ struct Plan {
     int64_t *cpos;           // caller's array
     int64_t nnz_c;
     void *mem;               // owned device memory: the next five arrays
-    unsigned *bin_counts;    // [2]
+    unsigned *bin_counts;    // [3]
     int64_t *cnt;            // per-row distinct count
     int32_t *bcrd32;
-    int32_t *list1, *list2;  // rows of bin 1 / bin 2
-    unsigned n1, n2;
+    int32_t *list1, *list2, *list3;  // rows of bins 1, 2 and 3
+    unsigned n1, n2, n3;
     uint32_t *bm_store;      // n2 * words, or null
     int words;
     MaskedPlan *masked;      // not null: the product is formed by dot products over the mask
@@ -132,8 +134,8 @@ static const int64_t NARROW_PART = 4096;                // entries per CTA
 __global__ void __launch_bounds__(BIN_THREADS)
 bin_rows_kernel(int64_t nrows, int passes, unsigned row_ctas, const int64_t *__restrict__ apos, const int64_t *__restrict__ acrd,
                 const int64_t *__restrict__ bpos, const int64_t *__restrict__ mpos,
-                int64_t *__restrict__ cnt, int32_t *__restrict__ list1, int32_t *__restrict__ list2,
-                unsigned *__restrict__ bin_counts, const int64_t *__restrict__ bcrd, int32_t *__restrict__ bcrd32, int64_t nnz_b)
+                int64_t stop, int64_t *__restrict__ cnt, int32_t *__restrict__ list1, int32_t *__restrict__ list2,
+                int32_t *__restrict__ list3, unsigned *__restrict__ bin_counts, const int64_t *__restrict__ bcrd, int32_t *__restrict__ bcrd32, int64_t nnz_b)
 {
     if (blockIdx.x >= row_ctas) {
         const int64_t first = (int64_t)(blockIdx.x - row_ctas) * NARROW_PART;
@@ -149,21 +151,21 @@ bin_rows_kernel(int64_t nrows, int passes, unsigned row_ctas, const int64_t *__r
     }
     __shared__ unsigned char bin_of[BIN_ROWS];
     __shared__ unsigned short local_at[BIN_ROWS];
-    __shared__ unsigned local_cnt[2], base[2], n_long;
+    __shared__ unsigned local_cnt[3], base[3], n_long;
     __shared__ unsigned short long_slot[BIN_ROWS];
     const int g = threadIdx.x / 8, l = threadIdx.x % 8;
     const unsigned gmask = 0xffu << ((threadIdx.x & 31) & ~7);
-    if (threadIdx.x < 2) local_cnt[threadIdx.x] = 0;
-    if (threadIdx.x == 2) n_long = 0;
+    if (threadIdx.x < 3) local_cnt[threadIdx.x] = 0;
+    if (threadIdx.x == 3) n_long = 0;
     __syncthreads();
     const int64_t row0 = (int64_t)blockIdx.x * (BIN_PASS * passes);
-    // the bin of a row from ub: its products, or more than HASH_ROW_MAX if it has more
+    // the bin of a row from ub: its products, or more than `stop` if it has more
     auto place = [&](int slot, int64_t r, int64_t ub) {
         if (mpos) {
             int64_t ml = mpos[r + 1] - mpos[r];
             if (ml < ub) ub = ml;
         }
-        int b = ub == 0 ? 0 : (ub <= HASH_ROW_MAX ? 1 : 2);
+        int b = ub == 0 ? 0 : (ub <= HASH_ROW_MAX ? 1 : ub <= stop ? 3 : 2);
         bin_of[slot] = (unsigned char)b;
         if (b == 0) cnt[r] = 0;
         else local_at[slot] = (unsigned short)atomicAdd(&local_cnt[b - 1], 1u);
@@ -194,7 +196,7 @@ bin_rows_kernel(int64_t nrows, int passes, unsigned row_ctas, const int64_t *__r
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) part += __shfl_xor_sync(gmask, (long long)part, o, 8);
             ub += part;
-            if (ub > HASH_ROW_MAX) break;
+            if (ub > stop) break;
         }
         if (l == 0) {
             if (later) long_slot[atomicAdd(&n_long, 1u)] = (unsigned short)slot;
@@ -210,10 +212,10 @@ bin_rows_kernel(int64_t nrows, int passes, unsigned row_ctas, const int64_t *__r
         bool over = false;
         for (int64_t p = apos[r]; p < ae && !over; p += 4 * BIN_THREADS) {
             ub += four(p + threadIdx.x, ae, BIN_THREADS);
-            over = __syncthreads_or(ub > HASH_ROW_MAX);
+            over = __syncthreads_or(ub > stop);
         }
-        // without a thread over the limit, the sum of all: no more than 256 * HASH_ROW_MAX
-        int64_t total = over ? HASH_ROW_MAX + 1 : 0;
+        // without a thread over the limit, the sum of all: no more than 256 * stop
+        int64_t total = over ? stop + 1 : 0;
         if (!over) {
             __shared__ unsigned sum;
             if (threadIdx.x == 0) sum = 0;
@@ -226,7 +228,7 @@ bin_rows_kernel(int64_t nrows, int passes, unsigned row_ctas, const int64_t *__r
         __syncthreads();
     }
     __syncthreads();
-    if (threadIdx.x < 2 && local_cnt[threadIdx.x]) base[threadIdx.x] = atomicAdd(&bin_counts[threadIdx.x], local_cnt[threadIdx.x]);
+    if (threadIdx.x < 3 && local_cnt[threadIdx.x]) base[threadIdx.x] = atomicAdd(&bin_counts[threadIdx.x], local_cnt[threadIdx.x]);
     __syncthreads();
     for (int slot = threadIdx.x; slot < BIN_PASS * passes; slot += BIN_THREADS) {
         int64_t r = row0 + slot;
@@ -234,6 +236,7 @@ bin_rows_kernel(int64_t nrows, int passes, unsigned row_ctas, const int64_t *__r
         int b = bin_of[slot];
         if (b == 1) list1[base[0] + local_at[slot]] = (int32_t)r;
         else if (b == 2) list2[base[1] + local_at[slot]] = (int32_t)r;
+        else if (b == 3) list3[base[2] + local_at[slot]] = (int32_t)r;
     }
 }
 
@@ -243,7 +246,8 @@ __global__ void publish_kernel(const unsigned *__restrict__ bin_counts, const in
     wait_for_previous();
     host[0] = bin_counts[0];
     host[1] = bin_counts[1];
-    if (nnz) *(int64_t *)(host + 2) = *nnz;
+    host[2] = bin_counts[2];
+    if (nnz) *(int64_t *)(host + 4) = *nnz;
 }
 
 // --------------------------------------------------------------------------
@@ -558,6 +562,142 @@ short_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restr
         __syncwarp();
     }
 }
+
+// --------------------------------------------------------------------------
+// Bin 3, without a mask: rows of up to MID_ROW_MAX products where a bitmap over B's columns fits beside them.
+//
+// A CTA of 128 threads per row.  The lengths of up to 128 rows of B are scanned and their products dealt to the threads one
+// by one, so that short and long rows of B cost the same per product.  A product marks its column and is kept; popcounts
+// of the words give every column its rank; the products are added up by rank in shared memory, and the row is written
+// in one coalesced pass.  The kept products also clear the bitmap.  Against a bin-2 CTA: no bitmap stored by one call
+// and read by the other, no cleared and re-read output, four times as many rows at a time.
+//
+// Bound: instructions, two passes over the words and about 60 per product.  50,000 rows of 900 products in 50,000 columns:
+// 1374 -> MIDNOW us for both calls.
+// --------------------------------------------------------------------------
+static const int MID_THREADS = 128;
+static const int MID_ROW_MAX = 1024;
+static const int MID_WORDS = 8192;
+
+template <bool NUMERIC>
+__global__ void __launch_bounds__(MID_THREADS)
+mid_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restrict__ rows, int words,
+                const int64_t *__restrict__ apos, const int64_t *__restrict__ acrd, const double *__restrict__ aval,
+                const int64_t *__restrict__ bpos, const int32_t *__restrict__ bcrd, const double *__restrict__ bval, int semi,
+                int64_t *__restrict__ cnt, const int64_t *__restrict__ cpos, int64_t *__restrict__ ccrd,
+                double *__restrict__ cval)
+{
+    constexpr int NW = MID_THREADS / 32, KEEP = NUMERIC ? MID_ROW_MAX : 1;
+    extern __shared__ uint32_t bm[];                   // words, then (numeric) a 16-bit rank for each
+    __shared__ int64_t s_rel[MID_THREADS];
+    __shared__ double s_av[NUMERIC ? MID_THREADS : 1], s_vals[KEEP], s_sums[KEEP];
+    __shared__ int s_upto[MID_THREADS], s_cols[MID_ROW_MAX], s_out[KEEP];
+    __shared__ unsigned s_warp[NW], s_count;
+    unsigned short *pre = (unsigned short *)(bm + words);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double ident = sr_identity(semi);
+    for (int w = tid; w < words; w += MID_THREADS) bm[w] = 0;
+    wait_for_previous();
+    const unsigned nlist = *nlist_dev;
+    for (unsigned it = blockIdx.x; it < nlist; it += gridDim.x) {
+        const int64_t r = rows[it], ae = apos[r + 1];
+        int n = 0;                                     // products so far
+        unsigned fresh = 0;
+        for (int64_t p0 = apos[r]; p0 < ae; p0 += MID_THREADS) {
+            int64_t s = 0;
+            int len = 0;
+            if (p0 + tid < ae) {
+                const int64_t k = acrd[p0 + tid];
+                if (NUMERIC) s_av[tid] = aval[p0 + tid];
+                s = bpos[k];
+                len = (int)(bpos[k + 1] - s);
+            }
+            int upto = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            if (lane == 31) s_warp[warp] = upto;
+            __syncthreads();
+            int total = 0;
+#pragma unroll
+            for (int w = 0; w < NW; w++) {
+                if (w < warp) upto += s_warp[w];
+                total += s_warp[w];
+            }
+            s_upto[tid] = upto;
+            s_rel[tid] = s - (upto - len);             // product x of the batch is entry s_rel[t] + x of B, for its own A entry
+            __syncthreads();
+#pragma unroll 2
+            for (int x = tid; x < total; x += MID_THREADS) {
+                int t = 0;                             // first A entry whose prefix sum exceeds x
+#pragma unroll
+                for (int step = MID_THREADS / 2; step > 0; step >>= 1)
+                    if (s_upto[t + step - 1] <= x) t += step;
+                const int64_t q = s_rel[t] + x;
+                const int32_t j = bcrd[q];
+                s_cols[n + x] = j;
+                if (NUMERIC) {
+                    s_vals[n + x] = sr_combine(semi, s_av[t], bval[q]);
+                    atomicOr(&bm[j >> 5], 1u << (j & 31));
+                } else {
+                    fresh += !((atomicOr(&bm[j >> 5], 1u << (j & 31)) >> (j & 31)) & 1u);
+                }
+            }
+            n += total;
+            __syncthreads();                           // the batch's arrays and the warps' sums are free again
+        }
+        if (!NUMERIC) {
+            if (tid == 0) s_count = 0;
+            fresh = __reduce_add_sync(0xffffffffu, fresh);
+            __syncthreads();
+            if (lane == 0 && fresh) atomicAdd(&s_count, fresh);
+        } else {
+            // words in runs of an odd number per thread: every bank once
+            const int per = ((words + MID_THREADS - 1) / MID_THREADS) | 1;
+            const int w0 = min(tid * per, words), w1 = min(w0 + per, words);
+            unsigned c = 0;
+            for (int w = w0; w < w1; w++) c += __popc(bm[w]);
+            unsigned incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) s_warp[warp] = incl;
+            const int64_t base = cpos[r];
+            const int out = (int)(cpos[r + 1] - base);
+            for (int i = tid; i < out; i += MID_THREADS) s_sums[i] = ident;
+            __syncthreads();
+            unsigned run = incl - c;
+#pragma unroll
+            for (int w = 0; w < NW; w++)
+                if (w < warp) run += s_warp[w];
+            for (int w = w0; w < w1; w++) {
+                pre[w] = (unsigned short)run;
+                run += __popc(bm[w]);
+            }
+            __syncthreads();
+            for (int i = tid; i < n; i += MID_THREADS) {
+                const int j = s_cols[i];
+                const unsigned rank = pre[j >> 5] + __popc(bm[j >> 5] & ((1u << (j & 31)) - 1u));
+                s_out[rank] = j;
+                sr_fold(semi, &s_sums[rank], s_vals[i]);
+            }
+            __syncthreads();
+            for (int i = tid; i < out; i += MID_THREADS) {
+                __stcs((long long *)ccrd + base + i, (long long)s_out[i]);
+                __stcs(cval + base + i, s_sums[i]);
+            }
+        }
+        for (int i = tid; i < n; i += MID_THREADS) bm[s_cols[i] >> 5] = 0;
+        __syncthreads();
+        if (!NUMERIC && tid == 0) cnt[r] = s_count;
+    }
+}
+
+static size_t mid_smem(int words, bool numeric) { return (size_t)words * (numeric ? 6 : 4); }
 
 // --------------------------------------------------------------------------
 // Bin 2: CTA per row, bitmap over B's columns.
@@ -1006,6 +1146,22 @@ static int bitmap_grid(unsigned nlist, size_t smem_bytes)
     return (int)(g < 1 ? 1 : g);
 }
 
+static unsigned cnt_grid(unsigned rows)
+{
+    const unsigned cap = (unsigned)sm_count() * 16;
+    return rows < cap ? rows : cap;
+}
+
+template <bool NUMERIC>
+static int launch_mid(const Plan *p, unsigned grid, int64_t *ccrd, double *cval, cudaStream_t st)
+{
+    const size_t smem = mid_smem(p->words, NUMERIC);
+    CB_CUDA(cudaFuncSetAttribute(mid_rows_kernel<NUMERIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CB_CUDA(launch_behind(mid_rows_kernel<NUMERIC>, dim3(grid), MID_THREADS, smem, st, p->bin_counts + 2, p->list3, p->words, p->apos,
+                          p->acrd, p->aval, p->bpos, p->bcrd32, p->bval, p->semi, p->cnt, p->cpos, ccrd, cval));
+    return 0;
+}
+
 int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t *apos,
                     const int64_t *acrd, const double *aval, const int64_t *bpos,
                     const int64_t *bcrd, const double *bval, const int64_t *mpos,
@@ -1050,21 +1206,24 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     auto pad = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
     const size_t b_cnt = pad(((size_t)nrows + 1) * 8), b_crd = pad((size_t)nnz_b * 4 + 8), b_list = pad((size_t)nrows * 4);
     char *mem = nullptr;
-    STEP(dev_alloc(&mem, 256 + b_cnt + b_crd + 2 * b_list, st));
+    const bool mid = !mpos && p->words <= MID_WORDS;
+    STEP(dev_alloc(&mem, 256 + b_cnt + b_crd + (mid ? 3 : 2) * b_list, st));
     p->mem = mem;
     p->bin_counts = (unsigned *)mem;
     p->cnt = (int64_t *)(mem + 256);
     p->bcrd32 = (int32_t *)(mem + 256 + b_cnt);
     p->list1 = (int32_t *)(mem + 256 + b_cnt + b_crd);
     p->list2 = (int32_t *)((char *)p->list1 + b_list);
-    STEP_CUDA(cudaMemsetAsync(p->bin_counts, 0, 2 * sizeof(unsigned), st));
+    p->list3 = (int32_t *)((char *)p->list2 + b_list);
+    STEP_CUDA(cudaMemsetAsync(p->bin_counts, 0, 3 * sizeof(unsigned), st));
     if (!rc && nrows + nnz_b > 0) {
         const int passes = nrows >= (int64_t)sm_count() * 8 * BIN_ROWS ? 4 : 1;
         const int64_t row_ctas = ceil_div(nrows, (int64_t)BIN_PASS * passes), ctas = row_ctas + ceil_div(nnz_b, NARROW_PART);
         if (ctas > 0x7fffffffLL) rc = fail("spgemm: too many entries");
         if (!rc)
-            bin_rows_kernel<<<(unsigned)ctas, BIN_THREADS, 0, st>>>(nrows, passes, (unsigned)row_ctas, apos, acrd, bpos, mpos, p->cnt,
-                                                                   p->list1, p->list2, p->bin_counts, bcrd, p->bcrd32, nnz_b);
+            bin_rows_kernel<<<(unsigned)ctas, BIN_THREADS, 0, st>>>(nrows, passes, (unsigned)row_ctas, apos, acrd, bpos, mpos,
+                                                                   mid ? MID_ROW_MAX : HASH_ROW_MAX, p->cnt, p->list1, p->list2,
+                                                                   p->list3, p->bin_counts, bcrd, p->bcrd32, nnz_b);
         STEP_CUDA(cudaGetLastError());
     }
     PinnedWords words;
@@ -1073,10 +1232,11 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     // The bitmaps of the bin-2 rows are kept for the numeric call, so their number is needed to allocate them: after a
     // synchronisation, unless bitmaps for every row are small change (then the kernels read the bin sizes themselves).
     p->n1 = p->n2 = (unsigned)nrows;
+    p->n3 = mid ? (unsigned)nrows : 0;
     if ((size_t)nrows * p->words * 4 > BM_STORE_SMALL) {
         STEP_CUDA(launch_behind(publish_kernel, dim3(1), 1, 0, st, p->bin_counts, nullptr, counts));
         STEP_CUDA(cudaStreamSynchronize(st));
-        if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; }
+        if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; p->n3 = counts[2]; }
     }
     if (!rc && p->n1) {
         unsigned grid = (unsigned)ceil_div(p->n1, HASH_WARPS);
@@ -1085,6 +1245,7 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
         STEP_CUDA(launch_behind(hash_rows_kernel<false, false>, dim3(grid), HASH_WARPS * 32, 0, st, p->bin_counts, p->list1, apos, acrd,
                                 aval, bpos, p->bcrd32, bval, mpos, p->mcrd, p->semi, p->cnt, nullptr, nullptr, nullptr));
     }
+    if (!rc && p->n3) STEP(launch_mid<false>(p, cnt_grid(p->n3), nullptr, nullptr, st));
     if (!rc && p->n2) {
         size_t store = (size_t)p->n2 * p->words * sizeof(uint32_t);
         // the symbolic pass's bitmaps are kept for the numeric pass while they fit the budget
@@ -1117,8 +1278,8 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     STEP_CUDA(launch_behind(publish_kernel, dim3(1), 1, 0, st, p->bin_counts, cpos + nrows, counts));
     STEP_CUDA(cudaStreamSynchronize(st));
     if (!rc) {
-        p->n1 = counts[0]; p->n2 = counts[1];
-        p->nnz_c = *(int64_t *)(counts + 2);
+        p->n1 = counts[0]; p->n2 = counts[1]; p->n3 = counts[2];
+        p->nnz_c = *(int64_t *)(counts + 4);
     }
 #undef STEP
 #undef STEP_CUDA
@@ -1187,6 +1348,7 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
             }
             if (cudaGetLastError() != cudaSuccess) rc = fail("spgemm numeric (hash) launch failed");
         }
+        if (!rc && p->n3) rc = launch_mid<true>(p, cnt_grid(p->n3), ccrd, cval, st);
         if (!rc && p->n2) {
             size_t smem = (size_t)p->words * sizeof(uint32_t) * 2;
             if (smem <= BM_SMEM_LIMIT) {
