@@ -7,7 +7,7 @@
 //   bin 1  bound <= HASH_ROW_MAX           -> one warp per row, hash table in
 //          shared memory (int32 keys + f64 accumulators); output order by rank
 //          counting among the row's distinct keys
-//   bin 3  bound <= MID_ROW_MAX, no mask, not too many columns -> 128 threads per row, a bitmap over the columns of B and
+//   bin 3  bound <= MID_ROW_MAX, no mask, not too many columns -> 128 or 256 threads per row, a bitmap over the columns of B and
 //          sums by rank in shared memory
 //   bin 2  everything else                 -> one CTA per row, a bitmap over the
 //          columns of B in shared memory (global memory when B has too many
@@ -566,44 +566,45 @@ short_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restr
 // --------------------------------------------------------------------------
 // Bin 3, without a mask: rows of up to MID_ROW_MAX products where a bitmap over B's columns fits beside them.
 //
-// A CTA of 128 threads per row.  The lengths of up to 128 rows of B are scanned and their products dealt to the threads one
+// A CTA of 128 or 256 threads per row.  The lengths of as many rows of B are scanned and their products dealt to the threads one
 // by one, so that short and long rows of B cost the same per product.  A product marks its column and is kept; popcounts
 // of the words give every column its rank; the products are added up by rank in shared memory, and the row is written
 // in one coalesced pass.  The kept products also clear the bitmap.  Against a bin-2 CTA: no bitmap stored by one call
 // and read by the other, no cleared and re-read output, four times as many rows at a time.
 //
 // Bound: instructions, two passes over the words and about 60 per product.  50,000 rows of 900 products in 50,000 columns:
-// 1374 -> MIDNOW us for both calls.
+// 1374 -> 845 us for both calls; the numeric one has the shared-memory pipe busy two thirds of the time.  A second bitmap of
+// the words with columns, to skip the others, cost more than it saved (966).
 // --------------------------------------------------------------------------
-static const int MID_THREADS = 128;
+static const int MID_MANY_WORDS = 2048;     // 256 threads from here on, as fewer CTAs fit: 180,000 rows of 20, 4250 -> 3410 us (at 50,000 columns 845 -> 900)
 static const int MID_ROW_MAX = 1024;
 static const int MID_WORDS = 8192;
 
-template <bool NUMERIC>
-__global__ void __launch_bounds__(MID_THREADS)
+template <int THREADS, bool NUMERIC>
+__global__ void __launch_bounds__(THREADS)
 mid_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restrict__ rows, int words,
                 const int64_t *__restrict__ apos, const int64_t *__restrict__ acrd, const double *__restrict__ aval,
                 const int64_t *__restrict__ bpos, const int32_t *__restrict__ bcrd, const double *__restrict__ bval, int semi,
                 int64_t *__restrict__ cnt, const int64_t *__restrict__ cpos, int64_t *__restrict__ ccrd,
                 double *__restrict__ cval)
 {
-    constexpr int NW = MID_THREADS / 32, KEEP = NUMERIC ? MID_ROW_MAX : 1;
+    constexpr int NW = THREADS / 32, KEEP = NUMERIC ? MID_ROW_MAX : 1;
     extern __shared__ uint32_t bm[];                   // words, then (numeric) a 16-bit rank for each
-    __shared__ int64_t s_rel[MID_THREADS];
-    __shared__ double s_av[NUMERIC ? MID_THREADS : 1], s_vals[KEEP], s_sums[KEEP];
-    __shared__ int s_upto[MID_THREADS], s_cols[MID_ROW_MAX], s_out[KEEP];
+    __shared__ int64_t s_rel[THREADS];
+    __shared__ double s_av[NUMERIC ? THREADS : 1], s_vals[KEEP], s_sums[KEEP];
+    __shared__ int s_upto[THREADS], s_cols[MID_ROW_MAX], s_out[KEEP];
     __shared__ unsigned s_warp[NW], s_count;
     unsigned short *pre = (unsigned short *)(bm + words);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double ident = sr_identity(semi);
-    for (int w = tid; w < words; w += MID_THREADS) bm[w] = 0;
+    for (int w = tid; w < words; w += THREADS) bm[w] = 0;
     wait_for_previous();
     const unsigned nlist = *nlist_dev;
     for (unsigned it = blockIdx.x; it < nlist; it += gridDim.x) {
         const int64_t r = rows[it], ae = apos[r + 1];
         int n = 0;                                     // products so far
         unsigned fresh = 0;
-        for (int64_t p0 = apos[r]; p0 < ae; p0 += MID_THREADS) {
+        for (int64_t p0 = apos[r]; p0 < ae; p0 += THREADS) {
             int64_t s = 0;
             int len = 0;
             if (p0 + tid < ae) {
@@ -630,10 +631,10 @@ mid_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restric
             s_rel[tid] = s - (upto - len);             // product x of the batch is entry s_rel[t] + x of B, for its own A entry
             __syncthreads();
 #pragma unroll 2
-            for (int x = tid; x < total; x += MID_THREADS) {
+            for (int x = tid; x < total; x += THREADS) {
                 int t = 0;                             // first A entry whose prefix sum exceeds x
 #pragma unroll
-                for (int step = MID_THREADS / 2; step > 0; step >>= 1)
+                for (int step = THREADS / 2; step > 0; step >>= 1)
                     if (s_upto[t + step - 1] <= x) t += step;
                 const int64_t q = s_rel[t] + x;
                 const int32_t j = bcrd[q];
@@ -655,7 +656,7 @@ mid_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restric
             if (lane == 0 && fresh) atomicAdd(&s_count, fresh);
         } else {
             // words in runs of an odd number per thread: every bank once
-            const int per = ((words + MID_THREADS - 1) / MID_THREADS) | 1;
+            const int per = ((words + THREADS - 1) / THREADS) | 1;
             const int w0 = min(tid * per, words), w1 = min(w0 + per, words);
             unsigned c = 0;
             for (int w = w0; w < w1; w++) c += __popc(bm[w]);
@@ -668,7 +669,7 @@ mid_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restric
             if (lane == 31) s_warp[warp] = incl;
             const int64_t base = cpos[r];
             const int out = (int)(cpos[r + 1] - base);
-            for (int i = tid; i < out; i += MID_THREADS) s_sums[i] = ident;
+            for (int i = tid; i < out; i += THREADS) s_sums[i] = ident;
             __syncthreads();
             unsigned run = incl - c;
 #pragma unroll
@@ -679,19 +680,19 @@ mid_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restric
                 run += __popc(bm[w]);
             }
             __syncthreads();
-            for (int i = tid; i < n; i += MID_THREADS) {
+            for (int i = tid; i < n; i += THREADS) {
                 const int j = s_cols[i];
                 const unsigned rank = pre[j >> 5] + __popc(bm[j >> 5] & ((1u << (j & 31)) - 1u));
                 s_out[rank] = j;
                 sr_fold(semi, &s_sums[rank], s_vals[i]);
             }
             __syncthreads();
-            for (int i = tid; i < out; i += MID_THREADS) {
+            for (int i = tid; i < out; i += THREADS) {
                 __stcs((long long *)ccrd + base + i, (long long)s_out[i]);
                 __stcs(cval + base + i, s_sums[i]);
             }
         }
-        for (int i = tid; i < n; i += MID_THREADS) bm[s_cols[i] >> 5] = 0;
+        for (int i = tid; i < n; i += THREADS) bm[s_cols[i] >> 5] = 0;
         __syncthreads();
         if (!NUMERIC && tid == 0) cnt[r] = s_count;
     }
@@ -1156,9 +1157,11 @@ template <bool NUMERIC>
 static int launch_mid(const Plan *p, unsigned grid, int64_t *ccrd, double *cval, cudaStream_t st)
 {
     const size_t smem = mid_smem(p->words, NUMERIC);
-    CB_CUDA(cudaFuncSetAttribute(mid_rows_kernel<NUMERIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CB_CUDA(launch_behind(mid_rows_kernel<NUMERIC>, dim3(grid), MID_THREADS, smem, st, p->bin_counts + 2, p->list3, p->words, p->apos,
-                          p->acrd, p->aval, p->bpos, p->bcrd32, p->bval, p->semi, p->cnt, p->cpos, ccrd, cval));
+    const bool many = p->words >= MID_MANY_WORDS;
+    auto kernel = many ? mid_rows_kernel<256, NUMERIC> : mid_rows_kernel<128, NUMERIC>;
+    CB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CB_CUDA(launch_behind(kernel, dim3(grid), many ? 256 : 128, smem, st, p->bin_counts + 2, p->list3, p->words, p->apos, p->acrd,
+                          p->aval, p->bpos, p->bcrd32, p->bval, p->semi, p->cnt, p->cpos, ccrd, cval));
     return 0;
 }
 
