@@ -994,11 +994,14 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
             if (threadIdx.x == 0) s_item = atomicAdd(&th->next, 1u);
             __syncthreads();
             const unsigned idx = s_item;
-            if (idx >= th->nitems) break;
-            const uint64_t v = items[idx];
-            it = (unsigned)v;
-            part = (unsigned)(v >> 32) & 0xffffu;
-            team = (unsigned)(v >> 48);
+            if (idx >= (items ? th->nitems : nlist)) break;
+            it = idx;
+            if (items) {
+                const uint64_t v = items[idx];
+                it = (unsigned)v;
+                part = (unsigned)(v >> 32) & 0xffffu;
+                team = (unsigned)(v >> 48);
+            }
         } else if (iter >= nlist) {
             break;
         }
@@ -1362,6 +1365,8 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
                 if (const char *e = getenv("COMET_B200_SPGEMM_TEAM_MB")) budget_mb = atof(e);
                 if (budget_mb < 0.001) budget_mb = 0.001;
                 const double per_entry = 8.0 * grid / (budget_mb * 1048576.0);
+                // no row of so few columns wants a team: two launches less
+                const bool alone = (double)p->ncols * per_entry <= 1.0;
                 const size_t cap = (size_t)p->n2 + (size_t)((double)p->nnz_c * per_entry) + 64;
                 void *tm = nullptr;
                 rc = cap > 0xfffffff0u ? fail("spgemm numeric: too many team items")
@@ -1371,9 +1376,11 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
                 if (!rc && cudaMemsetAsync(th, 0, sizeof(TeamHeader), st) != cudaSuccess)
                     rc = fail("spgemm numeric: clearing the team header failed");
                 if (!rc) {
-                    team_items_kernel<<<(unsigned)ceil_div(p->n2, 256), 256, 0, st>>>(
-                        p->n2, p->list2, p->cpos, per_entry, th, items, (unsigned)cap);
-                    launch_behind(team_clear_kernel, dim3((unsigned)sm_count() * 8), 256, 0, st, th, items, (unsigned)cap, p->list2,
+                    if (alone) items = nullptr;
+                    else
+                        team_items_kernel<<<(unsigned)ceil_div(p->n2, 256), 256, 0, st>>>(
+                            p->n2, p->list2, p->cpos, per_entry, th, items, (unsigned)cap);
+                    if (!alone) launch_behind(team_clear_kernel, dim3((unsigned)sm_count() * 8), 256, 0, st, th, items, (unsigned)cap, p->list2,
                                   p->cpos, p->semi, cval);
                     if (p->semi == COMET_B200_PLUS_TIMES) {
                         cudaFuncSetAttribute(bitmap_numeric_kernel<true, true>,
