@@ -29,7 +29,7 @@ spmm_long_rows_kernel(int64_t nrows, const int64_t *__restrict__ pos, int64_t li
     bool any = false;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x)
         any |= pos[r + 1] - pos[r] > limit;
-    if (any) *flag = call;
+    if (__syncthreads_or(any) && threadIdx.x == 0) *flag = call;       // 50,000 stores to one address took 100 us
 }
 
 template <typename V, int NI, int U, bool PAIR>
@@ -100,6 +100,25 @@ spmm_short_rows_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const
     }
 }
 
+// A call marks the word with its own number, so the word need not be cleared.  What an earlier use left there can only
+// be equal by chance, and then the kernels that take every matrix do the work.
+LongRows next_mark()
+{
+    static std::atomic<int64_t> calls{1};
+    void *flag = nullptr;
+    if (scratch(SLOT_FLAG, sizeof(int64_t), &flag)) return {nullptr, 0};
+    return {(const int64_t *)flag, calls.fetch_add(1) * 0x9e3779b97f4a7c1 + 0x5bd1e995};
+}
+
+int mark_long_rows(int64_t nrows, const int64_t *pos, int64_t limit, LongRows lr, cudaStream_t st)
+{
+    int64_t grid = ceil_div(nrows, 256);
+    if (grid > sm_count() * 8) grid = sm_count() * 8;
+    spmm_long_rows_kernel<<<(unsigned)grid, 256, 0, st>>>(nrows, pos, limit, (int64_t *)lr.flag, lr.call);
+    CB_LAUNCH_CHECK();
+    return 0;
+}
+
 template <typename V, int NI, int U, bool PAIR>
 static int launch_short(const SpmmCall &a, LongRows *lr)
 {
@@ -111,17 +130,9 @@ static int launch_short(const SpmmCall &a, LongRows *lr)
     if (limit < 128) limit = 128;
     if (limit > a.nnz / a.nrows * 3 + 16) limit = a.nnz / a.nrows * 3 + 16;
     if (limit > 0x7ffffff0) limit = 0x7ffffff0;        // a row's entries are counted in 32 bits
-    void *flag = nullptr;
-    CB_TRY(scratch(SLOT_FLAG, sizeof(int64_t), &flag));
-    // A call marks the word with its own number, so the word need not be cleared.  What an earlier use left there can only
-    // be equal by chance, and then the other kernels, which take every matrix, do the work.
-    static std::atomic<int64_t> calls{1};
-    lr->flag = (int64_t *)flag;
-    lr->call = calls.fetch_add(1) * 0x9e3779b97f4a7c1 + 0x5bd1e995;
-    int64_t g1 = ceil_div(a.nrows, 256);
-    if (g1 > sm_count() * 8) g1 = sm_count() * 8;
-    spmm_long_rows_kernel<<<(unsigned)g1, 256, 0, a.st>>>(a.nrows, a.pos, limit, (int64_t *)flag, lr->call);
-    CB_LAUNCH_CHECK();
+    *lr = next_mark();
+    if (!lr->flag) return -1;
+    CB_TRY(mark_long_rows(a.nrows, a.pos, limit, *lr, a.st));
     int64_t blocks = ceil_div(a.nrows, SHORT_THREADS / tp);
     if (blocks > resident / SHORT_THREADS) blocks = resident / SHORT_THREADS;
     const dim3 grid((unsigned)blocks, (unsigned)ceil_div(a.k, SHORT_SLICE));

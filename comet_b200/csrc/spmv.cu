@@ -10,11 +10,12 @@
 // a warp that adds its partial sum to y with one f64 atomic -- on a power-law
 // matrix the long rows sit next to each other and would otherwise all land in
 // the first few CTAs.
-// Between: equal tiles of A's path.  A power-law matrix of this size has its hub rows in a CTA or two, which one launch
-// waits for, and too few others to hide a list and its launches.  Microseconds, one launch / list / tiles:
+// From 2^18 to 2^20: equal tiles of A's path.  A power-law matrix of this size has its hub rows in a CTA or two, which one
+// launch waits for, and too few others to hide a list and its launches.
+// From 2^23 on a first kernel looks for long rows (3 us): without them the lane groups take the call and need no list, with
+// them the tiles do.  Microseconds, one launch / list / tiles:
 //   even rows: 262,144 entries 5.5 / 9 / 9    600,000 8.2 / 12 / 10.5    3.2 M 26 / 25 / 29    36 M 201 / 182 / 232
 //   R-MAT:     120,000 entries 18 / -  / 7.6  728,000 84 / 25 / 12       3 M 500 / 43 / 28     16 M 1150 / 133 / 107
-// The tiles would take large power-law matrices too, but nothing known at the launch tells those from large even ones.
 //
 // Bound: HBM, 8(n+1) + 16 nnz + 8 ncols + 8 nrows bytes per call, and the L1's rate for the gathered x, one line per entry
 // (57 us at one line a clock for 16 M entries of a power-law matrix).  Row pointers fetched a row ahead: R-MAT scale 20
@@ -31,6 +32,7 @@ static const int64_t DEFER_ROW = 64;       // with a work list: rows above this 
 static const int64_t SPMV_CHUNK = 256;     // entries per work-list chunk
 static const int64_t DEFER_MIN_NNZ = 1 << 20;
 static const int64_t TILES_MIN_NNZ = (1 << 18) + 1;
+static const int64_t LOOK_MIN_NNZ = 1 << 23;      // the look and two launches that return at once: 5 us, too much of 40
 static const int TILE_ITEMS = 8;           // steps per thread of a tile's CTA: 2^11 per tile
 
 template <bool PAIR>
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(SPMV_THREADS)
 spmv_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
             const int64_t *__restrict__ crd, const double *__restrict__ val,
             const double *__restrict__ x, double *__restrict__ y, int accumulate, int passes,
-            WorkHeader *hdr, Chunk *chunks, unsigned chunk_cap)
+            WorkHeader *hdr, Chunk *chunks, unsigned chunk_cap, LongRows lr)
 {
     constexpr int GROUPS = SPMV_THREADS / T;
     constexpr int ROWS = GROUPS * SPMV_PASSES;
@@ -90,7 +92,7 @@ spmv_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *_
     // touched before the wait, and the next kernel in the stream is allowed to set up from here on.  Without
     // the attribute both instructions do nothing.
     wait_for_previous();
-    let_next_start();
+    if (lr.flag && *lr.flag == lr.call) return;        // a matrix with long rows: the tiles'
     __syncthreads();
 
     const int64_t row0 = (int64_t)blockIdx.x * (GROUPS * passes);
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(SPMV_THREADS, 4)
 spmv_tiles_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
                   const int64_t *__restrict__ crd, const double *__restrict__ val, const double *__restrict__ x,
                   double *__restrict__ y, int accumulate, const int64_t *__restrict__ tile_row,
-                  const int64_t *__restrict__ tile_ent)
+                  const int64_t *__restrict__ tile_ent, LongRows lr)
 {
     constexpr int ITEMS = TILE_ITEMS, STEPS = SPMV_THREADS * ITEMS;
     __shared__ double prod[STEPS + STEPS / ITEMS];     // entry i at i + i / ITEMS: a thread's run of ITEMS hits every bank once
@@ -187,6 +189,7 @@ spmv_tiles_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int6
     __shared__ int warp_end[SPMV_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     wait_for_previous();
+    if (not_this(lr)) return;
     const int64_t r0 = tile_row[blockIdx.x], e0 = tile_ent[blockIdx.x];
     const int m = (int)(tile_row[blockIdx.x + 1] - r0), n = (int)(tile_ent[blockIdx.x + 1] - e0);
 
@@ -298,12 +301,12 @@ spmv_chunks_kernel(const int64_t *__restrict__ row_ids, const int64_t *__restric
 template <int T>
 static int launch_spmv(int64_t nrows, const int64_t *row_ids, const int64_t *pos, const int64_t *crd,
                        const double *val, const double *x, double *y, bool pair, bool vec,
-                       int accumulate, int64_t nnz, cudaStream_t st)
+                       int accumulate, int64_t nnz, LongRows lr, cudaStream_t st)
 {
     WorkHeader *hdr = nullptr;
     Chunk *chunks = nullptr;
     size_t cap = 0;
-    if (nnz >= DEFER_MIN_NNZ) {
+    if (nnz >= DEFER_MIN_NNZ && !lr.flag) {
         cap = (size_t)(nnz / SPMV_CHUNK + nnz / DEFER_ROW + 16);
         void *wl = nullptr;
         CB_TRY(scratch(SLOT_WORKLIST, sizeof(WorkHeader) + cap * sizeof(Chunk), &wl));
@@ -316,27 +319,14 @@ static int launch_spmv(int64_t nrows, const int64_t *row_ids, const int64_t *pos
     int passes = SPMV_PASSES;
     while (passes > 1 && ceil_div(nrows, (int64_t)GROUPS * passes) < (int64_t)sm_count() * 4) passes--;
     unsigned grid = (unsigned)ceil_div(nrows, (int64_t)GROUPS * passes);
-    // One-launch calls (no chunk list) are a few microseconds long.  With COMET_B200_SPMV_PDL=1 they are launched
-    // with programmatic stream serialization, which lets the next grid be set up under the tail of this one.
-    // Off by default: measured on B200 in a CUDA graph of back-to-back calls (16384 rows x 16) it gave 3.49 against
-    // 3.89 us per call at 10 calls and 4.04 against 3.56 us at 1000, so nothing consistent; the empty-kernel floor of
-    // the same graphs is 0.73 us per launch, the rest is the kernel's own chain of dependent loads.
-    static const bool pdl = [] { const char *e = getenv("COMET_B200_SPMV_PDL"); return e && e[0] == '1'; }();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(SPMV_THREADS);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (pdl && !hdr) ? 1 : 0;
     const unsigned ucap = (unsigned)cap;
-#define GO(P, V) CB_CUDA(cudaLaunchKernelEx(&cfg, spmv_kernel<T, P, V>, nrows, row_ids, pos, crd, val, x, y, accumulate, passes, hdr, chunks, ucap))
-    if (pair) { if (vec) GO(true, true); else GO(true, false); }
-    else      { if (vec) GO(false, true); else GO(false, false); }
-#undef GO
+    auto kernel = pair ? (vec ? spmv_kernel<T, true, true> : spmv_kernel<T, true, false>)
+                       : (vec ? spmv_kernel<T, false, true> : spmv_kernel<T, false, false>);
+    if (lr.flag)
+        CB_CUDA(launch_behind(kernel, dim3(grid), SPMV_THREADS, 0, st, nrows, row_ids, pos, crd, val, x, y, accumulate, passes, hdr,
+                              chunks, ucap, lr));
+    else
+        kernel<<<grid, SPMV_THREADS, 0, st>>>(nrows, row_ids, pos, crd, val, x, y, accumulate, passes, hdr, chunks, ucap, lr);
     CB_LAUNCH_CHECK();
     if (hdr) {
         const unsigned g2 = (unsigned)sm_count() * 8;
@@ -365,20 +355,28 @@ int spmv_rows(int64_t nrows, int64_t nnz, const int64_t *row_ids, const int64_t 
     if (const char *env = getenv("COMET_B200_SPMV_LANES")) {        // tuning knob: lanes per row
         const int want = atoi(env);
         if (want == 2 || want == 4 || want == 8 || want == 16 || want == 32) t = want;
-    } else if (nnz >= TILES_MIN_NNZ && nnz < DEFER_MIN_NNZ) {
+    }
+    auto tiles = [&](LongRows lr) {
         StreamPlan plan;
         static_assert(SPMV_THREADS * TILE_ITEMS == 1 << 11, "steps per tile");
-        CB_TRY(piece_plan(nrows, nnz, 11, row_ids, pos, y, 1, 1, accumulate, LongRows{nullptr, 0}, st, &plan));
+        CB_TRY(piece_plan(nrows, nnz, 11, row_ids, pos, y, 1, 1, accumulate, lr, st, &plan));
         if (plan.nblocks > 0x7fffffffLL) return fail("spmv: too many rows");
         CB_CUDA(launch_behind(pair ? spmv_tiles_kernel<true> : spmv_tiles_kernel<false>, dim3((unsigned)plan.nblocks),
-                              SPMV_THREADS, 0, st, nrows, row_ids, pos, crd, val, x, y, accumulate, plan.block_row, plan.block_ent));
+                              SPMV_THREADS, 0, st, nrows, row_ids, pos, crd, val, x, y, accumulate, plan.block_row,
+                              plan.block_ent, lr));
         return 0;
+    };
+    if (nnz >= TILES_MIN_NNZ && nnz < DEFER_MIN_NNZ) return tiles(LongRows{nullptr, 0});
+    LongRows lr = {nullptr, 0};
+    if (nnz >= LOOK_MIN_NNZ) {
+        lr = next_mark();
+        if (!lr.flag) return -1;
+        // a lane group finishes 64 entries, or four times the mean, while its neighbours are still busy
+        CB_TRY(mark_long_rows(nrows, pos, nnz / nrows * 4 > 64 ? nnz / nrows * 4 : 64, lr, st));
     }
-    if (t == 2) return launch_spmv<2>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
-    if (t == 4) return launch_spmv<4>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
-    if (t == 8) return launch_spmv<8>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
-    if (t == 16) return launch_spmv<16>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
-    return launch_spmv<32>(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, st);
+    auto rows = t == 2 ? launch_spmv<2> : t == 4 ? launch_spmv<4> : t == 8 ? launch_spmv<8> : t == 16 ? launch_spmv<16> : launch_spmv<32>;
+    CB_TRY(rows(nrows, row_ids, pos, crd, val, x, y, pair, vec, accumulate, nnz, lr, st));
+    return lr.flag ? tiles(lr) : 0;
 }
 
 }  // namespace cb200

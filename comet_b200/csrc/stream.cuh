@@ -48,6 +48,10 @@ struct StreamPlan {
 // accumulate == 0: rows cut by a boundary get zeros (k columns).  The plan lives in the device's work-list slot.
 int piece_plan(int64_t nrows, int64_t nnz, int s, const int64_t *row_ids, const int64_t *pos, double *c, int64_t ldc,
                int64_t k, int accumulate, LongRows lr, cudaStream_t st, StreamPlan *out);
+// A word for a call's mark and the call's number (spmm_short.cu); flag == null on error.
+LongRows next_mark();
+// Marks the call if a row has more than `limit` entries.
+int mark_long_rows(int64_t nrows, const int64_t *pos, int64_t limit, LongRows lr, cudaStream_t st);
 // Pieces for `warps` persistent warps.  Returns 1, 0 when the piece count does not fit 32 bits, -1 on error.
 int stream_plan(int64_t nrows, int64_t nnz, int64_t warps, const int64_t *row_ids, const int64_t *pos, double *c,
                 int64_t ldc, int64_t k, int accumulate, LongRows lr, cudaStream_t st, StreamPlan *out);

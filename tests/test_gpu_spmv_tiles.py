@@ -26,7 +26,7 @@ def _matrix(kind, nnz, ncols=9001):
     return sp.csr_matrix((rng.uniform(-1, 1, nnz), rng.integers(0, ncols, nnz), pos), shape=(ends.size, ncols))
 
 
-@pytest.mark.parametrize("nnz", [1, 50000, (1 << 18), (1 << 18) + 1, 300007, (1 << 20) - 1, (1 << 20), 1200000])
+@pytest.mark.parametrize("nnz", [1, 50000, (1 << 18), (1 << 18) + 1, 300007, (1 << 20) - 1, (1 << 20), 1200000, (1 << 23), 9000000])
 @pytest.mark.parametrize("kind", ["hubs", "tiles", "ragged"])
 def test_sizes(kind, nnz):
     m = _matrix(kind, nnz)
