@@ -322,7 +322,7 @@ class SpMM(Workload):
 
 class SpMV(Workload):
     name = "spmv"
-    launches_per_step = 1     # one kernel below 2^20 stored entries, two (rows + long-row chunks) above
+    launches_per_step = 1     # one kernel up to 2^18 stored entries (the default), two or four above
 
     def build(self):
         from comet_b200 import datasets
@@ -447,7 +447,7 @@ class SpMV(Workload):
 
 class SDDMM(Workload):
     name = "sddmm"
-    launches_per_step = 2     # short-row stream kernel + long-row chunk kernel
+    launches_per_step = 2     # plan kernel + entry pieces
 
     def build(self):
         from comet_b200 import datasets
@@ -531,7 +531,7 @@ def _tail_sample(weights, fraction):
 
 class SpGEMM(Workload):
     name = "spgemm"
-    launches_per_step = 9     # narrow, bin, hash+bitmap symbolic, 3 scan kernels, hash+bitmap numeric
+    launches_per_step = 14    # bin, 2 publish, hash+mid+bitmap symbolic, 3 scan kernels, short+mid+bitmap numeric, 2 team kernels
 
     def build(self):
         from comet_b200 import datasets, sharding
@@ -661,7 +661,7 @@ class SpGEMM(Workload):
 
 class Triangles(Workload):
     name = "triangles"
-    launches_per_step = 6     # index narrowing, binning, four counting kernels (units, slow rows, CTA rows, warp rows)
+    launches_per_step = 17    # columns present (2), 2 scans of 3, 2 narrowings, rows, routing, scatter, units, three counting kernels
 
     def build(self):
         from comet_b200 import datasets, sharding
