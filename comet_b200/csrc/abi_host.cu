@@ -150,16 +150,37 @@ static int get_sparse(const char *what, int isz, int32_t f1, int32_t f2, int64_t
     return 0;
 }
 
+// End of a host entry point: the stream's work is done and every staged copy has reached the caller's arrays, also where
+// one of the two failed.
+static int finish(cudaStream_t st)
+{
+    const cudaError_t e = cudaStreamSynchronize(st);
+    const int rc = copies_drain();
+    if (e != cudaSuccess) return fail("the work of a host call failed: %s", cudaGetErrorString(e));
+    return rc;
+}
+
 // Device allocations of one call; freed (stream-ordered) when the object dies
 // unless released to a longer-lived owner.
 struct DevBag {
     cudaStream_t st;
     std::vector<void *> ptrs;
+    bool finished = false;
     explicit DevBag(cudaStream_t s) : st(s) {}
     ~DevBag()
     {
-        if (open) uploads_join();          // an early return: the copies still read the caller's arrays
+        if (open) uploads_join();
+        // an early return: queued copies still read the caller's arrays or write to them, and the caller gets them back
+        if (!finished) {
+            cudaStreamSynchronize(st);
+            copies_drain();
+        }
         for (void *p : ptrs) cudaFreeAsync(p, st);
+    }
+    int finish()
+    {
+        finished = true;
+        return cb200::finish(st);
     }
     // Between begin() and commit() the uploads below run side by side; what is made from them on the device (widened
     // indices and values) is launched by commit(), and so must be everything else that reads them.
@@ -348,13 +369,6 @@ static int verify_coords(const char *what, DevBag &bag, const int64_t *cols, int
     return 0;
 }
 
-// End of a host entry point: the stream's work is done and every staged copy has reached the caller's arrays.
-static int finish(cudaStream_t st)
-{
-    CB_CUDA(cudaStreamSynchronize(st));
-    return copies_drain();
-}
-
 static int need_stream(cudaStream_t *st)
 {
     int n = 0;
@@ -437,7 +451,7 @@ static int spmv_host(const HostSparse &A, Arr x, Arr y, int semiring, int accumu
     CB_TRY(comet_b200_dev_spmv_f64_i64(dA.nrows_k, A.nnz, dA.row_ids, dA.pos, dA.crd, dA.val, dx, dy,
                                        semiring, accumulate, st));
     CB_TRY(bag.download_val(y.data, dy, (size_t)A.nrows));
-    return finish(st);
+    return bag.finish();
 }
 
 // Large SpMM through the host entry point is bound by PCIe: B goes up, C comes back.  The two
@@ -614,7 +628,7 @@ static int spmm_host(const HostSparse &A, const Mat &B, const Mat &C, int semiri
     CB_TRY(comet_b200_dev_spmm_f64_i64(dA.nrows_k, A.ncols, A.nnz, k, dA.row_ids, dA.pos, dA.crd,
                                        dA.val, dB, B.s0, dC, C.s0, semiring, accumulate, 0, st));
     if (cbytes) CB_TRY(bag.download_val(C.data, dC, cbytes / 8));
-    return finish(st);
+    return bag.finish();
 }
 
 static void copy_pattern(const HostSparse &src, const HostSparse &dst)
@@ -752,7 +766,7 @@ static void sddmm_impl(int mode, COMET_B200_SPARSE2D(S), int64_t X_rank, void *X
         return;
     if (bag.download_val(O.val, dOut, (size_t)S.nnz)) return;
     copy_pattern(S, O);
-    finish(st);
+    bag.finish();
 }
 
 static void elews_sd_impl(int isz, COMET_B200_SPARSE2D(A), int64_t B_rank, void *B_ptr,
@@ -785,7 +799,7 @@ static void elews_sd_impl(int isz, COMET_B200_SPARSE2D(A), int64_t B_rank, void 
         return;
     if (A.nnz && d2h(C.val, dOut, (size_t)A.nnz * 8, st)) return;
     copy_pattern(A, C);
-    finish(st);
+    bag.finish();
 }
 
 // C (dense) = A (sparse) .* B (dense): products land at A's stored positions, the rest of C keeps its values.
@@ -828,7 +842,7 @@ static void elews_to_dense_impl(int isz, COMET_B200_SPARSE2D(A), int64_t B_rank,
                                                                dA.val, dB, B.s0, dC, C.s0, st))
         return;
     if (cbytes && d2h(C.data, dC, cbytes, st)) return;
-    finish(st);
+    bag.finish();
 }
 
 // n int64 indices on the device -> the caller's array of isz-byte integers
@@ -920,7 +934,7 @@ static void transpose_impl(int isz, int32_t A1format, int32_t A2format, int64_t 
     }
     if (download_idx(bag, ocrd, (char *)b2crd.data, nnz, isz, st)) return;
     if (nnz && d2h(bval.data, oval, (size_t)nnz * 8, st)) return;
-    if (finish(st)) return;
+    if (bag.finish()) return;
     idx_set((char *)sizes.data, 0, isz, ncols);
     idx_set((char *)sizes.data, 1, isz, nrows);
 }
@@ -965,7 +979,7 @@ static void dense_sparse_impl(int isz, int64_t A_rank, void *A_ptr, COMET_B200_S
                                                   lda, dC, ldc, semiring, accumulate, st))
         return;
     if (cbytes && d2h(hc, dC, cbytes, st)) return;
-    finish(st);
+    bag.finish();
 }
 
 // cm != null (sharded): A, M and the output are this rank's row block, B is the replicated operand.
@@ -1024,7 +1038,7 @@ static int64_t sparse_out_symbolic(int isz, int kind, const HostSparse &A, const
         }
         pos_src = p32;
     }
-    if (d2h(cpos.data, pos_src, (size_t)(A.nrows + 1) * isz, st) || finish(st)) {
+    if (d2h(cpos.data, pos_src, (size_t)(A.nrows + 1) * isz, st) || bag.finish()) {
         comet_b200_handle_destroy(dev_handle);
         return fail("sparse output: copy of C2pos failed"), 0;
     }
@@ -1201,7 +1215,7 @@ static void masked_count_impl(int mode, COMET_B200_SPARSE2D(A), COMET_B200_SPARS
         return;
     if (comm_allreduce_sum_i64(cm, dcount, 1, st)) return;
     if (cudaMemcpyAsync(out.data, dcount, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess) { fail("masked count: copy failed"); return; }
-    finish(st);
+    bag.finish();
 }
 
 // ---------------------------------------------------------------------------
@@ -1352,5 +1366,5 @@ extern "C" int32_t comet_b200_host_coo_to_csr(int64_t nrows, int64_t ncols, int6
     CB_TRY(d2h(crd, dcrd, bytes, st));
     CB_TRY(d2h(val, dval, bytes, st));
     CB_TRY(d2h(pos, dpos, (size_t)(nrows + 1) * 8, st));
-    return finish(st);
+    return bag.finish();
 }

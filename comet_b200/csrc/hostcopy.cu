@@ -305,7 +305,10 @@ int staged(Pool *p, bool to_device, const Piece &pc, cudaStream_t st)
             } else {
                 cudaError_t e = flat ? cudaMemcpyAsync(s.buf, dev, nb * nr, cudaMemcpyDeviceToHost, st)
                                      : cudaMemcpy2DAsync(s.buf, nb, dev, dev_pitch, nb, nr, cudaMemcpyDeviceToHost, st);
-                if (e == cudaSuccess) e = cudaEventRecord(s.ev, st);
+                if (e == cudaSuccess) {
+                    e = cudaEventRecord(s.ev, st);
+                    if (e != cudaSuccess) cudaStreamSynchronize(st);        // the copy into the chunk
+                }
                 if (e != cudaSuccess) {
                     p->release(si);
                     return fail("staged copy to the host failed: %s", cudaGetErrorString(e));

@@ -1,0 +1,33 @@
+"""The host layer's own code (staged copies, result memory) built with g++ against a stand-in for the CUDA runtime
+(tests/cpu_checks/fake_cuda.hpp), whose calls can be made to fail."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CHECKS = os.path.join(ROOT, "tests", "cpu_checks")
+CSRC = os.path.join(ROOT, "comet_b200", "csrc")
+
+
+def build(exe, check, *sources):
+    # the entry points of other files are not called
+    subprocess.check_call(["g++", "-O1", "-g", "-std=c++17", "-pthread", "-I/usr/local/cuda/include", "-x", "c++",
+                           os.path.join(CHECKS, check)] + [os.path.join(CSRC, s) for s in sources] +
+                          ["-no-pie", "-Wl,--unresolved-symbols=ignore-in-object-files", "-o", exe])
+    return exe
+
+
+@pytest.fixture(scope="module")
+def download_errors(tmp_path_factory):
+    return build(str(tmp_path_factory.mktemp("checks") / "download_errors"), "download_errors_check.cpp", "abi_host.cu",
+                 "hostcopy.cu")
+
+
+@pytest.mark.parametrize("memory,call,n", [("pinned", "copy", 2), ("pinned", "copy", 3), ("pageable", "copy", 2),
+                                           ("pageable", "copy", 4), ("pageable", "copy", 6), ("pinned", "sync", 1),
+                                           ("pageable", "sync", 1)])
+def test_a_call_that_failed_no_longer_writes_to_its_results(download_errors, memory, call, n):
+    out = subprocess.run([download_errors, memory, call, str(n)], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert out.returncode == 0, out.stdout
+    assert out.stdout == "returned 1\n"
