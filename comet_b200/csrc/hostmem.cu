@@ -6,8 +6,8 @@
 // result of about the same size.  The pool never makes a caller wait: a request it has no block for is answered with
 // null (the caller uses ordinary memory), and from the second such request of a size on a background thread
 // page-locks one more block.  Blocks in use and kept together stay below 1 GiB and an eighth of the machine's memory;
-// beyond that kept blocks of other sizes are given up, and then requests are refused.  comet_b200_release_scratch()
-// gives back every block that is not in use.
+// beyond that kept blocks of other sizes are given up, which is the background thread's work too (cudaFreeHost waits for
+// the device), and then requests are refused.  comet_b200_release_scratch() gives back every block that is not in use.
 #include <unistd.h>
 
 #include <map>
@@ -52,8 +52,24 @@ size_t rounded(size_t bytes)
     return (bytes + step - 1) / step * step;
 }
 
-void grow(size_t size, int device)
+using Blocks = std::vector<std::pair<void *, size_t>>;
+
+// gives blocks back that are on no list any more; without the lock
+void give_back(const Blocks &blocks)
 {
+    if (blocks.empty()) return;
+    size_t bytes = 0;
+    for (const auto &b : blocks) {
+        cudaFreeHost(b.first);
+        bytes += b.second;
+    }
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_held -= bytes;
+}
+
+void grow(size_t size, int device, Blocks given_up)
+{
+    give_back(given_up);
     void *p = nullptr;
     const bool ok = cudaSetDevice(device) == cudaSuccess && cudaHostAlloc(&p, size, cudaHostAllocPortable) == cudaSuccess;
     if (!ok) (void)cudaGetLastError();
@@ -67,15 +83,16 @@ void grow(size_t size, int device)
 
 void result_release_kept()
 {
-    std::lock_guard<std::mutex> lk(g_mu);
-    for (auto &s : g_sizes) {
-        for (void *p : s.second.kept) {
-            cudaFreeHost(p);
-            g_held -= s.first;
+    Blocks all;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        for (auto &s : g_sizes) {
+            for (void *p : s.second.kept) all.emplace_back(p, s.first);
+            s.second.kept.clear();
+            s.second.misses = 0;
         }
-        s.second.kept.clear();
-        s.second.misses = 0;
     }
+    give_back(all);
 }
 
 }  // namespace cb200
@@ -94,21 +111,25 @@ extern "C" void *comet_b200_result_alloc(int64_t bytes)
         return p;
     }
     if (++s.misses < 2 || g_growing || size > limit()) return nullptr;
-    for (auto it = g_sizes.begin(); g_held + size > limit() && it != g_sizes.end(); ++it)
-        while (g_held + size > limit() && !it->second.kept.empty()) {
-            cudaFreeHost(it->second.kept.back());
-            it->second.kept.pop_back();
-            g_held -= it->first;
-        }
+    size_t kept = 0;
+    for (const auto &o : g_sizes) kept += o.first * o.second.kept.size();
     int device = 0;
-    if (g_held + size > limit() || cudaGetDevice(&device) != cudaSuccess) return nullptr;
+    if (g_held - kept + size > limit() || cudaGetDevice(&device) != cudaSuccess) return nullptr;
     // a process that ends waits for the block being made (registered after the CUDA runtime's own handler, so run before it)
     static const bool registered = std::atexit([] { if (g_grower.joinable()) g_grower.join(); }) == 0;
     if (!registered) return nullptr;
     if (g_grower.joinable()) g_grower.join();          // g_growing is false: it has ended, or is about to return
+    Blocks given_up;                                   // they count as held until they are free
+    size_t over = g_held + size > limit() ? g_held + size - limit() : 0;
+    for (auto it = g_sizes.begin(); over && it != g_sizes.end(); ++it)
+        while (over && !it->second.kept.empty()) {
+            given_up.emplace_back(it->second.kept.back(), it->first);
+            it->second.kept.pop_back();
+            over = over > it->first ? over - it->first : 0;
+        }
     g_held += size;
     g_growing = true;
-    g_grower = std::thread(grow, size, device);
+    g_grower = std::thread(grow, size, device, given_up);
     return nullptr;
 }
 

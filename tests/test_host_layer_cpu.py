@@ -31,3 +31,9 @@ def test_a_call_that_failed_no_longer_writes_to_its_results(download_errors, mem
     out = subprocess.run([download_errors, memory, call, str(n)], stdout=subprocess.PIPE, text=True, timeout=60)
     assert out.returncode == 0, out.stdout
     assert out.stdout == "returned 1\n"
+
+
+def test_the_result_pool_never_makes_a_caller_wait(tmp_path):
+    exe = build(str(tmp_path / "result_pool"), "result_pool_check.cpp", "hostmem.cu")
+    out = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert (out.returncode, out.stdout) == (0, "ok\n")
