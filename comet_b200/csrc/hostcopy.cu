@@ -24,6 +24,7 @@
 #include <mutex>
 #include <immintrin.h>
 #include <string.h>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -70,7 +71,10 @@ class Pool {
         if (n > 12) n = 12;
         slots_.reserve(SLAB_CHUNKS * MAX_SLABS);
         grow(1);
-        for (int i = 0; i < n; i++) workers_.emplace_back([this] { work(); });
+        try {
+            for (int i = 0; i < n; i++) workers_.emplace_back([this] { work(); });
+        } catch (const std::system_error &) {  // no more threads to be had: whoever waits for a copy carries queued ones out
+        }
     }
     bool usable() const { return slots_.size() >= 2; }
     int threads() const { return (int)workers_.size() + 1; }

@@ -12,6 +12,7 @@
 
 #include <map>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -127,9 +128,13 @@ extern "C" void *comet_b200_result_alloc(int64_t bytes)
             it->second.kept.pop_back();
             over = over > it->first ? over - it->first : 0;
         }
-    g_held += size;
-    g_growing = true;
-    g_grower = std::thread(grow, size, device, given_up);
+    try {
+        g_grower = std::thread(grow, size, device, given_up);
+        g_held += size;                                // it waits for the lock before it looks at either
+        g_growing = true;
+    } catch (const std::system_error &) {              // no thread to be had: everything stays as it was
+        for (const auto &b : given_up) g_sizes[b.second].kept.push_back(b.first);
+    }
     return nullptr;
 }
 

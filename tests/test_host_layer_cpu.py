@@ -37,3 +37,9 @@ def test_the_result_pool_never_makes_a_caller_wait(tmp_path):
     exe = build(str(tmp_path / "result_pool"), "result_pool_check.cpp", "hostmem.cu")
     out = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
     assert (out.returncode, out.stdout) == (0, "ok\n")
+
+
+def test_without_threads_the_caller_copies_and_nothing_is_thrown(tmp_path):
+    exe = build(str(tmp_path / "no_threads"), "no_threads_check.cpp", "hostcopy.cu", "hostmem.cu")
+    out = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert (out.returncode, out.stdout) == (0, "ok\n")
