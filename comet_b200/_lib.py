@@ -86,6 +86,7 @@ SIGNATURES = {
     "comet_b200_host_coo_to_csr": (c_int32, [c_int64] * 3 + [c_void_p] * 6),
     "comet_b200_result_alloc": (c_void_p, [c_int64]),
     "comet_b200_result_free": (None, [c_void_p]),
+    "comet_b200_result_size": (c_int64, [c_void_p]),
     "comet_b200_dev_gather_probe_f64_i64": (c_int32, [c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int32,
                                                       c_void_p, c_int64, c_void_p]),
 }

@@ -162,33 +162,24 @@ class _Packer:
 _EMPTY = np.zeros(0, dtype=np.int64)
 
 
-class _ResultBlock:
-    """Page-locked memory of the library's pool; goes back when the array made from it is gone."""
-    __slots__ = ("address", "free", "__array_interface__")
-
-    def __init__(self, address, nbytes):
-        self.address = address
-        self.free = _lib.load().comet_b200_result_free      # arrays may outlive this module's globals
-        self.__array_interface__ = {"data": (address, False), "shape": (nbytes,), "typestr": "|u1", "version": 3}
-
-    def __del__(self):
-        self.free(self.address)
-
-
 _RESULT_MIN = 1 << 18          # smaller results are not worth a block
+_POOL = ("comet_b200_result_alloc", "comet_b200_result_size", "comet_b200_result_free")
 
 
 def _result(shape, dtype):
     """A new array for a result that the call writes completely: in page-locked memory when the library has a block,
-    which the device then fills by DMA (an ordinary new array is first faulted in page by page)."""
+    which the device then fills by DMA (an ordinary new array is first faulted in page by page).  Either way the array
+    owns its memory."""
     dtype = np.dtype(dtype)
     n = dtype.itemsize
     for d in (shape if isinstance(shape, tuple) else (shape,)):
         n *= d
     if n >= _RESULT_MIN:
-        p = _lib.load().comet_b200_result_alloc(n)
-        if p:
-            return np.asarray(_ResultBlock(p, n)).view(dtype).reshape(shape)
+        _lib.load()
+        from . import _pycall
+        a = _pycall.new_result(*map(_lib.address, _POOL), dtype, shape)
+        if a is not None:
+            return a
     return np.empty(shape, dtype=dtype)
 
 

@@ -9,6 +9,8 @@ import subprocess
 import sys
 import sysconfig
 
+import numpy
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
@@ -79,7 +81,7 @@ def build_pycall(force=False):
     if not force and not _stale(PYCALL, [src]):
         return PYCALL
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           "-I" + sysconfig.get_paths()["include"], src, "-o", PYCALL]
+           "-I" + sysconfig.get_paths()["include"], "-I" + numpy.get_include(), src, "-o", PYCALL]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout)

@@ -148,3 +148,11 @@ extern "C" void comet_b200_result_free(void *p)
     g_sizes[it->second].kept.push_back(p);
     g_used.erase(it);
 }
+
+extern "C" int64_t comet_b200_result_size(void *p)
+{
+    using namespace cb200;
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_used.find(p);
+    return it == g_used.end() ? 0 : (int64_t)it->second;
+}

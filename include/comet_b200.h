@@ -634,9 +634,11 @@ COMET_B200_EXPORT int32_t comet_b200_host_coo_to_csr(int64_t nrows, int64_t ncol
 
 /* Page-locked memory for a result of `bytes` bytes, from a pool of at most 1 GiB that is kept between calls; NULL when the
    pool has no block of that size (it may have one the next time): use ordinary memory then.  Contents are undefined.
-   result_free gives a block back; both may be called from any thread. */
+   result_free gives a block back, result_size tells how many bytes a block in use has (0: not one of the pool's); all
+   may be called from any thread. */
 COMET_B200_EXPORT void *comet_b200_result_alloc(int64_t bytes);
 COMET_B200_EXPORT void comet_b200_result_free(void *p);
+COMET_B200_EXPORT int64_t comet_b200_result_size(void *p);
 
 /* Frees the library's scratch memory on the current device, and the kept result blocks. */
 COMET_B200_EXPORT void comet_b200_release_scratch(void);

@@ -1,5 +1,7 @@
 """Host arrays in and out: sizes at the edges of the staged copies (driver copy, one piece, several pieces, several
 chunks), sources at odd addresses, and result arrays from the page-locked pool."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -56,3 +58,23 @@ def test_sort_keys_of_every_width(shape, n):
     order = np.lexsort((np.arange(n), cols, rows))
     assert np.array_equal(C.a2pos, np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=shape[0]))]))
     assert np.array_equal(C.a2crd, cols[order]) and np.array_equal(C.val, vals[order])
+
+
+def test_results_from_the_pool_own_their_memory_and_can_be_resized():
+    A = api.SparseTensor("CSR", 60000, 60000, np.array([60000]), np.array([-1]), np.arange(60001), np.arange(60000),
+                         np.ones(60000))
+    x = np.arange(60000.0)
+    lib, ys = _lib.load(), []
+    for _ in range(400):                                    # the pool makes its blocks in the background
+        ys.append(api.spmv(A, x))
+        if lib.comet_b200_result_size(ys[-1].ctypes.data):
+            break
+        ys = ys[-1:]
+        time.sleep(0.005)
+    else:
+        pytest.fail("no result came from the pool")
+    y = ys.pop()
+    assert y.flags.owndata and y.base is None and np.array_equal(y, x)
+    p = y.ctypes.data
+    y.resize(200000, refcheck=False)
+    assert np.array_equal(y[:60000], x) and not y[60000:].any() and lib.comet_b200_result_size(p) == 0
