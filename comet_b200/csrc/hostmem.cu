@@ -2,12 +2,14 @@
 //
 // A new 64 MB array costs its user 37 ms of page faults on one core (4 KB pages; 2.5 ms on eight cores with large
 // ones) before or while the result is copied into it, and a pageable destination is staged on top; the DMA engine
-// writes a page-locked one in 1.2 ms.  Page-locking itself takes 30 ms per 64 MB, so blocks are kept for the next
-// result of about the same size.  The pool never makes a caller wait: a request it has no block for is answered with
+// writes a page-locked one in 1.2 ms.  Page-locking itself takes 11 ms per 64 MB, so blocks are kept for the next
+// result of about the same size.  A block is private memory that is page-locked afterwards, not cudaHostAlloc's: that is
+// mapped shared, so that a forked child would write to its parent's results (and takes 24 ms per 64 MB).  The pool never makes a caller wait: a request it has no block for is answered with
 // null (the caller uses ordinary memory), and from the second such request of a size on a background thread
 // page-locks one more block.  Blocks in use and kept together stay below 1 GiB and an eighth of the machine's memory;
-// beyond that kept blocks of other sizes are given up, which is the background thread's work too (cudaFreeHost waits for
+// beyond that kept blocks of other sizes are given up, which is the background thread's work too (it waits for
 // the device), and then requests are refused.  comet_b200_release_scratch() gives back every block that is not in use.
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <map>
@@ -45,12 +47,35 @@ size_t limit()
     return bytes;
 }
 
-// sizes are rounded up to eight steps per power of two
+// sizes are rounded up to whole pages and eight steps per power of two
 size_t rounded(size_t bytes)
 {
-    size_t step = 4096;
+    static const size_t page = sysconf(_SC_PAGESIZE) > 0 ? (size_t)sysconf(_SC_PAGESIZE) : 4096;
+    size_t step = page;
     while (step * 16 < bytes) step <<= 1;
     return (bytes + step - 1) / step * step;
+}
+
+// Page-locked memory of whole pages, large ones where they fit.
+void *make_block(size_t size)
+{
+    const size_t large = (size_t)2 << 20, align = size >= large ? large : 0;
+    char *m = (char *)mmap(nullptr, size + align, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (m == (char *)MAP_FAILED) return nullptr;
+    char *p = align ? (char *)(((uintptr_t)m + align - 1) & ~(uintptr_t)(align - 1)) : m;
+    if (p > m) munmap(m, p - m);
+    if (m + align > p) munmap(p + size, m + align - p);
+    if (align) madvise(p, size, MADV_HUGEPAGE);
+    if (cudaHostRegister(p, size, cudaHostRegisterPortable) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    munmap(p, size);
+    return nullptr;
+}
+
+void free_block(void *p, size_t size)
+{
+    cudaHostUnregister(p);
+    munmap(p, size);
 }
 
 using Blocks = std::vector<std::pair<void *, size_t>>;
@@ -61,7 +86,7 @@ void give_back(const Blocks &blocks)
     if (blocks.empty()) return;
     size_t bytes = 0;
     for (const auto &b : blocks) {
-        cudaFreeHost(b.first);
+        free_block(b.first, b.second);
         bytes += b.second;
     }
     std::lock_guard<std::mutex> lk(g_mu);
@@ -71,11 +96,9 @@ void give_back(const Blocks &blocks)
 void grow(size_t size, int device, Blocks given_up)
 {
     give_back(given_up);
-    void *p = nullptr;
-    const bool ok = cudaSetDevice(device) == cudaSuccess && cudaHostAlloc(&p, size, cudaHostAllocPortable) == cudaSuccess;
-    if (!ok) (void)cudaGetLastError();
+    void *p = cudaSetDevice(device) == cudaSuccess ? make_block(size) : nullptr;
     std::lock_guard<std::mutex> lk(g_mu);
-    if (ok) g_sizes[size].kept.push_back(p);
+    if (p) g_sizes[size].kept.push_back(p);
     else g_held -= size;
     g_growing = false;                     // last: the lock's release is all that follows
 }

