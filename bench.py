@@ -48,10 +48,10 @@ RTOL = 1e-12
 # capture at the full workload on one GPU) is kept in profiles/dram_traffic.json together with a hash of the
 # kernel sources it was taken from; it is reported only while those sources are unchanged.
 KERNEL_SOURCES = {
-    "spmm": ["spmm_stream.cu", "stream.cuh", "spmm.cu"],
-    "sddmm": ["sddmm.cu"],
-    "spgemm": ["spgemm.cu", "util.cu"],
-    "triangles": ["tc.cu"],
+    "spmm": ["spmm.cu", "spmm.cuh", "spmm_short.cu", "spmm_pieces.cu", "spmm_stream.cu", "stream.cuh", "common.cuh"],
+    "sddmm": ["sddmm.cu", "stream.cuh", "common.cuh"],
+    "spgemm": ["spgemm.cu", "semiring.cuh", "stream.cuh", "util.cu", "common.cuh"],
+    "triangles": ["tc.cu", "pairs.cuh", "semiring.cuh", "util.cu", "common.cuh"],
 }
 
 
