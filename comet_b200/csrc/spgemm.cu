@@ -578,7 +578,10 @@ short_rows_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__restr
 // --------------------------------------------------------------------------
 static const int MID_MANY_WORDS = 2048;     // 256 threads from here on, as fewer CTAs fit: 180,000 rows of 20, 4250 -> 3410 us (at 50,000 columns 845 -> 900)
 static const int MID_ROW_MAX = 1024;
-static const int MID_WORDS = 8192;
+// The bitmap and its ranks, beside the 29 KB the kernel has anyway in 227: 1,070,400 columns.  It is the faster one as far as it
+// goes, where one CTA is left on an SM too.  Both calls, rows of 20, in milliseconds here and in bin 2: 262,200 columns 7.1 and
+// 12.0, 400,000 12.0 and 25.5, 700,000 48 and 100, 1,000,000 90 and 287; rows of 30 and 1,000,000 columns 113 and 301.
+static const size_t MID_SMEM = 196 * 1024;
 
 template <int THREADS, bool NUMERIC>
 __global__ void __launch_bounds__(THREADS)
@@ -1212,7 +1215,7 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     auto pad = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
     const size_t b_cnt = pad(((size_t)nrows + 1) * 8), b_crd = pad((size_t)nnz_b * 4 + 8), b_list = pad((size_t)nrows * 4);
     char *mem = nullptr;
-    const bool mid = !mpos && p->words <= MID_WORDS;
+    const bool mid = !mpos && mid_smem(p->words, true) <= MID_SMEM;
     STEP(dev_alloc(&mem, 256 + b_cnt + b_crd + (mid ? 3 : 2) * b_list, st));
     p->mem = mem;
     p->bin_counts = (unsigned *)mem;

@@ -56,3 +56,8 @@ def test_rows_at_the_limits(kind, ncols, semiring):
         keys = sorted(want)
         assert np.array_equal(crd[pos[r]:pos[r + 1]], keys)
         assert np.allclose(val[pos[r]:pos[r + 1]], [want[j] for j in keys], rtol=1e-12, atol=1e-13)
+
+
+@pytest.mark.parametrize("ncols", [1070400, 1070401])      # the most columns whose bitmap fits the 257-to-1024 kernel, one more
+def test_the_widest_matrices(ncols):
+    test_rows_at_the_limits("mixed", ncols, api.PLUS_TIMES)
