@@ -39,6 +39,14 @@ namespace {
 // staging 14.  Waking a worker takes 12 us and the DMA engine reads the chunks while others are written, so few threads with
 // large pieces beat many with small ones (4.3 MB / 17 MB / 70 MB in and out: five threads and pieces of 1.5 MB 225 / 601 /
 // 3500 us, eight and 512 KB 272 / 639 / 3580).
+//
+// What a worker reads of the caller's arrays is in its core's caches afterwards, and the caller's next writes there have to
+// take the lines back.  A program that rewrites its operands before each call pays for that what the workers saved, and more
+// while the arrays fit the caches.  Microseconds to write operands of 4.2 / 10.2 / 25.6 MB and to multiply by them (SpMV,
+// rows of 16), by number of workers: none 249 + 375 / 612 + 735 / 1590 + 1940, one 409 + 310 / 890 + 530 / 2000 + 1220, two
+// 690 + 309 / 1193 + 481 / 2085 + 915, five 890 + 332 / 1820 + 520 / 2730 + 890; the driver's own copies 252 + 410 / 610 +
+// 767 / 1810 + 1980.  So there is a worker for every BYTES_PER_WORKER that wait to be copied, none for a few MB.
+const size_t BYTES_PER_WORKER = (size_t)8 << 20;
 const size_t CHUNK = (size_t)2 << 20;     // bytes per page-locked chunk
 const int SLAB_CHUNKS = 8;                // chunks are allocated 16 MiB at a time (7 ms each),
 const int MAX_SLABS = 4;                  // at most 64 MiB per device
@@ -126,15 +134,22 @@ class Pool {
     }
     Slot &slot(int i) { return slots_[i]; }
 
-    void submit(std::function<void()> fn, Batch *batch = nullptr)
+    void submit(std::function<void()> fn, size_t bytes, Batch *batch = nullptr)
     {
+        bool wake;
         {
             std::lock_guard<std::mutex> lk(mu_);
-            tasks_.push_back(Task{std::move(fn), batch});
+            tasks_.push_back(Task{std::move(fn), batch, bytes});
             pending_++;
+            pending_bytes_ += bytes;
             if (batch) batch->left++;
+            wake = awake_ < workers_.size() && (awake_ + 1) * BYTES_PER_WORKER <= pending_bytes_;
+            if (wake) {
+                awake_++;
+                calls_++;
+            }
         }
-        cv_task_.notify_one();
+        if (wake) cv_task_.notify_one();
     }
     // waits until the tasks of one batch have run, doing queued ones meanwhile
     void wait(Batch *batch)
@@ -166,6 +181,7 @@ class Pool {
         t.fn();
         lk.lock();
         pending_--;
+        pending_bytes_ -= t.bytes;
         if (t.batch) t.batch->left--;
         if (pending_ == 0 || (t.batch && t.batch->left == 0)) cv_done_.notify_all();
         return true;
@@ -175,13 +191,17 @@ class Pool {
         cudaSetDevice(device_);
         std::unique_lock<std::mutex> lk(mu_);
         while (true) {
-            cv_task_.wait(lk, [this] { return !tasks_.empty(); });
-            run_one(lk);
+            cv_task_.wait(lk, [this] { return calls_ > 0; });
+            calls_--;
+            while (run_one(lk)) {
+            }
+            awake_--;
         }
     }
     struct Task {
         std::function<void()> fn;
         Batch *batch = nullptr;
+        size_t bytes = 0;
     };
     int device_;
     std::vector<Slot> slots_;
@@ -191,6 +211,8 @@ class Pool {
     std::mutex mu_;
     std::condition_variable cv_free_, cv_task_, cv_done_;
     int pending_ = 0, slabs_ = 0;
+    size_t pending_bytes_ = 0;             // of tasks that have not run
+    size_t awake_ = 0, calls_ = 0;         // workers at work or called, calls not heard yet
     std::atomic<bool> failed_{false};
 };
 
@@ -305,7 +327,7 @@ int staged(Pool *p, bool to_device, const Piece &pc, cudaStream_t st)
                     if (e != cudaSuccess) p->fail_flag();
                     sl.dma_pending = true;
                     p->release(si);
-                }, batch);
+                }, nb * nr, batch);
             } else {
                 cudaError_t e = flat ? cudaMemcpyAsync(s.buf, dev, nb * nr, cudaMemcpyDeviceToHost, st)
                                      : cudaMemcpy2DAsync(s.buf, nb, dev, dev_pitch, nb, nr, cudaMemcpyDeviceToHost, st);
@@ -322,7 +344,7 @@ int staged(Pool *p, bool to_device, const Piece &pc, cudaStream_t st)
                     if (cudaEventSynchronize(sl.ev) != cudaSuccess) p->fail_flag();
                     else copy_rows(host, host_pitch, sl.buf, nb, nb, nr);
                     p->release(si);
-                });
+                }, nb * nr);
             }
         }
     }

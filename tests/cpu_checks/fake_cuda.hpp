@@ -16,6 +16,7 @@
 #include <functional>
 #include <map>
 #include <mutex>
+#include <set>
 #include <thread>
 
 namespace fake {
@@ -28,6 +29,7 @@ static std::atomic<int> frees{0}, freeing{0};
 static std::atomic<int> free_ms{0};            // what giving back page-locked memory takes
 
 static std::mutex pinned_mu;
+static std::set<std::thread::id> copiers;      // threads that have queued a copy
 static std::map<char *, size_t> pinned;
 
 inline bool is_pinned(const void *p)
@@ -168,6 +170,10 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p)
 cudaError_t cudaMemcpy2DAsync(void *dst, size_t dp, const void *src, size_t sp, size_t w, size_t h, cudaMemcpyKind kind, cudaStream_t st)
 {
     if (kind == cudaMemcpyDeviceToHost && fake::due(fake::fail_download)) return cudaErrorUnknown;
+    {
+        std::lock_guard<std::mutex> lk(fake::pinned_mu);
+        fake::copiers.insert(std::this_thread::get_id());
+    }
     auto copy = [=] {
         for (size_t r = 0; r < h; r++) memcpy((char *)dst + r * dp, (const char *)src + r * sp, w);
     };

@@ -43,3 +43,9 @@ def test_without_threads_the_caller_copies_and_nothing_is_thrown(tmp_path):
     exe = build(str(tmp_path / "no_threads"), "no_threads_check.cpp", "hostcopy.cu", "hostmem.cu")
     out = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
     assert (out.returncode, out.stdout) == (0, "ok\n")
+
+
+def test_operands_of_a_few_mb_are_copied_by_the_caller(tmp_path):
+    exe = build(str(tmp_path / "copy_workers"), "copy_workers_check.cpp", "hostcopy.cu")
+    out = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert (out.returncode, out.stdout) == (0, "1 several\n")
