@@ -22,7 +22,6 @@
 #include <deque>
 #include <functional>
 #include <mutex>
-#include <immintrin.h>
 #include <string.h>
 #include <system_error>
 #include <thread>
@@ -30,6 +29,7 @@
 
 #include "common.cuh"
 #include "hostcopy.cuh"
+#include "streamcopy.cuh"
 
 namespace cb200 {
 
@@ -253,33 +253,6 @@ struct Piece {
     char *dev;
     size_t rows, row_bytes, host_pitch, dev_pitch;
 };
-
-// Into a chunk that the DMA engine reads next: with streaming stores the bytes go to memory; left modified in the
-// caches of the cores that copied them, each line is first fetched from there (4.5 MB: 400 us of DMA instead of 90).
-__attribute__((target("avx2"))) void copy_streaming(char *dst, const char *src, size_t n)
-{
-    while (n && ((uintptr_t)dst & 31)) { *dst++ = *src++; n--; }
-    for (; n >= 128; n -= 128, src += 128, dst += 128) {
-        const __m256i a = _mm256_loadu_si256((const __m256i *)src), b = _mm256_loadu_si256((const __m256i *)(src + 32));
-        const __m256i c = _mm256_loadu_si256((const __m256i *)(src + 64)), d = _mm256_loadu_si256((const __m256i *)(src + 96));
-        _mm256_stream_si256((__m256i *)dst, a);
-        _mm256_stream_si256((__m256i *)(dst + 32), b);
-        _mm256_stream_si256((__m256i *)(dst + 64), c);
-        _mm256_stream_si256((__m256i *)(dst + 96), d);
-    }
-    _mm_sfence();
-    memcpy(dst, src, n);
-}
-
-void fill_chunk(char *dst, const char *src, size_t spitch, size_t row_bytes, size_t rows)
-{
-    static const bool streaming = __builtin_cpu_supports("avx2");
-    if (spitch == row_bytes) { row_bytes *= rows; rows = 1; }
-    for (size_t r = 0; r < rows; r++) {
-        if (streaming) copy_streaming(dst + r * row_bytes, src + r * spitch, row_bytes);
-        else memcpy(dst + r * row_bytes, src + r * spitch, row_bytes);
-    }
-}
 
 void copy_rows(char *dst, size_t dpitch, const char *src, size_t spitch, size_t row_bytes, size_t rows)
 {

@@ -49,3 +49,26 @@ def test_operands_of_a_few_mb_are_copied_by_the_caller(tmp_path):
     exe = build(str(tmp_path / "copy_workers"), "copy_workers_check.cpp", "hostcopy.cu")
     out = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
     assert (out.returncode, out.stdout) == (0, "1 several\n")
+
+
+@pytest.mark.parametrize("host", [[], ["-DNOT_X86"]])
+def test_chunks_are_filled_on_any_host(tmp_path, host):
+    exe = str(tmp_path / "streamcopy")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-o", exe, os.path.join(CHECKS, "streamcopy_check.cpp")] + host)
+    out = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert (out.returncode, out.stdout) == (0, "ok\n")
+
+
+def test_no_source_needs_an_x86_host():
+    """Intrinsics and their header stand behind the architecture's macro."""
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh", ".cpp")):
+            continue
+        depth = 0
+        with open(os.path.join(CSRC, name)) as f:
+            for line in f:
+                if line.startswith("#if"):
+                    depth = depth + 1 if depth or "__x86_64__" in line else 0
+                elif line.startswith("#endif"):
+                    depth = max(depth - 1, 0)
+                assert depth or not any(w in line for w in ("immintrin.h", "__m256", "_mm_", "_mm256_")), (name, line)
