@@ -3,23 +3,34 @@
 // A group of T lanes (T chosen from the mean row length) walks one row with
 // 128-bit loads of crd and val (two entries per load), the next row's pointers on their way.
 //
-// Up to 2^18 stored entries: one launch, no scratch memory; rows of more than 16 T entries are left to the end of the CTA,
-// where a warp, or for very long ones all 256 threads, walk them; the summation order per row is fixed.
+// One launch of lane groups, while A's path of entries and row ends has fewer tiles of 2^11 steps than the chip has SMs; no
+// scratch memory.  Rows of more than 16 T entries are left to the end of the CTA, where a warp, or for very long ones all 256
+// threads, walk them.
+// From there to 2^20 entries: the tiles, a CTA each, in one launch and without scratch memory too.  A power-law matrix of this
+// size has its hub rows in a CTA or two of lane groups, which the launch waits for.
+// Both give the same sums to the bit in every call.
 // From 2^20 on: rows longer than DEFER_ROW entries are cut into chunks that
 // go to a work list in scratch memory, and a second launch gives each chunk to
 // a warp that adds its partial sum to y with one f64 atomic -- on a power-law
 // matrix the long rows sit next to each other and would otherwise all land in
 // the first few CTAs.
-// From 2^18 to 2^20: equal tiles of A's path.  A power-law matrix of this size has its hub rows in a CTA or two, which one
-// launch waits for, and too few others to hide a list and its launches.
 // From 2^23 on a first kernel looks for long rows (3 us): without them the lane groups take the call and need no list, with
-// them the tiles do.  Microseconds, one launch / list / tiles:
-//   even rows: 262,144 entries 5.5 / 9 / 9    600,000 8.2 / 12 / 10.5    3.2 M 26 / 25 / 29    36 M 201 / 182 / 232
-//   R-MAT:     120,000 entries 18 / -  / 7.6  728,000 84 / 25 / 12       3 M 500 / 43 / 28     16 M 1150 / 133 / 107
+// them planned tiles do.
+//
+// Microseconds of back-to-back calls in a CUDA graph, lane groups in one launch / tiles in one launch:
+//   even rows of 16:  60,000 entries 2.8 / 5.5    262,144 3.8 / 6.2    600,000 5.3 / 8.6    960,000 7.3 / 10.3
+//   rows of 0 to 20:  500,000 6.5 / 7.1           rows of 60: 300,000 3.8 / 5.8
+//   R-MAT:            25,500 8 / 6.3    120,000 17 / 8.4    228,000 20 / 8.1    468,000 51 / 8.8    728,000 88 / 10.9
+//   100,000 rows of 4 and one of 300,000: 269 / 10.3
+// (launched one by one the calls are 8 to 10 apart either way).  Only the device knows how long the rows are, and tiles are
+// the ones that no matrix makes slow, so they take over as soon as they fill the chip.
+// With a list / planned tiles: even rows 3.2 M entries 25 / 29, 36 M 182 / 232; R-MAT 3 M 43 / 28, 16 M 133 / 107.
 //
 // Bound: HBM, 8(n+1) + 16 nnz + 8 ncols + 8 nrows bytes per call, and the L1's rate for the gathered x, one line per entry
 // (57 us at one line a clock for 16 M entries of a power-law matrix).  Row pointers fetched a row ahead: R-MAT scale 20
 // 146 -> 133 us, 36 M entries in even rows 202 -> 182.
+#include <atomic>
+
 #include "common.cuh"
 #include "stream.cuh"
 
@@ -31,9 +42,12 @@ static const int64_t LONG_ROW = 2048;
 static const int64_t DEFER_ROW = 64;       // with a work list: rows above this go to it
 static const int64_t SPMV_CHUNK = 256;     // entries per work-list chunk
 static const int64_t DEFER_MIN_NNZ = 1 << 20;
-static const int64_t TILES_MIN_NNZ = (1 << 18) + 1;
 static const int64_t LOOK_MIN_NNZ = 1 << 23;      // the look and two launches that return at once: 5 us, too much of 40
-static const int TILE_ITEMS = 8;           // steps per thread of a tile's CTA: 2^11 per tile
+static const int TILE_ITEMS = 8;           // steps per thread of a tile's CTA
+static const int TILE_SHIFT = 11;          // 2^11 per tile
+static const int ONCE_PAST = SPMV_THREADS; // one launch: a row that ends so many steps behind a tile is not cut
+static const int ONCE_TILES = 1024;        // one launch: most tiles
+static const int ONCE_SLOTS = 16;          // one launch: calls in a row that use memory of their own
 
 template <bool PAIR>
 __device__ __forceinline__ double combine(double a, double b)
@@ -168,30 +182,151 @@ spmv_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *_
     }
 }
 
-// Equal tiles of A's path (one step per stored entry and one per row end), a CTA each.  The products of a tile's entries are
-// made with all loads in flight and put into shared memory; every thread then walks eight steps of the merged list of
-// entries and row ends, and sums of rows that reach over threads travel by a segmented scan.  A row cut by a tile boundary
-// is added with atomics onto a zero written by the plan.
+// Equal tiles of A's path (one step per stored entry and one per row end; the merge path of Merrill and Garland, Merge-based
+// Parallel Sparse Matrix-Vector Multiplication, 2016), a CTA each.  The products of a tile's entries are
+// made with all loads in flight and put into shared memory; every thread then walks eight or nine steps of the merged list of
+// entries and row ends, and sums of rows that reach over threads travel by a segmented scan.
 //
-// Bound: at the sizes it is used for, the latency of plan, entries and gathers (6 us) and then the L1's rate of line
-// accesses.  R-MAT scale 16, 728,000 entries: 86 -> 12 us.
-template <bool PAIR>
+// With a plan (piece_plan) a row cut by a tile boundary is added with atomics onto a zero that the plan has written.
+//
+// ONCE, for matrices of up to ONCE_TILES tiles: one launch.  A CTA finds its rows itself: a first round of probes looks at
+// the rows around where they would lie if all were alike and at places spread over the rest, which is all that even rows
+// take; a second is enough below 100,000 rows.  A row that ends up to ONCE_PAST steps behind a boundary stays with the tile
+// before it, so only long rows are cut: their tiles leave the parts in `cuts`, and the last one to do so adds them up in
+// order.  Nobody waits, and the sums of every call are the same to the bit.
+//
+// Bound: up to 2^20 entries the chain of probes, row ends, entries and gathers of a CTA (6 us); beyond, the L1's rate of line
+// accesses.
+struct CutRows {
+    double part[2 * ONCE_TILES];           // [2 b] of the row from before tile b, [2 b + 1] of the row that goes on behind it
+    unsigned arrived[ONCE_TILES];          // by the tile that the row starts in; zero between calls
+};
+static __device__ CutRows g_cut_rows[ONCE_SLOTS];
+
+// The rows and entries in which a tile and the next one start.  128 threads look for each, two probes at a time.
+__device__ __forceinline__ void once_bounds(int64_t tile, int nrows, int64_t nnz, const int64_t *__restrict__ pos, int64_t (&row)[2],
+                                            int64_t (&ent)[2])
+{
+    __shared__ int s_lo[2][2], s_hi[2][2];             // by round, so that one barrier does
+    __shared__ int64_t s_end[2];
+    const int which = threadIdx.x >> 7, i = threadIdx.x & 127;
+    const int64_t steps = nnz + nrows, d = (tile + which) << TILE_SHIFT;
+    if (threadIdx.x < 4) {
+        s_lo[threadIdx.x >> 1][threadIdx.x & 1] = 0;
+        s_hi[threadIdx.x >> 1][threadIdx.x & 1] = nrows;
+    }
+    if (i == 0) s_end[which] = -1;
+    __syncthreads();
+    // the row in whose steps (its entries, then its end) step d lies: the first with pos[r + 1] + r >= d
+    int lo = 0, hi = nrows;
+    for (int round = 0; round < 32; round++) {
+        if (lo < hi) {
+            const int64_t span = hi - lo;
+            int p[2];
+            if (round == 0) {
+                p[0] = (int)((double)d / (double)steps * nrows) - 64 + i;
+                p[1] = (int)(span * i / 128);
+            } else {
+                p[0] = lo + (int)(span * (2 * i) / 256);
+                p[1] = lo + (int)(span * (2 * i + 1) / 256);
+            }
+            int64_t b[2], e[2];
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                p[j] = p[j] < lo ? lo : p[j] >= hi ? hi - 1 : p[j];
+                b[j] = pos[p[j]] + p[j] - 1;           // last step of the row before
+                e[j] = pos[p[j] + 1] + p[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                if (e[j] < d) lo = p[j] + 1 > lo ? p[j] + 1 : lo;
+                else hi = p[j] < hi ? p[j] : hi;
+                if (e[j] >= d && b[j] < d) {           // this one
+                    lo = hi = p[j];
+                    s_end[which] = e[j];
+                }
+            }
+            lo = __reduce_max_sync(0xffffffffu, lo);
+            hi = __reduce_min_sync(0xffffffffu, hi);
+            if ((threadIdx.x & 31) == 0) {
+                atomicMax(&s_lo[round & 1][which], lo);
+                atomicMin(&s_hi[round & 1][which], hi);
+            }
+        }
+        __syncthreads();
+        lo = s_lo[round & 1][which];
+        hi = s_hi[round & 1][which];
+        if (s_lo[round & 1][0] >= s_hi[round & 1][0] && s_lo[round & 1][1] >= s_hi[round & 1][1]) {
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int64_t r = s_lo[round & 1][j], end = s_end[j], at = (tile + j) << TILE_SHIFT;     // end -1: behind the last row
+                const bool past = end >= 0 && end + 1 - at <= ONCE_PAST && at > 0;
+                row[j] = end < 0 ? nrows : past ? r + 1 : r;
+                ent[j] = end < 0 ? nnz : past ? end - r : at - r;
+            }
+            return;
+        }
+        // the other buffer starts the next round from these: it can only narrow
+        if (i == 0) {
+            s_lo[(round + 1) & 1][which] = lo;
+            s_hi[(round + 1) & 1][which] = hi;
+        }
+        __syncthreads();
+    }
+}
+
+// ONCE: this tile's part of row r, which is cut.  A warp; true for the last one to come, which has the sum of all tiles' parts.
+__device__ __forceinline__ bool once_add(CutRows *cuts, int64_t tile, int after, double part, int64_t r,
+                                            const int64_t *__restrict__ pos, double *total)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t first = (pos[r] + r) >> TILE_SHIFT, last = (pos[r + 1] + r - ONCE_PAST) >> TILE_SHIFT;
+    unsigned n = 0;
+    if (lane == 0) {
+        cuts->part[2 * tile + after] = part;
+        __threadfence();
+        n = atomicAdd(&cuts->arrived[first], 1u);
+    }
+    n = __shfl_sync(0xffffffffu, n, 0);
+    if (n != (unsigned)(last - first)) return false;
+    __threadfence();
+    double sum = 0.0;
+    for (int64_t q = first + lane; q <= last; q += 32) sum += __ldcg(&cuts->part[2 * q + (q == first)]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) cuts->arrived[first] = 0;
+    *total = sum;
+    return true;
+}
+
+template <bool PAIR, bool ONCE>
 __global__ void __launch_bounds__(SPMV_THREADS, 4)
-spmv_tiles_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
+spmv_tiles_kernel(int64_t nrows, int64_t nnz, const int64_t *__restrict__ row_ids, const int64_t *__restrict__ pos,
                   const int64_t *__restrict__ crd, const double *__restrict__ val, const double *__restrict__ x,
                   double *__restrict__ y, int accumulate, const int64_t *__restrict__ tile_row,
-                  const int64_t *__restrict__ tile_ent, LongRows lr)
+                  const int64_t *__restrict__ tile_ent, LongRows lr, int slot)
 {
-    constexpr int ITEMS = TILE_ITEMS, STEPS = SPMV_THREADS * ITEMS;
-    __shared__ double prod[STEPS + STEPS / ITEMS];     // entry i at i + i / ITEMS: a thread's run of ITEMS hits every bank once
+    constexpr int ITEMS = ONCE ? ((1 << TILE_SHIFT) + ONCE_PAST) / SPMV_THREADS : TILE_ITEMS, STEPS = SPMV_THREADS * ITEMS;
+    constexpr int PAD = ITEMS % 2 ? STEPS : ITEMS;     // entry i at i + i / PAD: a thread's run of ITEMS hits every bank once
+    __shared__ double prod[STEPS + STEPS / PAD];
     __shared__ int ends[STEPS + 2];                    // ends of the rows that end in the tile, counted from its first entry
     __shared__ double warp_sum[SPMV_THREADS / 32];
     __shared__ int warp_end[SPMV_THREADS / 32];
+    __shared__ double cut_part[2];                     // ONCE: of the row from before, of the row that goes on
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     wait_for_previous();
     if (not_this(lr)) return;
-    const int64_t r0 = tile_row[blockIdx.x], e0 = tile_ent[blockIdx.x];
-    const int m = (int)(tile_row[blockIdx.x + 1] - r0), n = (int)(tile_ent[blockIdx.x + 1] - e0);
+    int64_t row[2], ent[2];
+    if (ONCE) {
+        once_bounds(blockIdx.x, (int)nrows, nnz, pos, row, ent);
+    } else {
+        row[0] = tile_row[blockIdx.x];
+        row[1] = tile_row[blockIdx.x + 1];
+        ent[0] = tile_ent[blockIdx.x];
+        ent[1] = tile_ent[blockIdx.x + 1];
+    }
+    const int64_t r0 = row[0], e0 = ent[0];
+    const int m = (int)(row[1] - r0), n = (int)(ent[1] - e0);
 
     int64_t c[ITEMS];
     double v[ITEMS];
@@ -210,7 +345,7 @@ spmv_tiles_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int6
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
         const int p = tid + i * SPMV_THREADS;
-        if (p < n) prod[p + p / ITEMS] = PAIR ? 1.0 : v[i] * __ldg(x + c[i]);
+        if (p < n) prod[p + p / PAD] = PAIR ? 1.0 : v[i] * __ldg(x + c[i]);
     }
     __syncthreads();
 
@@ -234,7 +369,7 @@ spmv_tiles_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int6
     int next = a < m ? ends[a] : n + 1;
     for (int t = d; t < last; t++) {
         if (e < next) {
-            acc += prod[e + e / ITEMS];
+            acc += prod[e + e / PAD];
             e++;
         } else {
             if (a == a0) head = acc;
@@ -270,8 +405,23 @@ spmv_tiles_kernel(int64_t nrows, const int64_t *__restrict__ row_ids, const int6
             in += warp_sum[w];
             if (warp_end[w]) break;
         }
-    if (has) store(r0 + a0, in + head, a0 == 0 && cut);
-    if (tid == SPMV_THREADS - 1 && r0 + m < nrows && e0 + n > pos[r0 + m]) store(r0 + m, has ? acc : in + acc, true);
+    if (!ONCE) {
+        if (has) store(r0 + a0, in + head, a0 == 0 && cut);
+        if (tid == SPMV_THREADS - 1 && r0 + m < nrows && e0 + n > pos[r0 + m]) store(r0 + m, has ? acc : in + acc, true);
+        return;
+    }
+    const bool goes_on = r0 + m < nrows && e0 + n > pos[r0 + m], through = goes_on && cut && m == 0;
+    if (has) {
+        if (a0 == 0 && cut) cut_part[0] = in + head;
+        else store(r0 + a0, in + head, false);
+    }
+    if (tid == SPMV_THREADS - 1 && goes_on) cut_part[through ? 0 : 1] = has ? acc : in + acc;
+    __syncthreads();
+    if (warp == 0 ? cut : warp == 1 && goes_on && !through) {
+        const int64_t r = warp == 0 ? r0 : r0 + m;
+        double total = 0.0;
+        if (once_add(g_cut_rows + slot, blockIdx.x, warp, cut_part[warp], r, pos, &total) && lane == 0) store(r, total, false);
+    }
 }
 
 template <bool PAIR, bool VEC>
@@ -348,7 +498,7 @@ int spmv_rows(int64_t nrows, int64_t nnz, const int64_t *row_ids, const int64_t 
     bool pair = semiring == COMET_B200_PLUS_PAIR;
     double mean = (double)nnz / (double)nrows;
     int t = mean <= 4.0 ? 2 : mean <= 8.0 ? 4 : mean <= 24.0 ? 8 : mean <= 48.0 ? 16 : 32;
-    if (nnz < TILES_MIN_NNZ) {
+    if (nnz < DEFER_MIN_NNZ) {
         // lanes that would idle otherwise shorten the longest rows (R-MAT scale 14: 28 -> 18 us)
         while (t < 32 && nrows * t * 2 <= (int64_t)sm_count() * 2048) t *= 2;
     }
@@ -358,15 +508,22 @@ int spmv_rows(int64_t nrows, int64_t nnz, const int64_t *row_ids, const int64_t 
     }
     auto tiles = [&](LongRows lr) {
         StreamPlan plan;
-        static_assert(SPMV_THREADS * TILE_ITEMS == 1 << 11, "steps per tile");
-        CB_TRY(piece_plan(nrows, nnz, 11, row_ids, pos, y, 1, 1, accumulate, lr, st, &plan));
+        static_assert(SPMV_THREADS * TILE_ITEMS == 1 << TILE_SHIFT, "steps per tile");
+        CB_TRY(piece_plan(nrows, nnz, TILE_SHIFT, row_ids, pos, y, 1, 1, accumulate, lr, st, &plan));
         if (plan.nblocks > 0x7fffffffLL) return fail("spmv: too many rows");
-        CB_CUDA(launch_behind(pair ? spmv_tiles_kernel<true> : spmv_tiles_kernel<false>, dim3((unsigned)plan.nblocks),
-                              SPMV_THREADS, 0, st, nrows, row_ids, pos, crd, val, x, y, accumulate, plan.block_row,
-                              plan.block_ent, lr));
+        CB_CUDA(launch_behind(pair ? spmv_tiles_kernel<true, false> : spmv_tiles_kernel<false, false>, dim3((unsigned)plan.nblocks),
+                              SPMV_THREADS, 0, st, nrows, nnz, row_ids, pos, crd, val, x, y, accumulate, plan.block_row,
+                              plan.block_ent, lr, 0));
         return 0;
     };
-    if (nnz >= TILES_MIN_NNZ && nnz < DEFER_MIN_NNZ) return tiles(LongRows{nullptr, 0});
+    const int64_t ntiles = ceil_div(nnz + nrows, (int64_t)1 << TILE_SHIFT);
+    if (nnz < DEFER_MIN_NNZ && ntiles >= sm_count() && ntiles <= ONCE_TILES) {
+        static std::atomic<unsigned> calls{0};
+        CB_CUDA(launch_behind(pair ? spmv_tiles_kernel<true, true> : spmv_tiles_kernel<false, true>, dim3((unsigned)ntiles),
+                              SPMV_THREADS, 0, st, nrows, nnz, row_ids, pos, crd, val, x, y, accumulate, nullptr, nullptr,
+                              LongRows{nullptr, 0}, (int)(calls++ % ONCE_SLOTS)));
+        return 0;
+    }
     LongRows lr = {nullptr, 0};
     if (nnz >= LOOK_MIN_NNZ) {
         lr = next_mark();

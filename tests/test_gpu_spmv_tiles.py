@@ -43,3 +43,56 @@ def test_sizes(kind, nnz):
     ids = dev.DeviceCSR(2 * n, ncols, *arrays, row_ids=up(np.arange(n, dtype=np.int64) * 2 + 1))
     y = dev.spmv(ids, up(x)).cpu().numpy()
     assert np.all(np.abs(y[1::2] - ref) <= room) and not y[::2].any()
+
+
+def _boundaries(nnz):
+    """Rows that end just before, on and behind the step up to which a row stays with the tile it starts in, rows that start on
+    a boundary, and a row over more tiles than a warp has lanes."""
+    lens, step = [], 0
+
+    def row(n):
+        nonlocal step
+        lens.append(int(n))
+        step += n + 1
+
+    for behind in (0, 1, 2, 254, 255, 256, 257, 258, 2047, 2048, 2300, 2304, 2305, 6000):
+        for start in (2047, 2048 - 17, 0, 1):
+            row((start - 1 - step) % 2048)             # the next row starts `start` steps into a tile
+            if start:
+                row(2048 - step % 2048 + behind - 1)   # and ends `behind` steps behind a boundary
+    row(80000)
+    total = sum(lens)
+    lens += [7] * ((nnz - total) // 7) + [(nnz - total) % 7]
+    return np.array(lens)
+
+
+@pytest.mark.parametrize("nnz", [310000, (1 << 20) - 1])
+@pytest.mark.parametrize("kind", ["boundaries", "hubs", "middle", "one_row", "ragged"])
+def test_sums_keep_their_order(kind, nnz):
+    rng = np.random.default_rng(nnz)
+    ncols = 9001
+    if kind == "boundaries":
+        lens = _boundaries(nnz)
+    elif kind == "one_row":
+        lens = np.array([0, nnz, 0])
+    elif kind == "middle":                             # around the length from which a row is the tiles', cut and not
+        lens = rng.integers(0, 1100, nnz // 400)
+        lens = np.minimum(lens, np.maximum(nnz - np.concatenate([[0], np.cumsum(lens)[:-1]]), 0))
+        lens[-1] += nnz - lens.sum()
+    else:
+        lens = np.diff(_matrix(kind, nnz).indptr)
+    pos = np.concatenate([[0], np.cumsum(lens)])
+    crd, val, x = rng.integers(0, ncols, nnz), rng.uniform(-1, 1, nnz), rng.uniform(-1, 1, ncols)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    A = dev.DeviceCSR(lens.size, ncols, up(pos), up(crd), up(val))
+    y, y0 = dev.spmv(A, up(x)), rng.uniform(-1, 1, lens.size)
+    added = dev.spmv(A, up(x), up(y0), accumulate=True)
+    for _ in range(20):
+        assert torch.equal(y, dev.spmv(A, up(x)))
+        assert torch.equal(added, dev.spmv(A, up(x), up(y0), accumulate=True))
+    # any order of a row's n terms is off by at most n 2^-53 of the sum of their sizes
+    sums = lambda v: np.add.reduceat(np.concatenate([v, [0.0]]), np.minimum(pos[:-1], nnz)) * (lens > 0)
+    ref, size = sums(val * x[crd]), sums(np.abs(val * x[crd]))
+    assert np.all(np.abs(y.cpu().numpy() - ref) <= (lens + 1) * 2.0 ** -52 * size)
+    assert np.all(np.abs(added.cpu().numpy() - ref - y0) <= (lens + 2) * 2.0 ** -52 * (size + np.abs(y0)))
+    assert np.array_equal(dev.spmv(A, up(x), semiring=api.PLUS_PAIR).cpu().numpy(), lens)
