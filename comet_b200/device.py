@@ -77,8 +77,8 @@ def _call(name, *args):
 def spmv(A, x, y=None, semiring=PLUS_TIMES, accumulate=False):
     _check_cuda(A.pos, A.crd, A.val, x, y)
     if y is None:
-        # rows a DCSR matrix does not store, and the values that are added to, start at zero; any other row is written
-        new = torch.zeros if A.row_ids is not None or accumulate else torch.empty
+        # rows the matrix does not store, and the values that are added to, start at zero; any other row is written
+        new = torch.zeros if A.row_ids is not None or A.nstored < A.nrows or accumulate else torch.empty
         y = new(A.nrows, dtype=torch.float64, device=x.device)
     _call("comet_b200_dev_spmv_f64_i64", A.nstored, A.nnz, _p(A.row_ids), A.pos.data_ptr(), A.crd.data_ptr(),
           A.val.data_ptr(), x.data_ptr(), y.data_ptr(), semiring, int(accumulate), _stream())

@@ -96,3 +96,15 @@ def test_sums_keep_their_order(kind, nnz):
     assert np.all(np.abs(y.cpu().numpy() - ref) <= (lens + 1) * 2.0 ** -52 * size)
     assert np.all(np.abs(added.cpu().numpy() - ref - y0) <= (lens + 2) * 2.0 ** -52 * (size + np.abs(y0)))
     assert np.array_equal(dev.spmv(A, up(x), semiring=api.PLUS_PAIR).cpu().numpy(), lens)
+
+
+def test_rows_behind_the_row_pointer_are_zero():
+    """A row pointer shorter than the matrix: the rows it says nothing about are zero, whatever the new result's memory held."""
+    n = 50000
+    pos, crd = torch.arange(1001, device="cuda"), torch.arange(1000, device="cuda")
+    A = dev.DeviceCSR(n, n, pos, crd, torch.ones(1000, device="cuda", dtype=torch.float64))
+    x = torch.ones(n, device="cuda", dtype=torch.float64)
+    dirty = torch.full((n,), 7.0, device="cuda", dtype=torch.float64)
+    del dirty                                          # the allocator gives it out again
+    y = dev.spmv(A, x)
+    assert bool((y[:1000] == 1).all()) and not y[1000:].any()
