@@ -222,13 +222,13 @@ int spmm_stream_tma(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const 
 // so the kernels for the others are launched too and return at once.  Of these the entry stream takes over from the pieces
 // where a row of B fills a warp, from 64 columns (R-MAT scale 20: K = 48 894 us against 880, K = 64 833 against 900, K = 65
 // 1421 against 1685).  From 96 columns on it is as fast as spmm_short_rows where that takes a call (400,000 rows of 8, K = 128:
-// 477 us against 502; 50,021 rows of up to 24: 55 against 54) and is launched alone. Below SPMM_FIXED_NNZ entries the
+// 477 us against 502; 50,021 rows of up to 24: 55 against 54) and is launched alone. Below SPMM_SMALL_NNZ entries the
 // launches themselves are what a call takes (3 us each for the host), and the pieces do without the other kernels' look.
 static int spmm_auto(const SpmmCall &a)
 {
-    const bool stream = !a.pair && a.k >= 64 && a.nnz >= SPMM_FIXED_NNZ;
+    const bool stream = !a.pair && a.k >= 64 && a.nnz >= SPMM_SMALL_NNZ;
     LongRows lr = {nullptr, 0};
-    if (a.nnz >= SPMM_FIXED_NNZ && (!stream || !a.vec || a.k < 96)) CB_TRY(spmm_short_rows(a, &lr));
+    if (a.nnz >= SPMM_SMALL_NNZ && (!stream || !a.vec || a.k < 96)) CB_TRY(spmm_short_rows(a, &lr));
     if (!stream) return spmm_pieces(a, lr);
     const int64_t slices = ceil_div(a.k, 256), width = ceil_div(ceil_div(a.k, slices), 2) * 2;
     for (int64_t col0 = 0; col0 < a.k; col0 += width) {

@@ -5,8 +5,10 @@
 
 namespace cb200 {
 
-// Calls with fewer entries (plus-times) give the same sums to the bit every time: no atomics.
-static const int64_t SPMM_FIXED_NNZ = 65536;
+// Fewer entries: the launches themselves are what a call takes.
+static const int64_t SPMM_SMALL_NNZ = 65536;
+// Most memory for the parts of rows that are cut (2 k doubles a piece); more entries than this allows get longer pieces.
+static const int64_t PARTS_BYTES = (int64_t)128 << 20;
 
 struct SpmmCall {
     int64_t nrows, ncols, nnz, k;
@@ -25,6 +27,10 @@ struct SpmmCall {
 int spmm_short_rows(const SpmmCall &a, LongRows *lr);
 // Equal pieces of A's path, a group of lanes each; any K and alignment (spmm_pieces.cu).
 int spmm_pieces(const SpmmCall &a, LongRows lr);
+// Scratch memory for the parts of the rows that pieces cut, two rows of k sums a piece: [0] of a row that started before it,
+// [1] of one that starts in it and goes on; and the kernel that adds them up, in order.
+int piece_parts(int64_t npieces, int64_t k, double **parts);
+int add_parts(const SpmmCall &a, const StreamPlan &plan, LongRows lr, const double *parts);
 // Rows of B staged in shared memory (spmm_stream.cu).  Returns 1 when it took the call, 0 when the shape is not one that
 // it handles, -1 on error.
 int spmm_stream(const SpmmCall &a, LongRows lr);

@@ -16,7 +16,9 @@
 // is written with plain stores; a row cut by a boundary is added with f64
 // atomics (onto zeros written by the plan kernel when the call does not
 // accumulate), so its summation order is not fixed and differences stay at
-// rounding level.
+// rounding level.  With 8-byte vectors (odd widths or addresses) the pieces
+// leave their parts of such rows in scratch memory instead, where
+// spmm_pieces.cu adds them up in order.
 //
 // Bound: the L2 -> SM rate (17 TB/s) for the gathered rows of B; the arrays alone would take 370 us of HBM time at R-MAT
 // scale 20, K = 128, the gather 960 us.  Constant offsets in the ring, short pieces for small matrices (stream_plan) and a plan
@@ -51,6 +53,7 @@ struct StreamShape {
     static const int STAGES = SB_RING_BYTES / STAGE;
     static const int RING = STAGE * STAGES;
     static const int WARP = RING + SB_SIDE_BYTES;
+    static const bool FIXED = Vec<V>::N == 1;
 };
 
 template <typename V, int NI, bool FULLK>
@@ -59,12 +62,13 @@ spmm_stream_kernel(int64_t nrows, unsigned nblocks, const int64_t *__restrict__ 
                    const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, const double *__restrict__ val,
                    const double *__restrict__ b, int64_t ldb, double *__restrict__ c, int64_t ldc, int k,
                    int accumulate, WorkHeader *hdr, const int64_t *__restrict__ block_row,
-                   const int64_t *__restrict__ block_ent, LongRows lr)
+                   const int64_t *__restrict__ block_ent, LongRows lr, double *__restrict__ parts)
 {
     wait_for_previous();
     if (not_this(lr)) return;
     using S = StreamShape<V, NI>;
     constexpr int SB_G = S::G, stages = S::STAGES;
+    constexpr bool FIXED = StreamShape<V, NI>::FIXED;
     constexpr uint32_t rowbytes = S::ROW, stagebytes = S::STAGE, ringbytes = S::RING;
     // per warp: a ring of `stages` stages of SB_G rows of B, then 32 column indices and 32 values of A
     extern __shared__ __align__(128) unsigned char sb_smem_raw[];
@@ -126,13 +130,14 @@ spmm_stream_kernel(int64_t nrows, unsigned nblocks, const int64_t *__restrict__ 
         // write out the finished row r and clear the accumulators
         auto flush = [&](bool whole) {
             const int64_t out = row_ids ? row_ids[r] : r;
-            double *crow = c + out * ldc;
+            double *crow = FIXED && !whole ? parts + (2 * (int64_t)blk + (rs >= 0 ? 1 : 0)) * k : c + out * ldc;
             if (whole && accumulate && rs == re) return;       // an empty row adds nothing
 #pragma unroll
             for (int i = 0; i < NI; i++) {
                 V *at = (V *)crow + lane + i * 32;
                 if (on[i]) {
-                    if (!whole) Vec<V>::atomic_to(at, acc[i]);
+                    if (!whole && FIXED) *at = acc[i];
+                    else if (!whole) Vec<V>::atomic_to(at, acc[i]);
                     else {
                         if (accumulate) Vec<V>::add_to(acc[i], __ldcs(at));
                         __stcs(at, acc[i]);
@@ -253,10 +258,13 @@ spmm_stream_kernel(int64_t nrows, unsigned nblocks, const int64_t *__restrict__ 
 template <typename V, int NI, bool FULLK>
 static int launch_stream(const SpmmCall &a, LongRows lr)
 {
+    constexpr bool FIXED = StreamShape<V, NI>::FIXED;
     StreamPlan plan;
-    const int planned = stream_plan(a.nrows, a.nnz, (int64_t)sm_count() * SB_WARPS, a.row_ids, a.pos, a.c, a.ldc, a.k,
-                                    a.accumulate, lr, a.st, &plan);
+    const int planned = stream_plan(a.nrows, a.nnz, (int64_t)sm_count() * SB_WARPS, FIXED ? PARTS_BYTES / (16 * a.k) : INT64_MAX,
+                                    a.row_ids, a.pos, FIXED ? nullptr : a.c, a.ldc, a.k, a.accumulate, lr, a.st, &plan);
     if (planned <= 0) return planned;
+    double *parts = nullptr;
+    if (FIXED && piece_parts(plan.nblocks, a.k, &parts)) return -1;
     auto kernel = spmm_stream_kernel<V, NI, FULLK>;
     const size_t smem = (size_t)SB_WARPS * StreamShape<V, NI>::WARP;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -267,11 +275,12 @@ static int launch_stream(const SpmmCall &a, LongRows lr)
     if (grid > sm_count()) grid = sm_count();
     const cudaError_t e = launch_behind(kernel, dim3((unsigned)grid), SB_WARPS * 32, smem, a.st, a.nrows, (unsigned)plan.nblocks,
                                         a.row_ids, a.pos, a.crd, a.val, a.b, a.ldb, a.c, a.ldc, (int)a.k, a.accumulate,
-                                        plan.hdr, plan.block_row, plan.block_ent, lr);
+                                        plan.hdr, plan.block_row, plan.block_ent, lr, parts);
     if (e != cudaSuccess) {
         fail("spmm: launch failed: %s", cudaGetErrorString(e));
         return -1;
     }
+    if (FIXED && add_parts(a, plan, lr, parts)) return -1;
     return 1;
 }
 

@@ -332,7 +332,7 @@ int spmm_stream_tma(int64_t nrows, int64_t ncols, int64_t nnz, int64_t k, const 
     }
 
     StreamPlan plan;
-    const int planned = stream_plan(nrows, nnz, (int64_t)sm_count() * ST_WARPS, row_ids, pos, c, ldc, (int)k, accumulate,
+    const int planned = stream_plan(nrows, nnz, (int64_t)sm_count() * ST_WARPS, INT64_MAX, row_ids, pos, c, ldc, (int)k, accumulate,
                                     LongRows{nullptr, 0}, st, &plan);
     if (planned <= 0) return planned;
     int64_t grid = ceil_div(plan.nblocks, ST_WARPS);

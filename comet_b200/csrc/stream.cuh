@@ -42,6 +42,7 @@ struct StreamPlan {
     int64_t *block_row;       // piece b starts in row block_row[b] ...
     int64_t *block_ent;       // ... at entry block_ent[b]; both have nblocks + 1 entries
     int64_t nblocks;
+    int s;                    // a piece has 2^s steps
 };
 
 // Cuts the (entries + rows) path into pieces of 2^s steps (spmm_pieces.cu) and clears the counter.  c != null and
@@ -52,8 +53,8 @@ int piece_plan(int64_t nrows, int64_t nnz, int s, const int64_t *row_ids, const 
 LongRows next_mark();
 // Marks the call if a row has more than `limit` entries.
 int mark_long_rows(int64_t nrows, const int64_t *pos, int64_t limit, LongRows lr, cudaStream_t st);
-// Pieces for `warps` persistent warps.  Returns 1, 0 when the piece count does not fit 32 bits, -1 on error.
-int stream_plan(int64_t nrows, int64_t nnz, int64_t warps, const int64_t *row_ids, const int64_t *pos, double *c,
+// Pieces for `warps` persistent warps, fewer than `most`.  Returns 1, 0 when the piece count does not fit 32 bits, -1 on error.
+int stream_plan(int64_t nrows, int64_t nnz, int64_t warps, int64_t most, const int64_t *row_ids, const int64_t *pos, double *c,
                 int64_t ldc, int64_t k, int accumulate, LongRows lr, cudaStream_t st, StreamPlan *out);
 
 #ifdef __CUDACC__

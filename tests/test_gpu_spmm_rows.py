@@ -75,3 +75,36 @@ def test_small_products_are_the_same_to_the_bit(k):
     assert all(torch.equal(C, dev.spmm(A, B)) for _ in range(5))
     if k > 6:                      # and a panel's sums are those of the whole product
         assert torch.equal(C[:, :6], dev.spmm(A, B[:, :6]))
+
+
+def _hubs(nnz):
+    """Short rows, and among them rows of one piece up to more units of pieces than a warp adds up alone."""
+    rng = np.random.default_rng(nnz)
+    hubs = [31, 33, 255, 257, 991, 1023, 1025, 1057, 8190, 8500, 16000, 17000, 39999]
+    lens = rng.integers(0, 9, (nnz - sum(hubs)) // 4)
+    lens[rng.permutation(lens.size)[:len(hubs)]] = hubs
+    cols = rng.integers(0, 5000, lens.sum())
+    pos = np.concatenate([[0], np.cumsum(lens)])
+    return sp.csr_matrix((rng.uniform(-1, 1, cols.size), cols, pos), shape=(lens.size, 5000))
+
+
+@pytest.mark.parametrize("k", [1, 4, 7, 17, 33, 48, 62, 65, 129, 201])
+@pytest.mark.parametrize("nnz", [100000, 900000])
+def test_sums_keep_their_order(nnz, k):
+    """Rows cut into pieces: every call adds in the same order, below 64 columns and for every odd width."""
+    m = _hubs(nnz)
+    lens = np.diff(m.indptr)[:, None]
+    rng = np.random.default_rng(k)
+    B, C0 = rng.uniform(-1, 1, (m.shape[1], k)), rng.uniform(-1, 1, (m.shape[0], k))
+    A, dB, dC = _device(m), torch.from_numpy(B).cuda(), torch.from_numpy(C0).cuda()
+    C, acc = dev.spmm(A, dB), dev.spmm(A, dB, dC.clone(), accumulate=True)
+    for _ in range(4):
+        assert torch.equal(C, dev.spmm(A, dB))
+        assert torch.equal(acc, dev.spmm(A, dB, dC.clone(), accumulate=True))
+    # either order of a row's n + 1 terms is off by at most (n + 1) 2^-53 of the sum of their sizes
+    n, size = lens + 1.0, sp.csr_matrix((np.abs(m.data), m.indices, m.indptr), shape=m.shape) @ np.abs(B)
+    assert np.all(np.abs(C.cpu().numpy() - m @ B) <= n * 2.0 ** -52 * size)
+    assert np.all(np.abs(acc.cpu().numpy() - (m @ B + C0)) <= (n + 1) * 2.0 ** -52 * (size + np.abs(C0)))
+    dC = torch.from_numpy(C0).cuda()
+    pairs = dev.spmm(A, dB, dC.clone(), semiring=api.PLUS_PAIR, accumulate=True)
+    assert torch.equal(pairs, torch.from_numpy(C0 + lens).cuda())
