@@ -296,7 +296,6 @@ int spmm_stream(const SpmmCall &a, LongRows lr)
         if (a.k == 256) return launch_stream<double2, 4, true>(a, lr);
         return launch_stream<double2, 4, false>(a, lr);
     }
-    if (a.k <= 32) return launch_stream<double, 1, false>(a, lr);
     if (a.k <= 64) return launch_stream<double, 2, false>(a, lr);
     if (a.k <= 96) return launch_stream<double, 3, false>(a, lr);
     if (a.k <= 128) return launch_stream<double, 4, false>(a, lr);
