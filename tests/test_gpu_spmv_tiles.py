@@ -108,3 +108,21 @@ def test_rows_behind_the_row_pointer_are_zero():
     del dirty                                          # the allocator gives it out again
     y = dev.spmv(A, x)
     assert bool((y[:1000] == 1).all()) and not y[1000:].any()
+
+
+@pytest.mark.parametrize("tiles,more", [(-1, 0), (-1, 1), (0, 0), (1024, 0), (1024, 1)])
+def test_where_the_tiles_take_over(tiles, more):
+    """As many tiles of 2048 steps (entries and row ends) as the chip has SMs, less one step; and the most that one launch
+    takes, and one more."""
+    steps = (tiles if tiles > 0 else torch.cuda.get_device_properties(0).multi_processor_count + tiles) * 2048 + more
+    nnz = min(steps - 5000, 1000003)
+    rng = np.random.default_rng(steps)
+    pos = np.sort(np.concatenate([[0, nnz], rng.integers(0, nnz + 1, steps - nnz - 1)]))
+    lens, crd, val, x = np.diff(pos), rng.integers(0, 9001, nnz), rng.uniform(-1, 1, nnz), rng.uniform(-1, 1, 9001)
+    assert lens.size + nnz == steps
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    A = dev.DeviceCSR(lens.size, 9001, up(pos), up(crd), up(val))
+    y = dev.spmv(A, up(x))
+    assert all(torch.equal(y, dev.spmv(A, up(x))) for _ in range(3))
+    ref, size = (np.bincount(np.repeat(np.arange(lens.size), lens), w, lens.size) for w in (val * x[crd], np.abs(val * x[crd])))
+    assert np.all(np.abs(y.cpu().numpy() - ref) <= (lens + 1) * 2.0 ** -52 * size)
