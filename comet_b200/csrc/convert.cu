@@ -10,7 +10,9 @@
 // the row pointer by binary search in the sorted keys.  A CSR matrix is already in row order, so its
 // transpose sorts by the column alone.
 //
-// The sort is this file's own.  One kernel makes the keys and counts the digits of all passes; a pass is one kernel:
+// The sort is this file's own code for published methods: least-significant-digit passes of one kernel each (Adinets and
+// Merrill, Onesweep, 2022) whose tiles find their places by decoupled look-back (Merrill and Garland, Single-pass Parallel
+// Prefix Scan with Decoupled Look-back, 2016).  One kernel makes the keys and counts the digits of all passes; a pass is one kernel:
 // a CTA ranks a tile of keys by their digit, learns from the tiles before it where its runs of equal digits
 // start (each tile publishes its digit counts, then their sums over all tiles so far, and looks back until it meets
 // such a sum), orders the tile in shared memory and writes it out run by run.  Tiles are numbered in the order in

@@ -4,9 +4,9 @@
 // Rows are binned by an upper bound on their number of distinct columns
 // (sum of the lengths of the B rows they touch, capped by the mask row):
 //   bin 0  no products                     -> empty row
-//   bin 1  bound <= HASH_ROW_MAX           -> one warp per row, hash table in
-//          shared memory (int32 keys + f64 accumulators); output order by rank
-//          counting among the row's distinct keys
+//   bin 1  bound <= HASH_ROW_MAX           -> one warp per row.  The symbolic call counts distinct columns with a hash table
+//          in shared memory; the numeric call sorts column and place of the products in registers and adds equal
+//          neighbours (with a mask: the hash table again, its keys sorted in registers)
 //   bin 3  bound <= MID_ROW_MAX, no mask, not too many columns -> 128 or 256 threads per row, a bitmap over the columns of B and
 //          sums by rank in shared memory
 //   bin 2  everything else                 -> one CTA per row, a bitmap over the

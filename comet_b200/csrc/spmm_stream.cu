@@ -21,8 +21,10 @@
 // spmm_pieces.cu adds them up in order.
 //
 // Bound: the L2 -> SM rate (17 TB/s) for the gathered rows of B; the arrays alone would take 370 us of HBM time at R-MAT
-// scale 20, K = 128, the gather 960 us.  Constant offsets in the ring, short pieces for small matrices (stream_plan) and a plan
-// kernel with a thread per row instead of a search per piece: 1240 -> 1140 us there, 111 -> 28 us at scale 14.
+// scale 20, K = 128, the gather 960 us.  That rate goes with the SM clock: calls with pauses between them take 1165 us at
+// 1965 MHz, calls one after the other for seconds 1340, as the power cap (1000 W) then holds the clock at 1470 MHz.  Constant
+// offsets in the ring, short pieces for small matrices (stream_plan) and a plan kernel with a thread per row instead of a search
+// per piece: 111 -> 28 us at scale 14, at scale 20 no more than the runs of one side differ (1336 -> 1324 in long alternation).
 #include "common.cuh"
 #include "spmm.cuh"
 

@@ -490,8 +490,7 @@ COMET_B200_EXPORT int32_t comet_b200_dev_spmv_f64_i64(int64_t nrows, int64_t nnz
 
 /* variant: 0 = automatic.  Bits 24-25 pick the kernel family: 0 = by shape and row lengths (row
    panels if the low bits ask for them and K < 64),
-   1 = entry stream whenever the shape allows it (K even, at most 256; worth asking for with
-   narrow B and a power-law A, where it is several times faster than the panels),
+   1 = entry stream whenever the shape allows it (K even, at most 256; what 0 takes from 64 columns on),
    2 = row panels, 3 = the entry stream with the rows of B staged by TMA bulk copies
    (cp.async.bulk completing on an mbarrier) instead of per-lane cp.async; with bit 26 set as well, one
    cp.async.bulk.tensor ... tile::gather4 copy per stage of four rows (a tensor map of B is built per call).  For the row panels the low bits are (panel width in columns) |
