@@ -322,7 +322,7 @@ class SpMM(Workload):
 
 class SpMV(Workload):
     name = "spmv"
-    launches_per_step = 1     # one kernel up to 2^18 stored entries (the default), two or four above
+    launches_per_step = 1     # one kernel up to 2^20 stored entries (the default has 2^18), two or four above
 
     def build(self):
         from comet_b200 import datasets
