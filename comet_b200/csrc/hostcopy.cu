@@ -45,8 +45,9 @@ namespace {
 // while the arrays fit the caches.  Microseconds to write operands of 4.2 / 10.2 / 25.6 MB and to multiply by them (SpMV,
 // rows of 16), by number of workers: none 249 + 375 / 612 + 735 / 1590 + 1940, one 409 + 310 / 890 + 530 / 2000 + 1220, two
 // 690 + 309 / 1193 + 481 / 2085 + 915, five 890 + 332 / 1820 + 520 / 2730 + 890; the driver's own copies 252 + 410 / 610 +
-// 767 / 1810 + 1980.  So there is a worker for every BYTES_PER_WORKER that wait to be copied, none for a few MB.
-const size_t BYTES_PER_WORKER = (size_t)8 << 20;
+// 767 / 1810 + 1980.  So the calling thread copies the first WORKERS_FROM bytes of what it is given alone, and there is one
+// more worker for every BYTES_PER_WORKER after them (with 4 MB instead of 8 the 25.6 MB take as long as the driver's copies).
+const size_t WORKERS_FROM = (size_t)8 << 20, BYTES_PER_WORKER = (size_t)8 << 20;
 const size_t CHUNK = (size_t)2 << 20;     // bytes per page-locked chunk
 const int SLAB_CHUNKS = 8;                // chunks are allocated 16 MiB at a time (7 ms each),
 const int MAX_SLABS = 4;                  // at most 64 MiB per device
@@ -139,11 +140,11 @@ class Pool {
         bool wake;
         {
             std::lock_guard<std::mutex> lk(mu_);
-            tasks_.push_back(Task{std::move(fn), batch, bytes});
-            pending_++;
-            pending_bytes_ += bytes;
+            tasks_.push_back(Task{std::move(fn), batch});
+            if (pending_++ == 0) busy_bytes_ = 0;
+            busy_bytes_ += bytes;
             if (batch) batch->left++;
-            wake = awake_ < workers_.size() && (awake_ + 1) * BYTES_PER_WORKER <= pending_bytes_;
+            wake = awake_ < workers_.size() && WORKERS_FROM + awake_ * BYTES_PER_WORKER <= busy_bytes_;
             if (wake) {
                 awake_++;
                 calls_++;
@@ -181,7 +182,6 @@ class Pool {
         t.fn();
         lk.lock();
         pending_--;
-        pending_bytes_ -= t.bytes;
         if (t.batch) t.batch->left--;
         if (pending_ == 0 || (t.batch && t.batch->left == 0)) cv_done_.notify_all();
         return true;
@@ -201,7 +201,6 @@ class Pool {
     struct Task {
         std::function<void()> fn;
         Batch *batch = nullptr;
-        size_t bytes = 0;
     };
     int device_;
     std::vector<Slot> slots_;
@@ -211,7 +210,7 @@ class Pool {
     std::mutex mu_;
     std::condition_variable cv_free_, cv_task_, cv_done_;
     int pending_ = 0, slabs_ = 0;
-    size_t pending_bytes_ = 0;             // of tasks that have not run
+    size_t busy_bytes_ = 0;                // given since there was nothing to do
     size_t awake_ = 0, calls_ = 0;         // workers at work or called, calls not heard yet
     std::atomic<bool> failed_{false};
 };
