@@ -73,3 +73,25 @@ def test_small_chunks_and_every_staged_direction(monkeypatch):
         _close(C.val, R.val, oracle.spgemm(_orc(A, True), _orc(A, True)).val)
     L = datasets.config_triangles(scale=12, edge_factor=8)
     assert api.triangle_count(L) == oracle.masked_pair_count(_orc(L), _orc(L), _orc(L))
+
+
+@pytest.mark.parametrize("locked", ["S", "X", "Y", "SXY", "XY"])
+@pytest.mark.parametrize("y_is_kj", [False, True])
+def test_sddmm_with_page_locked_operands(locked, y_is_kj):
+    """Which dense operands go up before the check of S and which after it depends on whether they are page-locked."""
+    A = datasets.rmat_csr(12, 16, seed=5)
+    X, Y = datasets.dense_uniform((A.nrows, 64), 2), datasets.dense_uniform((A.ncols, 64), 3)
+    ref = oracle.sddmm(_orc(A), X, Y)
+    scale = oracle.sddmm(_orc(A, True), np.abs(X), np.abs(Y))
+
+    def pin(name, a):
+        return torch.from_numpy(np.ascontiguousarray(a)).pin_memory().numpy() if name in locked else a
+
+    X, Y = pin("X", X), pin("Y", np.ascontiguousarray(Y.T) if y_is_kj else Y)
+    S = api.SparseTensor("CSR", A.nrows, A.ncols, A.a1pos, A.a1crd, pin("S", A.a2pos), pin("S", A.a2crd), pin("S", A.val))
+    _close(api.sddmm(S, X, Y, y_is_kj=y_is_kj), ref, scale)
+    crd = A.a2crd.copy()
+    crd[7] = A.ncols                                             # refused before anything gathers through it
+    bad = api.SparseTensor("CSR", A.nrows, A.ncols, A.a1pos, A.a1crd, A.a2pos, pin("S", crd), A.val)
+    with pytest.raises(Exception, match="outside"):
+        api.sddmm(bad, X, Y, y_is_kj=y_is_kj)
