@@ -32,6 +32,7 @@
 #include "common.cuh"
 #include "stream.cuh"
 #include "hostcopy.cuh"
+#include "hubs.cuh"
 #include "masked.cuh"
 #include "semiring.cuh"
 
@@ -44,6 +45,7 @@ static const int BM_THREADS = 512;          // CTA size of the bitmap kernels
 static const size_t BM_SMEM_LIMIT = 200 * 1024;
 static const size_t BM_STORE_BUDGET = (size_t)12 << 30;
 static const size_t BM_STORE_SMALL = (size_t)64 << 20;
+static const size_t HUB_WORK = (size_t)32 << 20;      // bytes of bitmaps of bin-2 rows from which on hubs.cuh takes them
 
 struct Plan {
     int kind;                // 0 = spgemm, 1 = elementwise CSR .* CSR
@@ -61,6 +63,7 @@ struct Plan {
     unsigned n1, n2, n3;
     uint32_t *bm_store;      // n2 * words, or null
     int words;
+    Hubs *hubs;              // not null: bin 2 goes by hubs.cuh
     MaskedPlan *masked;      // not null: the product is formed by dot products over the mask
     cudaStream_t last;       // stream of the latest call on this plan: its arrays are released in that stream's order
 };
@@ -74,6 +77,11 @@ static void plan_free(Plan *p, cudaStream_t st)
     if (!p) return;
     if (p->mem) cudaFreeAsync(p->mem, st);
     if (p->bm_store) cudaFreeAsync(p->bm_store, st);
+    if (p->hubs) {
+        if (p->hubs->mem) cudaFreeAsync(p->hubs->mem, st);
+        if (p->hubs->mem2) cudaFreeAsync(p->hubs->mem2, st);
+        delete p->hubs;
+    }
     masked_free(p->masked, st);
     delete p;
 }
@@ -725,25 +733,30 @@ static const int64_t LONG_B_ROW = 1024;
 
 static const unsigned BM_DENSE_ROW = 512;   // bits in 32 consecutive bitmap words from which crd is written word by word (measured: 96 / 192 / 320 / 512 / 768 / never = 22.9 / 21.8 / 21.5 / 21.45 / 21.65 / 21.7 ms numeric at config 4)
 static const int LONG_LIST = 1024;          // long rows of B remembered per pass over a row of A
+// Steps of 32 products whose loads are in flight, with 3 CTAs of 512 threads on an SM (R-MAT scale 18 squared, numeric / symbolic kernel in
+// ms): 1 19.3 / 4.6, 2 18.1 / 4.0, 4 17.4 / 3.8.  More of them with fewer warps is slower (2 CTAs, 6 steps 20.1), and so are more
+// warps with fewer steps (4 CTAs, 2 steps 20.1).
+static const int WALK_DEPTH = 4;
+static const int WALK_DEPTH_FOLD = 2;       // where the fold is a loop: R-MAT scale 17, 5 per row, min-plus 2.4 ms, with 4 steps 2.6
 
 // Calls f(j, bv, av) for every product of row r of A with B in this CTA's share: j and bv are the column and
 // value of an entry of row acrd[p] of B (bv = 0 when bval is null), av = aval[p] (0 when aval is null).  A team
 // of `team` CTAs deals the entries of the A row out over its warps one by one.  The loads are arranged so that
 // no warp waits on a chain: 32 entries of a warp's share look up their rows of B lane-parallel (acrd, then
-// bpos, once per batch), the first 32 entries of the next row of B are fetched before the current row is
-// worked on, and longer rows are walked two vectors per step with both loads issued first.
+// bpos, once per batch), and DEPTH steps of 32 products are fetched before the first of them is worked on.
+// hub_id (null: none): rows of B with a number >= 0 there are left out.
 // Short rows of B are walked by one warp; long ones are remembered in s_long and then walked by the
 // whole CTA.  s_ctl: [0] entries in s_long, [1] set when the list was too small (then the share is
 // scanned again for long rows).  All threads of the CTA must call this.
-template <typename F>
+template <int DEPTH, typename F>
 __device__ __forceinline__ void for_each_product(int64_t r, unsigned part, unsigned team,
                                                  const int64_t *__restrict__ apos,
                                                  const int64_t *__restrict__ acrd,
                                                  const double *__restrict__ aval,
                                                  const int64_t *__restrict__ bpos,
                                                  const int32_t *__restrict__ bcrd,
-                                                 const double *__restrict__ bval, int *s_long,
-                                                 unsigned *s_ctl, F f)
+                                                 const double *__restrict__ bval, const int32_t *__restrict__ hub_id,
+                                                 int *s_long, unsigned *s_ctl, F f)
 {
     constexpr int NW = BM_THREADS / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -762,7 +775,8 @@ __device__ __forceinline__ void for_each_product(int64_t r, unsigned part, unsig
         if (p < ae) {
             const int64_t k = acrd[p];
             s_l = bpos[k];
-            const int64_t len = bpos[k + 1] - s_l;
+            int64_t len = bpos[k + 1] - s_l;
+            if (hub_id && hub_id[k] >= 0) len = 0;
             if (aval) av_l = aval[p];
             if (len > LONG_B_ROW) {
                 const unsigned at = atomicAdd(&s_ctl[0], 1u);
@@ -772,41 +786,36 @@ __device__ __forceinline__ void for_each_product(int64_t r, unsigned part, unsig
                 n_l = (int)len;
             }
         }
-        const int64_t left = (ae - p0 + stride - 1) / stride;      // entries of the sequence from p0 on
-        const int n = left < 32 ? (int)left : 32;
-        // row t of the batch: start, length, value of A, and the first vector of its entries
-        int64_t s0 = __shfl_sync(0xffffffffu, (long long)s_l, 0);
-        int n0 = __shfl_sync(0xffffffffu, n_l, 0);
-        double a0 = shfl_f64(av_l, 0, 32);
-        int32_t j0 = 0;
-        double v0 = 0.0;
-        if (lane < n0) {
-            j0 = bcrd[s0 + lane];
-            if (bval) v0 = bval[s0 + lane];
-        }
-        for (int t = 0; t < n; t++) {
-            const int tn = (t + 1) & 31;                 // past the batch: lane 0 again, never used
-            const int64_t s1 = __shfl_sync(0xffffffffu, (long long)s_l, tn);
-            int n1 = __shfl_sync(0xffffffffu, n_l, tn);
-            if (t + 1 >= n) n1 = 0;
-            const double a1 = shfl_f64(av_l, tn, 32);
-            int32_t j1 = 0;
-            double v1 = 0.0;
-            if (lane < n1) {
-                j1 = bcrd[s1 + lane];
-                if (bval) v1 = bval[s1 + lane];
+        // the rows' entries in steps of 32, DEPTH steps' loads in flight whether they belong to one row or to several
+        unsigned left = __ballot_sync(0xffffffffu, n_l > 0);
+        int64_t at = 0;
+        int rem = 0;
+        double av = 0.0;
+        while (left || rem > 0) {
+            int32_t j[DEPTH];
+            double v[DEPTH], am[DEPTH];
+#pragma unroll
+            for (int i = 0; i < DEPTH; i++) {
+                if (rem <= 0 && left) {
+                    const int t = __ffs(left) - 1;
+                    left &= left - 1;
+                    at = __shfl_sync(0xffffffffu, (long long)s_l, t) + lane;
+                    rem = __shfl_sync(0xffffffffu, n_l, t);
+                    av = shfl_f64(av_l, t, 32);
+                }
+                am[i] = av;
+                j[i] = -1;
+                v[i] = 0.0;
+                if (lane < rem) {
+                    j[i] = bcrd[at];
+                    if (bval) v[i] = bval[at];
+                }
+                at += 32;
+                rem -= 32;
             }
-            if (lane < n0) f(j0, v0, a0);
-            for (int64_t q = s0 + 32 + lane; q < s0 + n0; q += 64) {
-                const bool two = q + 32 < s0 + n0;
-                const int32_t ja = bcrd[q];
-                const int32_t jb = two ? bcrd[q + 32] : 0;
-                const double va = bval ? bval[q] : 0.0;
-                const double vb = (bval && two) ? bval[q + 32] : 0.0;
-                f(ja, va, a0);
-                if (two) f(jb, vb, a0);
-            }
-            s0 = s1; n0 = n1; a0 = a1; j0 = j1; v0 = v1;
+#pragma unroll
+            for (int i = 0; i < DEPTH; i++)
+                if (j[i] >= 0) f(j[i], v[i], am[i]);
         }
     }
     __syncthreads();
@@ -833,7 +842,7 @@ __device__ __forceinline__ void for_each_product(int64_t r, unsigned part, unsig
             for (int64_t pl = p0; pl < p0 + NW && pl < ae; pl++) {
                 const int64_t k = acrd[pl];
                 const int64_t sl = bpos[k], el = bpos[k + 1];
-                if (el - sl <= LONG_B_ROW) continue;
+                if (el - sl <= LONG_B_ROW || (hub_id && hub_id[k] >= 0)) continue;
                 whole_cta(sl, el, aval ? aval[pl] : 0.0);
             }
     }
@@ -849,7 +858,7 @@ __device__ __forceinline__ void mark_products(uint32_t *bm, int64_t r, const int
 {
     int64_t ms = 0, me = 0;
     if (mpos) { ms = mpos[r]; me = mpos[r + 1]; }
-    for_each_product(r, 0u, 1u, apos, acrd, nullptr, bpos, bcrd, nullptr, s_long, s_ctl, [&](int32_t j, double, double) {
+    for_each_product<WALK_DEPTH>(r, 0u, 1u, apos, acrd, nullptr, bpos, bcrd, nullptr, nullptr, s_long, s_ctl, [&](int32_t j, double, double) {
         if (mpos && !in_mask(mcrd, ms, me, j)) return;
         atomicOr(&bm[j >> 5], 1u << (j & 31));          // testing the bit first was measured slower (6.4 vs 5.2 ms)
     });
@@ -968,9 +977,11 @@ team_clear_kernel(const TeamHeader *th, const uint64_t *__restrict__ items, unsi
     }
 }
 
-template <bool SMEM, bool PLUS_TIMES>
+// stride: words from one stored bitmap to the next.  MAPPED: colmap has the column of each number in bcrd.
+template <bool SMEM, bool PLUS_TIMES, bool MAPPED>
 __global__ void __launch_bounds__(BM_THREADS, SMEM ? 3 : 1)
-bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int words,
+bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int words, int stride, unsigned stage_n,
+                      const int32_t *__restrict__ colmap,
                       uint32_t *__restrict__ gbm, const int64_t *__restrict__ apos,
                       const int64_t *__restrict__ acrd, const double *__restrict__ aval,
                       const int64_t *__restrict__ bpos, const int32_t *__restrict__ bcrd,
@@ -988,6 +999,7 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
     uint32_t *bm = SMEM ? s_dyn : gbm + (size_t)blockIdx.x * 2 * words;
     uint32_t *pre = bm + words;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int32_t *stage = (int32_t *)s_dyn + (SMEM ? 2 * words : 0) + warp * stage_n;
     constexpr int NW = BM_THREADS / 32;
     wait_for_previous();
     for (unsigned iter = blockIdx.x;; iter += gridDim.x) {
@@ -1010,7 +1022,7 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
         }
         const int64_t r = list[it];
         if (bm_store) {
-            const uint32_t *keep = bm_store + (size_t)it * words;
+            const uint32_t *keep = bm_store + (size_t)it * stride;
             for (int w = threadIdx.x; w < words; w += BM_THREADS) bm[w] = __ldcs(keep + w);     // read once per member
             __syncthreads();
         } else {
@@ -1038,6 +1050,17 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
         for (int w2 = 0; w2 < warp; w2++) run += s_scan[w2];
         const int64_t base = cpos[r];
         const int64_t rown = cpos[r + 1] - base;
+        unsigned held = 0;                             // columns in the stage: those of the outputs before `upto`
+        auto flush = [&](unsigned upto) {
+            __syncwarp();
+            long long *out = (long long *)ccrd + base + upto - held;
+#pragma unroll 4
+            for (unsigned o = lane; o < held; o += 32) {
+                __stcs(out + o, (long long)__ldg(colmap + stage[o]));               // written once, not read here again
+            }
+            __syncwarp();
+            held = 0;
+        };
         for (int i = i0; i < i1; i++) {
             const int w = i * 32 + lane;
             uint32_t v = w < words ? bm[w] : 0u;
@@ -1051,10 +1074,15 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
             const unsigned excl = run + incl - c;
             if (w < words) pre[w] = excl;
             const unsigned rowtotal = __shfl_sync(0xffffffffu, incl, 31);
+            const unsigned before = run;
             run += rowtotal;
+            if (rowtotal == 0) continue;
             // the members of a team share the writing of crd by rows of 32 words
-            if (rowtotal == 0 || (team > 1 && (unsigned)i % team != part)) continue;
+            const bool ours = team == 1 || (unsigned)i % team == part;
+            if (MAPPED && held && (!ours || held + rowtotal > stage_n)) flush(before);
+            if (!ours) continue;
             if (rowtotal >= BM_DENSE_ROW) {
+                if (MAPPED && held) flush(before);
                 // many bits per word: one word at a time, lane b writes column 32 w + b at its rank, so a
                 // store instruction covers consecutive addresses
                 // (all 32 words in a fixed-trip loop: the shuffles of different words do not depend on each
@@ -1065,24 +1093,32 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
                 for (int l = 0; l < 32; l++) {
                     const uint32_t wv = __shfl_sync(0xffffffffu, v, l);
                     const unsigned wp = __shfl_sync(0xffffffffu, excl, l);
-                    if ((wv >> lane) & 1u) __stcs(out + wp + __popc(wv & below), (long long)(i * 32 + l) * 32 + lane);
+                    if ((wv >> lane) & 1u) {
+                        const int j = (i * 32 + l) * 32 + lane;
+                        __stcs(out + wp + __popc(wv & below), (long long)(MAPPED ? __ldg(colmap + j) : j));
+                    }
+                }
+            } else if (!MAPPED || rowtotal > stage_n) {
+                unsigned at = excl;
+                for (; v; v &= v - 1, at++) {
+                    const int j = w * 32 + __ffs(v) - 1;
+                    __stcs((long long *)ccrd + base + at, (long long)(MAPPED ? __ldg(colmap + j) : j));
                 }
             } else {
-                unsigned at = excl;
-                while (v) {
-                    const int b = __ffs(v) - 1;
-                    v &= v - 1;
-                    __stcs((long long *)ccrd + base + at, (long long)w * 32 + b);   // written once, not read here again
-                    at++;
-                }
+                // the columns go through shared memory, so that the stores are coalesced and the look-ups independent (R-MAT scale
+                // 18 squared 21.5 -> 18.6 ms)
+                unsigned at = held + excl - before;
+                for (; v; v &= v - 1) stage[at++] = w * 32 + __ffs(v) - 1;
+                held += rowtotal;
             }
         }
+        if (MAPPED && held) flush(run);
         if (team == 1)
             for (int64_t t = threadIdx.x; t < rown; t += BM_THREADS) cval[base + t] = sr_identity(semi);
         __syncthreads();
         // accumulate every product at the rank of its column
         double *crow = cval + base;
-        for_each_product(r, part, team, apos, acrd, aval, bpos, bcrd, bval, s_long, s_ctl, [&](int32_t j, double bv, double av) {
+        for_each_product<PLUS_TIMES ? WALK_DEPTH : WALK_DEPTH_FOLD>(r, part, team, apos, acrd, aval, bpos, bcrd, bval, nullptr, s_long, s_ctl, [&](int32_t j, double bv, double av) {
             uint32_t word = bm[j >> 5];
             uint32_t bit = 1u << (j & 31);
             if (!(word & bit)) return;          // filtered out by the mask
@@ -1093,6 +1129,84 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
         __syncthreads();
     }
     (void)mpos; (void)mcrd;
+}
+
+// --------------------------------------------------------------------------
+// Bin 2 by hubs (hubs.cuh).
+// --------------------------------------------------------------------------
+
+// The hubs that the next entries of a row of A name, from *p on, to s_hub, their count to *s_n, in any order.  Stops when a further
+// step of BM_THREADS entries might not fit.  Called by the whole CTA.
+__device__ __forceinline__ int hub_list(int64_t *p, int64_t ae, const int64_t *__restrict__ acrd, const int32_t *__restrict__ hub_id,
+                                        int *s_hub, unsigned *s_n)
+{
+    __syncthreads();                                   // the list is no longer read
+    if (threadIdx.x == 0) *s_n = 0;
+    __syncthreads();
+    int64_t at = *p;
+    for (; at < ae && (int)*s_n <= LONG_LIST - BM_THREADS; at += BM_THREADS) {
+        __syncthreads();                               // all have read the count
+        if (at + threadIdx.x < ae) {
+            const int h = hub_id[acrd[at + threadIdx.x]];
+            if (h >= 0) s_hub[atomicAdd(s_n, 1u)] = h;
+        }
+        __syncthreads();
+    }
+    *p = at;
+    return (int)*s_n;
+}
+
+// bm = the columns of row r's products; hub_id == null: B has no hubs
+__device__ __forceinline__ void hub_mark_row(uint32_t *bm, int stride, int64_t r, const int64_t *__restrict__ apos,
+                                             const int64_t *__restrict__ acrd, const int64_t *__restrict__ bpos,
+                                             const int32_t *__restrict__ bcrd, const int32_t *__restrict__ hub_id,
+                                             const uint32_t *__restrict__ hub_bm, int *s_long, unsigned *s_n,
+                                             unsigned *s_ctl)
+{
+    int *s_hub = s_long;                               // one list after the other
+    const int64_t ae = apos[r + 1];
+    int64_t p = apos[r];
+    for (bool first = true; first || (hub_id && p < ae); first = false) {
+        const int n = hub_id ? hub_list(&p, ae, acrd, hub_id, s_hub, s_n) : 0;
+        for (int g = threadIdx.x; g < stride / 4; g += BM_THREADS) {
+            uint4 v = first ? make_uint4(0, 0, 0, 0) : ((uint4 *)bm)[g];
+#pragma unroll 8
+            for (int i = 0; i < n; i++) {
+                const uint4 o = __ldg((const uint4 *)(hub_bm + (size_t)s_hub[i] * stride) + g);
+                v.x |= o.x; v.y |= o.y; v.z |= o.z; v.w |= o.w;
+            }
+            ((uint4 *)bm)[g] = v;
+        }
+    }
+    __syncthreads();
+    for_each_product<WALK_DEPTH>(r, 0u, 1u, apos, acrd, nullptr, bpos, bcrd, nullptr, hub_id, s_long, s_ctl,
+                     [&](int32_t j, double, double) { atomicOr(&bm[j >> 5], 1u << (j & 31)); });
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(BM_THREADS)
+hub_symbolic_kernel(unsigned nlist, const int32_t *__restrict__ list, Hubs hb, const int64_t *__restrict__ apos,
+                    const int64_t *__restrict__ acrd, const int64_t *__restrict__ bpos, int64_t *__restrict__ cnt,
+                    uint32_t *__restrict__ bm_store)
+{
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    __shared__ unsigned s_warp[BM_THREADS / 32];
+    __shared__ int s_long[LONG_LIST];
+    __shared__ unsigned s_ctl[2], s_n;
+    const int32_t *id = *hb.count ? hb.id : nullptr;
+    for (unsigned it = blockIdx.x; it < nlist; it += gridDim.x) {
+        const int64_t r = list[it];
+        hub_mark_row(s_dyn, hb.stride, r, apos, acrd, bpos, hb.crd, id, hb.bm, s_long, &s_n, s_ctl);
+        unsigned c = 0;
+        uint4 *keep = bm_store ? (uint4 *)(bm_store + (size_t)it * hb.stride) : nullptr;
+        for (int g = threadIdx.x; g < hb.stride / 4; g += BM_THREADS) {
+            const uint4 v = ((const uint4 *)s_dyn)[g];
+            c += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+            if (keep) __stcs(keep + g, v);
+        }
+        const unsigned total = block_sum_u32(c, s_warp);
+        if (threadIdx.x == 0) cnt[r] = total;
+    }
 }
 
 // --------------------------------------------------------------------------
@@ -1171,6 +1285,88 @@ static int launch_mid(const Plan *p, unsigned grid, int64_t *ccrd, double *cval,
     return 0;
 }
 
+// Prepares B's long rows (p->hubs stays null where the columns that B stores are too many, or B has no long rows and hardly a column
+// without entries).  Synchronises.
+static int hub_prepare(Plan *p, int64_t nrows, cudaStream_t st)
+{
+    Hubs *hb = new Hubs();
+    memset(hb, 0, sizeof(Hubs));
+    p->hubs = hb;                                      // freed with the plan
+    const int64_t words = ceil_div(p->ncols, 32);
+    auto pad = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+    const size_t b_bits = pad((size_t)words * 4), b_map = pad((size_t)p->ncols * 4), b_crd = pad((size_t)p->nnz_b * 4 + 16);
+    char *m = nullptr;
+    CB_TRY(dev_alloc(&m, 256 + 2 * b_bits + b_map + b_crd, st));
+    hb->mem = m;
+    hb->prep = (HubPrep *)m;
+    hb->count = (unsigned *)(m + 128);
+    hb->present = (uint32_t *)(m + 256);
+    hb->before = (int32_t *)(m + 256 + b_bits);
+    hb->colmap = (int32_t *)(m + 256 + 2 * b_bits);
+    hb->crd = (int32_t *)(m + 256 + 2 * b_bits + b_map);
+    CB_CUDA(cudaMemsetAsync(m, 0, 256 + b_bits, st));
+    const int64_t least = ceil_div(p->nnz_b, 4096), most = (int64_t)sm_count() * 2;
+    const unsigned grid = (unsigned)(least < most ? least : most);
+    if (words * 4 <= 96 * 1024) {
+        CB_CUDA(cudaFuncSetAttribute(hub_present_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(words * 4)));
+        hub_present_kernel<true><<<grid, 1024, (size_t)words * 4, st>>>(p->nnz_b, p->bcrd32, words, hb->present, nrows, p->apos,
+                                                                      p->acrd, p->bpos, hb->prep);
+    } else {
+        hub_present_kernel<false><<<grid, 1024, 0, st>>>(p->nnz_b, p->bcrd32, words, hb->present, nrows, p->apos, p->acrd,
+                                                          p->bpos, hb->prep);
+    }
+    CB_LAUNCH_CHECK();
+    hub_before_kernel<<<1, 1024, 0, st>>>(words, hb->present, hb->before, hb->prep);
+    CB_LAUNCH_CHECK();
+    HubPrep prep;
+    {
+        PinnedWords host;
+        if (!host.p) return fail("spgemm: no page-locked memory");
+        CB_CUDA(cudaMemcpyAsync(host.p, hb->prep, sizeof(prep), cudaMemcpyDeviceToHost, st));
+        CB_CUDA(cudaStreamSynchronize(st));
+        memcpy(&prep, host.p, sizeof(prep));
+    }
+    // the look-up of every coordinate costs what an eighth of the words does (200,000 columns, all stored: 3.3 -> 4.0 ms)
+    const bool renumber = (int64_t)prep.ncols * 8 <= p->ncols * 7;
+    hb->words = (int)(renumber ? ceil_div((int64_t)prep.ncols, 32) : words);
+    hb->stride = (hb->words + 3) & ~3;
+    hb->nrows_b = prep.nrows_b;
+    const int64_t entries = hb->words / 8 > HUB_MIN_ENTRIES ? hb->words / 8 : HUB_MIN_ENTRIES;
+    if (hb->words > HUB_MAX_WORDS || (!renumber && prep.longest < entries)) {
+        cudaFreeAsync(hb->mem, st);
+        delete hb;
+        p->hubs = nullptr;
+        return 0;
+    }
+    if (renumber) {
+        hub_renumber_kernel<<<(unsigned)sm_count() * 8, 256, 0, st>>>(p->nnz_b, p->bcrd32, words, hb->present, hb->before, hb->crd,
+                                                                      hb->colmap);
+        CB_LAUNCH_CHECK();
+    } else {
+        hb->crd = p->bcrd32;
+        hb->colmap = nullptr;
+    }
+    const size_t each = (size_t)hb->stride * 4 + 4;
+    size_t cap = (size_t)(p->nnz_b / entries) + 1;
+    if (cap > HUB_MEMORY / each) cap = HUB_MEMORY / each;
+    hb->cap = (unsigned)cap;
+    const size_t b_id = pad((size_t)hb->nrows_b * 4), b_rows = pad(cap * 4);
+    m = nullptr;
+    CB_TRY(dev_alloc(&m, b_id + b_rows + cap * hb->stride * 4, st));
+    hb->mem2 = m;
+    hb->id = (int32_t *)m;
+    int32_t *rows = (int32_t *)(m + b_id);
+    hb->bm = (uint32_t *)(m + b_id + b_rows);
+    hub_find_kernel<<<(unsigned)ceil_div(hb->nrows_b, 256), 256, 0, st>>>(hb->nrows_b, p->bpos, entries, hb->cap, hb->count, hb->id,
+                                                                        rows);
+    CB_LAUNCH_CHECK();
+    CB_CUDA(cudaFuncSetAttribute(hub_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hb->stride * 4));
+    hub_build_kernel<<<(unsigned)(cap < (size_t)sm_count() * 2 ? cap : (size_t)sm_count() * 2), 512, (size_t)hb->stride * 4, st>>>(
+        hb->count, hb->cap, rows, p->bpos, hb->crd, hb->stride, hb->bm);
+    CB_LAUNCH_CHECK();
+    return 0;
+}
+
 int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t *apos,
                     const int64_t *acrd, const double *aval, const int64_t *bpos,
                     const int64_t *bcrd, const double *bval, const int64_t *mpos,
@@ -1242,10 +1438,11 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     // synchronisation, unless bitmaps for every row are small change (then the kernels read the bin sizes themselves).
     p->n1 = p->n2 = (unsigned)nrows;
     p->n3 = mid ? (unsigned)nrows : 0;
+    bool counted = false;
     if ((size_t)nrows * p->words * 4 > BM_STORE_SMALL) {
         STEP_CUDA(launch_behind(publish_kernel, dim3(1), 1, 0, st, p->bin_counts, nullptr, counts));
         STEP_CUDA(cudaStreamSynchronize(st));
-        if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; p->n3 = counts[2]; }
+        if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; p->n3 = counts[2]; counted = true; }
     }
     if (!rc && p->n1) {
         unsigned grid = (unsigned)ceil_div(p->n1, HASH_WARPS);
@@ -1255,8 +1452,10 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
                                 aval, bpos, p->bcrd32, bval, mpos, p->mcrd, p->semi, p->cnt, nullptr, nullptr, nullptr));
     }
     if (!rc && p->n3) STEP(launch_mid<false>(p, cnt_grid(p->n3), nullptr, nullptr, st));
+    if (counted && !mpos && p->n2 && (size_t)p->n2 * p->words * 4 >= HUB_WORK && ncols_b <= HUB_MAX_COLS && nnz_b < 0x7fffffffLL)
+        STEP(hub_prepare(p, nrows, st));
     if (!rc && p->n2) {
-        size_t store = (size_t)p->n2 * p->words * sizeof(uint32_t);
+        size_t store = (size_t)p->n2 * (p->hubs ? p->hubs->stride : p->words) * sizeof(uint32_t);
         // the symbolic pass's bitmaps are kept for the numeric pass while they fit the budget
         // (COMET_B200_SPGEMM_BITMAP_GB overrides it; 0 makes the numeric pass mark its rows again)
         size_t budget = BM_STORE_BUDGET;
@@ -1265,8 +1464,13 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
             cudaError_t e = cudaMallocAsync((void **)&p->bm_store, store, st);
             if (e != cudaSuccess) { p->bm_store = nullptr; (void)cudaGetLastError(); }
         }
-        size_t smem = (size_t)p->words * sizeof(uint32_t);
-        if (2 * smem <= BM_SMEM_LIMIT) {
+        size_t smem = (size_t)(p->hubs ? p->hubs->stride : p->words) * sizeof(uint32_t);
+        if (p->hubs) {
+            STEP_CUDA(cudaFuncSetAttribute(hub_symbolic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (!rc)
+                hub_symbolic_kernel<<<bitmap_grid(p->n2, smem + 5 * 1024), BM_THREADS, smem, st>>>(p->n2, p->list2, *p->hubs, apos,
+                                                                                                  acrd, bpos, p->cnt, p->bm_store);
+        } else if (2 * smem <= BM_SMEM_LIMIT) {
             int grid = bitmap_grid(p->n2, smem);
             STEP_CUDA(cudaFuncSetAttribute(bitmap_symbolic_kernel<true>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1359,17 +1563,30 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
         }
         if (!rc && p->n3) rc = launch_mid<true>(p, cnt_grid(p->n3), ccrd, cval, st);
         if (!rc && p->n2) {
-            size_t smem = (size_t)p->words * sizeof(uint32_t) * 2;
+            const int words = p->hubs ? p->hubs->words : p->words, stride = p->hubs ? p->hubs->stride : p->words;
+            const int32_t *colmap = p->hubs ? p->hubs->colmap : nullptr, *bcrd32 = p->hubs ? p->hubs->crd : p->bcrd32;
+            size_t smem = (size_t)words * sizeof(uint32_t) * 2;
+            const size_t stage = (size_t)BM_THREADS / 32 * BM_DENSE_ROW * 4;
             if (smem <= BM_SMEM_LIMIT) {
+
                 // full occupancy grid even for few rows: teams give every CTA work
-                int grid = bitmap_grid(0xffffffffu, smem);
+                // three CTAs are what the registers leave room for; coordinates are staged in the shared memory that is left
+                // (200,000 rows of up to 60: 4.2 ms with three and what is left, 5.2 with a full stage and two).  Columns that need no
+                // look-up are written as they are found (3.3 against 3.5).
+                const size_t sm = (size_t)228 * 1024, own = 6 * 1024;
+                size_t per_sm = sm / (smem + own);
+                per_sm = per_sm < 1 ? 1 : per_sm > 3 ? 3 : per_sm;
+                size_t stage_n = colmap ? (sm / per_sm - own - smem) / (BM_THREADS / 32 * 4) : 0;
+                if (stage_n > BM_DENSE_ROW) stage_n = BM_DENSE_ROW;
+                smem += stage_n * (BM_THREADS / 32 * 4);
+                const int grid = sm_count() * (int)per_sm;
                 // team size of a row = its output entries * 8 bytes * CTAs in flight / budget
                 double budget_mb = 60.0;                 // measured best on R-MAT scale 18 (25 / 40 / 60 / 160 MB)
                 if (const char *e = getenv("COMET_B200_SPGEMM_TEAM_MB")) budget_mb = atof(e);
                 if (budget_mb < 0.001) budget_mb = 0.001;
                 const double per_entry = 8.0 * grid / (budget_mb * 1048576.0);
                 // no row of so few columns wants a team: two launches less
-                const bool alone = (double)p->ncols * per_entry <= 1.0;
+                const bool alone = (double)words * 32 * per_entry <= 1.0;
                 const size_t cap = (size_t)p->n2 + (size_t)((double)p->nnz_c * per_entry) + 64;
                 void *tm = nullptr;
                 rc = cap > 0xfffffff0u ? fail("spgemm numeric: too many team items")
@@ -1385,28 +1602,22 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
                             p->n2, p->list2, p->cpos, per_entry, th, items, (unsigned)cap);
                     if (!alone) launch_behind(team_clear_kernel, dim3((unsigned)sm_count() * 8), 256, 0, st, th, items, (unsigned)cap, p->list2,
                                   p->cpos, p->semi, cval);
-                    if (p->semi == COMET_B200_PLUS_TIMES) {
-                        cudaFuncSetAttribute(bitmap_numeric_kernel<true, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                        launch_behind(bitmap_numeric_kernel<true, true>, dim3(grid), BM_THREADS, smem, st, p->n2, p->list2, p->words,
-                                      nullptr, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32, p->bval, p->mpos, p->mcrd,
-                                      p->semi, p->bm_store, p->cpos, ccrd, cval, th, items);
-                    } else {
-                        cudaFuncSetAttribute(bitmap_numeric_kernel<true, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                        launch_behind(bitmap_numeric_kernel<true, false>, dim3(grid), BM_THREADS, smem, st, p->n2, p->list2, p->words,
-                                      nullptr, p->apos, p->acrd, p->aval, p->bpos, p->bcrd32, p->bval, p->mpos, p->mcrd,
-                                      p->semi, p->bm_store, p->cpos, ccrd, cval, th, items);
-                    }
+                    const bool times = p->semi == COMET_B200_PLUS_TIMES;
+                    auto kernel = colmap ? (times ? bitmap_numeric_kernel<true, true, true> : bitmap_numeric_kernel<true, false, true>)
+                                         : (times ? bitmap_numeric_kernel<true, true, false> : bitmap_numeric_kernel<true, false, false>);
+                    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                    launch_behind(kernel, dim3(grid), BM_THREADS, smem, st, p->n2, p->list2, words, stride, (unsigned)stage_n, colmap,
+                                  nullptr, p->apos, p->acrd, p->aval, p->bpos, bcrd32, p->bval, p->mpos, p->mcrd, p->semi, p->bm_store,
+                                  p->cpos, ccrd, cval, th, items);
                 }
             } else {
                 int grid = bitmap_grid(p->n2, 0);
                 void *gbm = nullptr;
                 rc = scratch(SLOT_BITMAP, (size_t)grid * smem, &gbm);
                 if (!rc)
-                    bitmap_numeric_kernel<false, false><<<grid, BM_THREADS, 0, st>>>(
-                        p->n2, p->list2, p->words, (uint32_t *)gbm, p->apos, p->acrd, p->aval, p->bpos,
-                        p->bcrd32, p->bval, p->mpos, p->mcrd, p->semi, p->bm_store, p->cpos, ccrd, cval, nullptr,
+                    bitmap_numeric_kernel<false, false, false><<<grid, BM_THREADS, 0, st>>>(
+                        p->n2, p->list2, words, stride, 0, nullptr, (uint32_t *)gbm, p->apos, p->acrd, p->aval, p->bpos,
+                        bcrd32, p->bval, p->mpos, p->mcrd, p->semi, p->bm_store, p->cpos, ccrd, cval, nullptr,
                         nullptr);
             }
             if (!rc && cudaGetLastError() != cudaSuccess) rc = fail("spgemm numeric (bitmap) launch failed");
