@@ -11,6 +11,10 @@
 // semiring a second pass over the mask entries with hits folds the products; then every row's entries are written in
 // mask order, which is ascending.
 //
+// Where A, B and M are one symmetric pattern (the adjacency matrix of a graph: the device looks every entry's mate up, 15 us), B needs
+// no transposing, the entries (i,j) and (j,i) have the same count and are counted once, with the longer list as the set, so nothing has
+// to be routed to the other side; a second pass folds the values of both.
+//
 // Taken when A's rows ascend strictly (checked on the device; a set or a list with repeats would count them wrong, and
 // so would B's, whose check is part of the transpose), when the bitmaps cover A's columns, and when the bound
 // sum |M_i| |A_i| on the elements streamed is at most MASKED_DOT_COST times the products of the push form: a mask much
@@ -32,8 +36,10 @@ struct MaskedStats {
     unsigned long long nrows_b;            // rows of B that A names
     unsigned long long products, bound;
     unsigned long long desc_all, desc_edge;           // places where A's coordinates do not ascend: all, and at row starts
-    long long nnz_a, nnz_m;
+    unsigned nnz_a, nnz_m;                 // 0xffffffff: that or more
+    unsigned long long one_sided;          // entries of A without a mate, see masked_mates_kernel
 };
+static_assert(sizeof(MaskedStats) <= 64, "fits a page-locked word block");
 
 struct MaskedPlan {
     char *mem;
@@ -46,6 +52,7 @@ struct MaskedPlan {
     int64_t *tpos, *bptr, *place;
     TcUnit *units, *mids;
     const int64_t *apos, *mpos;
+    int32_t *mate;                         // not null: A, B and M are one symmetric pattern; place of (j,i) for every entry (i,j)
 };
 
 static unsigned flat_grid(int64_t n)
@@ -90,8 +97,9 @@ masked_stats_kernel(int64_t nrows, const int64_t *__restrict__ apos, const int64
         if (edge) atomicAdd(&stats->desc_edge, (unsigned long long)edge);
     }
     if (t0 == 0) {
-        stats->nnz_a = n;
-        stats->nnz_m = mpos[nrows];
+        const int64_t m = mpos[nrows];
+        stats->nnz_a = n < 0xffffffffLL ? (unsigned)n : 0xffffffffu;
+        stats->nnz_m = m < 0xffffffffLL ? (unsigned)m : 0xffffffffu;
     }
 }
 
@@ -116,6 +124,44 @@ masked_rows_kernel(int64_t nrows, const int64_t *__restrict__ bpos, const int64_
     if ((threadIdx.x & 31) == 0) {
         if (all) atomicAdd(desc, all);
         if (edge) atomicAdd(desc + 1, edge);
+    }
+}
+
+// A square pattern of strictly ascending rows: the place of (j,i) for every entry (i,j), and the number of entries that have none.
+// A thread per entry: its row by a search in the row pointer, its mate by one in row j.
+__global__ void __launch_bounds__(256)
+masked_mates_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, int64_t room,
+                    int32_t *__restrict__ mate, MaskedStats *stats)
+{
+    const int64_t n = pos[nrows];
+    unsigned none = n > room;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n && p < room; p += (int64_t)gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = nrows - 1;
+        while (lo < hi) {                              // the first row that ends behind p
+            const int64_t mid = (lo + hi) >> 1;
+            if (pos[mid + 1] <= p) lo = mid + 1; else hi = mid;
+        }
+        const int64_t i = lo, j = crd[p], e = pos[j + 1];
+        lo = pos[j];
+        hi = e;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (crd[mid] < i) lo = mid + 1; else hi = mid;
+        }
+        if (lo < e && crd[lo] == i) mate[p] = (int32_t)lo;
+        else none++;
+    }
+    none = __reduce_add_sync(0xffffffffu, none);
+    if ((threadIdx.x & 31) == 0 && none) atomicAdd(&stats->one_sided, (unsigned long long)none);
+}
+
+// the entries left out have their mates' counts (an entry and its mate write the same)
+__global__ void __launch_bounds__(256)
+masked_mirror_kernel(int64_t n, const int32_t *__restrict__ mate, int32_t *cnt)
+{
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t c = cnt[mate[p]];
+        if (c > cnt[p]) cnt[p] = c;
     }
 }
 
@@ -153,7 +199,7 @@ template <class Out>
 static int run_pairs(MaskedPlan *m, const Out &out, cudaStream_t st)
 {
     // "A" of the pairs is the mask, "M" is A, "B" is the transposed B
-    const TcShape sh = {m->ncols, false, true};
+    const TcShape sh = {m->mate ? 0 : m->ncols, false, true, m->mate != nullptr};
     const int width = (int)m->width;
     const size_t smem = (size_t)2 * TC_SET_BUF * 4 + (size_t)((width >> 5) + 1) * 4;
     if (smem > 52 * 1024)
@@ -177,6 +223,7 @@ void masked_free(MaskedPlan *plan, cudaStream_t st)
 {
     if (!plan) return;
     if (plan->mem) cudaFreeAsync(plan->mem, st);
+    if (plan->mate) cudaFreeAsync(plan->mate, st);
     delete plan;
 }
 
@@ -191,19 +238,39 @@ int masked_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     CB_CUDA(cudaMemsetAsync(sp, 0, sizeof(MaskedStats), st));
     masked_stats_kernel<<<(unsigned)sm_count() * 4, 256, 0, st>>>(nrows, apos, acrd, bpos, mpos, (MaskedStats *)sp);
     CB_LAUNCH_CHECK();
+    // one matrix in all three places: it may be symmetric, as the adjacency matrix of a graph is
+    int32_t *mate = nullptr;
+    if (nrows == ncols_b && apos == bpos && apos == mpos && acrd == bcrd && acrd == mcrd &&
+        cudaMallocAsync((void **)&mate, (size_t)nnz_b * 4, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        mate = nullptr;
+    }
+    MaskedPlan *m = new MaskedPlan();
+    m->mate = mate;                        // freed with the plan
+    if (mate) masked_mates_kernel<<<flat_grid(nnz_b), 256, 0, st>>>(nrows, apos, acrd, nnz_b, mate, (MaskedStats *)sp);
     MaskedStats s;
     {
         PinnedWords words;
-        if (!words.p) return fail("spgemm: no page-locked memory");
-        CB_CUDA(cudaMemcpyAsync(words.p, sp, sizeof(s), cudaMemcpyDeviceToHost, st));
-        CB_CUDA(cudaStreamSynchronize(st));
+        int rc = words.p ? 0 : fail("spgemm: no page-locked memory");
+        if (!rc && (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(words.p, sp, sizeof(s), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                    cudaStreamSynchronize(st) != cudaSuccess))
+            rc = fail("spgemm: looking the operands over failed");
+        if (rc) {
+            masked_free(m, st);
+            return rc;
+        }
         memcpy(&s, words.p, sizeof(s));
     }
-    if (s.nnz_a <= 0 || s.nnz_m <= 0 || s.nnz_a >= 0x7fffffffLL || s.nnz_m >= 0x7fffffffLL || s.desc_all != s.desc_edge ||
-        (int64_t)s.nrows_b > TC_MAX_COLS || (double)s.bound > MASKED_DOT_COST * (double)s.products)
+    if (s.nnz_a == 0 || s.nnz_m == 0 || s.nnz_a >= 0x7fffffffu || s.nnz_m >= 0x7fffffffu || s.desc_all != s.desc_edge ||
+        (int64_t)s.nrows_b > TC_MAX_COLS || (double)s.bound > MASKED_DOT_COST * (double)s.products) {
+        masked_free(m, st);
         return 0;
-
-    MaskedPlan *m = new MaskedPlan();
+    }
+    if (m->mate && s.one_sided) {
+        cudaFreeAsync(m->mate, st);
+        m->mate = nullptr;
+    }
+    const bool sym = m->mate != nullptr;
     m->nrows = nrows; m->ncols = ncols_b; m->nnz_m = s.nnz_m; m->width = (int64_t)s.nrows_b; m->nnz_b = nnz_b;
     m->apos = apos; m->mpos = mpos;
     const size_t nunits = (size_t)(s.nnz_m / 16 + (s.nnz_a < nrows * TC_WARP_MAX ? s.nnz_a / TC_WARP_MAX : nrows) +
@@ -214,11 +281,14 @@ int masked_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     // cleared: headers (the second one only collects what tc_rows_kernel counts), list counts, hits
     const size_t o_hdr = want(3 * sizeof(TcHeader)), o_bcount = want((size_t)ncols_b * 4), o_cnt = want((size_t)s.nnz_m * 4);
     const size_t cleared = total;
-    const size_t o_a32 = want((size_t)s.nnz_a * 4 + 16), o_m32 = want((size_t)s.nnz_m * 4 + 16),
-                 o_trow = want((size_t)nnz_b * 4 + 16), o_tidx = want((size_t)nnz_b * 4), o_tpos = want((size_t)(ncols_b + 1) * 8),
-                 o_bptr = want((size_t)(ncols_b + 1) * 8), o_blist = want((size_t)s.nnz_m * 8), o_small = want((size_t)nrows * 4), o_place = want((size_t)(s.nnz_m + 1) * 8),
+    const size_t o_a32 = want((size_t)s.nnz_a * 4 + 16), o_small = want((size_t)nrows * 4), o_place = want(((size_t)s.nnz_m + 1) * 8),
                  o_units = want(nunits * sizeof(TcUnit)), o_mids = want(nunits * sizeof(TcUnit));
-    const size_t o_rows = want((size_t)(nnz_b > s.nnz_m ? nnz_b : s.nnz_m) * 4), o_slot = want((size_t)s.nnz_m * 4);
+    // not needed for a symmetric pattern, which is its own transpose and has no B side
+    auto want_too = [&](size_t bytes) { return sym ? 0 : want(bytes); };
+    const size_t o_m32 = want_too((size_t)s.nnz_m * 4 + 16), o_trow = want_too((size_t)nnz_b * 4 + 16), o_tidx = want_too((size_t)nnz_b * 4),
+                 o_tpos = want_too((size_t)(ncols_b + 1) * 8), o_bptr = want_too((size_t)(ncols_b + 1) * 8),
+                 o_blist = want_too((size_t)s.nnz_m * 8), o_rows = want_too((size_t)(nnz_b > s.nnz_m ? nnz_b : s.nnz_m) * 4),
+                 o_slot = want_too((size_t)s.nnz_m * 4);
     if (cudaMallocAsync((void **)&m->mem, total, st) != cudaSuccess) {
         (void)cudaGetLastError();
         m->mem = nullptr;
@@ -234,32 +304,43 @@ int masked_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     m->bptr = (int64_t *)at(o_bptr); m->blist = (int2 *)at(o_blist); m->small = (int32_t *)at(o_small);
     m->place = (int64_t *)at(o_place);
     m->units = (TcUnit *)at(o_units); m->mids = (TcUnit *)at(o_mids);
+    if (sym) {
+        m->m32 = m->trow = m->a32;
+        m->tidx = m->mate;
+        m->tpos = const_cast<int64_t *>(apos);
+    }
     int32_t *bcount = (int32_t *)at(o_bcount), *rows = (int32_t *)at(o_rows), *slot = (int32_t *)at(o_slot);
 
     auto build = [&]() {
         CB_CUDA(cudaMemsetAsync(m->mem, 0, cleared, st));
         CB_TRY(narrow_any_i64_to_i32(acrd, m->a32, s.nnz_a, st));
-        CB_TRY(narrow_any_i64_to_i32(mcrd, m->m32, s.nnz_m, st));
-        masked_rows_kernel<<<flat_grid(m->width * 16), 256, 0, st>>>(m->width, bpos, bcrd, rows, (unsigned *)m->err + 1);
-        CB_LAUNCH_CHECK();
-        CB_TRY(transpose_index(nnz_b, bpos + m->width, ncols_b, bcrd, rows, m->tpos, m->trow, m->tidx, m->err, st));
-        const TcShape sh = {ncols_b, false, true};
-        tc_rows_kernel<<<flat_grid(nrows * 16), 256, 0, st>>>(0, nrows, mpos, apos, acrd, rows, m->hdr + 1);
-        CB_LAUNCH_CHECK();
-        tc_route_kernel<<<flat_grid(s.nnz_m), 256, 0, st>>>(0, nrows, mpos, m->m32, rows, m->tpos, apos, sh, m->hdr, slot, bcount);
-        CB_LAUNCH_CHECK();
-        CB_TRY(exclusive_scan_i32(bcount, m->bptr, ncols_b, st));
-        tc_scatter_kernel<<<flat_grid(s.nnz_m), 256, 0, st>>>(0, nrows, mpos, m->m32, rows, slot, m->bptr, m->blist);
-        CB_LAUNCH_CHECK();
+        const TcShape sh = {ncols_b, false, true, false};
+        if (!sym) {
+            CB_TRY(narrow_any_i64_to_i32(mcrd, m->m32, s.nnz_m, st));
+            masked_rows_kernel<<<flat_grid(m->width * 16), 256, 0, st>>>(m->width, bpos, bcrd, rows, (unsigned *)m->err + 1);
+            CB_LAUNCH_CHECK();
+            CB_TRY(transpose_index(nnz_b, bpos + m->width, ncols_b, bcrd, rows, m->tpos, m->trow, m->tidx, m->err, st));
+            tc_rows_kernel<<<flat_grid(nrows * 16), 256, 0, st>>>(0, nrows, mpos, apos, acrd, rows, m->hdr + 1);
+            CB_LAUNCH_CHECK();
+            tc_route_kernel<<<flat_grid(s.nnz_m), 256, 0, st>>>(0, nrows, mpos, m->m32, rows, m->tpos, apos, sh, m->hdr, slot, bcount);
+            CB_LAUNCH_CHECK();
+            CB_TRY(exclusive_scan_i32(bcount, m->bptr, ncols_b, st));
+            tc_scatter_kernel<<<flat_grid(s.nnz_m), 256, 0, st>>>(0, nrows, mpos, m->m32, rows, slot, m->bptr, m->blist);
+            CB_LAUNCH_CHECK();
+        }
         auto clamp = [](int64_t v, int64_t lo, int64_t hi) { return (unsigned)(v < lo ? lo : (v > hi ? hi : v)); };
         const int64_t most = nrows > ncols_b ? nrows : ncols_b;
-        tc_units_kernel<<<(unsigned)ceil_div(most, 256), 256, 0, st>>>(0, nrows, ncols_b, mpos, apos, m->tpos, m->bptr, m->hdr,
+        tc_units_kernel<<<(unsigned)ceil_div(most, 256), 256, 0, st>>>(0, nrows, sym ? 0 : ncols_b, mpos, apos, m->tpos, m->bptr, m->hdr,
                                                                       m->small, m->mids, m->units,
                                                                       clamp(s.nnz_m / (sm_count() * 192), 32, 512),
                                                                       clamp(s.nnz_m / (sm_count() * 64), 64, 4096));
         CB_LAUNCH_CHECK();
         const TcCountPairs out = {m->cnt};
         CB_TRY(run_pairs(m, out, st));
+        if (sym) {
+            masked_mirror_kernel<<<flat_grid(s.nnz_m), 256, 0, st>>>(s.nnz_m, m->mate, m->cnt);
+            CB_LAUNCH_CHECK();
+        }
         CB_TRY(exclusive_scan_nonzero(m->cnt, m->place, s.nnz_m, st));
         masked_pos_kernel<<<flat_grid(nrows + 1), 256, 0, st>>>(nrows, mpos, m->place, cpos);
         CB_LAUNCH_CHECK();
@@ -283,9 +364,9 @@ int masked_numeric(MaskedPlan *m, const double *aval, const double *bval, const 
             return fail("spgemm numeric: device allocation failed");
         tval = val + m->nnz_m;             // B's values in column order
         masked_gather_kernel<<<flat_grid(m->nnz_b), 256, 0, st>>>(m->nnz_b, m->tidx, bval, tval);
-        const TcValuePairs out = {m->cnt, val, aval, tval, semi};
         int rc = cudaMemsetAsync(&m->hdr->next_small, 0, 3 * sizeof(unsigned), st) == cudaSuccess ? 0 : fail("spgemm numeric: clearing the counters failed");
-        if (!rc) rc = run_pairs(m, out, st);
+        if (!rc) rc = m->mate ? run_pairs(m, TcValuePairs<true>{m->cnt, m->mate, val, aval, tval, semi}, st)
+                              : run_pairs(m, TcValuePairs<false>{m->cnt, nullptr, val, aval, tval, semi}, st);
         if (rc) {
             cudaFreeAsync(val, st);
             return rc;

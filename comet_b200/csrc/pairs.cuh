@@ -35,7 +35,14 @@ struct TcShape {
     int64_t bcap;         // rows of B that can be sets
     bool cut;             // A and M are one matrix
     bool distinct;        // a coordinate that row i of A repeats is one pair (otherwise one per occurrence)
+    bool half;            // A, M and B (rows of B as the pairs have them) are one symmetric pattern: of the pairs (i,k) and (k,i) the one
+                          // whose set is the longer list is taken, and none goes to the B side
 };
+
+__device__ __forceinline__ bool tc_left_out(const TcShape &sh, int64_t i, int64_t k, int64_t ml, int64_t bl)
+{
+    return sh.half && (bl > ml || (bl == ml && k > i));
+}
 
 // M repeats no coordinate: every place where its coordinates do not ascend is the start of a row
 __device__ __forceinline__ bool tc_swap_ok(const TcHeader *hdr) { return hdr->desc_all == hdr->desc_edge; }
@@ -358,9 +365,12 @@ struct TcCountPairs {                      // cnt[p], cleared before
     __device__ void finish(unsigned long long *, int) {}
 };
 
-struct TcValuePairs {                      // val[p] for the pairs with hits: the products of equal positions, folded
+// val[p] for the pairs with hits: the products of equal positions, folded.  BOTH: a pair taken for two (TcShape::half): val[mate[p]] too,
+// from the values of A along the list and of B along the set.
+template <bool BOTH>
+struct TcValuePairs {
     static const bool PAIRS = true, VALUES = true;
-    const int32_t *cnt;
+    const int32_t *cnt, *mate;
     double *val;
     const double *aval, *bval;             // values of the rows of A (the lists "M_i") and of the transposed B ("B_k")
     int semi;
@@ -372,15 +382,18 @@ struct TcValuePairs {                      // val[p] for the pairs with hits: th
                            int64_t set_at)
     {
         const double *sval = (bside ? bval : aval) + set_at, *lval = bside ? aval : bval;
-        double own = 0.0, part = sr_identity(semi);
+        double own = 0.0, part = sr_identity(semi), own2 = 0.0, part2 = part;
         unsigned left = __ballot_sync(0xffffffffu, len > 0);
         int64_t at = 0;
         int rem = 0, t = -1, cur = -1;
         auto flush = [&]() {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) part = sr_fold_value(semi, part, __shfl_xor_sync(0xffffffffu, part, o));
-            if (lane == cur) own = part;
-            part = sr_identity(semi);
+            for (int o = 16; o > 0; o >>= 1) {
+                part = sr_fold_value(semi, part, __shfl_xor_sync(0xffffffffu, part, o));
+                if (BOTH) part2 = sr_fold_value(semi, part2, __shfl_xor_sync(0xffffffffu, part2, o));
+            }
+            if (lane == cur) { own = part; own2 = part2; }
+            part = part2 = sr_identity(semi);
         };
         while (left || rem > 0) {
             int32_t j[4];
@@ -408,13 +421,19 @@ struct TcValuePairs {                      // val[p] for the pairs with hits: th
                     cur = of[i];
                 }
                 if (probe(j[i])) {
-                    const double sv = __ldg(sval + where(j[i])), lv = __ldg(lval + from[i]);
+                    const int at_set = where(j[i]);
+                    const double sv = __ldg(sval + at_set), lv = __ldg(lval + from[i]);
                     part = sr_fold_value(semi, part, bside ? sr_combine(semi, lv, sv) : sr_combine(semi, sv, lv));
+                    if (BOTH)
+                        part2 = sr_fold_value(semi, part2, sr_combine(semi, __ldg(aval + from[i]), __ldg(bval + set_at + at_set)));
                 }
             }
         }
         if (cur >= 0) flush();
-        if (len > 0) val[p] = own;
+        if (len > 0) {
+            val[p] = own;
+            if (BOTH) val[mate[p]] = own2;
+        }
     }
     __device__ void finish(unsigned long long *, int) {}
 };
@@ -497,7 +516,9 @@ tc_warp_kernel(TcHeader *hdr, const int32_t *__restrict__ small, const int64_t *
                     s = bpos[k];
                     const int64_t bl = bpos[k + 1] - s;
                     const bool again = sh.distinct && p0 + lane > as && acrd[p0 + lane - 1] == k;
-                    if (!again && out.wanted(p0 + lane) && !tc_b_side(swap, me - ms, p0 + lane - as, bl, k, sh)) len = (int)bl;
+                    if (!again && out.wanted(p0 + lane) && !tc_left_out(sh, i, k, me - ms, bl) &&
+                        !tc_b_side(swap, me - ms, p0 + lane - as, bl, k, sh))
+                        len = (int)bl;
                 }
                 if (!__any_sync(0xffffffffu, len > 0)) continue;
                 if (!filled) {
@@ -518,7 +539,7 @@ tc_warp_kernel(TcHeader *hdr, const int32_t *__restrict__ small, const int64_t *
 // `first` is the unit's first entry of A's row (mask side) or first place in blist.  On the B side a list ends, at the
 // latest, where the entry of M_i at the pair's own place o in row i already lies behind the set's last column.
 template <class Out>
-__device__ __forceinline__ void tc_unit_lists(const Out &out, bool bside, int64_t first, int64_t off, int b, int n, int lists,
+__device__ __forceinline__ void tc_unit_lists(const Out &out, int64_t row, bool bside, int64_t first, int64_t off, int b, int n, int lists,
                                               int lane, bool swap, int64_t ml, int32_t last, TcShape sh,
                                               const int64_t *__restrict__ apos, const int32_t *__restrict__ acrd,
                                               const int64_t *__restrict__ bpos, const int64_t *__restrict__ mpos,
@@ -544,7 +565,7 @@ __device__ __forceinline__ void tc_unit_lists(const Out &out, bool bside, int64_
         if (!out.wanted(p) || (sh.distinct && off + b + lane > 0 && __ldg(acrd + p - 1) == k)) return;
         s = __ldg(bpos + k);
         const int64_t bl = __ldg(bpos + k + 1) - s;
-        len = tc_b_side(swap, ml, off + b + lane, bl, k, sh) ? 0 : (int)bl;
+        len = tc_left_out(sh, row, k, ml, bl) || tc_b_side(swap, ml, off + b + lane, bl, k, sh) ? 0 : (int)bl;
     }
 }
 
@@ -584,7 +605,7 @@ tc_mid_kernel(TcHeader *hdr, const TcUnit *__restrict__ mids, const int64_t *__r
             int64_t s;
             int len;
             int64_t p;
-            tc_unit_lists(out, bside, row_at, u.off, b, 32, lists, lane, swap, se - ss, last, sh, apos, acrd, bpos, mpos, mcrd,
+            tc_unit_lists(out, u.row, bside, row_at, u.off, b, 32, lists, lane, swap, se - ss, last, sh, apos, acrd, bpos, mpos, mcrd,
                           blist, s, len, p);
             tc_stream_set<TC_MID_LOG2>(out, s_tab[w], s_place[Out::VALUES ? w : 0], how, lcrd, s, len, lane, scrd + ss, p, bside,
                                        ss, (int)(se - ss));
@@ -706,7 +727,7 @@ tc_bitmap_kernel(TcHeader *hdr, const TcUnit *__restrict__ units, const int64_t 
                 if ((int)b >= lists) break;
                 int64_t s, p;
                 int n;
-                tc_unit_lists(out, bside, row_at, u.off, (int)b, step, lists, lane, swap, ml, bside ? s_last : 0, sh, apos, acrd,
+                tc_unit_lists(out, u.row, bside, row_at, u.off, (int)b, step, lists, lane, swap, ml, bside ? s_last : 0, sh, apos, acrd,
                               bpos, mpos, mcrd, blist, s, n, p);
                 auto where = [&](int32_t x) {
                     if (!Out::VALUES || !pre) return tc_search(set, len, x);

@@ -116,7 +116,7 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     // two agree for the square operands this is called with (pairs beyond it stay on the mask side)
     const int64_t bcap = ncols > row_hi ? ncols : row_hi;
     const bool compact = ncols > TC_MAX_COLS;
-    const TcShape sh = {bcap, acrd == mcrd && apos == mpos, false};
+    const TcShape sh = {bcap, acrd == mcrd && apos == mpos, false, false};
     const int64_t words = ceil_div(ncols, 32);
     auto grid_for = [](int64_t n) {
         const int64_t blocks = ceil_div(n, 256), cap = (int64_t)sm_count() * 16;
