@@ -56,11 +56,13 @@ enum Slot {
     SLOT_MISC,
     SLOT_FLAG,           // a word that tells kernels of one call which of them the operands are for
     SLOT_TEAMS,          // team item list of the SpGEMM numeric pass
+    SLOT_TRIANGLES,      // a triangular matrix in another order of its vertices (order.cuh)
     SLOT_H2D_0, SLOT_H2D_1, SLOT_H2D_2, SLOT_H2D_3, SLOT_H2D_4, SLOT_H2D_5,
     SLOT_H2D_6, SLOT_H2D_7, SLOT_H2D_8, SLOT_H2D_9, SLOT_H2D_10, SLOT_H2D_11,
     SLOT_COUNT
 };
 int scratch(Slot slot, size_t bytes, void **ptr);   // status; *ptr valid until the slot grows
+bool scratch_if_room(Slot slot, size_t bytes, void **ptr);   // for what a call can do without: false, and no error, where it does not fit
 void scratch_release_all();
 void result_release_kept();                          // page-locked result blocks that are not in use (hostmem.cu)
 

@@ -199,7 +199,7 @@ template <class Out>
 static int run_pairs(MaskedPlan *m, const Out &out, cudaStream_t st)
 {
     // "A" of the pairs is the mask, "M" is A, "B" is the transposed B
-    const TcShape sh = {m->mate ? 0 : m->ncols, false, true, m->mate != nullptr};
+    const TcShape sh = {m->mate ? 0 : m->ncols, false, true, m->mate != nullptr, false};
     const int width = (int)m->width;
     const size_t smem = (size_t)2 * TC_SET_BUF * 4 + (size_t)((width >> 5) + 1) * 4;
     if (smem > 52 * 1024)
@@ -314,7 +314,7 @@ int masked_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     auto build = [&]() {
         CB_CUDA(cudaMemsetAsync(m->mem, 0, cleared, st));
         CB_TRY(narrow_any_i64_to_i32(acrd, m->a32, s.nnz_a, st));
-        const TcShape sh = {ncols_b, false, true, false};
+        const TcShape sh = {ncols_b, false, true, false, false};
         if (!sym) {
             CB_TRY(narrow_any_i64_to_i32(mcrd, m->m32, s.nnz_m, st));
             masked_rows_kernel<<<flat_grid(m->width * 16), 256, 0, st>>>(m->width, bpos, bcrd, rows, (unsigned *)m->err + 1);

@@ -29,6 +29,7 @@ struct TcHeader {
     unsigned nsmall, nmid, nunits;         // short mask rows, hash-set units, bitmap units
     unsigned next_small, next_mid, next_unit;         // next one to hand out
     unsigned desc_all, desc_edge;          // positions where M's coordinates do not ascend: all, and those at row starts
+    unsigned ordered;                      // A, B and M are the rest of a matrix in another order (order.cuh): rows in any order
 };
 
 struct TcShape {
@@ -37,6 +38,7 @@ struct TcShape {
     bool distinct;        // a coordinate that row i of A repeats is one pair (otherwise one per occurrence)
     bool half;            // A, M and B (rows of B as the pairs have them) are one symmetric pattern: of the pairs (i,k) and (k,i) the one
                           // whose set is the longer list is taken, and none goes to the B side
+    bool ask;             // `cut` is off if TcHeader::ordered
 };
 
 __device__ __forceinline__ bool tc_left_out(const TcShape &sh, int64_t i, int64_t k, int64_t ml, int64_t bl)
@@ -50,9 +52,9 @@ __device__ __forceinline__ bool tc_swap_ok(const TcHeader *hdr) { return hdr->de
 // The pair of entry number o of row i of A goes to the B side: B_k is the longer one.  What is compared is the part of
 // M_i that would be streamed: when A and M are one matrix whose row i is cut at column k (`cut`: a strict lower
 // triangle squared, where no column of B_k reaches k), that is its first o entries.
-__device__ __forceinline__ bool tc_b_side(bool swap, int64_t ml, int64_t o, int64_t bl, int64_t k, const TcShape &sh)
+__device__ __forceinline__ bool tc_b_side(bool swap, int64_t ml, int64_t o, int64_t bl, int64_t k, const TcShape &sh, bool cut)
 {
-    return swap && bl > TC_WARP_MAX && bl > (sh.cut ? o : ml) && k < sh.bcap;
+    return swap && bl > TC_WARP_MAX && bl > (cut ? o : ml) && k < sh.bcap;
 }
 
 // --- cuckoo set: tables T0 = tab[0, H) and T1 = tab[H, 2H), H = 2^(LOG2-1) -------------------------
@@ -149,12 +151,13 @@ tc_rows_kernel(int64_t row_lo, int64_t row_hi, const int64_t *__restrict__ apos,
 {
     const int l = threadIdx.x & 15;
     const int64_t first = mpos[row_lo];
+    const bool check = l == 0 && !hdr->ordered;
     unsigned desc = 0;
     const int64_t ng = ((int64_t)gridDim.x * blockDim.x) >> 4;
     for (int64_t r = row_lo + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4); r < row_hi; r += ng) {
         const int64_t e = apos[r + 1];
         for (int64_t p = apos[r] + l; p < e; p += 16) arow[p] = (int32_t)r;
-        if (l == 0) {
+        if (check) {
             const int64_t s = mpos[r];
             if (s > first && mpos[r + 1] > s && mcrd[s] <= mcrd[s - 1]) desc++;
         }
@@ -169,6 +172,7 @@ tc_route_kernel(int64_t row_lo, int64_t row_hi, const int64_t *__restrict__ apos
                 TcShape sh, const TcHeader *hdr, int32_t *__restrict__ slot, int32_t *__restrict__ bcount)
 {
     const bool swap = tc_swap_ok(hdr);
+    const bool cut = sh.cut && !(sh.ask && hdr->ordered);
     const int64_t end = apos[row_hi];
     for (int64_t p = apos[row_lo] + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < end;
          p += (int64_t)gridDim.x * blockDim.x) {
@@ -176,7 +180,7 @@ tc_route_kernel(int64_t row_lo, int64_t row_hi, const int64_t *__restrict__ apos
         const int64_t ml = mpos[i + 1] - mpos[i], bl = bpos[k + 1] - bpos[k];
         int32_t at = -1;
         const bool again = sh.distinct && p > apos[i] && acrd[p - 1] == k;
-        if (ml > 0 && !again && tc_b_side(swap, ml, p - apos[i], bl, k, sh)) at = atomicAdd(bcount + k, 1);
+        if (ml > 0 && !again && tc_b_side(swap, ml, p - apos[i], bl, k, sh, cut)) at = atomicAdd(bcount + k, 1);
         slot[p] = at;
     }
 }
@@ -496,6 +500,7 @@ tc_warp_kernel(TcHeader *hdr, const int32_t *__restrict__ small, const int64_t *
     __shared__ unsigned long long s_part[TC_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool swap = tc_swap_ok(hdr);
+    const bool cut = sh.cut && !(sh.ask && hdr->ordered);
     const unsigned n = hdr->nsmall;
     while (true) {
         unsigned idx = 0;
@@ -516,8 +521,8 @@ tc_warp_kernel(TcHeader *hdr, const int32_t *__restrict__ small, const int64_t *
                     s = bpos[k];
                     const int64_t bl = bpos[k + 1] - s;
                     const bool again = sh.distinct && p0 + lane > as && acrd[p0 + lane - 1] == k;
-                    if (!again && out.wanted(p0 + lane) && !tc_left_out(sh, i, k, me - ms, bl) &&
-                        !tc_b_side(swap, me - ms, p0 + lane - as, bl, k, sh))
+                    if (!again && out.wanted(p0 + lane) && !(Out::PAIRS && tc_left_out(sh, i, k, me - ms, bl)) &&
+                        !tc_b_side(swap, me - ms, p0 + lane - as, bl, k, sh, cut))
                         len = (int)bl;
                 }
                 if (!__any_sync(0xffffffffu, len > 0)) continue;
@@ -540,7 +545,7 @@ tc_warp_kernel(TcHeader *hdr, const int32_t *__restrict__ small, const int64_t *
 // latest, where the entry of M_i at the pair's own place o in row i already lies behind the set's last column.
 template <class Out>
 __device__ __forceinline__ void tc_unit_lists(const Out &out, int64_t row, bool bside, int64_t first, int64_t off, int b, int n, int lists,
-                                              int lane, bool swap, int64_t ml, int32_t last, TcShape sh,
+                                              int lane, bool swap, bool cut, int64_t ml, int32_t last, const TcShape &sh,
                                               const int64_t *__restrict__ apos, const int32_t *__restrict__ acrd,
                                               const int64_t *__restrict__ bpos, const int64_t *__restrict__ mpos,
                                               const int32_t *__restrict__ mcrd, const int2 *__restrict__ blist, int64_t &s,
@@ -558,14 +563,14 @@ __device__ __forceinline__ void tc_unit_lists(const Out &out, int64_t row, bool 
         }
         s = __ldg(mpos + io.x);
         len = (int)(__ldg(mpos + io.x + 1) - s);
-        if (sh.cut && io.y < len && __ldg(mcrd + s + io.y) > last) len = io.y;
+        if (cut && io.y < len && __ldg(mcrd + s + io.y) > last) len = io.y;
     } else {
         p = first + b + lane;
         const int64_t k = __ldg(acrd + p);
         if (!out.wanted(p) || (sh.distinct && off + b + lane > 0 && __ldg(acrd + p - 1) == k)) return;
         s = __ldg(bpos + k);
         const int64_t bl = __ldg(bpos + k + 1) - s;
-        len = tc_left_out(sh, row, k, ml, bl) || tc_b_side(swap, ml, off + b + lane, bl, k, sh) ? 0 : (int)bl;
+        len = (Out::PAIRS && tc_left_out(sh, row, k, ml, bl)) || tc_b_side(swap, ml, off + b + lane, bl, k, sh, cut) ? 0 : (int)bl;
     }
 }
 
@@ -582,6 +587,7 @@ tc_mid_kernel(TcHeader *hdr, const TcUnit *__restrict__ mids, const int64_t *__r
     __shared__ unsigned long long s_part[TC_MID_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool swap = tc_swap_ok(hdr);
+    const bool cut = sh.cut && !(sh.ask && hdr->ordered);
     const unsigned n = hdr->nmid;
     while (true) {
         unsigned idx = 0;
@@ -605,7 +611,7 @@ tc_mid_kernel(TcHeader *hdr, const TcUnit *__restrict__ mids, const int64_t *__r
             int64_t s;
             int len;
             int64_t p;
-            tc_unit_lists(out, u.row, bside, row_at, u.off, b, 32, lists, lane, swap, se - ss, last, sh, apos, acrd, bpos, mpos, mcrd,
+            tc_unit_lists(out, u.row, bside, row_at, u.off, b, 32, lists, lane, swap, cut, se - ss, last, sh, apos, acrd, bpos, mpos, mcrd,
                           blist, s, len, p);
             tc_stream_set<TC_MID_LOG2>(out, s_tab[w], s_place[Out::VALUES ? w : 0], how, lcrd, s, len, lane, scrd + ss, p, bside,
                                        ss, (int)(se - ss));
@@ -639,6 +645,7 @@ tc_bitmap_kernel(TcHeader *hdr, const TcUnit *__restrict__ units, const int64_t 
     uint32_t *pre = Out::VALUES && with_prefix ? bm + words : nullptr;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool swap = tc_swap_ok(hdr);
+    const bool cut = sh.cut && !(sh.ask && hdr->ordered);
     const unsigned nunits = hdr->nunits;
     for (int t = threadIdx.x; t < words; t += THREADS) bm[t] = 0;
 
@@ -727,7 +734,7 @@ tc_bitmap_kernel(TcHeader *hdr, const TcUnit *__restrict__ units, const int64_t 
                 if ((int)b >= lists) break;
                 int64_t s, p;
                 int n;
-                tc_unit_lists(out, u.row, bside, row_at, u.off, (int)b, step, lists, lane, swap, ml, bside ? s_last : 0, sh, apos, acrd,
+                tc_unit_lists(out, u.row, bside, row_at, u.off, (int)b, step, lists, lane, swap, cut, ml, bside ? s_last : 0, sh, apos, acrd,
                               bpos, mpos, mcrd, blist, s, n, p);
                 auto where = [&](int32_t x) {
                     if (!Out::VALUES || !pre) return tc_search(set, len, x);

@@ -73,6 +73,25 @@ static DeviceState *state()
     return &g_dev[d];
 }
 
+bool scratch_if_room(Slot slot, size_t bytes, void **ptr)
+{
+    std::lock_guard<std::mutex> lk(g_mu);
+    DeviceState *s = state();
+    if (!s) return false;
+    if (s->cap[slot] < bytes) {
+        void *p = nullptr;                 // beside the old buffer, which stays if this fails
+        if (cudaMalloc(&p, (bytes + 255) & ~(size_t)255) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        if (s->ptr[slot] && (cudaDeviceSynchronize() != cudaSuccess || cudaFree(s->ptr[slot]) != cudaSuccess)) return false;
+        s->ptr[slot] = p;
+        s->cap[slot] = (bytes + 255) & ~(size_t)255;
+    }
+    *ptr = s->ptr[slot];
+    return true;
+}
+
 int scratch(Slot slot, size_t bytes, void **ptr)
 {
     std::lock_guard<std::mutex> lk(g_mu);

@@ -27,10 +27,12 @@
 // flag found while M is narrowed), and a B_k that sets a bit twice has its hits counted by a linear scan.
 //
 // Counts are exact int64; no floating point is involved.
-// Measured on B200, R-MAT edge factor 16 lower triangles (mask side only, cuckoo sets in every bin -> this):
-// scale 14 0.27 -> 0.16 ms, scale 18 1.96 -> 0.76, scale 20 10.2 -> 3.15, scale 22 61.9 -> 18.3.  At scale 22 the bitmap kernel takes 12.0 of
-// it (shared-memory pipe and issue slots both near 70 %: 6.7 wavefronts and 25 instructions per 32 probes), the hash
-// sets 3.6, routing and scattering the pairs 1.4, narrowing and renumbering 1.1.
+// A matrix counted with itself that is large and triangular, as a graph's lower triangle, is renumbered first (order.cuh); only what lies
+// beyond its hub columns is left to the kernels here.
+//
+// Measured on B200, R-MAT edge factor 16 lower triangles (mask side only, cuckoo sets in every bin -> both sides, bitmaps -> renumbered):
+// scale 14 0.27 -> 0.16 ms, scale 18 1.96 -> 0.76, scale 20 10.2 -> 3.15 -> 2.38, scale 22 61.9 -> 18.4 -> 11.4.
+#include "order.cuh"
 #include "pairs.cuh"
 
 namespace cb200 {
@@ -41,8 +43,9 @@ namespace cb200 {
 static const int TC_SEEN_SLOTS = 8192;
 
 __global__ void __launch_bounds__(512)
-tc_present_kernel(int64_t n, const int64_t *__restrict__ mcrd, uint32_t *__restrict__ present)
+tc_present_kernel(int64_t n, const int64_t *__restrict__ mcrd, uint32_t *__restrict__ present, const TcHeader *mode)
 {
+    if (mode && mode->ordered) return;
     __shared__ int32_t s_seen[TC_SEEN_SLOTS];
     for (int t = threadIdx.x; t < TC_SEEN_SLOTS; t += blockDim.x) s_seen[t] = -1;
     __syncthreads();
@@ -69,8 +72,9 @@ tc_popc_kernel(int64_t words, const uint32_t *__restrict__ present, int32_t *__r
 __global__ void __launch_bounds__(256)
 tc_narrow_kernel(int64_t n, const int64_t *__restrict__ crd, int32_t *__restrict__ out,
                  const uint32_t *__restrict__ present, const int64_t *__restrict__ before, int64_t words,
-                 const int64_t *__restrict__ pos, int64_t row_lo, int64_t row_hi, TcHeader *hdr)
+                 const int64_t *__restrict__ pos, int64_t row_lo, int64_t row_hi, TcHeader *hdr, const TcHeader *mode)
 {
+    if (mode && mode->ordered) return;
     int64_t lo = 0, hi = 0;
     if (hdr) { lo = pos[row_lo]; hi = pos[row_hi] - 1; }
     unsigned desc = 0;
@@ -100,6 +104,87 @@ tc_narrow_kernel(int64_t n, const int64_t *__restrict__ crd, int32_t *__restrict
     if (hdr && desc) atomicAdd(&hdr->desc_all, desc);
 }
 
+struct TriArrays {
+    TriCounters *counters;
+    uint32_t *degree, *bits;
+    int32_t *rank, *hub_count, *rest_count, *bits_at;
+    int64_t *hub_pos, *rest_pos;
+    unsigned short *hub;
+    int2 *edge;
+    int32_t *place;
+    unsigned long long room;               // words of `bits`
+};
+
+// eight bytes an entry hold all bitmaps of R-MAT graphs; rows that find no room do without
+static size_t tri_room(int64_t nnz) { return nnz * 2 < ((int64_t)1 << 28) ? (size_t)nnz * 2 : (size_t)1 << 28; }
+static size_t tri_pad(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+static size_t tri_bytes(int64_t nrows, int64_t nnz)
+{
+    return tri_pad(sizeof(TriCounters)) + 5 * tri_pad((size_t)nrows * 4) + 2 * tri_pad((size_t)(nrows + 1) * 8) + tri_pad((size_t)nnz * 2) +
+           tri_room(nnz) * 4;
+}
+
+// Decides whether the matrix is counted in another order, and numbers its vertices and edges (mem: tri_bytes; edge, place: room for n of them).
+static int tri_prepare(int64_t nrows, int64_t nnz, const int64_t *pos, const int64_t *crd, TcHeader *hdr, void *mem, int2 *edge, int32_t *place,
+                       TriArrays *t, cudaStream_t st)
+{
+    const size_t b_n = tri_pad((size_t)nrows * 4), b_pos = tri_pad((size_t)(nrows + 1) * 8), b_tc = tri_pad(sizeof(TriCounters)),
+                 b_hub = tri_pad((size_t)nnz * 2), cleared = b_tc + 3 * b_n;
+    t->room = tri_room(nnz);
+    char *at = (char *)mem;
+    auto take = [&](size_t bytes) { char *q = at; at += bytes; return (void *)q; };
+    t->counters = (TriCounters *)take(b_tc);
+    t->degree = (uint32_t *)take(b_n);
+    t->hub_count = (int32_t *)take(b_n);
+    t->rest_count = (int32_t *)take(b_n);
+    t->rank = (int32_t *)take(b_n);
+    t->bits_at = (int32_t *)take(b_n);
+    t->hub_pos = (int64_t *)take(b_pos);
+    t->rest_pos = (int64_t *)take(b_pos);
+    t->hub = (unsigned short *)take(b_hub);
+    t->bits = (uint32_t *)at;
+    t->edge = edge;
+    t->place = place;
+    CB_CUDA(cudaMemsetAsync(mem, 0, cleared, st));
+    const unsigned full = (unsigned)sm_count() * 8;
+    auto grid = [&](int64_t items, int per) {
+        const int64_t n = ceil_div(items, per);
+        return (unsigned)(n < (int64_t)full ? n : (int64_t)full);
+    };
+    tri_degree_kernel<<<grid(nnz, 512), 256, 0, st>>>(nnz, crd, t->degree, hdr);
+    CB_LAUNCH_CHECK();
+    tri_hist_kernel<<<grid(nrows, 2048), 512, 0, st>>>(nrows, pos, crd, t->degree, hdr, t->counters);
+    CB_LAUNCH_CHECK();
+    tri_decide_kernel<<<1, TRI_BUCKETS, 0, st>>>(nnz, hdr, t->counters);
+    CB_LAUNCH_CHECK();
+    tri_rank_kernel<<<grid(nrows, 2048), 512, 0, st>>>(nrows, t->degree, hdr, t->counters, t->rank);
+    CB_LAUNCH_CHECK();
+    tri_edges_kernel<<<(unsigned)ceil_div(nnz, 4096), 256, 0, st>>>(nrows, nnz, pos, crd, t->rank, hdr, t->counters, t->edge,
+                                                                   t->place, t->hub_count, t->rest_count);
+    CB_LAUNCH_CHECK();
+    CB_TRY(exclusive_scan_i32(t->hub_count, t->hub_pos, nrows, st));
+    CB_TRY(exclusive_scan_i32(t->rest_count, t->rest_pos, nrows, st));
+    tri_keep_kernel<<<grid(nrows + 1, 256), 256, 0, st>>>(nrows, pos, hdr, t->rest_pos);
+    CB_LAUNCH_CHECK();
+    return 0;
+}
+
+// Counts the triangles of the hub columns; the rest of the rows goes to a32 and, renumbered, m32.
+static int tri_count(int64_t nrows, int64_t nnz, TcHeader *hdr, TriArrays *t, int32_t *a32, int32_t *m32,
+                     int64_t *columns, int64_t *count_dev, cudaStream_t st)
+{
+    const unsigned sms = (unsigned)sm_count();
+    tri_scatter_kernel<<<sms * 8, 256, 0, st>>>(nnz, t->edge, t->place, t->hub_pos, t->rest_pos, hdr, t->counters, t->hub, a32, m32,
+                                                columns);
+    CB_LAUNCH_CHECK();
+    tri_bitmap_kernel<<<sms * 6, TRI_WARPS * 32, 0, st>>>(nrows, t->hub_pos, t->hub, hdr, t->counters, t->room, t->bits_at, t->bits);
+    CB_LAUNCH_CHECK();
+    tri_count_kernel<<<sms * 5, TRI_WARPS * 32, 0, st>>>(nrows, t->hub_pos, t->hub, t->rest_pos, a32, t->bits_at, t->bits, hdr,
+                                                         t->counters, (unsigned long long *)count_dev);
+    CB_LAUNCH_CHECK();
+    return 0;
+}
+
 int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz_a, int64_t nnz_b,
                       int64_t nnz_m, const int64_t *apos, const int64_t *acrd, const int64_t *bpos,
                       const int64_t *bcrd, const int64_t *mpos, const int64_t *mcrd,
@@ -116,7 +201,6 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     // two agree for the square operands this is called with (pairs beyond it stay on the mask side)
     const int64_t bcap = ncols > row_hi ? ncols : row_hi;
     const bool compact = ncols > TC_MAX_COLS;
-    const TcShape sh = {bcap, acrd == mcrd && apos == mpos, false, false};
     const int64_t words = ceil_div(ncols, 32);
     auto grid_for = [](int64_t n) {
         const int64_t blocks = ceil_div(n, 256), cap = (int64_t)sm_count() * 16;
@@ -124,6 +208,12 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     };
     const bool same_bm = bcrd == mcrd && nnz_b == nnz_m, same_am = acrd == mcrd && nnz_a == nnz_m;
     const bool same_ab = acrd == bcrd && nnz_a == nnz_b;
+    // one matrix in all three places: its triangles, if it is triangular, in another order of the vertices
+    bool order = same_am && same_bm && apos == mpos && bpos == mpos && row_lo == 0 && row_hi == ncols &&
+                       nnz_a >= TRI_MIN_ENTRIES && nnz_a / TRI_MIN_PER_ROW >= ncols && nnz_a < 0x7fffffffLL;
+    void *tri_mem = nullptr;
+    if (order) order = scratch_if_room(SLOT_TRIANGLES, tri_bytes(row_hi, nnz_a), &tri_mem);       // else in the order it has
+    const TcShape sh = {bcap, acrd == mcrd && apos == mpos, false, false, order};
 
     // scratch: header, rows of A, list places, B side lists and their pointers, unit list
     const size_t nunits = (size_t)(nnz_a / 16 + (nnz_m < nrows * TC_WARP_MAX ? nnz_m / TC_WARP_MAX : nrows) +
@@ -150,8 +240,11 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     TcUnit *units = (TcUnit *)((char *)bins + pad((size_t)nrows * 4)), *mids = units + nunits;
     CB_CUDA(cudaMemsetAsync(hdr, 0, counts_bytes, st));           // header, list counts, column bits
 
+    TriArrays tri;
+    if (order) CB_TRY(tri_prepare(row_hi, nnz_a, apos, acrd, hdr, tri_mem, blist, slot, &tri, st));
+
     if (compact) {
-        tc_present_kernel<<<(unsigned)sm_count() * 4, 512, 0, st>>>(nnz_m, mcrd, present);
+        tc_present_kernel<<<(unsigned)sm_count() * 4, 512, 0, st>>>(nnz_m, mcrd, present, order ? hdr : nullptr);
         CB_LAUNCH_CHECK();
         tc_popc_kernel<<<grid_for(words), 256, 0, st>>>(words, present, popc);
         CB_LAUNCH_CHECK();
@@ -159,7 +252,7 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     }
     auto narrow = [&](const int64_t *crd, int64_t n, void *out, bool columns, bool check) {
         tc_narrow_kernel<<<grid_for(ceil_div(n, 2)), 256, 0, st>>>(n, crd, (int32_t *)out, columns ? present : nullptr, before,
-                                                                  words, mpos, row_lo, row_hi, check ? hdr : nullptr);
+                                                                  words, mpos, row_lo, row_hi, check ? hdr : nullptr, order ? hdr : nullptr);
         return cudaGetLastError() == cudaSuccess ? 0 : fail("masked count: narrowing failed");
     };
     CB_TRY(scratch(SLOT_NARROW_M, (size_t)nnz_m * 4 + 16, &m32));
@@ -169,13 +262,17 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
         CB_TRY(scratch(SLOT_NARROW_B, (size_t)nnz_b * 4 + 16, &b32));
         CB_TRY(narrow(bcrd, nnz_b, b32, true, false));
     }
-    if (same_am && !compact) a32 = m32;
-    else if (same_ab && !compact) a32 = b32;
+    if (same_am && !compact && !order) a32 = m32;
+    else if (same_ab && !compact && !order) a32 = b32;
     else {
         CB_TRY(scratch(SLOT_NARROW_A, (size_t)nnz_a * 4 + 16, &a32));
         CB_TRY(narrow(acrd, nnz_a, a32, false, false));
     }
     const int32_t *A = (const int32_t *)a32, *B = (const int32_t *)b32, *M = (const int32_t *)m32;
+    if (order) {
+        CB_TRY(tri_count(row_hi, nnz_a, hdr, &tri, (int32_t *)a32, (int32_t *)m32, compact ? before + words : nullptr, count_dev, st));
+        apos = bpos = mpos = tri.rest_pos;
+    }
     tc_rows_kernel<<<grid_for(nrows * 16), 256, 0, st>>>(row_lo, row_hi, apos, mpos, mcrd, arow, hdr);
     CB_LAUNCH_CHECK();
     tc_route_kernel<<<grid_for(nnz_a), 256, 0, st>>>(row_lo, row_hi, apos, A, arow, bpos, mpos, sh, hdr, slot, bcount);
