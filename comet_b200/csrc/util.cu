@@ -192,60 +192,42 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply(const InT *__restrict
     }
 }
 
-// One CTA for short arrays, 8192 elements a step: the loads of eight rows of 1024 are coalesced and in flight together, the
-// 256 sums of their warps are scanned by one warp (16384 elements: 14 us; three kernels 11 us and two more launch gaps).
-static const int64_t SCAN_ONE_CTA = 32768;
+// Short arrays in one launch: a CTA per 2048 elements, which adds up all elements before its own itself (the last of 16 CTAs reads
+// 32 a thread, eight in flight) instead of waiting for the CTAs before it.  Its warps then need one barrier.  16,384 elements 5 us, 32,768 6
+// (one CTA with 8192 a step 14 and 26, three kernels 11 and two more launch gaps).
+static const int64_t SCAN_FEW_CTAS = 32768;
+static const int SCAN_FEW_TILE = 2048;
 
 template <typename InT>
-__global__ void __launch_bounds__(1024) scan_one_cta(const InT *__restrict__ in, int64_t *__restrict__ out, int64_t n)
+__global__ void __launch_bounds__(1024) scan_few_ctas(const InT *__restrict__ in, int64_t *__restrict__ out, int64_t n)
 {
-    __shared__ int64_t sums[8 * 32];
-    __shared__ int64_t total;
+    __shared__ int64_t s_before[32], s_own[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t carry = 0;
-    for (int64_t base = 0; base < n; base += 8192) {
-        int64_t v[8], incl[8];
+    const int64_t first = (int64_t)blockIdx.x * SCAN_FEW_TILE, at = first + 2 * threadIdx.x;
+    const int64_t v0 = at < n ? (int64_t)in[at] : 0, v1 = at + 1 < n ? (int64_t)in[at + 1] : 0;
+    int64_t before = 0;
+#pragma unroll 8
+    for (int64_t i = threadIdx.x; i < first; i += 1024) before += (int64_t)in[i];
+    int64_t incl = v0 + v1;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int64_t at = base + i * 1024 + threadIdx.x;
-            v[i] = at < n ? (int64_t)in[at] : 0;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            incl[i] = v[i];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t t = __shfl_up_sync(0xffffffffu, (long long)incl[i], o);
-                if (lane >= o) incl[i] += t;
-            }
-            if (lane == 31) sums[i * 32 + warp] = incl[i];
-        }
-        __syncthreads();
-        if (warp == 0) {
-            int64_t w[8], s = 0;
-#pragma unroll
-            for (int i = 0; i < 8; i++) { w[i] = sums[lane * 8 + i]; s += w[i]; }
-            int64_t before = s;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t t = __shfl_up_sync(0xffffffffu, (long long)before, o);
-                if (lane >= o) before += t;
-            }
-            if (lane == 31) total = before;
-            before -= s;
-#pragma unroll
-            for (int i = 0; i < 8; i++) { sums[lane * 8 + i] = before; before += w[i]; }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int64_t at = base + i * 1024 + threadIdx.x;
-            if (at < n) out[at] = carry + sums[i * 32 + warp] + incl[i] - v[i];
-        }
-        carry += total;
-        __syncthreads();
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t t = __shfl_up_sync(0xffffffffu, (long long)incl, o);
+        if (lane >= o) incl += t;
+        before += __shfl_xor_sync(0xffffffffu, (long long)before, o);
     }
-    if (threadIdx.x == 0) out[n] = carry;
+    if (lane == 31) {
+        s_before[warp] = before;
+        s_own[warp] = incl;
+    }
+    __syncthreads();
+    // what lies before this warp: everything before the tile, and the tile's warps before it
+    int64_t base = s_before[lane] + (lane < warp ? s_own[lane] : 0);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) base += __shfl_xor_sync(0xffffffffu, (long long)base, o);
+    const int64_t mine = base + incl - v0 - v1;
+    if (at < n) out[at] = mine;
+    if (at + 1 < n) out[at + 1] = mine + v0;
+    if (at < n && at + 2 >= n) out[n] = mine + v0 + v1;
 }
 
 template <typename InT>
@@ -255,8 +237,8 @@ static int exclusive_scan(const InT *in, int64_t *out, int64_t n, cudaStream_t s
         CB_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), st));
         return 0;
     }
-    if (n <= SCAN_ONE_CTA) {
-        scan_one_cta<<<1, 1024, 0, st>>>(in, out, n);
+    if (n <= SCAN_FEW_CTAS) {
+        scan_few_ctas<<<(unsigned)ceil_div(n, SCAN_FEW_TILE), 1024, 0, st>>>(in, out, n);
         CB_LAUNCH_CHECK();
         return 0;
     }
