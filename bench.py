@@ -531,7 +531,7 @@ def _tail_sample(weights, fraction):
 
 class SpGEMM(Workload):
     name = "spgemm"
-    launches_per_step = 14    # bin, 2 publish, hash+mid+bitmap symbolic, 3 scan kernels, short+mid+bitmap numeric, 2 team kernels
+    launches_per_step = 19    # bin, 2 publish, hash+mid+hub symbolic, 5 for the hubs, 3 scan kernels, short+mid+bitmap numeric, 2 team kernels
 
     def build(self):
         from comet_b200 import datasets, sharding
@@ -661,7 +661,7 @@ class SpGEMM(Workload):
 
 class Triangles(Workload):
     name = "triangles"
-    launches_per_step = 17    # columns present (2), 2 scans of 3, 2 narrowings, rows, routing, scatter, units, three counting kernels
+    launches_per_step = 32    # renumbering (6), hub columns (3), columns present (2), 4 scans of 3, 2 narrowings, rows, routing, scatter, units, three counting kernels
 
     def build(self):
         from comet_b200 import datasets, sharding

@@ -43,7 +43,7 @@ def _operands(ncols, step, repeats):
 
 
 @pytest.mark.parametrize("semiring", [api.PLUS_TIMES, api.MIN_PLUS])
-@pytest.mark.parametrize("ncols,step", [(200001, 1), (262144, 3), (819232, 1), (900000, 2), (300000, 60000)])
+@pytest.mark.parametrize("ncols,step", [(200001, 1), (262144, 3), (819200, 1), (819232, 1), (900000, 2), (300000, 60000)])
 def test_long_rows_of_b(ncols, step, semiring, monkeypatch):
     if semiring == api.MIN_PLUS:
         monkeypatch.setenv("COMET_B200_SPGEMM_BITMAP_GB", "0")
