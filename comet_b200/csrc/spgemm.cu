@@ -4,8 +4,8 @@
 // Rows are binned by an upper bound on their number of distinct columns
 // (sum of the lengths of the B rows they touch, capped by the mask row):
 //   bin 0  no products                     -> empty row
-//   bin 1  bound <= HASH_ROW_MAX           -> one warp per row.  The symbolic call counts distinct columns with a hash table
-//          in shared memory; the numeric call sorts column and place of the products in registers and adds equal
+//   bin 1  bound <= HASH_ROW_MAX           -> one warp per row.  The symbolic call counts distinct columns with a bitmap (few
+//          columns) or a hash table in shared memory; the numeric call sorts column and place of the products in registers and adds equal
 //          neighbours (with a mask: the hash table again, its keys sorted in registers)
 //   bin 3  bound <= MID_ROW_MAX, no mask, not too many columns -> 128 or 256 threads per row, a bitmap over the columns of B and
 //          sums by rank in shared memory
@@ -15,6 +15,7 @@
 //          column's rank, so crd comes out sorted with no sort and val[rank] is
 //          accumulated in place with f64 atomics on the output row, which the
 //          CTA has just zeroed and which therefore sits in L2.
+//          From HUB_WORK bytes of bitmaps on, without a mask, B's long rows are prepared first (hubs.cuh).
 // This mirrors COMET's workspace transformation (dense row workspace + mark
 // array, sort of the touched columns) with a bit per column instead of a mark
 // word per column, and replaces std::sort by ranking.
@@ -806,7 +807,9 @@ static const int LONG_LIST = 1024;          // long rows of B remembered per pas
 // ms): 1 19.3 / 4.6, 2 18.1 / 4.0, 4 17.4 / 3.8.  More of them with fewer warps is slower (2 CTAs, 6 steps 20.1), and so are more
 // warps with fewer steps (4 CTAs, 2 steps 20.1).
 static const int WALK_DEPTH = 4;
-static const int WALK_DEPTH_FOLD = 2;       // where the fold is a loop: R-MAT scale 17, 5 per row, min-plus 2.4 ms, with 4 steps 2.6
+// Where the fold is a loop, steps side by side only meet in it (min-plus, numeric kernel in ms, 1 / 2 / 4: R-MAT scale 14, 16 per row
+// 0.85 / 0.93 / 0.94; scale 17, 5 per row 2.4 / 2.4 / 2.6).
+static const int WALK_DEPTH_FOLD = 1;
 
 // Calls f(j, bv, av) for every product of row r of A with B in this CTA's share: j and bv are the column and
 // value of an entry of row acrd[p] of B (bv = 0 when bval is null), av = aval[p] (0 when aval is null).  A team
