@@ -636,6 +636,7 @@ few_columns_kernel(const unsigned *__restrict__ nlist_dev, const int32_t *__rest
         }
         fresh = __reduce_add_sync(0xffffffffu, fresh);
         if (lane == 0) cnt[r] = fresh;
+        __syncwarp();                                  // the other lanes' columns and marks: a reduction orders no memory
         for (int x = lane; x < n; x += 32) bits[cols[x] >> 5] = 0;
         __syncwarp();
     }

@@ -1,0 +1,47 @@
+"""Kernels in which the lanes of a warp hand each other values through shared memory, with their own text compiled by g++ against
+tests/cpu_checks/fake_warp.hpp and run under ThreadSanitizer: results are compared, and an access that no barrier orders is a failure."""
+import os
+import re
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CHECKS = os.path.join(ROOT, "tests", "cpu_checks")
+CSRC = os.path.join(ROOT, "comet_b200", "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return f.read()
+
+
+def function(name, text):
+    """The definition of a function, from its first line (a template's or its qualifiers') to its closing brace."""
+    at = re.search(r"^[^\n;{}/]*\b%s\(" % name, text, re.M).start()
+    start = max(text.rfind("\n\n", 0, at), text.rfind("\n}\n", 0, at) + 1)
+    end = text.index("\n}\n", at) + 3
+    return re.sub(r"extern __shared__", "extern", text[start:end]) + "\n"
+
+
+def constant(name, text):
+    return re.search(r"^static const [a-z0-9_]+ %s = .*?;" % name, text, re.M).group(0) + "\n"
+
+
+def run(tmp_path, check, code, *args):
+    with open(str(tmp_path / "kernels.inc"), "w") as f:
+        f.write(code)
+    exe = str(tmp_path / "check")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-g", "-fsanitize=thread", "-pthread", "-Wno-unknown-pragmas", "-I" + str(tmp_path),
+                           "-I" + CHECKS, "-I" + os.path.join(ROOT, "include"), os.path.join(CHECKS, check), "-o", exe])
+    out = subprocess.run([exe] + list(args), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=600)
+    assert "data race" not in out.stdout, out.stdout[:3000]
+    assert out.returncode == 0 and out.stdout == "ok\n", out.stdout[:3000]
+
+
+def test_short_rows_of_few_columns(tmp_path):
+    text = source("spgemm.cu")
+    kernel = function("few_columns_kernel", text)
+    # several lanes may store the same 0 to a word, which is a race in C++ and none on the device; what they read has to be ordered
+    clear = "bits[cols[x] >> 5] = 0;"
+    assert kernel.count(clear) == 1
+    kernel = kernel.replace(clear, "__atomic_store_n(&bits[cols[x] >> 5], 0u, __ATOMIC_RELAXED);")
+    run(tmp_path, "few_columns_check.cpp", constant("HASH_ROW_MAX", text) + constant("HASH_WARPS", text) + kernel)
