@@ -137,10 +137,12 @@ __device__ __forceinline__ unsigned tc_fill(int32_t *tab, const int32_t *__restr
         if (repeats && t > ms && crd[t - 1] >= key) ok = false;
         ok = tc_cuckoo_insert<LOG2>(tab, key) && ok;
     }
+    __syncwarp();                          // the other lanes' columns: a vote orders no memory
     if (__all_sync(0xffffffffu, ok)) return TC_CUCKOO;
     clear();
     bool twice = false;
     for (int64_t t = ms + lane; t < me; t += 32) twice |= tc_linear_insert<LOG2>(tab, crd[t]);
+    __syncwarp();
     return __any_sync(0xffffffffu, twice) && repeats ? TC_REPEATS : TC_LINEAR;
 }
 

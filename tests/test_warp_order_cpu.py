@@ -4,6 +4,8 @@ import os
 import re
 import subprocess
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CHECKS = os.path.join(ROOT, "tests", "cpu_checks")
 CSRC = os.path.join(ROOT, "comet_b200", "csrc")
@@ -26,6 +28,13 @@ def constant(name, text):
     return re.search(r"^static const [a-z0-9_]+ %s = .*?;" % name, text, re.M).group(0) + "\n"
 
 
+def body(name, until=None):
+    """A header without its includes, up to a line."""
+    text = source(name)
+    text = text[:text.index(until)] + "}\n" if until else text
+    return re.sub(r"^#(include|pragma).*$", "", text, flags=re.M).replace("extern __shared__", "extern").replace("static __global__", "__global__")
+
+
 def run(tmp_path, check, code, *args):
     with open(str(tmp_path / "kernels.inc"), "w") as f:
         f.write(code)
@@ -45,3 +54,10 @@ def test_short_rows_of_few_columns(tmp_path):
     assert kernel.count(clear) == 1
     kernel = kernel.replace(clear, "__atomic_store_n(&bits[cols[x] >> 5], 0u, __ATOMIC_RELAXED);")
     run(tmp_path, "few_columns_check.cpp", constant("HASH_ROW_MAX", text) + constant("HASH_WARPS", text) + kernel)
+
+
+@pytest.mark.parametrize("kernel", ["warp", "mid"])
+@pytest.mark.parametrize("out", ["all", "pairs", "values"])
+def test_sets_of_a_warp(tmp_path, kernel, out):
+    run(tmp_path, "warp_sets_check.cpp", body("semiring.cuh") + body("pairs.cuh", "template <int THREADS, bool SEGMENTED, class Out>\nstatic int"),
+        kernel, out)
