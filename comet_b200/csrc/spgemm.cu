@@ -256,7 +256,7 @@ __global__ void publish_kernel(const unsigned *__restrict__ bin_counts, const in
     host[0] = bin_counts[0];
     host[1] = bin_counts[1];
     host[2] = bin_counts[2];
-    if (nnz) *(int64_t *)(host + 4) = *nnz;
+    *(int64_t *)(host + 4) = *nnz;
 }
 
 // --------------------------------------------------------------------------
@@ -1360,7 +1360,7 @@ static int launch_mid(const Plan *p, unsigned grid, int64_t *ccrd, double *cval,
 
 // Prepares B's long rows (p->hubs stays null where the columns that B stores are too many, or B has no long rows and hardly a column
 // without entries).  Synchronises.
-static int hub_prepare(Plan *p, int64_t nrows, cudaStream_t st)
+static int hub_prepare(Plan *p, int64_t nrows, int64_t nnz_a, cudaStream_t st)
 {
     Hubs *hb = new Hubs();
     memset(hb, 0, sizeof(Hubs));
@@ -1385,7 +1385,9 @@ static int hub_prepare(Plan *p, int64_t nrows, cudaStream_t st)
     hb->colmap = (int32_t *)(m + 256 + 2 * b_bits);
     hb->crd = (int32_t *)(m + 256 + 2 * b_bits + b_map);
     CB_CUDA(cudaMemsetAsync(m, 0, 256 + b_bits, st));
-    const int64_t least = ceil_div(p->nnz_b, 4096), most = (int64_t)sm_count() * 2;
+    // the kernel walks A as well as B: a tall A times a small B has its work there (100,000 rows of 300 times 600 of 6, both calls
+    // 15.6 ms with the one CTA that B alone would get)
+    const int64_t least = ceil_div(nnz_a > p->nnz_b ? nnz_a : p->nnz_b, 4096), most = (int64_t)sm_count() * 2;
     const unsigned grid = (unsigned)(least < most ? least : most);
     if (words * 4 <= 96 * 1024) {
         CB_CUDA(cudaFuncSetAttribute(hub_present_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(words * 4)));
@@ -1514,10 +1516,11 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     p->n1 = p->n2 = (unsigned)nrows;
     p->n3 = mid ? (unsigned)nrows : 0;
     bool counted = false;
+    int64_t nnz_a = 0;
     if ((size_t)nrows * p->words * 4 > BM_STORE_SMALL) {
-        STEP_CUDA(launch_behind(publish_kernel, dim3(1), 1, 0, st, p->bin_counts, nullptr, counts));
+        STEP_CUDA(launch_behind(publish_kernel, dim3(1), 1, 0, st, p->bin_counts, apos + nrows, counts));
         STEP_CUDA(cudaStreamSynchronize(st));
-        if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; p->n3 = counts[2]; counted = true; }
+        if (!rc) { p->n1 = counts[0]; p->n2 = counts[1]; p->n3 = counts[2]; nnz_a = *(int64_t *)(counts + 4); counted = true; }
     }
     if (!rc && p->n1) {
         unsigned grid = (unsigned)ceil_div(p->n1, HASH_WARPS);
@@ -1532,7 +1535,7 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     }
     if (!rc && p->n3) STEP(launch_mid<false>(p, cnt_grid(p->n3), nullptr, nullptr, st));
     if (counted && !mpos && p->n2 && (size_t)p->n2 * p->words * 4 >= HUB_WORK && ncols_b <= HUB_MAX_COLS && nnz_b < 0x7fffffffLL)
-        STEP(hub_prepare(p, nrows, st));
+        STEP(hub_prepare(p, nrows, nnz_a, st));
     if (!rc && p->n2) {
         size_t store = (size_t)p->n2 * (p->hubs ? p->hubs->stride : p->words) * sizeof(uint32_t);
         // the symbolic pass's bitmaps are kept for the numeric pass while they fit the budget

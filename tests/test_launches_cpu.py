@@ -1,0 +1,38 @@
+"""What the host side allocates and launches, with the library's own objects linked to a stand-in for the CUDA runtime
+(tests/cpu_checks/fake_launch.hpp)."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CHECKS = os.path.join(ROOT, "tests", "cpu_checks")
+
+
+def link(tmp_path_factory, check, *objects):
+    from comet_b200 import build
+    build.build_library()
+    exe = str(tmp_path_factory.mktemp("checks") / check[:-4])
+    # functions of the files that are not linked are not called
+    subprocess.check_call(["g++", "-O1", "-g", "-std=c++17", "-I/usr/local/cuda/include", os.path.join(CHECKS, check)] +
+                          [os.path.join(build.OBJ, o) for o in objects] +
+                          ["-no-pie", "-Wl,--unresolved-symbols=ignore-in-object-files", "-o", exe])
+    return exe
+
+
+def output(*command):
+    out = subprocess.run([str(c) for c in command], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=120)
+    assert out.returncode == 0, out.stdout
+    return out.stdout.strip()
+
+
+@pytest.fixture(scope="module")
+def hub_grid(tmp_path_factory):
+    return link(tmp_path_factory, "hub_grid_check.cpp", "spgemm.o")
+
+
+# two blocks an SM at most; below, one for every 4096 entries of the longer operand
+@pytest.mark.parametrize("nrows,nnz_a,nnz_b,ncols,blocks", [(20000, 6000000, 2400, 200000, 296), (100000, 30000000, 3600, 150000, 296),
+                                                            (20000, 400000, 2400, 200000, 98), (20000, 40000, 4000000, 200000, 296)])
+def test_a_tall_operand_is_looked_over_by_the_whole_chip(hub_grid, nrows, nnz_a, nnz_b, ncols, blocks):
+    assert int(output(hub_grid, nrows, nnz_a, nnz_b, ncols)) == blocks
