@@ -808,8 +808,10 @@ static const int LONG_LIST = 1024;          // long rows of B remembered per pas
 // ms): 1 19.3 / 4.6, 2 18.1 / 4.0, 4 17.4 / 3.8.  More of them with fewer warps is slower (2 CTAs, 6 steps 20.1), and so are more
 // warps with fewer steps (4 CTAs, 2 steps 20.1).
 static const int WALK_DEPTH = 4;
-// Where the fold is a loop, steps side by side only meet in it (min-plus, numeric kernel in ms, 1 / 2 / 4: R-MAT scale 14, 16 per row
-// 0.85 / 0.93 / 0.94; scale 17, 5 per row 2.4 / 2.4 / 2.6).
+// Where the fold is a loop, and where the bitmaps are in memory, steps side by side only meet in it: one is folded with the next one's
+// loads ahead.  Numeric kernel in ms with 1 (nothing ahead) / 2 / 4: min-plus, R-MAT scale 14, 16 per row 0.85 / 0.93 / 0.94; scale 17, 5 per
+// row 2.4 / 2.4 / 2.6.  Both calls in us with nothing and with the next step ahead: min-plus, scale 13, 16 per row 566, 526; plus-times, 40 rows
+// of 24,000 products in 8,000,000 columns 930, 852.
 static const int WALK_DEPTH_FOLD = 1;
 
 // Calls f(j, bv, av) for every product of row r of A with B in this CTA's share: j and bv are the column and
@@ -864,31 +866,46 @@ __device__ __forceinline__ void for_each_product(int64_t r, unsigned part, unsig
         int64_t at = 0;
         int rem = 0;
         double av = 0.0;
-        while (left || rem > 0) {
-            int32_t j[DEPTH];
-            double v[DEPTH], am[DEPTH];
-#pragma unroll
-            for (int i = 0; i < DEPTH; i++) {
-                if (rem <= 0 && left) {
-                    const int t = __ffs(left) - 1;
-                    left &= left - 1;
-                    at = __shfl_sync(0xffffffffu, (long long)s_l, t) + lane;
-                    rem = __shfl_sync(0xffffffffu, n_l, t);
-                    av = shfl_f64(av_l, t, 32);
-                }
-                am[i] = av;
-                j[i] = -1;
-                v[i] = 0.0;
-                if (lane < rem) {
-                    j[i] = bcrd[at];
-                    if (bval) v[i] = bval[at];
-                }
-                at += 32;
-                rem -= 32;
+        auto step = [&](int32_t &j, double &v, double &a) {
+            if (rem <= 0 && left) {
+                const int t = __ffs(left) - 1;
+                left &= left - 1;
+                at = __shfl_sync(0xffffffffu, (long long)s_l, t) + lane;
+                rem = __shfl_sync(0xffffffffu, n_l, t);
+                av = shfl_f64(av_l, t, 32);
             }
+            a = av;
+            j = -1;
+            v = 0.0;
+            if (lane < rem) {
+                j = bcrd[at];
+                if (bval) v = bval[at];
+            }
+            at += 32;
+            rem -= 32;
+        };
+        if (DEPTH == 1) {
+            int32_t j = -1;
+            double v = 0.0, a = 0.0;
+            if (left) step(j, v, a);
+            for (bool more = true; more;) {
+                more = left || rem > 0;
+                int32_t j1 = -1;
+                double v1 = 0.0, a1 = 0.0;
+                if (more) step(j1, v1, a1);
+                if (j >= 0) f(j, v, a);
+                j = j1; v = v1; a = a1;
+            }
+        } else {
+            while (left || rem > 0) {
+                int32_t j[DEPTH];
+                double v[DEPTH], am[DEPTH];
 #pragma unroll
-            for (int i = 0; i < DEPTH; i++)
-                if (j[i] >= 0) f(j[i], v[i], am[i]);
+                for (int i = 0; i < DEPTH; i++) step(j[i], v[i], am[i]);
+#pragma unroll
+                for (int i = 0; i < DEPTH; i++)
+                    if (j[i] >= 0) f(j[i], v[i], am[i]);
+            }
         }
     }
     __syncthreads();
