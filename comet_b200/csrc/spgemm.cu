@@ -1274,7 +1274,10 @@ __device__ __forceinline__ void hub_mark_row(uint32_t *bm, int stride, int64_t r
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(BM_THREADS)
+// Four CTAs on an SM: rows of a few thousand products wait for barriers and for loads, so that registers for a fourth CTA are worth more than
+// the 24 bytes they put on the stack.  Both calls with three (39 registers) and four (32): 200,000 rows of 2000 products in 100,000
+// columns 8.13 and 7.64 ms (7.89 before there were hubs), R-MAT scale 18 squared 23.3 and 22.3.
+__global__ void __launch_bounds__(BM_THREADS, 4)
 hub_symbolic_kernel(unsigned nlist, const int32_t *__restrict__ list, Hubs hb, const int64_t *__restrict__ apos,
                     const int64_t *__restrict__ acrd, const int64_t *__restrict__ bpos, int64_t *__restrict__ cnt,
                     uint32_t *__restrict__ bm_store)
