@@ -803,6 +803,10 @@ __device__ __forceinline__ unsigned block_sum_u32(unsigned v, unsigned *s_warp)
 static const int64_t LONG_B_ROW = 1024;
 
 static const unsigned BM_DENSE_ROW = 512;   // bits in 32 consecutive bitmap words from which crd is written word by word (measured: 96 / 192 / 320 / 512 / 768 / never = 22.9 / 21.8 / 21.5 / 21.45 / 21.65 / 21.7 ms numeric at config 4)
+// Columns that need a look-up: the least that a warp's stage is worth having for.  Rows of 32 words with more than it holds go out like those
+// of BM_DENSE_ROW, one word at a time (one by one with a look-up each 2000 rows of 100,000 products in 350,000 columns took 3.08 ms; 2.42
+// so, and 2.53 before columns were renumbered).
+static const unsigned STAGE_MIN = 128;
 static const int LONG_LIST = 1024;          // long rows of B remembered per pass over a row of A
 // Steps of 32 products whose loads are in flight, with 3 CTAs of 512 threads on an SM (R-MAT scale 18 squared, numeric / symbolic kernel in
 // ms): 1 19.3 / 4.6, 2 18.1 / 4.0, 4 17.4 / 3.8.  More of them with fewer warps is slower (2 CTAs, 6 steps 20.1), and so are more
@@ -1171,7 +1175,7 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
             const bool ours = team == 1 || (unsigned)i % team == part;
             if (MAPPED && held && (!ours || held + rowtotal > stage_n)) flush(before);
             if (!ours) continue;
-            if (rowtotal >= BM_DENSE_ROW) {
+            if (rowtotal >= BM_DENSE_ROW || (MAPPED && rowtotal > stage_n)) {
                 if (MAPPED && held) flush(before);
                 // many bits per word: one word at a time, lane b writes column 32 w + b at its rank, so a
                 // store instruction covers consecutive addresses
@@ -1188,11 +1192,11 @@ bitmap_numeric_kernel(unsigned nlist, const int32_t *__restrict__ list, int word
                         __stcs(out + wp + __popc(wv & below), (long long)(MAPPED ? __ldg(colmap + j) : j));
                     }
                 }
-            } else if (!MAPPED || rowtotal > stage_n) {
+            } else if (!MAPPED) {
                 unsigned at = excl;
                 for (; v; v &= v - 1, at++) {
                     const int j = w * 32 + __ffs(v) - 1;
-                    __stcs((long long *)ccrd + base + at, (long long)(MAPPED ? __ldg(colmap + j) : j));
+                    __stcs((long long *)ccrd + base + at, (long long)j);
                 }
             } else {
                 // the columns go through shared memory, so that the stores are coalesced and the look-ups independent (R-MAT scale
@@ -1668,17 +1672,18 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
             const int words = p->hubs ? p->hubs->words : p->words, stride = p->hubs ? p->hubs->stride : p->words;
             const int32_t *colmap = p->hubs ? p->hubs->colmap : nullptr, *bcrd32 = p->hubs ? p->hubs->crd : p->bcrd32;
             size_t smem = (size_t)words * sizeof(uint32_t) * 2;
-            const size_t stage = (size_t)BM_THREADS / 32 * BM_DENSE_ROW * 4;
             if (smem <= BM_SMEM_LIMIT) {
-
                 // full occupancy grid even for few rows: teams give every CTA work
                 // three CTAs are what the registers leave room for; coordinates are staged in the shared memory that is left
                 // (200,000 rows of up to 60: 4.2 ms with three and what is left, 5.2 with a full stage and two).  Columns that need no
-                // look-up are written as they are found (3.3 against 3.5).
+                // look-up are written as they are found (3.3 against 3.5).  A stage of a few columns is worth less than a CTA: 2000 rows of
+                // 100,000 products in 450,000 columns 2.39 ms with three CTAs and 43 columns, 2.27 with two and 512.
                 const size_t sm = (size_t)228 * 1024, own = 6 * 1024;
                 size_t per_sm = sm / (smem + own);
                 per_sm = per_sm < 1 ? 1 : per_sm > 3 ? 3 : per_sm;
-                size_t stage_n = colmap ? (sm / per_sm - own - smem) / (BM_THREADS / 32 * 4) : 0;
+                auto stage_of = [&](size_t ctas) { return (sm / ctas - own - smem) / (BM_THREADS / 32 * 4); };
+                while (colmap && per_sm > 1 && stage_of(per_sm) < STAGE_MIN) per_sm--;
+                size_t stage_n = colmap ? stage_of(per_sm) : 0;
                 if (stage_n > BM_DENSE_ROW) stage_n = BM_DENSE_ROW;
                 smem += stage_n * (BM_THREADS / 32 * 4);
                 const int grid = sm_count() * (int)per_sm;

@@ -1,0 +1,55 @@
+// A product of rows that all go to the bitmaps over B's columns: what is launched to look A and B over, and for the numeric call.
+// Arguments: rows of A, entries of A, entries of B, columns, columns that B stores.  Prints the blocks of the kernel that looks them over
+// (0: not launched), the blocks an SM of the numeric kernel, and the columns of a warp's stage.
+#include "fake_launch.hpp"
+
+#include "../../comet_b200/csrc/hostcopy.cuh"
+#include "../../comet_b200/csrc/masked.cuh"
+
+namespace cb200 {
+PinnedWords::PinnedWords() { p = calloc(64, 1); }
+PinnedWords::~PinnedWords() { free(p); }
+int scratch(Slot, size_t bytes, void **ptr) { *ptr = malloc(bytes); return 0; }
+int exclusive_scan_i64(const int64_t *, int64_t *, int64_t, cudaStream_t) { return 0; }
+void masked_free(MaskedPlan *, cudaStream_t) {}
+}  // namespace cb200
+
+struct HubPrep { unsigned ncols, pad; long long nrows_b, longest; };       // as hubs.cuh has it
+
+int main(int argc, char **argv)
+{
+    const int64_t nrows = atoll(argv[1]), nnz_a = atoll(argv[2]), nnz_b = atoll(argv[3]), ncols = atoll(argv[4]), stored = atoll(argv[5]);
+    std::vector<int64_t> apos((size_t)nrows + 1, 0), bcrd((size_t)nnz_b + 2, 0), cpos((size_t)nrows + 1, 0);
+    apos[(size_t)nrows] = nnz_a;
+    cpos[(size_t)nrows] = nrows * 10000;
+    unsigned stage = 0;
+    fake::on_launch = [&](const std::string &name, void **args) {
+        if (name.find("publish_kernel") != std::string::npos) {
+            unsigned *host = *(unsigned **)args[2];
+            host[1] = (unsigned)nrows;
+            const int64_t *n = *(const int64_t **)args[1];
+            if (n) *(int64_t *)(host + 4) = *n;
+        } else if (name.find("hub_before_kernel") != std::string::npos) {
+            HubPrep *prep = *(HubPrep **)args[3];
+            prep->ncols = (unsigned)stored;
+            prep->nrows_b = 1000;
+            prep->longest = 10;
+        } else if (name.find("bitmap_numeric_kernel") != std::string::npos) {
+            stage = *(unsigned *)args[4];
+        }
+    };
+    int64_t nnz = 0, handle = 0;
+    if (comet_b200_dev_spgemm_symbolic_f64_i64(nrows, ncols, nnz_b, apos.data(), nullptr, nullptr, apos.data(), bcrd.data(), nullptr, nullptr,
+                                               nullptr, COMET_B200_PLUS_TIMES, cpos.data(), &nnz, &handle, nullptr) ||
+        comet_b200_dev_spgemm_numeric_f64_i64(handle, nullptr, nullptr, 0, nullptr)) {
+        printf("%s\n", cb200::g_err);
+        return 1;
+    }
+    unsigned looked = 0, numeric = 0;
+    for (auto &l : fake::launches) {
+        if (l.name.find("hub_present_kernel") != std::string::npos) looked = l.grid.x;
+        if (l.name.find("bitmap_numeric_kernel") != std::string::npos) numeric = l.grid.x / 148;
+    }
+    printf("%u %u %u\n", looked, numeric, stage);
+    return 0;
+}

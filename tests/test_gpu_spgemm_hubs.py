@@ -65,3 +65,25 @@ def test_long_rows_of_b(ncols, step, semiring, monkeypatch):
                 b = slice(B.indptr[k], B.indptr[k + 1])
                 np.minimum.at(out, B.indices[b], a + B.data[b])
             assert np.array_equal(val[pos[r]:pos[r + 1]], out[crd[pos[r]:pos[r + 1]]])
+
+
+@pytest.mark.parametrize("stored", [146000, 240000, 262000])
+def test_rows_with_more_columns_than_the_stage_holds(stored):
+    """Columns that need a look-up, rows of 32 words with from a few to all of their 1024 columns: staged, word by word, and both in turn."""
+    rng = np.random.default_rng(stored)
+    columns = np.sort(rng.choice(300000, stored, replace=False))
+    brows = [np.sort(rng.choice(columns, 600, replace=False)) for _ in range(400)]
+    brows[0] = columns                                                    # all of them are stored
+    brows += [columns[:7000], columns[3000:3400], columns[-2000:]]
+    B = _csr(brows, rng.uniform(0.5, 1, sum(map(len, brows))), (len(brows), 300000))
+    arows = [np.sort(rng.choice(np.arange(1, 403), n, replace=False)) for n in (40, 80, 110, 130, 160, 200, 300, 402) * 6]
+    arows += [np.array([0]), np.array([400, 401, 402])] + [np.sort(rng.choice(np.arange(1, 400), 2, replace=False)) for _ in range(1900)]
+    A = _csr(arows, rng.uniform(-1, 1, sum(map(len, arows))), (len(arows), len(brows)))
+    C = dev.spgemm(_device(A), _device(B))
+    pos, crd, val = C.pos.cpu().numpy(), C.crd.cpu().numpy(), C.val.cpu().numpy()
+    want = sp.csr_matrix((np.ones(A.nnz), A.indices, A.indptr), A.shape) @ sp.csr_matrix((np.ones(B.nnz), B.indices, B.indptr), B.shape)
+    ref, mag = A @ B, abs(A) @ abs(B)
+    want.sort_indices(), ref.sort_indices(), mag.sort_indices()
+    assert np.array_equal(pos, want.indptr) and np.array_equal(crd, want.indices)
+    # a sum of n products in any order: n * 2^-53 of the sum of their magnitudes, n up to 402
+    assert np.all(np.abs(val - ref.data) <= 402 * 2.0 ** -53 * mag.data)

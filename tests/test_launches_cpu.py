@@ -27,12 +27,21 @@ def output(*command):
 
 
 @pytest.fixture(scope="module")
-def hub_grid(tmp_path_factory):
-    return link(tmp_path_factory, "hub_grid_check.cpp", "spgemm.o")
+def hub_launch(tmp_path_factory):
+    return link(tmp_path_factory, "hub_launch_check.cpp", "spgemm.o")
 
 
 # two blocks an SM at most; below, one for every 4096 entries of the longer operand
 @pytest.mark.parametrize("nrows,nnz_a,nnz_b,ncols,blocks", [(20000, 6000000, 2400, 200000, 296), (100000, 30000000, 3600, 150000, 296),
                                                             (20000, 400000, 2400, 200000, 98), (20000, 40000, 4000000, 200000, 296)])
-def test_a_tall_operand_is_looked_over_by_the_whole_chip(hub_grid, nrows, nnz_a, nnz_b, ncols, blocks):
-    assert int(output(hub_grid, nrows, nnz_a, nnz_b, ncols)) == blocks
+def test_a_tall_operand_is_looked_over_by_the_whole_chip(hub_launch, nrows, nnz_a, nnz_b, ncols, blocks):
+    assert int(output(hub_launch, nrows, nnz_a, nnz_b, ncols, 1000).split()[0]) == blocks
+
+
+@pytest.mark.parametrize("stored", [1, 100000, 219000, 221000, 254061, 270000, 286069, 300000, 400000, 819200])
+def test_columns_that_need_a_look_up_have_a_stage(hub_launch, stored):
+    """Shared memory holds the bitmap, its ranks and a stage of 128 columns a warp at least, whatever the number of CTAs."""
+    _, ctas, stage = map(int, output(hub_launch, 6000, 600000, 500000, 1000000, stored).split())
+    assert ctas >= 1 and 128 <= stage <= 512
+    dynamic = (stored + 31) // 32 * 8 + stage * 16 * 4
+    assert ctas * (dynamic + 4176 + 1024) <= 228 * 1024 and dynamic + 4176 <= 227 * 1024
