@@ -47,6 +47,10 @@ static const size_t BM_SMEM_LIMIT = 200 * 1024;
 static const size_t BM_STORE_BUDGET = (size_t)12 << 30;
 static const size_t BM_STORE_SMALL = (size_t)64 << 20;
 static const size_t HUB_WORK = (size_t)32 << 20;      // bytes of bitmaps of bin-2 rows from which on hubs.cuh takes them
+// and bytes of them per entry of B: looking B over takes some 10 us per million entries, in vain where it has no long rows and stores nearly all
+// of its columns. B of 8 M entries, bytes per entry and both calls without / with it: 9 560 / 700 us, 12 397 / 464, 25 714 / 789, 50 1959 / 2070.
+// Where it pays there are 83 (20,000 rows of 300 times 300 of 8) and more.
+static const size_t HUB_ENTRY = 64;
 
 struct Plan {
     int kind;                // 0 = spgemm, 1 = elementwise CSR .* CSR
@@ -1558,7 +1562,8 @@ int spgemm_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
                                 aval, bpos, p->bcrd32, bval, mpos, p->mcrd, p->semi, p->cnt, nullptr, nullptr, nullptr));
     }
     if (!rc && p->n3) STEP(launch_mid<false>(p, cnt_grid(p->n3), nullptr, nullptr, st));
-    if (counted && !mpos && p->n2 && (size_t)p->n2 * p->words * 4 >= HUB_WORK && ncols_b <= HUB_MAX_COLS && nnz_b < 0x7fffffffLL)
+    const size_t hub_bytes = counted && !mpos ? (size_t)p->n2 * p->words * 4 : 0;
+    if (hub_bytes >= HUB_WORK && hub_bytes / HUB_ENTRY >= (size_t)nnz_b && ncols_b <= HUB_MAX_COLS && nnz_b < 0x7fffffffLL)
         STEP(hub_prepare(p, nrows, nnz_a, st));
     if (!rc && p->n2) {
         size_t store = (size_t)p->n2 * (p->hubs ? p->hubs->stride : p->words) * sizeof(uint32_t);

@@ -33,7 +33,10 @@ def hub_launch(tmp_path_factory):
 
 # two blocks an SM at most; below, one for every 4096 entries of the longer operand
 @pytest.mark.parametrize("nrows,nnz_a,nnz_b,ncols,blocks", [(20000, 6000000, 2400, 200000, 296), (100000, 30000000, 3600, 150000, 296),
-                                                            (20000, 400000, 2400, 200000, 98), (20000, 40000, 4000000, 200000, 296)])
+                                                            (20000, 400000, 2400, 200000, 98), (20000, 40000, 4000000, 200000, 296),
+                                                            # few rows against a large B: 25 bytes of bitmaps per entry of B, 63 and 64
+                                                            (3200, 640000, 8000000, 500000, 0), (4032, 640000, 4000032, 500000, 0),
+                                                            (4032, 640000, 3937500, 500000, 296)])
 def test_a_tall_operand_is_looked_over_by_the_whole_chip(hub_launch, nrows, nnz_a, nnz_b, ncols, blocks):
     assert int(output(hub_launch, nrows, nnz_a, nnz_b, ncols, 1000).split()[0]) == blocks
 
