@@ -1016,6 +1016,10 @@ struct TeamHeader {
     unsigned pad;
 };
 static const unsigned TEAM_MAX = 64;
+// Shares of the L2 that one CTA's row may take: a team of two clears and scans the row twice, which is more than what it saves where the row is
+// a little above one share. Rows of 1.06 shares 4.95 ms in teams and 4.25 alone, 1.2 1.91 and 1.73, 1.33 2.06 and 1.94, 1.45 2.23 and
+// 2.29, 1.6 2.58 and 3.13 (6000 and 20,000 rows of 20,000 to 35,000 products in 300,000 columns, both calls).
+static const double TEAM_ALONE = 1.4;
 
 __device__ __forceinline__ uint64_t team_pack(unsigned it, unsigned part, unsigned t)
 {
@@ -1033,7 +1037,7 @@ team_items_kernel(unsigned nlist, const int32_t *__restrict__ list, const int64_
     if (it < nlist) {
         const int64_t r = list[it];
         const double want = (double)(cpos[r + 1] - cpos[r]) * ctas_per_budget_entry;
-        t = want <= 1.0 ? 1u : (want >= (double)TEAM_MAX ? TEAM_MAX : (unsigned)ceil(want));
+        t = want <= TEAM_ALONE ? 1u : (want >= (double)TEAM_MAX ? TEAM_MAX : (unsigned)ceil(want));
     }
     unsigned incl = t;
     for (int o = 1; o < 32; o <<= 1) {
@@ -1698,7 +1702,7 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
                 if (budget_mb < 0.001) budget_mb = 0.001;
                 const double per_entry = 8.0 * grid / (budget_mb * 1048576.0);
                 // no row of so few columns wants a team: two launches less
-                const bool alone = (double)words * 32 * per_entry <= 1.0;
+                const bool alone = (double)words * 32 * per_entry <= TEAM_ALONE;
                 const size_t cap = (size_t)p->n2 + (size_t)((double)p->nnz_c * per_entry) + 64;
                 void *tm = nullptr;
                 rc = cap > 0xfffffff0u ? fail("spgemm numeric: too many team items")
