@@ -137,10 +137,14 @@ tri_decide_kernel(int64_t nnz, TcHeader *hdr, TriCounters *tc)
     }
     const unsigned before = t ? s_n[t - 1] : 0u;
     tc->hist[t] = before;
-    // the vertices up to the bucket that reaches TRI_HUBS hold a quarter of all degrees, or there are no more vertices than that
+    // the first TRI_HUBS vertices hold a quarter of all degrees, or there are no more vertices than that.  Of the bucket that reaches TRI_HUBS
+    // as many count as still fit: where all vertices are alike it holds every one of them (12 entries in each of 700,000 rows, counted
+    // in another order: 713 -> 960 us).
     const bool last = s_n[t] >= TRI_HUBS || t == TRI_BUCKETS - 1;
-    if (last && (t == 0 || s_n[t - 1] < TRI_HUBS)) {
-        const bool skewed = s_n[TRI_BUCKETS - 1] <= TRI_HUBS || s_h[t] * 4 >= 2 * (unsigned long long)nnz;
+    if (last && before < TRI_HUBS) {
+        const double of = s_n[t] > TRI_HUBS ? (double)(TRI_HUBS - before) / (s_n[t] - before) : 1.0;
+        const double held = (t ? (double)s_h[t - 1] : 0.0) + of * (double)(s_h[t] - (t ? s_h[t - 1] : 0ull));
+        const bool skewed = s_n[TRI_BUCKETS - 1] <= TRI_HUBS || held * 4.0 >= 2.0 * (double)nnz;
         const bool triangular = (tc->not_lower == 0 || tc->not_upper == 0) && hdr->desc_all == hdr->desc_edge;
         hdr->ordered = skewed && triangular;
         hdr->desc_all = hdr->desc_edge = 0;     // counted again if not

@@ -32,7 +32,14 @@ def body(name, until=None):
     """A header without its includes, up to a line."""
     text = source(name)
     text = text[:text.index(until)] + "}\n" if until else text
-    return re.sub(r"^#(include|pragma).*$", "", text, flags=re.M).replace("extern __shared__", "extern").replace("static __global__", "__global__")
+    text = re.sub(r"^#(include|pragma).*$", "", text, flags=re.M).replace("extern __shared__", "extern").replace("static __global__", "__global__")
+    return re.sub(r"\*\(volatile [a-z ]+ \*\)(&[\w>-]+)", r"__atomic_load_n(\1, __ATOMIC_RELAXED)", text)
+
+
+def same_zero(store, text):
+    """Several lanes may store the same 0 to a word, which is a race in C++ and none on the device; what they read has to be ordered."""
+    assert text.count(store + " = 0;") == 1
+    return text.replace(store + " = 0;", "__atomic_store_n(&%s, 0u, __ATOMIC_RELAXED);" % store)
 
 
 def run(tmp_path, check, code, *args):
@@ -48,11 +55,7 @@ def run(tmp_path, check, code, *args):
 
 def test_short_rows_of_few_columns(tmp_path):
     text = source("spgemm.cu")
-    kernel = function("few_columns_kernel", text)
-    # several lanes may store the same 0 to a word, which is a race in C++ and none on the device; what they read has to be ordered
-    clear = "bits[cols[x] >> 5] = 0;"
-    assert kernel.count(clear) == 1
-    kernel = kernel.replace(clear, "__atomic_store_n(&bits[cols[x] >> 5], 0u, __ATOMIC_RELAXED);")
+    kernel = same_zero("bits[cols[x] >> 5]", function("few_columns_kernel", text))
     run(tmp_path, "few_columns_check.cpp", constant("HASH_ROW_MAX", text) + constant("HASH_WARPS", text) + kernel)
 
 
@@ -61,3 +64,13 @@ def test_short_rows_of_few_columns(tmp_path):
 def test_sets_of_a_warp(tmp_path, kernel, out):
     run(tmp_path, "warp_sets_check.cpp", body("semiring.cuh") + body("pairs.cuh", "template <int THREADS, bool SEGMENTED, class Out>\nstatic int"),
         kernel, out)
+
+
+@pytest.mark.parametrize("graph", ["skewed", "upper", "no room", "even", "regular"])
+def test_triangles_in_another_order(tmp_path, graph):
+    order = same_zero("bm[hub[s + q] >> 5]", body("order.cuh"))
+    for wide, narrow in (("TRI_HUBS = 16384", "TRI_HUBS = 256"), ("TRI_BITMAP = 64", "TRI_BITMAP = 16")):
+        assert order.count(wide) == 1
+        order = order.replace(wide, narrow)
+    run(tmp_path, "triangle_order_check.cpp", body("semiring.cuh") + body("pairs.cuh", "template <int THREADS, bool SEGMENTED, class Out>\nstatic int") +
+        order, graph)
