@@ -62,16 +62,18 @@ tri_degree_kernel(int64_t n, const int64_t *__restrict__ crd, uint32_t *__restri
     unsigned desc = 0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x * 2;
     for (int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2; p < n; p += stride) {
-        int64_t a;
+        int64_t a, b;
         if (p + 1 < n) {
             const longlong2 v = __ldcs((const longlong2 *)(crd + p));
             a = v.x;
-            desc += v.y <= a;
-            if (p + 2 < n) desc += crd[p + 2] <= v.y;
+            b = v.y;
+            desc += b <= a;
+            if (p + 2 < n) desc += crd[p + 2] <= b;
         } else {
-            a = crd[p];
+            a = b = crd[p];
         }
-        if ((p / 2 + p / 64) % (TRI_SAMPLE / 2) == 0) atomicAdd(degree + a, (unsigned)TRI_SAMPLE);
+        // either of the two: a column that ends every row of an even number of entries is always the second
+        if ((p / 2 + p / 64) % (TRI_SAMPLE / 2) == 0) atomicAdd(degree + ((unsigned)(p / 2) * 0x9E3779B1u >> 31 ? b : a), (unsigned)TRI_SAMPLE);
     }
     desc = __reduce_add_sync(0xffffffffu, desc);
     if ((threadIdx.x & 31) == 0 && desc) atomicAdd(&hdr->desc_all, desc);

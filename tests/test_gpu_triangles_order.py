@@ -82,3 +82,30 @@ def test_against_the_oracle():
     L = oracle.SparseArrays("CSR", n, n, np.array([n]), np.array([-1]), pos, crd, np.ones(crd.size))
     assert D.nnz >= 6000000
     assert int(dev.masked_pair_count(D, D, D)) == oracle.masked_pair_count_rowparallel(L, L, L)
+
+
+@pytest.mark.parametrize("hub", [0, 1])
+def test_a_column_at_the_same_place_of_every_row(hub):
+    """Rows of an even number of entries that all end in the last column, and rows of one length that lies in one bucket of degrees."""
+    n = 400000
+    i, j = _graph("skewed", n, 9000000, 11)
+    i, j = j, i                                          # rows are the lower numbers
+    keep = j != n - 1
+    i, j = i[keep], j[keep]
+    if hub:
+        order = torch.argsort(i * n + j)
+        i, j = i[order], j[order]
+        count = torch.bincount(i, minlength=n)
+        first = torch.cumsum(count, 0) - count
+        drop = first[(count % 2 == 0) & (count > 0)]     # one entry less where the number is even
+        keep = torch.ones(i.numel(), dtype=torch.bool, device="cuda")
+        keep[drop] = False
+        i, j = i[keep], j[keep]
+        rows = torch.nonzero(torch.bincount(i, minlength=n)).flatten()
+        i, j = torch.cat([i, rows]), torch.cat([j, torch.full_like(rows, n - 1)])
+    else:
+        rows = torch.arange(n - 20, device="cuda").repeat_interleave(16)
+        i, j = rows, rows + 1 + torch.arange(16, device="cuda").repeat(n - 20)
+    D = _device(i, j, n)
+    assert D.nnz >= max(6000000, 10 * n)
+    assert int(dev.masked_pair_count(D, D, D)) == _by_blocks(D, [0, n // 3, n])
