@@ -56,11 +56,11 @@ int main(int argc, char **argv)
     if (what == "skewed" || what == "no room") g = skewed(700, 9000, 3, false);
     else if (what == "upper") g = skewed(700, 9000, 3, true);
     else if (what == "even") g = skewed(4000, 60000, 1, false);
-    else if (what == "regular") {                    // a ring of 2000 vertices with 6 neighbours on either side
+    else if (what == "regular") {                    // a ring of 8000 vertices with 6 neighbours on either side
         std::vector<std::pair<int64_t, int64_t>> e;
-        for (int64_t i = 0; i < 2000; i++)
-            for (int64_t d = 1; d <= 6; d++) e.push_back({std::max(i, (i + d) % 2000), std::min(i, (i + d) % 2000)});
-        g = finish(2000, e, false);
+        for (int64_t i = 0; i < 8000; i++)
+            for (int64_t d = 1; d <= 6; d++) e.push_back({std::max(i, (i + d) % 8000), std::min(i, (i + d) % 8000)});
+        g = finish(8000, e, false);
     } else {                                         // rows of even length, all of which end in the last column
         g = skewed(700, 9000, 3, true);
         std::vector<std::pair<int64_t, int64_t>> e;
