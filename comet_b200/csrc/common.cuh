@@ -62,7 +62,15 @@ enum Slot {
     SLOT_COUNT
 };
 int scratch(Slot slot, size_t bytes, void **ptr);   // status; *ptr valid until the slot grows
-bool scratch_if_room(Slot slot, size_t bytes, void **ptr);   // for what a call can do without: false, and no error, where it does not fit
+// Scratch that a call can do without: p is null, and there is no error, where it does not fit.  The call asks for it after all that it cannot do
+// without; it is the call's while the object lives, and from then on it is given back when some other call finds no room (scratch()).
+struct ScratchIfRoom {
+    void *p = nullptr;
+    void take(Slot slot, size_t bytes);
+    ScratchIfRoom() {}
+    ~ScratchIfRoom();
+    ScratchIfRoom(const ScratchIfRoom &) = delete;
+};
 void scratch_release_all();
 void result_release_kept();                          // page-locked result blocks that are not in use (hostmem.cu)
 
@@ -82,6 +90,7 @@ int narrow_f64_to_f32(const double *src, float *dst, int64_t n, cudaStream_t st)
 int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st);
 int exclusive_scan_nonzero(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st);   // counts entries that are not 0
 int exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, cudaStream_t st);
+int exclusive_scan_room(int64_t n);                  // scans of up to n elements need no more scratch after this
 // sorted COO row coordinates -> row pointer; *sorted_flag_dev set to 0 if rows are not ascending
 int coo_rows_to_pos(const int64_t *rows, int64_t nnz, int64_t nrows, int64_t *pos, int *flag_dev,
                     cudaStream_t st);

@@ -270,11 +270,11 @@ tri_edges_kernel(int64_t nrows, int64_t nnz, const int64_t *__restrict__ pos, co
     if (lane == 0 && top > (unsigned)*(volatile unsigned long long *)&tc->columns) atomicMax(&tc->columns, (unsigned long long)top);
 }
 
-// The entries into their rows.  columns != null: where pairs.cuh looks for the number of columns.
+// The entries into their rows.  columns != null: where pairs.cuh looks for the number of columns.  m32 may be a32 (columns keep their numbers).
 static __global__ void __launch_bounds__(256)
 tri_scatter_kernel(int64_t nnz, const int2 *__restrict__ edge, const int32_t *__restrict__ place, const int64_t *__restrict__ hub_pos,
                    const int64_t *__restrict__ rest_pos, const TcHeader *hdr, const TriCounters *tc,
-                   unsigned short *__restrict__ hub, int32_t *__restrict__ a32, int32_t *__restrict__ m32, int64_t *columns)
+                   unsigned short *__restrict__ hub, int32_t *a32, int32_t *m32, int64_t *columns)
 {
     if (!hdr->ordered) return;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
@@ -298,7 +298,7 @@ tri_scatter_kernel(int64_t nnz, const int2 *__restrict__ edge, const int32_t *__
                     hub[at[u]] = (unsigned short)e[u].y;
                 } else {
                     a32[at[u]] = e[u].y;
-                    m32[at[u]] = e[u].y - TRI_HUBS;
+                    if (m32 != a32) m32[at[u]] = e[u].y - TRI_HUBS;
                 }
             }
     }

@@ -62,6 +62,7 @@ struct DeviceState {
     cudaStream_t stream;
     cudaStream_t aux[2];
     int sms;
+    int optional_users;                    // calls that have SLOT_TRIANGLES in use (ScratchIfRoom)
 };
 static DeviceState g_dev[kMaxDevices];
 static std::mutex g_mu;
@@ -73,23 +74,52 @@ static DeviceState *state()
     return &g_dev[d];
 }
 
-bool scratch_if_room(Slot slot, size_t bytes, void **ptr)
+static size_t with_headroom(size_t bytes)  // so that slowly growing inputs do not reallocate
+{
+    return (bytes + bytes / 8 + 255) & ~(size_t)255;
+}
+
+// A slot's buffer is released; a kernel of an earlier call may still read it.
+static bool give_back(DeviceState *s, Slot slot)
+{
+    if (!s->ptr[slot]) return true;
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaFree(s->ptr[slot]) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    s->ptr[slot] = nullptr;
+    s->cap[slot] = 0;
+    return true;
+}
+
+void ScratchIfRoom::take(Slot slot, size_t bytes)
 {
     std::lock_guard<std::mutex> lk(g_mu);
     DeviceState *s = state();
-    if (!s) return false;
+    if (!s || p) return;
     if (s->cap[slot] < bytes) {
-        void *p = nullptr;                 // beside the old buffer, which stays if this fails
-        if (cudaMalloc(&p, (bytes + 255) & ~(size_t)255) != cudaSuccess) {
+        if (s->optional_users || !give_back(s, slot)) return;
+        size_t want = with_headroom(bytes);
+        if (cudaMalloc(&s->ptr[slot], want) != cudaSuccess) {
             (void)cudaGetLastError();
-            return false;
+            want = (bytes + 255) & ~(size_t)255;
+            if (cudaMalloc(&s->ptr[slot], want) != cudaSuccess) {
+                (void)cudaGetLastError();
+                s->ptr[slot] = nullptr;
+                return;
+            }
         }
-        if (s->ptr[slot] && (cudaDeviceSynchronize() != cudaSuccess || cudaFree(s->ptr[slot]) != cudaSuccess)) return false;
-        s->ptr[slot] = p;
-        s->cap[slot] = (bytes + 255) & ~(size_t)255;
+        s->cap[slot] = want;
     }
-    *ptr = s->ptr[slot];
-    return true;
+    p = s->ptr[slot];
+    s->optional_users++;
+}
+
+ScratchIfRoom::~ScratchIfRoom()
+{
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (DeviceState *s = state()) s->optional_users--;
 }
 
 int scratch(Slot slot, size_t bytes, void **ptr)
@@ -106,9 +136,12 @@ int scratch(Slot slot, size_t bytes, void **ptr)
             s->ptr[slot] = nullptr;
             s->cap[slot] = 0;
         }
-        size_t want = bytes + bytes / 8;   // head-room so slowly growing inputs do not reallocate
-        want = (want + 255) & ~(size_t)255;
+        const size_t want = with_headroom(bytes);
         cudaError_t e = cudaMalloc(&s->ptr[slot], want);
+        if (e != cudaSuccess && s->ptr[SLOT_TRIANGLES] && !s->optional_users) {       // what earlier calls could do without
+            (void)cudaGetLastError();
+            if (give_back(s, SLOT_TRIANGLES)) e = cudaMalloc(&s->ptr[slot], want);
+        }
         if (e != cudaSuccess)
             return fail("cudaMalloc of %zu bytes of scratch failed: %s", want, cudaGetErrorString(e));
         s->cap[slot] = want;

@@ -169,7 +169,8 @@ static int tri_prepare(int64_t nrows, int64_t nnz, const int64_t *pos, const int
     return 0;
 }
 
-// Counts the triangles of the hub columns; the rest of the rows goes to a32 and, renumbered, m32.
+// Counts the triangles of the hub columns; the rest of the rows goes to a32 and, where that is another array, counted from the first of its
+// columns, to m32.
 static int tri_count(int64_t nrows, int64_t nnz, TcHeader *hdr, TriArrays *t, int32_t *a32, int32_t *m32,
                      int64_t *columns, int64_t *count_dev, cudaStream_t st)
 {
@@ -209,11 +210,8 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     const bool same_bm = bcrd == mcrd && nnz_b == nnz_m, same_am = acrd == mcrd && nnz_a == nnz_m;
     const bool same_ab = acrd == bcrd && nnz_a == nnz_b;
     // one matrix in all three places: its triangles, if it is triangular, in another order of the vertices
-    bool order = same_am && same_bm && apos == mpos && bpos == mpos && row_lo == 0 && row_hi == ncols &&
+    const bool suits = same_am && same_bm && apos == mpos && bpos == mpos && row_lo == 0 && row_hi == ncols &&
                        nnz_a >= TRI_MIN_ENTRIES && nnz_a / TRI_MIN_PER_ROW >= ncols && nnz_a < 0x7fffffffLL;
-    void *tri_mem = nullptr;
-    if (order) order = scratch_if_room(SLOT_TRIANGLES, tri_bytes(row_hi, nnz_a), &tri_mem);       // else in the order it has
-    const TcShape sh = {bcap, acrd == mcrd && apos == mpos, false, false, order};
 
     // scratch: header, rows of A, list places, B side lists and their pointers, unit list
     const size_t nunits = (size_t)(nnz_a / 16 + (nnz_m < nrows * TC_WARP_MAX ? nnz_m / TC_WARP_MAX : nrows) +
@@ -238,10 +236,22 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     CB_TRY(scratch(SLOT_BINS, pad((size_t)nrows * 4) + 2 * nunits * sizeof(TcUnit), &bins));
     int32_t *small = (int32_t *)bins;
     TcUnit *units = (TcUnit *)((char *)bins + pad((size_t)nrows * 4)), *mids = units + nunits;
+    CB_TRY(scratch(SLOT_NARROW_M, (size_t)nnz_m * 4 + 16, &m32));
+    if (same_bm) b32 = m32;
+    else CB_TRY(scratch(SLOT_NARROW_B, (size_t)nnz_b * 4 + 16, &b32));
+    if (same_am && !compact) a32 = m32;
+    else if (same_ab && !compact) a32 = b32;
+    else CB_TRY(scratch(SLOT_NARROW_A, (size_t)nnz_a * 4 + 16, &a32));
+    CB_TRY(exclusive_scan_room(bcap > words ? bcap : words));
+    // after all that the count cannot do without
+    ScratchIfRoom tri_mem;
+    if (suits) tri_mem.take(SLOT_TRIANGLES, tri_bytes(row_hi, nnz_a));
+    const bool order = tri_mem.p != nullptr;               // else in the order it has
+    const TcShape sh = {bcap, acrd == mcrd && apos == mpos, false, false, order};
     CB_CUDA(cudaMemsetAsync(hdr, 0, counts_bytes, st));           // header, list counts, column bits
 
     TriArrays tri;
-    if (order) CB_TRY(tri_prepare(row_hi, nnz_a, apos, acrd, hdr, tri_mem, blist, slot, &tri, st));
+    if (order) CB_TRY(tri_prepare(row_hi, nnz_a, apos, acrd, hdr, tri_mem.p, blist, slot, &tri, st));
 
     if (compact) {
         tc_present_kernel<<<(unsigned)sm_count() * 4, 512, 0, st>>>(nnz_m, mcrd, present, order ? hdr : nullptr);
@@ -255,19 +265,9 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
                                                                   words, mpos, row_lo, row_hi, check ? hdr : nullptr, order ? hdr : nullptr);
         return cudaGetLastError() == cudaSuccess ? 0 : fail("masked count: narrowing failed");
     };
-    CB_TRY(scratch(SLOT_NARROW_M, (size_t)nnz_m * 4 + 16, &m32));
     CB_TRY(narrow(mcrd, nnz_m, m32, true, true));
-    if (same_bm) b32 = m32;
-    else {
-        CB_TRY(scratch(SLOT_NARROW_B, (size_t)nnz_b * 4 + 16, &b32));
-        CB_TRY(narrow(bcrd, nnz_b, b32, true, false));
-    }
-    if (same_am && !compact && !order) a32 = m32;
-    else if (same_ab && !compact && !order) a32 = b32;
-    else {
-        CB_TRY(scratch(SLOT_NARROW_A, (size_t)nnz_a * 4 + 16, &a32));
-        CB_TRY(narrow(acrd, nnz_a, a32, false, false));
-    }
+    if (b32 != m32) CB_TRY(narrow(bcrd, nnz_b, b32, true, false));
+    if (a32 != m32 && a32 != b32) CB_TRY(narrow(acrd, nnz_a, a32, false, false));
     const int32_t *A = (const int32_t *)a32, *B = (const int32_t *)b32, *M = (const int32_t *)m32;
     if (order) {
         CB_TRY(tri_count(row_hi, nnz_a, hdr, &tri, (int32_t *)a32, (int32_t *)m32, compact ? before + words : nullptr, count_dev, st));

@@ -255,6 +255,12 @@ static int exclusive_scan(const InT *in, int64_t *out, int64_t n, cudaStream_t s
     return 0;
 }
 
+int exclusive_scan_room(int64_t n)
+{
+    void *p = nullptr;
+    return n <= SCAN_FEW_CTAS ? 0 : scratch(SLOT_SCAN, (size_t)ceil_div(n, SCAN_TILE) * sizeof(int64_t), &p);
+}
+
 int exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st) { return exclusive_scan(in, out, n, st); }
 
 // positions of the non-zero entries

@@ -48,3 +48,16 @@ def test_columns_that_need_a_look_up_have_a_stage(hub_launch, stored):
     assert ctas >= 1 and 128 <= stage <= 512
     dynamic = (stored + 31) // 32 * 8 + stage * 16 * 4
     assert ctas * (dynamic + 4176 + 1024) <= 228 * 1024 and dynamic + 4176 <= 227 * 1024
+
+
+@pytest.mark.parametrize("n,nnz", [(500000, 8000000), (1600000, 20000000)])
+def test_a_count_goes_on_without_memory_it_can_do_without(tmp_path_factory, n, nnz):
+    assert output(link(tmp_path_factory, "triangle_memory_check.cpp", "tc.o"), n, nnz) == "ok"
+
+
+def test_scratch_that_a_call_can_do_without(tmp_path):
+    exe = str(tmp_path / "scratch")
+    subprocess.check_call(["g++", "-O1", "-g", "-std=c++17", "-pthread", "-I/usr/local/cuda/include", "-x", "c++", os.path.join(CHECKS, "scratch_check.cpp"),
+                           os.path.join(ROOT, "comet_b200", "csrc", "runtime.cu"), "-no-pie",
+                           "-Wl,--unresolved-symbols=ignore-in-object-files", "-o", exe])
+    assert output(exe) == "ok"
