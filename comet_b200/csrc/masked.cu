@@ -38,6 +38,7 @@ struct MaskedStats {
     unsigned long long desc_all, desc_edge;           // places where A's coordinates do not ascend: all, and at row starts
     unsigned nnz_a, nnz_m;                 // 0xffffffff: that or more
     unsigned long long one_sided;          // entries of A without a mate, see masked_mates_kernel
+    unsigned long long balance;            // not 0: some vertex has not as many entries in its row as in its column
 };
 static_assert(sizeof(MaskedStats) <= 64, "fits a page-locked word block");
 
@@ -61,24 +62,36 @@ static unsigned flat_grid(int64_t n)
     return (unsigned)(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));
 }
 
+// a vertex's weight in MaskedStats::balance
+__device__ __forceinline__ unsigned long long masked_weight(int64_t k)
+{
+    unsigned long long h = (unsigned long long)(k + 1) * 0x9E3779B97F4A7C15ull;
+    h ^= h >> 29;
+    return h * 0xBF58476D1CE4E5B9ull;
+}
+
+// same: A, B and M are one square matrix.  It cannot be symmetric unless the weights of its entries' columns add up to those of their
+// rows, which rules out nearly every other one without a look-up (masked_mates_kernel took 130 us of 1847 on a lower triangle of 4 M entries).
 __global__ void __launch_bounds__(256)
 masked_stats_kernel(int64_t nrows, const int64_t *__restrict__ apos, const int64_t *__restrict__ acrd,
-                    const int64_t *__restrict__ bpos, const int64_t *__restrict__ mpos, MaskedStats *stats)
+                    const int64_t *__restrict__ bpos, const int64_t *__restrict__ mpos, bool same, MaskedStats *stats)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n = apos[nrows];
-    unsigned long long top = 0, products = 0, bound = 0;
+    unsigned long long top = 0, products = 0, bound = 0, balance = 0;
     unsigned desc = 0, edge = 0;
     for (int64_t p = t0; p < n; p += stride) {
         const int64_t k = acrd[p];
         if ((unsigned long long)(k + 1) > top) top = (unsigned long long)(k + 1);
         products += (unsigned long long)(bpos[k + 1] - bpos[k]);
         if (p + 1 < n && acrd[p + 1] <= k) desc++;
+        if (same) balance += masked_weight(k);
     }
     for (int64_t r = t0; r < nrows; r += stride) {
         const int64_t s = apos[r], e = apos[r + 1];
         bound += (unsigned long long)(e - s) * (unsigned long long)(mpos[r + 1] - mpos[r]);
         if (s > 0 && e > s && acrd[s] <= acrd[s - 1]) edge++;
+        if (same) balance -= (unsigned long long)(e - s) * masked_weight(r);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -86,6 +99,7 @@ masked_stats_kernel(int64_t nrows, const int64_t *__restrict__ apos, const int64
         top = v > top ? v : top;
         products += __shfl_xor_sync(0xffffffffu, products, o);
         bound += __shfl_xor_sync(0xffffffffu, bound, o);
+        balance += __shfl_xor_sync(0xffffffffu, balance, o);
     }
     desc = __reduce_add_sync(0xffffffffu, desc);
     edge = __reduce_add_sync(0xffffffffu, edge);
@@ -93,6 +107,7 @@ masked_stats_kernel(int64_t nrows, const int64_t *__restrict__ apos, const int64
         atomicMax(&stats->nrows_b, top);
         if (products) atomicAdd(&stats->products, products);
         if (bound) atomicAdd(&stats->bound, bound);
+        if (balance) atomicAdd(&stats->balance, balance);
         if (desc) atomicAdd(&stats->desc_all, (unsigned long long)desc);
         if (edge) atomicAdd(&stats->desc_edge, (unsigned long long)edge);
     }
@@ -133,6 +148,10 @@ __global__ void __launch_bounds__(256)
 masked_mates_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, int64_t room,
                     int32_t *__restrict__ mate, MaskedStats *stats)
 {
+    if (stats->balance) {                              // some entry has none
+        if (blockIdx.x == 0 && threadIdx.x == 0) stats->one_sided = 1;
+        return;
+    }
     const int64_t n = pos[nrows];
     unsigned none = n > room;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n && p < room; p += (int64_t)gridDim.x * blockDim.x) {
@@ -236,12 +255,12 @@ int masked_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     void *sp = nullptr;
     CB_TRY(scratch(SLOT_MISC, sizeof(MaskedStats), &sp));
     CB_CUDA(cudaMemsetAsync(sp, 0, sizeof(MaskedStats), st));
-    masked_stats_kernel<<<(unsigned)sm_count() * 4, 256, 0, st>>>(nrows, apos, acrd, bpos, mpos, (MaskedStats *)sp);
-    CB_LAUNCH_CHECK();
     // one matrix in all three places: it may be symmetric, as the adjacency matrix of a graph is
+    const bool same = nrows == ncols_b && apos == bpos && apos == mpos && acrd == bcrd && acrd == mcrd;
+    masked_stats_kernel<<<(unsigned)sm_count() * 4, 256, 0, st>>>(nrows, apos, acrd, bpos, mpos, same, (MaskedStats *)sp);
+    CB_LAUNCH_CHECK();
     int32_t *mate = nullptr;
-    if (nrows == ncols_b && apos == bpos && apos == mpos && acrd == bcrd && acrd == mcrd &&
-        cudaMallocAsync((void **)&mate, (size_t)nnz_b * 4, st) != cudaSuccess) {
+    if (same && cudaMallocAsync((void **)&mate, (size_t)nnz_b * 4, st) != cudaSuccess) {
         (void)cudaGetLastError();
         mate = nullptr;
     }

@@ -74,3 +74,9 @@ def test_triangles_in_another_order(tmp_path, graph):
         order = order.replace(wide, narrow)
     run(tmp_path, "triangle_order_check.cpp", body("semiring.cuh") + body("pairs.cuh", "template <int THREADS, bool SEGMENTED, class Out>\nstatic int") +
         order, graph)
+
+
+def test_mates_of_a_symmetric_pattern(tmp_path):
+    text = source("masked.cu")
+    struct = re.search(r"^struct MaskedStats \{.*?^\};\n", text, re.M | re.S).group(0)
+    run(tmp_path, "masked_mates_check.cpp", struct + "".join(function(f, text) for f in ("masked_weight", "masked_stats_kernel", "masked_mates_kernel")))
