@@ -222,10 +222,10 @@ static int run_pairs(MaskedPlan *m, const Out &out, cudaStream_t st)
     const int width = (int)m->width;
     const size_t smem = (size_t)2 * TC_SET_BUF * 4 + (size_t)((width >> 5) + 1) * 4;
     if (smem > 52 * 1024)
-        CB_TRY((launch_bitmap<1024, false>(smem, smem > 108 * 1024 ? 1 : 2, m->hdr, m->units, m->mpos, m->m32, m->tpos, m->trow,
+        CB_TRY((launch_bitmap<1024, false>(smem, m->hdr, m->units, m->mpos, m->m32, m->tpos, m->trow,
                                            m->apos, m->a32, m->bptr, m->blist, sh, width, nullptr, out, st)));
     else
-        CB_TRY((launch_bitmap<512, false>(smem, 4, m->hdr, m->units, m->mpos, m->m32, m->tpos, m->trow, m->apos, m->a32, m->bptr,
+        CB_TRY((launch_bitmap<512, false>(smem, m->hdr, m->units, m->mpos, m->m32, m->tpos, m->trow, m->apos, m->a32, m->bptr,
                                           m->blist, sh, width, nullptr, out, st)));
     tc_mid_kernel<<<(unsigned)sm_count() * 6, TC_MID_WARPS * 32, 0, st>>>(m->hdr, m->mids, m->mpos, m->m32, m->tpos, m->trow,
                                                                           m->apos, m->a32, m->bptr, m->blist, sh, out);

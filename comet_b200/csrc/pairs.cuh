@@ -626,8 +626,12 @@ tc_mid_kernel(TcHeader *hdr, const TcUnit *__restrict__ mids, const int64_t *__r
 // Units: a bitmap of the set, its lists drawn by the warps in batches of 32.  SEGMENTED: the columns do not fit one
 // bitmap, the unit is repeated per segment of `width` columns.  The next unit's set is fetched into shared memory by
 // warp 0 while the others stream, so that between two units only the bits change.
+// 32 warps an SM, as many as are launched: 64 registers a thread, which no variant spills for.  With the 109 that the value pass for both
+// halves takes otherwise, one CTA of 16 warps ran (R-MAT scale 15 / 16, 16 per row, symmetric, under itself, plus-times 1450 -> 1235 and
+// 3000 -> 2300 us); the one-sided pass spilled 112 bytes (not symmetric 728 -> 714 and 1715 -> 1690).  Three CTAs of 16 warps for
+// counts cost 96 bytes of spills and gain nothing (plus-pair at scale 15 373 and 373 us).
 template <int THREADS, bool SEGMENTED, class Out>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 tc_bitmap_kernel(TcHeader *hdr, const TcUnit *__restrict__ units, const int64_t *__restrict__ apos,
                  const int32_t *__restrict__ acrd, const int64_t *__restrict__ bpos, const int32_t *__restrict__ bcrd,
                  const int64_t *__restrict__ mpos, const int32_t *__restrict__ mcrd, const int64_t *__restrict__ bptr,
@@ -780,7 +784,7 @@ tc_bitmap_kernel(TcHeader *hdr, const TcUnit *__restrict__ units, const int64_t 
 }
 
 template <int THREADS, bool SEGMENTED, class Out>
-static int launch_bitmap(size_t smem, int per_sm, TcHeader *hdr, const TcUnit *units, const int64_t *apos,
+static int launch_bitmap(size_t smem, TcHeader *hdr, const TcUnit *units, const int64_t *apos,
                          const int32_t *acrd, const int64_t *bpos, const int32_t *bcrd, const int64_t *mpos,
                          const int32_t *mcrd, const int64_t *bptr, const int2 *blist, TcShape sh, int width,
                          const int64_t *ncols_dev, const Out &out, cudaStream_t st)
@@ -791,7 +795,7 @@ static int launch_bitmap(size_t smem, int per_sm, TcHeader *hdr, const TcUnit *u
     const bool with_prefix = Out::VALUES && both <= (size_t)210 * 1024;
     if (with_prefix) smem = both;
     CB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<(unsigned)(sm_count() * per_sm), THREADS, smem, st>>>(hdr, units, apos, acrd, bpos, bcrd, mpos, mcrd, bptr, blist,
+    k<<<(unsigned)(sm_count() * (1024 / THREADS)), THREADS, smem, st>>>(hdr, units, apos, acrd, bpos, bcrd, mpos, mcrd, bptr, blist,
                                                              sh, width, ncols_dev, with_prefix, out);
     CB_LAUNCH_CHECK();
     return 0;

@@ -290,15 +290,15 @@ int masked_pair_count(int64_t row_lo, int64_t row_hi, int64_t ncols, int64_t nnz
     const int width = (int)(compact ? TC_MAX_COLS : ncols);
     const size_t smem = (size_t)2 * TC_SET_BUF * 4 + (size_t)((width >> 5) + 1) * 4;
     const int64_t *ncols_dev = compact ? before + words : nullptr;
-    // one CTA of 32 warps per SM when the bitmap fills the shared memory, otherwise two of 32 or four of 16
+    // one CTA of 32 warps per SM where two bitmaps do not fit well, otherwise two of 16
     if (compact)
-        CB_TRY((launch_bitmap<1024, true>(smem, 1, hdr, units, apos, A, bpos, B, mpos, M, bptr, blist, sh, width, ncols_dev,
+        CB_TRY((launch_bitmap<1024, true>(smem, hdr, units, apos, A, bpos, B, mpos, M, bptr, blist, sh, width, ncols_dev,
                                           out, st)));
     else if (smem > 52 * 1024)
-        CB_TRY((launch_bitmap<1024, false>(smem, smem > 108 * 1024 ? 1 : 2, hdr, units, apos, A, bpos, B, mpos, M, bptr, blist,
+        CB_TRY((launch_bitmap<1024, false>(smem, hdr, units, apos, A, bpos, B, mpos, M, bptr, blist,
                                            sh, width, ncols_dev, out, st)));
     else
-        CB_TRY((launch_bitmap<512, false>(smem, 4, hdr, units, apos, A, bpos, B, mpos, M, bptr, blist, sh, width, ncols_dev,
+        CB_TRY((launch_bitmap<512, false>(smem, hdr, units, apos, A, bpos, B, mpos, M, bptr, blist, sh, width, ncols_dev,
                                           out, st)));
     tc_mid_kernel<<<(unsigned)sm_count() * 6, TC_MID_WARPS * 32, 0, st>>>(hdr, mids, apos, A, bpos, B, mpos, M, bptr, blist,
                                                                           sh, out);
