@@ -21,6 +21,7 @@
 // is the whole matrix as it is, and the kernels of the first part have nothing to do.
 #pragma once
 #include "pairs.cuh"
+#include "stream.cuh"
 
 namespace cb200 {
 
@@ -32,14 +33,15 @@ static const int TRI_LOOK = 1;                  // look-ups of 32 entries agains
 static const int TRI_SAMPLE = 16;
 static const int TRI_BUCKETS = 512;             // degrees: 16 per octave
 // Where it pays (us before and after, R-MAT scale x edges per vertex): 18x5 322 566, 19x9 873 999, 20x6 1119 1375, 21x6 2533 2431,
-// 19x12 1176 1129, 19x16 1636 1269, 20x16 3245 2385, 21x16 7792 4878, 22x16 18450 11370.
+// 19x13 1280 1128, 19x16 1745 1230, 20x16 3200 2378, 21x16 7760 4765, 22x16 18480 11250.
 static const int64_t TRI_MIN_ENTRIES = 6000000;
 static const int64_t TRI_MIN_PER_ROW = 10;
 static const int TRI_WARPS = 8;
 static const int TRI_SINGLE = 1 << 17;
 
 struct TriCounters {                            // cleared before
-    unsigned not_lower, not_upper;              // rows that are not
+    unsigned not_lower, not_upper;              // rows that are not (some of them counted twice)
+    unsigned desc_all, desc_edge;               // places where the coordinates do not ascend: all, and those at row starts
     unsigned next, pad;
     unsigned long long words;                   // of the bitmaps given out
     unsigned long long columns;                 // of the rest
@@ -55,39 +57,51 @@ __device__ __forceinline__ int tri_bucket(unsigned degree)      // larger degree
 }
 
 // Column counts, of one entry in TRI_SAMPLE (the order has to be about right, and all of them take 1.3 ms on 64 M entries: the hubs'
-// counters are a queue), and the places where the coordinates do not ascend.
+// counters are a queue).  Of 64 entries four neighbours are taken, any four: a column that is always at the same place of its row is met
+// as often as others.  A CTA looks at the ends of rows from all over the matrix first and counts nothing if that cannot be triangular, which
+// nearly all CTAs find out where it is not.
 static __global__ void __launch_bounds__(256)
-tri_degree_kernel(int64_t n, const int64_t *__restrict__ crd, uint32_t *__restrict__ degree, TcHeader *hdr)
+tri_degree_kernel(int64_t nrows, int64_t n, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, uint32_t *__restrict__ degree,
+                  TriCounters *tc)
 {
-    unsigned desc = 0;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x * 2;
-    for (int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2; p < n; p += stride) {
-        int64_t a, b;
-        if (p + 1 < n) {
-            const longlong2 v = __ldcs((const longlong2 *)(crd + p));
-            a = v.x;
-            b = v.y;
-            desc += b <= a;
-            if (p + 2 < n) desc += crd[p + 2] <= b;
-        } else {
-            a = b = crd[p];
-        }
-        // either of the two: a column that ends every row of an even number of entries is always the second
-        if ((p / 2 + p / 64) % (TRI_SAMPLE / 2) == 0) atomicAdd(degree + ((unsigned)(p / 2) * 0x9E3779B1u >> 31 ? b : a), (unsigned)TRI_SAMPLE);
+    __shared__ unsigned s_lower, s_upper;
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    if (threadIdx.x == 0) s_lower = s_upper = 0;
+    __syncthreads();
+    const int64_t r = ((int64_t)threadIdx.x * gridDim.x + blockIdx.x) * nrows / stride, s = pos[r], e = pos[r + 1];
+    const unsigned lower = __reduce_add_sync(0xffffffffu, (unsigned)(e > s && crd[e - 1] >= r));
+    const unsigned upper = __reduce_add_sync(0xffffffffu, (unsigned)(e > s && crd[s] <= r));
+    if ((threadIdx.x & 31) == 0) {
+        if (lower) atomicAdd(&s_lower, lower);
+        if (upper) atomicAdd(&s_upper, upper);
     }
-    desc = __reduce_add_sync(0xffffffffu, desc);
-    if ((threadIdx.x & 31) == 0 && desc) atomicAdd(&hdr->desc_all, desc);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_lower) atomicAdd(&tc->not_lower, s_lower);
+        if (s_upper) atomicAdd(&tc->not_upper, s_upper);
+    }
+    if (s_lower && s_upper) return;
+    for (int64_t g = t0; g * (4 * TRI_SAMPLE) < n; g += stride) {
+        const int64_t p = (g * TRI_SAMPLE + ((unsigned)g * 0x9E3779B1u >> 28)) * 4;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (p + i < n) atomicAdd(degree + crd[p + i], (unsigned)TRI_SAMPLE);
+    }
 }
+static_assert(TRI_SAMPLE == 16, "four bits of the hash");
 
 // Row lengths to the degrees, their histogram, and the checks by row.
 static __global__ void __launch_bounds__(512)
 tri_hist_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, uint32_t *__restrict__ degree,
-                TcHeader *hdr, TriCounters *tc)
+                TriCounters *tc)
 {
-    __shared__ unsigned s_hist[TRI_BUCKETS];
-    __shared__ unsigned long long s_held[TRI_BUCKETS];
-    for (int t = threadIdx.x; t < TRI_BUCKETS; t += blockDim.x) { s_hist[t] = 0; s_held[t] = 0; }
+    __shared__ unsigned s_hist[TRI_BUCKETS], s_held[TRI_BUCKETS];      // of 2^32 degrees at most
+    __shared__ bool s_neither;
+    wait_for_previous();
+    if (threadIdx.x == 0) s_neither = *(volatile unsigned *)&tc->not_lower && *(volatile unsigned *)&tc->not_upper;
+    for (int t = threadIdx.x; t < TRI_BUCKETS; t += blockDim.x) s_hist[t] = s_held[t] = 0;
     __syncthreads();
+    if (s_neither) return;
     unsigned edge = 0, lower = 0, upper = 0;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = pos[r], e = pos[r + 1];
@@ -101,7 +115,7 @@ tri_hist_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *_
             degree[r] = d;
         }
         atomicAdd(&s_hist[tri_bucket(d)], 1u);
-        if (d) atomicAdd(&s_held[tri_bucket(d)], (unsigned long long)d);
+        if (d) atomicAdd(&s_held[tri_bucket(d)], d);
     }
     lower = __reduce_add_sync(0xffffffffu, lower);
     upper = __reduce_add_sync(0xffffffffu, upper);
@@ -109,13 +123,13 @@ tri_hist_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *_
     if ((threadIdx.x & 31) == 0) {
         if (lower) atomicAdd(&tc->not_lower, lower);
         if (upper) atomicAdd(&tc->not_upper, upper);
-        if (edge) atomicAdd(&hdr->desc_edge, edge);
+        if (edge) atomicAdd(&tc->desc_edge, edge);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < TRI_BUCKETS; t += blockDim.x)
         if (s_hist[t]) {
             atomicAdd(&tc->hist[t], s_hist[t]);
-            atomicAdd(&tc->held[t], s_held[t]);
+            atomicAdd(&tc->held[t], (unsigned long long)s_held[t]);
         }
 }
 
@@ -126,6 +140,7 @@ tri_decide_kernel(int64_t nnz, TcHeader *hdr, TriCounters *tc)
     __shared__ unsigned s_n[TRI_BUCKETS];
     __shared__ unsigned long long s_h[TRI_BUCKETS];
     const int t = threadIdx.x;
+    wait_for_previous();
     s_n[t] = tc->hist[t];
     s_h[t] = tc->held[t];
     __syncthreads();
@@ -147,16 +162,16 @@ tri_decide_kernel(int64_t nnz, TcHeader *hdr, TriCounters *tc)
         const double of = s_n[t] > TRI_HUBS ? (double)(TRI_HUBS - before) / (s_n[t] - before) : 1.0;
         const double held = (t ? (double)s_h[t - 1] : 0.0) + of * (double)(s_h[t] - (t ? s_h[t - 1] : 0ull));
         const bool skewed = s_n[TRI_BUCKETS - 1] <= TRI_HUBS || held * 4.0 >= 2.0 * (double)nnz;
-        const bool triangular = (tc->not_lower == 0 || tc->not_upper == 0) && hdr->desc_all == hdr->desc_edge;
-        hdr->ordered = skewed && triangular;
-        hdr->desc_all = hdr->desc_edge = 0;     // counted again if not
+        hdr->ordered = skewed && (tc->not_lower == 0 || tc->not_upper == 0);       // if the coordinates ascend, see tri_totals_kernel
     }
 }
 
-// A vertex's new number: by falling degree, any order within a bucket.
+// A vertex's new number: by falling degree, any order within a bucket.  Clears the rows' counts.
 static __global__ void __launch_bounds__(512)
-tri_rank_kernel(int64_t nrows, const uint32_t *__restrict__ degree, const TcHeader *hdr, TriCounters *tc, int32_t *__restrict__ rank)
+tri_rank_kernel(int64_t nrows, const uint32_t *__restrict__ degree, const TcHeader *hdr, TriCounters *tc, int32_t *__restrict__ rank,
+                int32_t *__restrict__ hub_count, int32_t *__restrict__ rest_count)
 {
+    wait_for_previous();
     if (!hdr->ordered) return;
     __shared__ unsigned s_count[TRI_BUCKETS], s_base[TRI_BUCKETS];
     const int64_t stride = (int64_t)gridDim.x * 2048;
@@ -169,7 +184,10 @@ tri_rank_kernel(int64_t nrows, const uint32_t *__restrict__ degree, const TcHead
         for (int i = 0; i < 4; i++) {
             const int64_t r = r0 + i * 512 + threadIdx.x;
             bucket[i] = r < nrows ? tri_bucket(degree[r]) : -1;
-            if (r < nrows) at[i] = atomicAdd(&s_count[bucket[i]], 1u);
+            if (r < nrows) {
+                at[i] = atomicAdd(&s_count[bucket[i]], 1u);
+                hub_count[r] = rest_count[r] = 0;
+            }
         }
         __syncthreads();
         for (int t = threadIdx.x; t < TRI_BUCKETS; t += 512)
@@ -183,12 +201,13 @@ tri_rank_kernel(int64_t nrows, const uint32_t *__restrict__ degree, const TcHead
 }
 
 // The edges in their new numbers, how many entries every row will have in the hub columns and in the others, and each entry's place
-// among them.  A warp takes 512 entries, 128 of them in flight, and finds their rows among 32 row ends in the lanes.
+// among them; and the places where the coordinates do not ascend.  A warp takes 512 entries, 128 of them in flight, and finds their rows among 32 row ends in the lanes.
 static __global__ void __launch_bounds__(256)
 tri_edges_kernel(int64_t nrows, int64_t nnz, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd,
                  const int32_t *__restrict__ rank, const TcHeader *hdr, TriCounters *tc, int2 *__restrict__ edge,
                  int32_t *__restrict__ place, int32_t *__restrict__ hub_count, int32_t *__restrict__ rest_count)
 {
+    wait_for_previous();
     if (!hdr->ordered) return;
     const int lane = threadIdx.x & 31;
     const int64_t first = (((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5) * 512;
@@ -212,13 +231,15 @@ tri_edges_kernel(int64_t nrows, int64_t nnz, const int64_t *__restrict__ pos, co
         own = w0 + lane < nrows ? rank[w0 + lane] : 0;
     };
     rows_from(0);
-    unsigned top = 0;
+    unsigned top = 0, desc = 0;
     for (int p0 = 0; p0 < n; p0 += 128) {
         int32_t rj[4], ri[4], at[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const int p = p0 + u * 32 + lane;
-            rj[u] = rank[crd[p < n ? p : n - 1]];
+            const int64_t j = crd[p < n ? p : n - 1];
+            rj[u] = rank[j];
+            desc += p < n && first + p + 1 < nnz && crd[p + 1] <= j;
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
@@ -267,7 +288,119 @@ tri_edges_kernel(int64_t nrows, int64_t nnz, const int64_t *__restrict__ pos, co
         }
     }
     top = __reduce_max_sync(0xffffffffu, top);
+    desc = __reduce_add_sync(0xffffffffu, desc);
+    if (lane == 0 && desc) atomicAdd(&tc->desc_all, desc);
     if (lane == 0 && top > (unsigned)*(volatile unsigned long long *)&tc->columns) atomicMax(&tc->columns, (unsigned long long)top);
+}
+
+// Where the rows' entries begin in the hub columns (blockIdx.y 0) and in the others (1): sums of TRI_TILE rows, the sums before them, places.
+// Where the order stays, the rest is the whole matrix as it is.
+static const int TRI_TILE = 2048;
+
+static __global__ void __launch_bounds__(256)
+tri_sums_kernel(int64_t nrows, const int32_t *__restrict__ hub_count, const int32_t *__restrict__ rest_count, const TcHeader *hdr,
+                int64_t *__restrict__ sums)
+{
+    __shared__ int64_t s_sum[8];
+    wait_for_previous();
+    if (!hdr->ordered) return;
+    const int32_t *in = blockIdx.y ? rest_count : hub_count;
+    int64_t sum = 0;
+#pragma unroll
+    for (int i = 0; i < TRI_TILE / 256; i++) {
+        const int64_t r = (int64_t)blockIdx.x * TRI_TILE + i * 256 + threadIdx.x;
+        if (r < nrows) sum += in[r];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, (long long)sum, o);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) sum += s_sum[w];
+        sums[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = sum;
+    }
+}
+
+// One CTA.  The edges' kernel has been through all coordinates: if they do not ascend, the order stays.
+static __global__ void __launch_bounds__(1024)
+tri_totals_kernel(int64_t nrows, int64_t tiles, TcHeader *hdr, const TriCounters *tc, int64_t *__restrict__ sums, int64_t *__restrict__ hub_pos,
+                  int64_t *__restrict__ rest_pos)
+{
+    __shared__ int64_t s_sum[32];
+    wait_for_previous();
+    if (!hdr->ordered) return;
+    __syncthreads();                             // all have read it
+    if (tc->desc_all != tc->desc_edge) {
+        if (threadIdx.x == 0) hdr->ordered = 0;
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int y = 0; y < 2; y++, sums += tiles) {
+        int64_t carry = 0;
+        for (int64_t base = 0; base < tiles; base += 1024) {
+            const int64_t t = base + threadIdx.x, own = t < tiles ? sums[t] : 0;
+            int64_t incl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t v = __shfl_up_sync(0xffffffffu, (long long)incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) s_sum[warp] = incl;
+            __syncthreads();
+            int64_t before = carry + incl - own;
+            for (int w = 0; w < 32; w++) {
+                if (w < warp) before += s_sum[w];
+                carry += s_sum[w];
+            }
+            if (t < tiles) sums[t] = before;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) (y ? rest_pos : hub_pos)[nrows] = carry;
+    }
+}
+
+static __global__ void __launch_bounds__(256)
+tri_places_kernel(int64_t nrows, const int32_t *__restrict__ hub_count, const int32_t *__restrict__ rest_count, const int64_t *__restrict__ pos,
+                  const TcHeader *hdr, const int64_t *__restrict__ sums, int64_t *__restrict__ hub_pos, int64_t *__restrict__ rest_pos)
+{
+    __shared__ int64_t s_sum[8];
+    wait_for_previous();
+    const int64_t base = (int64_t)blockIdx.x * TRI_TILE;
+    if (!hdr->ordered) {
+        if (blockIdx.y == 0) return;
+#pragma unroll
+        for (int i = 0; i < TRI_TILE / 256; i++) {
+            const int64_t r = base + i * 256 + threadIdx.x;
+            if (r <= nrows) rest_pos[r] = pos[r];
+        }
+        return;
+    }
+    const int32_t *in = blockIdx.y ? rest_count : hub_count;
+    int64_t *out = blockIdx.y ? rest_pos : hub_pos;
+    const int64_t r0 = base + threadIdx.x * (TRI_TILE / 256);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t own[TRI_TILE / 256];
+    int64_t incl = 0;
+#pragma unroll
+    for (int i = 0; i < TRI_TILE / 256; i++) {
+        own[i] = r0 + i < nrows ? in[r0 + i] : 0;
+        incl += own[i];
+    }
+    int64_t at = -incl;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t v = __shfl_up_sync(0xffffffffu, (long long)incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    at += incl + sums[(int64_t)blockIdx.y * gridDim.x + blockIdx.x];
+    for (int w = 0; w < warp; w++) at += s_sum[w];
+#pragma unroll
+    for (int i = 0; i < TRI_TILE / 256; i++) {
+        if (r0 + i < nrows) out[r0 + i] = at;
+        at += own[i];
+    }
 }
 
 // The entries into their rows.  columns != null: where pairs.cuh looks for the number of columns.  m32 may be a32 (columns keep their numbers).
@@ -276,6 +409,7 @@ tri_scatter_kernel(int64_t nnz, const int2 *__restrict__ edge, const int32_t *__
                    const int64_t *__restrict__ rest_pos, const TcHeader *hdr, const TriCounters *tc,
                    unsigned short *__restrict__ hub, int32_t *a32, int32_t *m32, int64_t *columns)
 {
+    wait_for_previous();
     if (!hdr->ordered) return;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
     if (t0 == 0 && columns) *columns = (int64_t)tc->columns;
@@ -313,6 +447,7 @@ tri_bitmap_kernel(int64_t nrows, const int64_t *__restrict__ hub_pos, const unsi
                   TriCounters *tc, unsigned long long room, int32_t *__restrict__ bits_at, uint32_t *__restrict__ bits)
 {
     __shared__ __align__(16) uint32_t s_bits[TRI_WARPS][TRI_HUBS / 32];
+    wait_for_previous();
     if (!hdr->ordered) return;
     const int lane = threadIdx.x & 31;
     uint32_t *bm = s_bits[threadIdx.x >> 5];
@@ -361,6 +496,7 @@ tri_count_kernel(int64_t nrows, const int64_t *__restrict__ hub_pos, const unsig
 {
     __shared__ __align__(16) uint32_t s_bits[TRI_WARPS][TRI_HUBS / 32];
     __shared__ unsigned long long s_part[TRI_WARPS];
+    wait_for_previous();
     if (!hdr->ordered) return;
     const int lane = threadIdx.x & 31;
     uint32_t *bm = s_bits[threadIdx.x >> 5];
@@ -491,15 +627,6 @@ tri_count_kernel(int64_t nrows, const int64_t *__restrict__ hub_pos, const unsig
         }
     }
     tc_add_count(total, s_part, TRI_WARPS, count);
-}
-
-// The rest is the whole matrix where the order of its vertices stays.
-static __global__ void __launch_bounds__(256)
-tri_keep_kernel(int64_t nrows, const int64_t *__restrict__ pos, const TcHeader *hdr, int64_t *__restrict__ rest_pos)
-{
-    if (hdr->ordered) return;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= nrows; r += (int64_t)gridDim.x * blockDim.x)
-        rest_pos[r] = pos[r];
 }
 
 }  // namespace cb200

@@ -86,8 +86,8 @@ T from_bits(unsigned long long b)
     return v;
 }
 
-// runs one block (number b of n) of `threads` threads
-inline void run_block(unsigned threads, unsigned b, unsigned n, const std::function<void()> &kernel)
+// runs one block (number b of n, in row y) of `threads` threads
+inline void run_block(unsigned threads, unsigned b, unsigned n, const std::function<void()> &kernel, unsigned y = 0)
 {
     std::vector<Warp> w(threads / 32);
     for (auto &x : w)
@@ -101,7 +101,7 @@ inline void run_block(unsigned threads, unsigned b, unsigned n, const std::funct
     for (unsigned i = 0; i < threads; i++)
         t.emplace_back([&, i] {
             threadIdx = {i, 0, 0};
-            blockIdx = {b, 0, 0};
+            blockIdx = {b, y, 0};
             kernel();
         });
     for (auto &x : t) x.join();

@@ -1,5 +1,6 @@
 // The kernels that count a triangular matrix in another order of its vertices, on small graphs and with 256 hub columns: whether a graph
-// is taken, where its longest vertex goes, and the count, with and without room for bitmaps.
+// is taken, where its longest vertex goes, and the count, with and without room for bitmaps; and matrices that keep their order, because
+// they are not skewed, not triangular, or do not ascend.
 #include "fake_warp.hpp"
 
 #include <comet_b200.h>
@@ -53,8 +54,8 @@ int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "skewed";
     Graph g;
-    if (what == "skewed" || what == "no room") g = skewed(700, 9000, 3, false);
-    else if (what == "upper") g = skewed(700, 9000, 3, true);
+    if (what == "skewed" || what == "no room" || what == "unordered" || what == "repeats") g = skewed(700, 9000, 3, false);
+    else if (what == "upper" || what == "one below") g = skewed(700, 9000, 3, true);
     else if (what == "even") g = skewed(4000, 60000, 1, false);
     else if (what == "regular") {                    // a ring of 8000 vertices with 6 neighbours on either side
         std::vector<std::pair<int64_t, int64_t>> e;
@@ -77,30 +78,51 @@ int main(int argc, char **argv)
             if ((g.pos[(size_t)r + 1] - g.pos[(size_t)r]) % 2) { printf("row %ld is odd\n", (long)r); return 1; }
     }
     const int64_t n = g.n, nnz = g.nnz();
+    auto long_row = [&](int64_t from) {              // a row behind `from` of 5 entries and more
+        while (g.pos[(size_t)from + 1] - g.pos[(size_t)from] < 5) from++;
+        return from;
+    };
+    if (what == "unordered") std::swap(g.crd[(size_t)g.pos[(size_t)long_row(333)] + 1], g.crd[(size_t)g.pos[(size_t)long_row(333)] + 2]);
+    if (what == "repeats") g.crd[(size_t)g.pos[(size_t)long_row(333)] + 1] = g.crd[(size_t)g.pos[(size_t)long_row(333)]];
+    if (what == "one below") g.crd[(size_t)g.pos[(size_t)long_row(333)]] = 5;
     const int64_t *pos = g.pos.data(), *crd = g.crd.data();
     TcHeader hdr = {};
     TriCounters tc = {};
     std::vector<uint32_t> degree((size_t)n, 0), bits((size_t)nnz * 2);
-    std::vector<int32_t> hub_count((size_t)n, 0), rest_count((size_t)n, 0), rank((size_t)n, -1), bits_at((size_t)n, -5), place((size_t)nnz);
+    std::vector<int32_t> hub_count((size_t)n, -9), rest_count((size_t)n, -9), rank((size_t)n, -1), bits_at((size_t)n, -5), place((size_t)nnz);
     std::vector<int2> edge((size_t)nnz);
     std::vector<int64_t> hub_pos((size_t)n + 1), rest_pos((size_t)n + 1);
     std::vector<unsigned short> hub((size_t)nnz);
     std::vector<int32_t> a32((size_t)nnz, -1), m32((size_t)nnz, -1);
     unsigned long long count = 0;
     const unsigned long long room = what == "no room" ? 300 : (unsigned long long)nnz * 2;
-    fake::run_block(64, 0, 1, [&] { tri_degree_kernel(nnz, crd, degree.data(), &hdr); });
-    fake::run_block(512, 0, 1, [&] { tri_hist_kernel(n, pos, crd, degree.data(), &hdr, &tc); });
+    fake::run_block(64, 0, 1, [&] { tri_degree_kernel(n, nnz, pos, crd, degree.data(), &tc); });
+    fake::run_block(512, 0, 1, [&] { tri_hist_kernel(n, pos, crd, degree.data(), &tc); });
     fake::run_block(512, 0, 1, [&] { tri_decide_kernel(nnz, &hdr, &tc); });
     const bool taken = hdr.ordered;
-    if (taken != (what != "even" && what != "regular")) {
+    if (taken != (what != "even" && what != "regular" && what != "one below")) {
         printf("taken: %d\n", (int)taken);
         return 1;
     }
+    const int64_t tiles = (n + 1 + TRI_TILE - 1) / TRI_TILE;
+    std::vector<int64_t> sums((size_t)tiles * 2);
+    auto places = [&] {
+        for (unsigned y = 0; y < 2; y++)
+            for (unsigned b = 0; b < (unsigned)tiles; b++)
+                fake::run_block(256, b, (unsigned)tiles, [&] { tri_sums_kernel(n, hub_count.data(), rest_count.data(), &hdr, sums.data()); }, y);
+        fake::run_block(1024, 0, 1, [&] { tri_totals_kernel(n, tiles, &hdr, &tc, sums.data(), hub_pos.data(), rest_pos.data()); });
+        for (unsigned y = 0; y < 2; y++)
+            for (unsigned b = 0; b < (unsigned)tiles; b++)
+                fake::run_block(256, b, (unsigned)tiles, [&] {
+                    tri_places_kernel(n, hub_count.data(), rest_count.data(), pos, &hdr, sums.data(), hub_pos.data(), rest_pos.data());
+                }, y);
+    };
     if (!taken) {
-        printf("ok\n");
+        places();
+        printf(hdr.ordered || rest_pos != g.pos ? "rows\n" : "ok\n");
         return 0;
     }
-    fake::run_block(512, 0, 1, [&] { tri_rank_kernel(n, degree.data(), &hdr, &tc, rank.data()); });
+    fake::run_block(512, 0, 1, [&] { tri_rank_kernel(n, degree.data(), &hdr, &tc, rank.data(), hub_count.data(), rest_count.data()); });
     std::vector<int64_t> whole((size_t)n, 0);
     for (int64_t i = 0; i < n; i++)
         for (int64_t j : g.rows[(size_t)i]) { whole[(size_t)i]++; whole[(size_t)j]++; }
@@ -114,9 +136,15 @@ int main(int argc, char **argv)
         fake::run_block(256, b, blocks, [&] {
             tri_edges_kernel(n, nnz, pos, crd, rank.data(), &hdr, &tc, edge.data(), place.data(), hub_count.data(), rest_count.data());
         });
-    for (int64_t k = 0; k < n; k++) {
-        hub_pos[(size_t)k + 1] = hub_pos[(size_t)k] + hub_count[(size_t)k];
-        rest_pos[(size_t)k + 1] = rest_pos[(size_t)k] + rest_count[(size_t)k];
+    places();
+    if (what == "unordered" || what == "repeats") {
+        printf(hdr.ordered || rest_pos != g.pos ? "rows\n" : "ok\n");
+        return 0;
+    }
+    if (!hdr.ordered) { printf("given up\n"); return 1; }
+    for (int64_t k = 0, hubs = 0, others = 0; k <= n; k++) {
+        if (hub_pos[(size_t)k] != hubs || rest_pos[(size_t)k] != others) { printf("row %ld\n", (long)k); return 1; }
+        if (k < n) { hubs += hub_count[(size_t)k]; others += rest_count[(size_t)k]; }
     }
     fake::run_block(64, 0, 1, [&] {
         tri_scatter_kernel(nnz, edge.data(), place.data(), hub_pos.data(), rest_pos.data(), &hdr, &tc, hub.data(), a32.data(), m32.data(), nullptr);

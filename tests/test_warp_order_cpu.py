@@ -66,7 +66,7 @@ def test_sets_of_a_warp(tmp_path, kernel, out):
         kernel, out)
 
 
-@pytest.mark.parametrize("graph", ["skewed", "upper", "no room", "even", "regular", "ends in a hub"])
+@pytest.mark.parametrize("graph", ["skewed", "upper", "no room", "even", "regular", "ends in a hub", "unordered", "repeats", "one below"])
 def test_triangles_in_another_order(tmp_path, graph):
     order = same_zero("bm[hub[s + q] >> 5]", body("order.cuh"))
     for wide, narrow in (("TRI_HUBS = 16384", "TRI_HUBS = 256"), ("TRI_BITMAP = 64", "TRI_BITMAP = 16")):
