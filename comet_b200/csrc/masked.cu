@@ -143,7 +143,9 @@ masked_rows_kernel(int64_t nrows, const int64_t *__restrict__ bpos, const int64_
 }
 
 // A square pattern of strictly ascending rows: the place of (j,i) for every entry (i,j), and the number of entries that have none.
-// A thread per entry: its row by a search in the row pointer, its mate by one in row j.
+// A thread per entry: its row by a search in the row pointer, its mate by one in row j.  Ends with the first entry that has none (as many in
+// every row as in every column, but not symmetric: 16 neighbours on one side of each of 200,000 vertices of a ring, plus-pair, without a
+// search 648 us, with all of them 755, so 672).
 __global__ void __launch_bounds__(256)
 masked_mates_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, int64_t room,
                     int32_t *__restrict__ mate, MaskedStats *stats)
@@ -154,7 +156,8 @@ masked_mates_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_
     }
     const int64_t n = pos[nrows];
     unsigned none = n > room;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n && p < room; p += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n && p < room && !none && !*(volatile unsigned long long *)&stats->one_sided;
+         p += (int64_t)gridDim.x * blockDim.x) {
         int64_t lo = 0, hi = nrows - 1;
         while (lo < hi) {                              // the first row that ends behind p
             const int64_t mid = (lo + hi) >> 1;

@@ -51,6 +51,12 @@ int main()
     if (symmetric || looked) { printf("one entry without a mate\n"); return 1; }
     run(cycle);                                   // as many in every row as in every column
     if (symmetric) { printf("a cycle\n"); return 1; }
+    cycle.resize(3000);                           // and a ring without a direction behind it, whose entries need not be looked up any more
+    for (int i = n; i < 3000; i++) cycle[i] = {i > n ? i - 1 : n + 1, i + 1 < 3000 ? i + 1 : i - 1};
+    cycle[n] = {n + 1};
+    cycle[2999] = {2998};
+    run(cycle);
+    if (symmetric || looked) { printf("a cycle and a ring\n"); return 1; }
     printf("ok\n");
     return 0;
 }

@@ -33,6 +33,10 @@ def body(name, until=None):
     text = source(name)
     text = text[:text.index(until)] + "}\n" if until else text
     text = re.sub(r"^#(include|pragma).*$", "", text, flags=re.M).replace("extern __shared__", "extern").replace("static __global__", "__global__")
+    return relaxed(text)
+
+
+def relaxed(text):
     return re.sub(r"\*\(volatile [a-z ]+ \*\)(&[\w>-]+)", r"__atomic_load_n(\1, __ATOMIC_RELAXED)", text)
 
 
@@ -77,6 +81,6 @@ def test_triangles_in_another_order(tmp_path, graph):
 
 
 def test_mates_of_a_symmetric_pattern(tmp_path):
-    text = source("masked.cu")
+    text = relaxed(source("masked.cu"))
     struct = re.search(r"^struct MaskedStats \{.*?^\};\n", text, re.M | re.S).group(0)
     run(tmp_path, "masked_mates_check.cpp", struct + "".join(function(f, text) for f in ("masked_weight", "masked_stats_kernel", "masked_mates_kernel")))
