@@ -661,7 +661,7 @@ class SpGEMM(Workload):
 
 class Triangles(Workload):
     name = "triangles"
-    launches_per_step = 32    # renumbering (6), hub columns (3), columns present (2), 4 scans of 3, 2 narrowings, rows, routing, scatter, units, three counting kernels
+    launches_per_step = 28    # renumbering (5), rows' places (3), hub columns (3), columns present (2), 2 scans of 3, 2 narrowings, rows, routing, scatter, units, three counting kernels
 
     def build(self):
         from comet_b200 import datasets, sharding

@@ -87,3 +87,23 @@ def test_rows_with_more_columns_than_the_stage_holds(stored):
     assert np.array_equal(pos, want.indptr) and np.array_equal(crd, want.indices)
     # a sum of n products in any order: n * 2^-53 of the sum of their magnitudes, n up to 402
     assert np.all(np.abs(val - ref.data) <= 402 * 2.0 ** -53 * mag.data)
+
+
+def test_more_long_rows_than_there_is_memory_for():
+    """128 MB hold the bitmaps of 1310 rows of B in 819,200 columns; the others are walked like short rows."""
+    rng = np.random.default_rng(5)
+    lens = [3200, 3199, 4000] + [3300] * 1397 + [40] * 300
+    brows = [np.unique(rng.integers(0, 819200, n)) for n in lens]
+    brows[0] = np.sort(rng.choice(819200, 3200, replace=False))
+    brows[3:1400] = [np.sort(rng.choice(819200, 3300, replace=False)) for _ in range(1397)]
+    B = _csr(brows, rng.uniform(0.5, 1, sum(map(len, brows))), (len(brows), 819200))
+    arows = [np.sort(rng.choice(len(brows), 4, replace=False)) for _ in range(3300)]
+    A = _csr(arows, rng.uniform(-1, 1, sum(map(len, arows))), (len(arows), len(brows)))
+    assert np.count_nonzero(np.diff(B.indptr) >= 3200) > 1310 and A.shape[0] * 102400 > 64 * B.nnz
+    C = dev.spgemm(_device(A), _device(B))
+    pos, crd, val = C.pos.cpu().numpy(), C.crd.cpu().numpy(), C.val.cpu().numpy()
+    ref, mag = A @ B, abs(A) @ abs(B)
+    ref.sort_indices(), mag.sort_indices()
+    assert np.array_equal(pos, mag.indptr) and np.array_equal(crd, mag.indices) and np.array_equal(crd, ref.indices)
+    # a sum of n products in any order: n * 2^-53 of the sum of their magnitudes, n up to 4
+    assert np.all(np.abs(val - ref.data) <= 4 * 2.0 ** -53 * mag.data)

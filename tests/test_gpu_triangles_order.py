@@ -109,3 +109,33 @@ def test_a_column_at_the_same_place_of_every_row(hub):
     D = _device(i, j, n)
     assert D.nnz >= max(6000000, 10 * n)
     assert int(dev.masked_pair_count(D, D, D)) == _by_blocks(D, [0, n // 3, n])
+
+
+def test_more_rows_than_there_is_memory_for():
+    """Rows of 64 and more entries in the hub columns, twice as many as there is room for bitmaps of."""
+    n, m = 110000, 128
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(12)
+    i = torch.arange(n, device="cuda").repeat_interleave(m)
+    j = (torch.rand(n * m, generator=gen, device="cuda", dtype=torch.float64) * torch.where(torch.arange(n * m, device="cuda") % 16 == 0, n, 16000)).long()
+    key = torch.unique(torch.maximum(i, j) * n + torch.minimum(i, j))
+    i, j = torch.div(key, n, rounding_mode="floor"), key % n
+    i, j = i[i != j], j[i != j]
+    D = _device(i, j, n)
+    rows = int((torch.bincount(i[j < 16000], minlength=n) >= 64).sum())
+    assert D.nnz >= max(6000000, 10 * n) and (rows - 16384) * 512 > D.nnz * 2
+    pos, crd = D.pos.cpu().numpy(), D.crd.cpu().numpy()
+    L = oracle.SparseArrays("CSR", n, n, np.array([n]), np.array([-1]), pos, crd, np.ones(crd.size))
+    assert int(dev.masked_pair_count(D, D, D)) == oracle.masked_pair_count_rowparallel(L, L, L)
+
+
+def test_rows_that_do_not_ascend():
+    """Found out when the vertices have their new numbers already."""
+    n = 60000
+    i, j = _graph("skewed", n, 8000000, 8)
+    D = _device(i, j, n)
+    want = int(dev.masked_pair_count(D, D, D))
+    p = int(D.pos[torch.diff(D.pos).argmax()])
+    D.crd[p + 1:p + 3] = D.crd[p + 1:p + 3].flip(0)
+    assert D.nnz >= max(6000000, 10 * n)
+    assert int(dev.masked_pair_count(D, D, D)) == want
