@@ -37,7 +37,7 @@ struct MaskedStats {
     unsigned long long products, bound;
     unsigned long long desc_all, desc_edge;           // places where A's coordinates do not ascend: all, and at row starts
     unsigned nnz_a, nnz_m;                 // 0xffffffff: that or more
-    unsigned long long one_sided;          // entries of A without a mate, see masked_mates_kernel
+    unsigned long long one_sided;          // not 0: some entry of A has no mate, see masked_mates_kernel
     unsigned long long balance;            // not 0: some vertex has not as many entries in its row as in its column
 };
 static_assert(sizeof(MaskedStats) <= 64, "fits a page-locked word block");
@@ -142,7 +142,7 @@ masked_rows_kernel(int64_t nrows, const int64_t *__restrict__ bpos, const int64_
     }
 }
 
-// A square pattern of strictly ascending rows: the place of (j,i) for every entry (i,j), and the number of entries that have none.
+// A square pattern of strictly ascending rows: the place of (j,i) for every entry (i,j), or that some entry has none.
 // A thread per entry: its row by a search in the row pointer, its mate by one in row j.  Ends with the first entry that has none (as many in
 // every row as in every column, but not symmetric: 16 neighbours on one side of each of 200,000 vertices of a ring, plus-pair, without a
 // search 648 us, with all of them 755, so 672).
@@ -150,14 +150,14 @@ __global__ void __launch_bounds__(256)
 masked_mates_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, int64_t room,
                     int32_t *__restrict__ mate, MaskedStats *stats)
 {
+    const int64_t n = pos[nrows];
     if (stats->balance) {                              // some entry has none
         if (blockIdx.x == 0 && threadIdx.x == 0) stats->one_sided = 1;
         return;
     }
-    const int64_t n = pos[nrows];
     unsigned none = n > room;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n && p < room && !none && !*(volatile unsigned long long *)&stats->one_sided;
-         p += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n && p < room; p += (int64_t)gridDim.x * blockDim.x) {
+        const bool found = *(volatile unsigned long long *)&stats->one_sided != 0;       // looked at when this entry is done
         int64_t lo = 0, hi = nrows - 1;
         while (lo < hi) {                              // the first row that ends behind p
             const int64_t mid = (lo + hi) >> 1;
@@ -171,7 +171,8 @@ masked_mates_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_
             if (crd[mid] < i) lo = mid + 1; else hi = mid;
         }
         if (lo < e && crd[lo] == i) mate[p] = (int32_t)lo;
-        else none++;
+        else none = 1;
+        if (none || found) break;
     }
     none = __reduce_add_sync(0xffffffffu, none);
     if ((threadIdx.x & 31) == 0 && none) atomicAdd(&stats->one_sided, (unsigned long long)none);
