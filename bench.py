@@ -51,7 +51,7 @@ KERNEL_SOURCES = {
     "spmm": ["spmm.cu", "spmm.cuh", "spmm_short.cu", "spmm_pieces.cu", "spmm_stream.cu", "stream.cuh", "common.cuh"],
     "sddmm": ["sddmm.cu", "stream.cuh", "common.cuh"],
     "spgemm": ["spgemm.cu", "hubs.cuh", "semiring.cuh", "stream.cuh", "util.cu", "common.cuh"],
-    "triangles": ["tc.cu", "order.cuh", "pairs.cuh", "semiring.cuh", "util.cu", "common.cuh"],
+    "triangles": ["tc.cu", "order.cuh", "pairs.cuh", "semiring.cuh", "stream.cuh", "util.cu", "common.cuh"],
 }
 
 
