@@ -5,7 +5,7 @@
 //   columns   B's columns are renumbered to those that B stores, in order (scale 18: 148,500 of 262,144), so that a row's
 //             bitmap, its ranks and the walk over them shrink by as much
 //   bitmaps   of those rows of B ("hubs"): the symbolic call ORs them into a row's bitmap in registers, 128 bits a load,
-//             instead of marking their columns bit by bit with atomics (5.3 -> 3.7 ms).  The line of 512 entries: 256 6.1 ms,
+//             instead of marking their columns bit by bit with atomics (5.3 -> 3.7 ms, 3.3 with four CTAs an SM).  The line of 512 entries: 256 6.1 ms,
 //             384 3.8, 768 3.8, 1024 4.1; on scale 15 0.30, 0.27 (512: 0.27), 0.37, 0.37.  With wide bitmaps an OR takes longer than the
 //             marks of 512 entries, hence at least an eighth of an entry per word.
 // Tried and not kept: sums by rank in shared memory, a range of columns per warp and the part of every hub that falls into it

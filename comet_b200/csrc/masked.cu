@@ -11,7 +11,7 @@
 // semiring a second pass over the mask entries with hits folds the products; then every row's entries are written in
 // mask order, which is ascending.
 //
-// Where A, B and M are one symmetric pattern (the adjacency matrix of a graph: the device looks every entry's mate up, 15 us), B needs
+// Where A, B and M are one symmetric pattern (the adjacency matrix of a graph: the device looks every entry's mate up, 39 us), B needs
 // no transposing, the entries (i,j) and (j,i) have the same count and are counted once, with the longer list as the set, so nothing has
 // to be routed to the other side; a second pass folds the values of both.
 //
@@ -19,9 +19,10 @@
 // so would B's, whose check is part of the transpose), when the bitmaps cover A's columns, and when the bound
 // sum |M_i| |A_i| on the elements streamed is at most MASKED_DOT_COST times the products of the push form: a mask much
 // denser than the product it masks is cheaper to push.
-// Measured on B200: that graph under plus-pair 18.7 -> 0.62 ms, under plus-times 19.5 -> 1.66; scale 9, edge factor 8
-// 0.72 -> 0.25 ms (some thirty launches and two synchronisations).  The set kernels take 0.36 ms of the 0.62, the
-// transpose 0.09.
+// Measured on B200, push form and now: a symmetric graph of scale 15, edge factor 16, under plus-pair 18.7 -> 0.36 ms, under plus-times
+// 19.5 -> 1.21.  Of the 0.36 the set kernels take 0.21 (bitmaps 0.105, hash sets 0.076 and 0.031), the checks and the mates 0.06.  Not
+// symmetric, of the same scale: 0.45 and 0.99; set kernels 0.22, transposing 0.06, routing 0.03.  Scale 9, edge factor 8: 0.19 and 0.50
+// symmetric, 0.22 and 0.38 not (13 or 24 launches in the symbolic call, two synchronisations).
 #include <string.h>
 
 #include "hostcopy.cuh"

@@ -13,9 +13,9 @@
 //   j >= HUBS   the rest of the rows, by the kernels of pairs.cuh (which need neither sorted rows nor the cut at column k).
 // Nothing is sorted: entries are put into their rows in any order.
 //
-// Bound: the first part issues instructions 80 % of the time (scale 20), 35 per step of 4096 columns; with fewer of them (row i's bits in
+// Bound: the first part issues 2.9 of four instructions a clock (scale 20), 35 per step of 4096 columns; with fewer of them (row i's bits in
 // registers, four rows k a step 7.1 ms; only the groups of 128 columns that row i has 7.3) it waits for the L2 instead.  At scale 22 the
-// renumbering takes 2.9 ms of 11.4, the first part 5.5, the rest 2.9.
+// renumbering takes 2.8 ms of 11.3, the first part 5.5, the rest 2.9.
 //
 // Whether a matrix is triangular, and skewed enough for this to pay, is found out on the device (TcHeader::ordered); if not, the rest
 // is the whole matrix as it is, and the kernels of the first part have nothing to do.
@@ -56,8 +56,8 @@ __device__ __forceinline__ int tri_bucket(unsigned degree)      // larger degree
     return TRI_BUCKETS - 1 - (e * 16 - 48 + (int)((degree >> (e - 4)) & 15));
 }
 
-// Column counts, of one entry in TRI_SAMPLE (the order has to be about right, and all of them take 1.3 ms on 64 M entries: the hubs'
-// counters are a queue).  Of 64 entries four neighbours are taken, any four: a column that is always at the same place of its row is met
+// Column counts, of one entry in TRI_SAMPLE (the order has to be about right; all of them take 1.3 ms on 64 M entries, where the hubs'
+// counters are a queue, this 0.17).  Of 64 entries four neighbours are taken, any four: a column that is always at the same place of its row is met
 // as often as others.  A CTA looks at the ends of rows from all over the matrix first and counts nothing if that cannot be triangular, which
 // nearly all CTAs find out where it is not.
 static __global__ void __launch_bounds__(256)

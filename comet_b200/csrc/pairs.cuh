@@ -628,7 +628,7 @@ tc_mid_kernel(TcHeader *hdr, const TcUnit *__restrict__ mids, const int64_t *__r
 // warp 0 while the others stream, so that between two units only the bits change.
 // 32 warps an SM, as many as are launched: 64 registers a thread, which no variant spills for.  With the 109 that the value pass for both
 // halves takes otherwise, one CTA of 16 warps ran (R-MAT scale 15 / 16, 16 per row, symmetric, under itself, plus-times 1450 -> 1235 and
-// 3000 -> 2300 us); the one-sided pass spilled 112 bytes (not symmetric 728 -> 714 and 1715 -> 1690).  Three CTAs of 16 warps for
+// 3000 -> 2300 us); the one-sided pass spilled 112 bytes (not symmetric, 15 / 16, 1000 -> 985 and 1715 -> 1695).  Three CTAs of 16 warps for
 // counts cost 96 bytes of spills and gain nothing (plus-pair at scale 15 373 and 373 us).
 template <int THREADS, bool SEGMENTED, class Out>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)

@@ -31,7 +31,7 @@
 // beyond its hub columns is left to the kernels here.
 //
 // Measured on B200, R-MAT edge factor 16 lower triangles (mask side only, cuckoo sets in every bin -> both sides, bitmaps -> renumbered):
-// scale 14 0.27 -> 0.16 ms, scale 18 1.96 -> 0.76, scale 20 10.2 -> 3.15 -> 2.38, scale 22 61.9 -> 18.4 -> 11.4.
+// scale 14 0.27 -> 0.16 ms, scale 18 1.96 -> 0.76, scale 20 10.2 -> 3.15 -> 2.38, scale 22 61.9 -> 18.4 -> 11.3.
 #include "order.cuh"
 #include "pairs.cuh"
 
