@@ -1020,6 +1020,10 @@ static const unsigned TEAM_MAX = 64;
 // a little above one share. Rows of 1.06 shares 4.95 ms in teams and 4.25 alone, 1.2 1.91 and 1.73, 1.33 2.06 and 1.94, 1.45 2.23 and
 // 2.29, 1.6 2.58 and 3.13 (6000 and 20,000 rows of 20,000 to 35,000 products in 300,000 columns, both calls).
 static const double TEAM_ALONE = 1.4;
+// With fewer rows than twice the CTAs that run, teams also fill the chip: any row above one share gets one, with shares as for four CTAs an SM.
+// Rows of 18,000 entries in 120,000 columns, both calls, before columns were renumbered, without and with this: 20 rows 110, 140, 113; 300 170, 172, 166;
+// 500 220, 222, 206; 900 340, 316, 326; 1800 580, 521, 548.  20,000 in 60,000: 20 rows 122, 138, 106; 500 258, 285, 252; 900 386, 390, 385; 1800 675, 648, 652.
+static const unsigned TEAM_FEW = 2;
 
 __device__ __forceinline__ uint64_t team_pack(unsigned it, unsigned part, unsigned t)
 {
@@ -1028,7 +1032,7 @@ __device__ __forceinline__ uint64_t team_pack(unsigned it, unsigned part, unsign
 
 __global__ void __launch_bounds__(256)
 team_items_kernel(unsigned nlist, const int32_t *__restrict__ list, const int64_t *__restrict__ cpos,
-                  double ctas_per_budget_entry, TeamHeader *th, uint64_t *items, unsigned cap)
+                  double ctas_per_budget_entry, double alone_to, TeamHeader *th, uint64_t *items, unsigned cap)
 {
     // consecutive list entries in consecutive slots (one warp-wide scan per 32 rows keeps the list ordered)
     const unsigned it = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1037,7 +1041,7 @@ team_items_kernel(unsigned nlist, const int32_t *__restrict__ list, const int64_
     if (it < nlist) {
         const int64_t r = list[it];
         const double want = (double)(cpos[r + 1] - cpos[r]) * ctas_per_budget_entry;
-        t = want <= TEAM_ALONE ? 1u : (want >= (double)TEAM_MAX ? TEAM_MAX : (unsigned)ceil(want));
+        t = want <= alone_to ? 1u : (want >= (double)TEAM_MAX ? TEAM_MAX : (unsigned)ceil(want));
     }
     unsigned incl = t;
     for (int o = 1; o < 32; o <<= 1) {
@@ -1700,9 +1704,11 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
                 double budget_mb = 60.0;                 // measured best on R-MAT scale 18 (25 / 40 / 60 / 160 MB)
                 if (const char *e = getenv("COMET_B200_SPGEMM_TEAM_MB")) budget_mb = atof(e);
                 if (budget_mb < 0.001) budget_mb = 0.001;
-                const double per_entry = 8.0 * grid / (budget_mb * 1048576.0);
+                const bool few = p->n2 < (unsigned)grid * TEAM_FEW;
+                const double alone_to = few ? 1.0 : TEAM_ALONE;
+                const double per_entry = 8.0 * (few ? bitmap_grid(0xffffffffu, (size_t)words * 8) : grid) / (budget_mb * 1048576.0);
                 // no row of so few columns wants a team: two launches less
-                const bool alone = (double)words * 32 * per_entry <= TEAM_ALONE;
+                const bool alone = (double)words * 32 * per_entry <= alone_to;
                 const size_t cap = (size_t)p->n2 + (size_t)((double)p->nnz_c * per_entry) + 64;
                 void *tm = nullptr;
                 rc = cap > 0xfffffff0u ? fail("spgemm numeric: too many team items")
@@ -1715,7 +1721,7 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
                     if (alone) items = nullptr;
                     else
                         team_items_kernel<<<(unsigned)ceil_div(p->n2, 256), 256, 0, st>>>(
-                            p->n2, p->list2, p->cpos, per_entry, th, items, (unsigned)cap);
+                            p->n2, p->list2, p->cpos, per_entry, alone_to, th, items, (unsigned)cap);
                     if (!alone) launch_behind(team_clear_kernel, dim3((unsigned)sm_count() * 8), 256, 0, st, th, items, (unsigned)cap, p->list2,
                                   p->cpos, p->semi, cval);
                     const bool times = p->semi == COMET_B200_PLUS_TIMES;

@@ -1,6 +1,7 @@
 // A product of rows that all go to the bitmaps over B's columns: what is launched to look A and B over, and for the numeric call.
 // Arguments: rows of A, entries of A, entries of B, columns, columns that B stores.  Prints the blocks of the kernel that looks them over
-// (0: not launched), the blocks an SM of the numeric kernel, and the columns of a warp's stage.
+// (0: not launched), the blocks an SM of the numeric kernel, and the columns of a warp's stage; with a sixth argument whether rows are given
+// to teams.
 #include "fake_launch.hpp"
 
 #include "../../comet_b200/csrc/hostcopy.cuh"
@@ -50,6 +51,7 @@ int main(int argc, char **argv)
         if (l.name.find("hub_present_kernel") != std::string::npos) looked = l.grid.x;
         if (l.name.find("bitmap_numeric_kernel") != std::string::npos) numeric = l.grid.x / 148;
     }
-    printf("%u %u %u\n", looked, numeric, stage);
+    if (argc > 6) printf("%d\n", fake::launched("team_items_kernel"));
+    else printf("%u %u %u\n", looked, numeric, stage);
     return 0;
 }

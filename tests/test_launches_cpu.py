@@ -50,6 +50,12 @@ def test_columns_that_need_a_look_up_have_a_stage(hub_launch, stored):
     assert ctas * (dynamic + 4176 + 1024) <= 228 * 1024 and dynamic + 4176 <= 227 * 1024
 
 
+# 1.13 shares of the L2 a row with three CTAs on an SM, 1.5 with four
+@pytest.mark.parametrize("nrows,teams", [(20, 1), (443, 1), (887, 1), (888, 0), (20000, 0)])
+def test_few_rows_are_given_to_teams(hub_launch, nrows, teams):
+    assert int(output(hub_launch, nrows, nrows * 100, 400000, 20000, 20000, "teams")) == teams
+
+
 @pytest.mark.parametrize("n,nnz", [(500000, 8000000), (1600000, 20000000)])
 def test_a_count_goes_on_without_memory_it_can_do_without(tmp_path_factory, n, nnz):
     assert output(link(tmp_path_factory, "triangle_memory_check.cpp", "tc.o"), n, nnz) == "ok"
