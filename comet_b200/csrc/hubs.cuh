@@ -19,6 +19,12 @@
 namespace cb200 {
 
 static const int HUB_MIN_ENTRIES = 512;
+// Products per word of the rows' bitmaps from which on long rows, and columns of which between 5/8 and 7/8 are stored, are worth it where the
+// numeric kernel gains no CTA on an SM: coordinates cost a look-up each, which few products pay for.  R-MAT scale 15 squared has 22 (70 % stored,
+// both calls 1316 us renumbered, 1430 not); 12,351 rows of 13,000 products in 791,000 columns, 74 % stored, 0.5 (4199 and 3951); min-plus, 115,713
+// rows of 1900 in 268,835 columns, 75 %, 0.2 (7760 and 7060); long rows in columns that keep their numbers, 3300 rows of 13,200 in 800,000 columns,
+// 0.5 (with bitmaps of them 1550, without 1250).
+static const int HUB_PRODUCTS = 4;
 static const int HUB_MAX_WORDS = 25600;             // with their ranks, what bin 2 holds in shared memory
 static const int64_t HUB_MAX_COLS = (int64_t)1 << 23;
 static const size_t HUB_MEMORY = (size_t)128 << 20; // bitmaps of all hubs
@@ -28,6 +34,7 @@ struct HubPrep {             // filled on the device, read by the host
     unsigned pad;
     long long nrows_b;       // rows of B that A can name
     long long longest;       // entries of the longest of them
+    long long products;      // of A and B
 };
 
 struct Hubs {
@@ -47,7 +54,7 @@ struct Hubs {
 
 #ifdef __CUDACC__
 
-// Columns that B stores (a bit each), the largest row that A names, and the longest.  SMEM: the bits are collected per CTA, so that the hub
+// Columns that B stores (a bit each), the largest row that A names, the longest, and the number of products.  SMEM: the bits are collected per CTA, so that the hub
 // columns' words are not a queue for the whole chip.
 template <bool SMEM>
 __global__ void __launch_bounds__(1024)
@@ -71,11 +78,12 @@ hub_present_kernel(int64_t nnz_b, const int32_t *__restrict__ bcrd, int64_t word
         }
     }
     const int64_t nnz_a = apos[nrows];
-    long long top = 0, longest = 0;
+    long long top = 0, longest = 0, products = 0;
     for (int64_t p = t0; p < nnz_a; p += stride) {
         const long long k = acrd[p] + 1, len = bpos[k] - bpos[k - 1];
         top = k > top ? k : top;
         longest = len > longest ? len : longest;
+        products += len;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -83,10 +91,12 @@ hub_present_kernel(int64_t nnz_b, const int32_t *__restrict__ bcrd, int64_t word
         top = v > top ? v : top;
         const long long l = __shfl_xor_sync(0xffffffffu, longest, o);
         longest = l > longest ? l : longest;
+        products += __shfl_xor_sync(0xffffffffu, products, o);
     }
     if ((threadIdx.x & 31) == 0 && top) {
         atomicMax(&prep->nrows_b, top);
         atomicMax(&prep->longest, longest);
+        atomicAdd((unsigned long long *)&prep->products, (unsigned long long)products);
     }
     if (SMEM) {
         __syncthreads();

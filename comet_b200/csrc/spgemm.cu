@@ -1394,8 +1394,28 @@ static int launch_mid(const Plan *p, unsigned grid, int64_t *ccrd, double *cval,
     return 0;
 }
 
-// Prepares B's long rows (p->hubs stays null where the columns that B stores are too many, or B has no long rows and hardly a column
-// without entries).  Synchronises.
+// CTAs of the numeric kernel on an SM, and the columns of a warp's stage that are left room for where columns need a look-up (mapped)
+struct NumericCtas {
+    size_t per_sm, stage;
+};
+static NumericCtas numeric_ctas(int64_t words, bool mapped)
+{
+    // three CTAs are what the registers leave room for; coordinates are staged in the shared memory that is left
+    // (200,000 rows of up to 60: 4.2 ms with three and what is left, 5.2 with a full stage and two).  Columns that need no
+    // look-up are written as they are found (3.3 against 3.5).  A stage of a few columns is worth less than a CTA: 2000 rows of
+    // 100,000 products in 450,000 columns 2.39 ms with three CTAs and 43 columns, 2.27 with two and 512.
+    const size_t smem = (size_t)words * sizeof(uint32_t) * 2, sm = (size_t)228 * 1024, own = 6 * 1024;
+    if (smem > BM_SMEM_LIMIT) return {0, 0};
+    size_t per_sm = sm / (smem + own);
+    per_sm = per_sm < 1 ? 1 : per_sm > 3 ? 3 : per_sm;
+    auto stage_of = [&](size_t ctas) { return (sm / ctas - own - smem) / (BM_THREADS / 32 * 4); };
+    while (mapped && per_sm > 1 && stage_of(per_sm) < STAGE_MIN) per_sm--;
+    const size_t stage = mapped ? stage_of(per_sm) : 0;
+    return {per_sm, stage > BM_DENSE_ROW ? (size_t)BM_DENSE_ROW : stage};
+}
+
+// Prepares B's long rows (p->hubs stays null where the columns that B stores are too many, or where these keep their numbers and B has no long
+// rows or A names few).  Synchronises.  In vain that costs 20 to 65 us.
 static int hub_prepare(Plan *p, int64_t nrows, int64_t nnz_a, cudaStream_t st)
 {
     Hubs *hb = new Hubs();
@@ -1444,13 +1464,18 @@ static int hub_prepare(Plan *p, int64_t nrows, int64_t nnz_a, cudaStream_t st)
         CB_CUDA(cudaStreamSynchronize(st));
         memcpy(&prep, host.p, sizeof(prep));
     }
-    // the look-up of every coordinate costs what an eighth of the words does (200,000 columns, all stored: 3.3 -> 4.0 ms)
-    const bool renumber = (int64_t)prep.ncols * 8 <= p->ncols * 7;
+    // the look-up of every coordinate costs what an eighth of the words does (200,000 columns, all stored: 3.3 -> 4.0 ms), and more where rows
+    // have few products for their words: HUB_PRODUCTS
+    const bool much = prep.products / HUB_PRODUCTS >= (long long)p->n2 * words;
+    const int64_t stored = (int64_t)prep.ncols * 8;
+    const bool renumber = stored <= p->ncols * 5 ||
+                          (stored <= p->ncols * 7 &&
+                           (much || numeric_ctas(ceil_div((int64_t)prep.ncols, 32), true).per_sm > numeric_ctas(words, false).per_sm));
     hb->words = (int)(renumber ? ceil_div((int64_t)prep.ncols, 32) : words);
     hb->stride = (hb->words + 3) & ~3;
     hb->nrows_b = prep.nrows_b;
     const int64_t entries = hb->words / 8 > HUB_MIN_ENTRIES ? hb->words / 8 : HUB_MIN_ENTRIES;
-    if (hb->words > HUB_MAX_WORDS || (!renumber && prep.longest < entries)) return without();
+    if (hb->words > HUB_MAX_WORDS || (!renumber && (!much || prep.longest < entries))) return without();
     if (renumber) {
         hub_renumber_kernel<<<(unsigned)sm_count() * 8, 256, 0, st>>>(p->nnz_b, p->bcrd32, words, hb->present, hb->before, hb->crd,
                                                                       hb->colmap);
@@ -1687,19 +1712,10 @@ int sparse_out_numeric(int64_t handle, int64_t *ccrd, double *cval, int keep, cu
             size_t smem = (size_t)words * sizeof(uint32_t) * 2;
             if (smem <= BM_SMEM_LIMIT) {
                 // full occupancy grid even for few rows: teams give every CTA work
-                // three CTAs are what the registers leave room for; coordinates are staged in the shared memory that is left
-                // (200,000 rows of up to 60: 4.2 ms with three and what is left, 5.2 with a full stage and two).  Columns that need no
-                // look-up are written as they are found (3.3 against 3.5).  A stage of a few columns is worth less than a CTA: 2000 rows of
-                // 100,000 products in 450,000 columns 2.39 ms with three CTAs and 43 columns, 2.27 with two and 512.
-                const size_t sm = (size_t)228 * 1024, own = 6 * 1024;
-                size_t per_sm = sm / (smem + own);
-                per_sm = per_sm < 1 ? 1 : per_sm > 3 ? 3 : per_sm;
-                auto stage_of = [&](size_t ctas) { return (sm / ctas - own - smem) / (BM_THREADS / 32 * 4); };
-                while (colmap && per_sm > 1 && stage_of(per_sm) < STAGE_MIN) per_sm--;
-                size_t stage_n = colmap ? stage_of(per_sm) : 0;
-                if (stage_n > BM_DENSE_ROW) stage_n = BM_DENSE_ROW;
+                const NumericCtas ctas = numeric_ctas(words, colmap != nullptr);
+                const size_t stage_n = ctas.stage;
                 smem += stage_n * (BM_THREADS / 32 * 4);
-                const int grid = sm_count() * (int)per_sm;
+                const int grid = sm_count() * (int)ctas.per_sm;
                 // team size of a row = its output entries * 8 bytes * CTAs in flight / budget
                 double budget_mb = 60.0;                 // measured best on R-MAT scale 18 (25 / 40 / 60 / 160 MB)
                 if (const char *e = getenv("COMET_B200_SPGEMM_TEAM_MB")) budget_mb = atof(e);

@@ -1,7 +1,7 @@
 // A product of rows that all go to the bitmaps over B's columns: what is launched to look A and B over, and for the numeric call.
 // Arguments: rows of A, entries of A, entries of B, columns, columns that B stores.  Prints the blocks of the kernel that looks them over
-// (0: not launched), the blocks an SM of the numeric kernel, and the columns of a warp's stage; with a sixth argument whether rows are given
-// to teams.
+// (0: not launched), the blocks an SM of the numeric kernel, and the columns of a warp's stage; a sixth argument is the number of
+// products, or asks whether rows are given to teams.
 #include "fake_launch.hpp"
 
 #include "../../comet_b200/csrc/hostcopy.cuh"
@@ -15,7 +15,7 @@ int exclusive_scan_i64(const int64_t *, int64_t *, int64_t, cudaStream_t) { retu
 void masked_free(MaskedPlan *, cudaStream_t) {}
 }  // namespace cb200
 
-struct HubPrep { unsigned ncols, pad; long long nrows_b, longest; };       // as hubs.cuh has it
+struct HubPrep { unsigned ncols, pad; long long nrows_b, longest, products; };       // as hubs.cuh has it
 
 int main(int argc, char **argv)
 {
@@ -35,6 +35,7 @@ int main(int argc, char **argv)
             prep->ncols = (unsigned)stored;
             prep->nrows_b = 1000;
             prep->longest = 10;
+            prep->products = argc > 6 ? atoll(argv[6]) : 0;
         } else if (name.find("bitmap_numeric_kernel") != std::string::npos) {
             stage = *(unsigned *)args[4];
         }
@@ -51,7 +52,7 @@ int main(int argc, char **argv)
         if (l.name.find("hub_present_kernel") != std::string::npos) looked = l.grid.x;
         if (l.name.find("bitmap_numeric_kernel") != std::string::npos) numeric = l.grid.x / 148;
     }
-    if (argc > 6) printf("%d\n", fake::launched("team_items_kernel"));
+    if (argc > 6 && !strcmp(argv[6], "teams")) printf("%d\n", fake::launched("team_items_kernel"));
     else printf("%u %u %u\n", looked, numeric, stage);
     return 0;
 }

@@ -89,21 +89,36 @@ def test_rows_with_more_columns_than_the_stage_holds(stored):
     assert np.all(np.abs(val - ref.data) <= 402 * 2.0 ** -53 * mag.data)
 
 
-def test_more_long_rows_than_there_is_memory_for():
-    """128 MB hold the bitmaps of 1310 rows of B in 819,200 columns; the others are walked like short rows."""
-    rng = np.random.default_rng(5)
-    lens = [3200, 3199, 4000] + [3300] * 1397 + [40] * 300
-    brows = [np.unique(rng.integers(0, 819200, n)) for n in lens]
-    brows[0] = np.sort(rng.choice(819200, 3200, replace=False))
-    brows[3:1400] = [np.sort(rng.choice(819200, 3300, replace=False)) for _ in range(1397)]
-    B = _csr(brows, rng.uniform(0.5, 1, sum(map(len, brows))), (len(brows), 819200))
-    arows = [np.sort(rng.choice(len(brows), 4, replace=False)) for _ in range(3300)]
-    A = _csr(arows, rng.uniform(-1, 1, sum(map(len, arows))), (len(arows), len(brows)))
-    assert np.count_nonzero(np.diff(B.indptr) >= 3200) > 1310 and A.shape[0] * 102400 > 64 * B.nnz
+def _product_is_right(A, B, terms):
+    """Structure, and sums of up to `terms` products in any order: terms * 2^-53 of the sum of their magnitudes."""
     C = dev.spgemm(_device(A), _device(B))
     pos, crd, val = C.pos.cpu().numpy(), C.crd.cpu().numpy(), C.val.cpu().numpy()
     ref, mag = A @ B, abs(A) @ abs(B)
     ref.sort_indices(), mag.sort_indices()
     assert np.array_equal(pos, mag.indptr) and np.array_equal(crd, mag.indices) and np.array_equal(crd, ref.indices)
-    # a sum of n products in any order: n * 2^-53 of the sum of their magnitudes, n up to 4
-    assert np.all(np.abs(val - ref.data) <= 4 * 2.0 ** -53 * mag.data)
+    assert np.all(np.abs(val - ref.data) <= terms * 2.0 ** -53 * mag.data)
+
+
+def test_more_long_rows_than_there_is_memory_for():
+    """128 MB hold the bitmaps of 1310 rows of B in 819,200 columns that are stored; the others are walked like short rows."""
+    rng = np.random.default_rng(5)
+    stored = (np.arange(819200) * 1.7).astype(np.int64)                   # of 1,400,000 columns
+    lens = [819200, 3200, 3199] + [3300] * 1400 + [40] * 300
+    brows = [stored] + [np.sort(stored[rng.choice(819200, n, replace=False)]) for n in lens[1:]]
+    B = _csr(brows, rng.uniform(0.5, 1, sum(lens)), (len(brows), 1400000))
+    arows = [np.array([0])] + [np.sort(rng.choice(np.arange(1, len(brows)), 4, replace=False)) for _ in range(3300)]
+    A = _csr(arows, rng.uniform(-1, 1, sum(map(len, arows))), (len(arows), len(brows)))
+    assert np.count_nonzero(np.diff(B.indptr) >= 3200) > 1310 and A.shape[0] * 175000 > 64 * B.nnz
+    _product_is_right(A, B, 4)
+
+
+def test_long_rows_in_columns_that_keep_their_numbers():
+    """All columns stored, and five products per word of the bitmaps."""
+    rng = np.random.default_rng(6)
+    lens = [511, 512, 513] + [2000] * 700 + [30] * 100
+    brows = [np.sort(rng.choice(100000, n, replace=False)) for n in lens]
+    B = _csr(brows, rng.uniform(0.5, 1, sum(lens)), (len(brows), 100000))
+    arows = [np.array([0]), np.array([1, 2]), np.arange(len(brows))] + [np.sort(rng.choice(len(brows), 10, replace=False)) for _ in range(8000)]
+    A = _csr(arows, rng.uniform(-1, 1, sum(map(len, arows))), (len(arows), len(brows)))
+    assert np.diff(B.indptr)[A.indices].sum() > 4 * A.shape[0] * 3125 and A.shape[0] * 12500 > 64 * B.nnz
+    _product_is_right(A, B, len(brows))

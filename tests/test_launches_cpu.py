@@ -50,6 +50,13 @@ def test_columns_that_need_a_look_up_have_a_stage(hub_launch, stored):
     assert ctas * (dynamic + 4176 + 1024) <= 228 * 1024 and dynamic + 4176 <= 227 * 1024
 
 
+# bitmaps of 6000 * 6250 words; 62.5 and 87.5 % of the columns
+@pytest.mark.parametrize("stored,products,staged", [(125000, 0, 1), (125001, 0, 0), (150000, 149999999, 0), (150000, 150000000, 1), (175000, 150000000, 1),
+                                                    (175001, 150000000, 0)])
+def test_columns_are_renumbered_where_it_pays(hub_launch, stored, products, staged):
+    assert (int(output(hub_launch, 6000, 600000, 400000, 200000, stored, products).split()[2]) > 0) == staged
+
+
 # 1.13 shares of the L2 a row with three CTAs on an SM, 1.5 with four
 @pytest.mark.parametrize("nrows,teams", [(20, 1), (443, 1), (887, 1), (888, 0), (20000, 0)])
 def test_few_rows_are_given_to_teams(hub_launch, nrows, teams):
