@@ -28,6 +28,7 @@
 #include "hostcopy.cuh"
 #include "masked.cuh"
 #include "pairs.cuh"
+#include "stream.cuh"
 
 namespace cb200 {
 
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(256)
 masked_mates_kernel(int64_t nrows, const int64_t *__restrict__ pos, const int64_t *__restrict__ crd, int64_t room,
                     int32_t *__restrict__ mate, MaskedStats *stats)
 {
+    wait_for_previous();
     const int64_t n = pos[nrows];
     if (stats->balance) {                              // some entry has none
         if (blockIdx.x == 0 && threadIdx.x == 0) stats->one_sided = 1;
@@ -271,7 +273,7 @@ int masked_symbolic(int64_t nrows, int64_t ncols_b, int64_t nnz_b, const int64_t
     }
     MaskedPlan *m = new MaskedPlan();
     m->mate = mate;                        // freed with the plan
-    if (mate) masked_mates_kernel<<<flat_grid(nnz_b), 256, 0, st>>>(nrows, apos, acrd, nnz_b, mate, (MaskedStats *)sp);
+    if (mate) launch_behind(masked_mates_kernel, dim3(flat_grid(nnz_b)), 256, 0, st, nrows, apos, acrd, nnz_b, mate, (MaskedStats *)sp);
     MaskedStats s;
     {
         PinnedWords words;
