@@ -504,12 +504,15 @@ tc_warp_kernel(TcHeader *hdr, const int32_t *__restrict__ small, const int64_t *
     const bool swap = tc_swap_ok(hdr);
     const bool cut = sh.cut && !(sh.ask && hdr->ordered);
     const unsigned n = hdr->nsmall;
+    // Four rows a draw keep the counter from being a queue; fewer than all warps would draw go one by one, or most warps have none (a symmetric
+    // graph of 1934 vertices and 70,000 entries, plus-times 790 -> 456 us; R-MAT scale 13 x 16, plus-pair 330 -> 280).
+    const unsigned step = n >= gridDim.x * TC_WARPS * 4 ? 4u : 1u;
     while (true) {
         unsigned idx = 0;
-        if (lane == 0) idx = atomicAdd(&hdr->next_small, 4u);
+        if (lane == 0) idx = atomicAdd(&hdr->next_small, step);
         idx = __shfl_sync(0xffffffffu, idx, 0);
         if (idx >= n) break;
-        const unsigned stop = idx + 4 < n ? idx + 4 : n;
+        const unsigned stop = idx + step < n ? idx + step : n;
         for (; idx < stop; idx++) {
             const int64_t i = small[idx];
             const int64_t as = apos[i], ae = apos[i + 1], ms = mpos[i], me = mpos[i + 1];
