@@ -21,8 +21,8 @@
 // denser than the product it masks is cheaper to push.
 // Measured on B200, push form and now: a symmetric graph of scale 15, edge factor 16, under plus-pair 18.7 -> 0.36 ms, under plus-times
 // 19.5 -> 1.21.  Of the 0.36 the set kernels take 0.21 (bitmaps 0.105, hash sets 0.076 and 0.031), the checks and the mates 0.06.  Not
-// symmetric, of the same scale: 0.45 and 0.99; set kernels 0.22, transposing 0.06, routing 0.03.  Scale 9, edge factor 8: 0.19 and 0.50
-// symmetric, 0.22 and 0.38 not (13 or 24 launches in the symbolic call, two synchronisations).
+// symmetric, of the same scale: 0.42 and 0.88; set kernels 0.19, transposing 0.06, routing 0.03.  Scale 9, edge factor 8: 0.16 and 0.33
+// symmetric, 0.19 and 0.28 not (13 or 24 launches in the symbolic call, two synchronisations).
 #include <string.h>
 
 #include "hostcopy.cuh"
